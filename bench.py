@@ -237,7 +237,8 @@ def roofline_sweep(w, ms_per_colour, peaks, mixed, resident=False, layout=None):
     FP64 sweep: per active cell DIVDT, 4 cross-term weights, AN, AS, 3 factors read
     (80 B) and P written (8 B), plus the other colour's lagged P (8 B) and, for the
     second colour, its new P (8 B): 100 B x active cells on average.
-    The per-colour kernels launch once per colour.  The resident kernel runs the
+    The per-colour kernels launch once per colour.  The FP64 ring runs a step's whole
+    iteration in one launch (achieved = 100 B x cells / time per sweep).  The resident kernel runs the
     refine_sweeps sweeps of a refinement interval in one launch with its lines'
     operands held on chip: its algorithmic bytes per launch are the same per-sweep
     figure times the sweeps it runs, so achieved = 32 B x cells / time per sweep."""
@@ -253,7 +254,13 @@ def roofline_sweep(w, ms_per_colour, peaks, mixed, resident=False, layout=None):
     out = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
            "traffic": None, "kernel": "k_pois32" if mixed else "k_pois64",
            "avg_launch_us": ms_per_colour * 1e3, "bytes_per_launch": per_colour, "peak_source": peak_src}
-    if resident:
+    if resident and not mixed:
+        out.update({"kernel": "k_ring64", "avg_launch_us": 2 * ms_per_colour * 1e3 * w["nswpp"],
+                    "bytes_per_launch": 2 * per_colour * w["nswpp"], "per_sweep_us": 2 * ms_per_colour * 1e3,
+                    "bytes_per_sweep": 2 * per_colour,
+                    "note": "the whole FP64 Poisson iteration of a step in one launch, operands on chip; timed "
+                            "without its residuals; bound by FP64 issue"})
+    elif resident:
         spl = w["refine_sweeps"]
         pairs = bool(layout) and layout.get("sweeps_per_exchange") == 2
         out.update({"kernel": "k_pois32_resident2" if pairs else "k_pois32_resident", "sweeps_per_launch": spl,
@@ -376,8 +383,8 @@ def run_ours(args):
     e2e_value = units / (e2e_ms * 1e-3) / 1e6
     roof = roofline_sweep(w, res["mixed"]["sweep_ms"], peaks, True, res["mixed"]["resident"],
                           res["mixed"]["layout"])
-    roof64 = roofline_sweep(w, res["fp64"]["sweep_ms"], peaks, False)
-    if roof64:
+    roof64 = roofline_sweep(w, res["fp64"]["sweep_ms"], peaks, False, res["fp64"]["resident"])
+    if roof64 and not res["fp64"]["resident"]:
         roof64["fp64_issue"] = fp64_pipe("fp64_pipe_cylinder2d_512x384", "k_pois64")
         roof64["fp64_issue_residual"] = fp64_pipe("fp64_pipe_cylinder2d_512x384", "k_pres64")
     traffic_file = os.path.join(ROOT, "profiles", (roof["kernel"] if roof else "k_pois32") +

@@ -81,6 +81,7 @@ void make_target(fvm_batch *b)
         t.nblk_res = std::max(t.nblk_res, c->nblk_res);
         t.nblk_res64 = std::max(t.nblk_res64, c->nblk_res64);
         t.nblk_mres = std::max(t.nblk_mres, c->nblk_mres);
+        t.ring_ppb = std::max(t.ring_ppb, c->d.ring_ppb);
     }
 }
 

@@ -114,6 +114,7 @@ int fvm_create(const fvm_params *p, fvm_ctx **out)
     }
     int rc = fvm::setup_allocate(c);
     if (rc == FVM_OK) rc = fvm::resident_setup(c);
+    if (rc == FVM_OK) rc = fvm::ring_setup(c);
     if (rc != FVM_OK) {
         fvm_destroy(c);
         return rc;

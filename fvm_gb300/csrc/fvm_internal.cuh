@@ -15,11 +15,10 @@
 namespace fvm {
 
 constexpr int WARP = 32;
-constexpr int RES_CELLS = 2;   // cells per thread of the mixed and adjoint Poisson residual kernels
-// cells per thread of the FP64 path's residual (k_pres64): eight amortise the block
-// reduction over more cells and leave room for the overlapping sweep launches (FP64
-// step 39.7 -> 35.7 ms on 512 x 384; two, for the mixed path's k_mres, measured best)
-constexpr int RES64_CELLS = 8;
+constexpr int RES_CELLS = 2;   // cells per thread of the adjoint Poisson residual kernels
+// Most blocks of the FP64 Poisson ring (and of the FP64 residual, which sums its lines
+// in the same groups)
+constexpr int RING_MAX_BLOCKS = 256;
 // Tile of the mixed path's residual kernel k_mres: 32 radial x 8 circumferential
 // cells per 256-thread block, the pressure of the tile and its halo split into
 // double-float once in shared memory.
@@ -85,7 +84,8 @@ struct Dev {
     int refine_sweeps;  // MIXED: FP32 sweeps per FP64 refinement
     int adi_refine;     // MIXED: defect-correction passes of a predictor line
     int nblk_res;       // blocks of this case in the residual kernels (RES_CELLS per thread)
-    int nblk_res64;     // blocks of this case in the FP64 path's residual (RES64_CELLS per thread)
+    int nblk_res64;     // FP64 path: blocks of the Poisson ring and of the residual
+    int ring_ppb;       // FP64 path: line pairs per block of both
     int nblk_mres;      // blocks of this case in the mixed path's residual (MRES_TI x MRES_TJ tiles)
     int case_id;        // position in a batch
     BatchCtl *bctl;     // batch control (nullptr in a single-context launch)
@@ -175,6 +175,7 @@ struct fvm_ctx {
     int pgraph_batch = 0;
     int nblk_res = 0;      // blocks of the residual kernels
     int nblk_res64 = 0;    // blocks of the FP64 path's residual kernel
+    int ring_blocks = 0;   // blocks of the FP64 Poisson ring (0: the per-colour path)
     int nblk_mres = 0;     // blocks of the mixed path's residual kernel
     // instrumentation
     cudaEvent_t ev_a = nullptr, ev_b = nullptr;   // span around the first sweep group of a replay
@@ -231,7 +232,7 @@ struct Tgt {
     const Dev *one = nullptr;    // single context: its device view (passed by value)
     DevTable tab{nullptr};       // batch: device table of the cases' views
     int nz = 1;                  // cases
-    int NI = 0, NJ = 0, n = 0, nblk_res = 0, nblk_res64 = 0, nblk_mres = 0;   // launch extents
+    int NI = 0, NJ = 0, n = 0, nblk_res = 0, nblk_res64 = 0, nblk_mres = 0, ring_ppb = 1;   // launch extents
     LineSys tr{}, tt{};          // tiles (NW, M) of the radial and circumferential line families
     int mixed = 0, thermal = 1, iter_t_bug = 1, refine_sweeps = 1, res_every = 2;
 };
@@ -311,6 +312,11 @@ int resident_sweeps_on(fvm_ctx *c, const ResSys &sys, int sweeps, int apply, int
 int resident_sweeps(const Tgt &t, int sweeps, int apply, int max_polls, unsigned tag_skew,
                     cudaGraphConditionalHandle cond, int has_cond, int check_done, int decide = 0);
 int resident_reset(fvm_ctx *c);
+size_t exchange_words(const fvm_ctx *c);   // 64-bit words of d.XW
+// FP64 Poisson iteration in one launch (fvm_ring.cu)
+int ring_setup(fvm_ctx *c);
+int ring_pairs(const fvm_ctx *c);   // line pairs per block
+int ring_launch(fvm_ctx *c, int mode, int count);
 }  // namespace fvm
 
 // ---------------------------------------------------------------------------------
@@ -405,6 +411,27 @@ __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, 
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+
+// The FP64 Poisson operations in one fixed rounding order (the per-colour kernels and
+// the ring give the same bits).  Source of cell (i,j): DIVDT minus the lagged cross term
+// (dd_p: weights CNE, CSE, CNW, CSW of its four diagonal neighbours).
+__device__ __forceinline__ double pois_source(double dv, double c1, double p1, double c2, double p2, double c3, double p3,
+                                              double c4, double p4)
+{
+    return fma_rn(-c4, p4, fma_rn(-c3, p3, fma_rn(-c2, p2, fma_rn(-c1, p1, dv))));
+}
+// Right-hand side of a line: AN P(j+1) + (AS P(j-1) + SU).
+__device__ __forceinline__ double pois_rhs(double an, double pn, double as, double ps, double su)
+{
+    return fma_rn(an, pn, fma_rn(as, ps, su));
+}
+// Residual of a cell (iter_p.f90:42-44), its magnitude and that of AP P added to ra, pa.
+__device__ __forceinline__ void pois_resid(double ae, double pe, double aw, double pw, double an, double pn, double as,
+                                           double ps, double su, double ap, double p, double &ra, double &pa)
+{
+    ra += fabs(fma_rn(-ap, p, fma_rn(as, ps, fma_rn(an, pn, fma_rn(aw, pw, fma_rn(ae, pe, su))))));
+    pa += fabs(mul_rn(ap, p));
+}
 
 // Right-hand side of a line of the FP32 Poisson correction sweep:
 // (AN x(j+1) + AS x(j-1)) + r, in one fixed rounding order.

@@ -141,20 +141,67 @@ __device__ void refresh_row_ghosts(const Dev &d, const double *src, double *dst,
     }
 }
 
-// Lagged Poisson cross term (dif_diagonal.f90:13-23) from the gathered weights.
-__device__ __forceinline__ double dd_p(const Dev &d, const double *P, int i, int j)
+// Source of cell (i,j) of the Poisson equation, dv = DIVDT there: ITER_P subtracts the
+// lagged cross term (dif_diagonal.f90:13-23, from the gathered weights) with the same
+// positional pairing as DIF (iter_p.f90:27-30): that of cell (i-1,j-1), or zero.
+__device__ __forceinline__ double pois_src_at(const Dev &d, const double *P, double dv, int i, int j)
 {
-    int c = IDX(i, j);
-    return ((d.CNE[c] * P[IDX(i + 1, j + 1)] + d.CSE[c] * P[IDX(i + 1, j - 1)]) + d.CNW[c] * P[IDX(i - 1, j + 1)])
-           + d.CSW[c] * P[IDX(i - 1, j - 1)];
+    if (d.dd_pos) {
+        if (i < 2 || j < 2) return dv;
+        i--;
+        j--;
+    }
+    const int c = IDX(i, j);
+    return pois_source(dv, d.CNE[c], P[IDX(i + 1, j + 1)], d.CSE[c], P[IDX(i + 1, j - 1)], d.CNW[c],
+                       P[IDX(i - 1, j + 1)], d.CSW[c], P[IDX(i - 1, j - 1)]);
 }
 
-// Cross term that ITER_P subtracts from the source of cell (i,j): the same
-// positional pairing as DIF (iter_p.f90:27-30), cell (i-1,j-1) or zero.
-__device__ __forceinline__ double dd_src(const Dev &d, const double *P, int i, int j)
+// Sums of the FP64 residual, the same in the per-colour kernel and in the ring: the
+// threads of a line (shuffle trees, then the line's warps in order; result on thread 0
+// of the group), a block's lines in order, the blocks over one warp (lane b takes blocks
+// b, b+32, ..., then the tree).
+template <int NW, class Sync>
+__device__ __forceinline__ void line_sum2(double &a, double &b, double *wa, double *wb, int t, Sync sync)
 {
-    if (!d.dd_pos) return dd_p(d, P, i, j);
-    return (i > 1 && j > 1) ? dd_p(d, P, i - 1, j - 1) : 0.0;
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        b += __shfl_down_sync(0xffffffffu, b, o);
+    }
+    if (NW > 1) {
+        if ((t & (WARP - 1)) == 0) {
+            wa[t / WARP] = a;
+            wb[t / WARP] = b;
+        }
+        sync();
+        if (t == 0)
+            for (int q = 1; q < NW; q++) {
+                a += wa[q];
+                b += wb[q];
+            }
+    }
+}
+__device__ __forceinline__ void pairs_sum2(const double *lines, int nl, double &a, double &b)
+{
+    a = 0.0;
+    b = 0.0;
+    for (int q = 0; q < nl; q++) {
+        a += lines[2 * q];
+        b += lines[2 * q + 1];
+    }
+}
+template <class Load>
+__device__ __forceinline__ void blocks_sum2(Load load, int nb, double &a, double &b)
+{
+    a = 0.0;
+    b = 0.0;
+    for (int q = threadIdx.x & (WARP - 1); q < nb; q += WARP) {
+        a += load(2 * q);
+        b += load(2 * q + 1);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        b += __shfl_down_sync(0xffffffffu, b, o);
+    }
 }
 
 // Cross-warp part of a block sum: lane 0 of every warp holds its warp's sums; warp 0
@@ -331,16 +378,6 @@ __device__ __forceinline__ PredLine pred_line(const Dev &d, int field, int dir)
     L.wallF = field == FVM_FIELD_U ? d.UFW : (field == FVM_FIELD_V ? d.VFW : d.TFW);
     L.farF = field == FVM_FIELD_U ? d.FFU : (field == FVM_FIELD_V ? d.FFV : d.FFT);
     return L;
-}
-
-// Five-point Poisson residual (iter_p.f90:42-44) of P with the line neighbours
-// read through periodic wrap; AE(NI-1)=0 and AW(1)=0 are folded in the coefficients.
-__device__ __forceinline__ double pres_at(const Dev &d, const double *P, double su, int i, int j)
-{
-    const Coef &cf = d.cP;
-    int c = IDX(i, j);
-    return ((((cf.AE[c] * P[IDX(i + 1, j)] + cf.AW[c] * P[IDX(i - 1, j)]) + cf.AN[c] * P[IDX(i, jwrap(d, j + 1))])
-             + cf.AS[c] * P[IDX(i, jwrap(d, j - 1))]) + su) - cf.AP[c] * P[c];
 }
 
 }  // namespace fvm

@@ -597,12 +597,20 @@ int resident_sweeps_on(fvm_ctx *c, const ResSys &sys, int sweeps, int apply, int
     return launch_sys(c, sys, c->stream, sweeps, apply, 0, 0u, 0, 0, check_done);
 }
 
+// Exchange words of a context: two slots of every line in the largest tile (32 x 4
+// warps x 4 elements), one word per FP32 value or two per FP64 value, and the FP64
+// ring's two slots of block sums.
+size_t exchange_words(const fvm_ctx *c)
+{
+    const size_t line = 2 * size_t(c->NJ - 1) * WARP * 4 * 4;
+    return c->p.precision == FVM_MIXED ? line : 2 * line + 2 * 4 * size_t(RING_MAX_BLOCKS);
+}
+
 // After a wait ran out: the blocks' sweep counts may disagree, so clear the
 // exchange words, the counts and the fault flag (stream-ordered).
 int resident_reset(fvm_ctx *c)
 {
-    const size_t words = 2 * size_t(c->NJ - 1) * WARP * 4 * 4;
-    FVM_CUDA(c, cudaMemsetAsync(c->d.XW, 0, words * sizeof(unsigned long long), c->stream));
+    FVM_CUDA(c, cudaMemsetAsync(c->d.XW, 0, exchange_words(c) * sizeof(unsigned long long), c->stream));
     FVM_CUDA(c, cudaMemsetAsync(c->d.XCNT, 0, size_t(c->NJ) * sizeof(unsigned int), c->stream));
     FVM_CUDA(c, cudaMemsetAsync(&c->d.pctl->fault, 0, sizeof(int), c->stream));
     return FVM_OK;

@@ -1,0 +1,545 @@
+// fvm_ring.cu -- the FP64 Poisson iteration of a step in one launch (iter_p.f90:22-51,
+// lisolv.f90:18-33, bcp.f90:8-42).
+//
+// The per-colour path (k_pois64, k_pres64) launches two grids per sweep.  A colour of
+// the 128 x 96 grid took as long as one of 512 x 384 (about 7 us): launch latency, the
+// operands' L2 round trips and the FP64 recurrences, not the arithmetic.  Here the
+// lines j = 1..NJ-1 are dealt to a ring of blocks in pairs (odd line, even line), at
+// most one block per SM, and each block keeps the factors, couplings, cross-term
+// weights, source and pressure of its lines on chip for the whole iteration: sweeps,
+// residuals and the convergence decision.  Only boundary lines and the residual's
+// block sums travel between blocks.
+//
+// Order of the values.  Sweep n solves the odd lines from the neighbours' P^(n-1),
+// then the even lines from the odd lines' P^n.  The lagged cross term of cell (i,j)
+// is dd_p of cell (i-1,j-1) (the positional pairing of the reference's whole-array
+// operand) and reads rows j and j-2, columns i and i-2, of P^(n-1); ghost column 0 and
+// ghost row 0 hold values one BCP older, so they are P^(n-2)(1,j) and P^(n-2)(i,NJ-1).
+// A line's pressure is therefore kept in three versions.  Every operation is k_pois64's
+// and k_pres64's in the same rounding order: both paths give the same bits.
+//
+// A block with lines j0 .. j1 needs from others: line j0-1 (even, version n-1: coupling
+// of j0, cross term of j0+1), line j0-2 (odd, version n-1: cross term of j0) and line
+// j1+1 (odd, version n: coupling of j1).  Each published FP64 value is two 64-bit words
+// (half of the value | tag << 32) written and polled with relaxed gpu-scope accesses, so a
+// matching tag carries its half with no flag or fence; tags are the blocks' sweep
+// counts (XCNT), words alternate between two slots, and a slot is rewritten two sweeps
+// later, which the writer can only reach after every reader has passed: line j at sweep
+// n+2 needs neighbours that needed the readers' sweep n+1.  While one colour is solved
+// the other colour's groups form their next cross terms.  The residual's block sums
+// travel the same way and every block adds them in the same order, so all blocks take
+// the same decision.  Every wait is bounded; one that runs out sets the fault flag, the
+// pressure is left alone and the host reports FVM_ERR_TIMEOUT.
+//
+// Bound: FP64.  A warp's FP64 instruction holds its quarter of the SM's FP64 pipe for 64
+// cycles (measured: a dependent chain of DFMAs, and the same chain beside three others
+// on the quarter, run at 67 and 259 cycles a step), so a line costs 64 cycles times the FP64
+// instructions of its warps, 11 per element beside the scans, and a block's one or two
+// concurrent lines are spread over all four quarters (radial_tile).  The other part is the
+// exchange, 0.41 us one way through L2, twice a sweep.  The products of the constant
+// factors that the line solve's scans carry are formed once per launch and kept in
+// shared memory: per sweep only the value part of the scans is left.
+// Measured (step with 512 or 2048 sweeps, residual every 8): 128 x 96 FP64 7.51 -> 2.27 ms
+// (14.3 -> 3.9 us per sweep), 512 x 384 39.6 -> 16.6 ms (18 -> 7.6 us; 196,608 cells x 11
+// instructions at the chip's 0.63 T/s: 3.4 us).
+#include <algorithm>
+#include <type_traits>
+
+#include "fvm_internal.cuh"
+#include "fvm_ops.cuh"
+
+namespace fvm {
+namespace {
+
+constexpr int STAGES = 5;   // Kogge-Stone stages of a warp
+constexpr int kRingPolls = 1 << 21;   // bound of a wait: about a second of polling at L2 latency
+
+template <int M, int NW>
+struct RingLayout {
+    static constexpr int TG = WARP * NW, LW = TG * M;
+    static constexpr int CST = 2 * (STAGES + 1) + 2 * M;   // per-thread scan constants
+    // lines (3 versions), the halo lines j0-1 and j0-2 (3 versions each), per line the
+    // scan constants, the warps' total products and the fold buffers
+    static size_t doubles(int nl) { return size_t(3) * (nl + 2) * LW + size_t(nl) * (size_t(CST) * TG + 4 * NW); }
+    static size_t bytes(int nl) { return sizeof(double) * doubles(nl); }
+    static constexpr int MAXT = 4 * TG;   // at most two pairs per block
+};
+
+__device__ __forceinline__ void ld_words(const ulonglong2 *p, unsigned long long &a, unsigned long long &b)
+{
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p));
+}
+__device__ __forceinline__ void st_words(ulonglong2 *p, double v, unsigned tag)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v), t = (unsigned long long)tag << 32;
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(t | (b & 0xffffffffull)), "l"(t | (b >> 32))
+                 : "memory");
+}
+__device__ __forceinline__ double of_words(unsigned long long a, unsigned long long b)
+{
+    return __hiloint2double((int)(unsigned)b, (int)(unsigned)a);
+}
+
+// The M elements of a line that thread t owns, once their words carry the tag; false
+// when the wait ran out.  One L2 round trip per poll: all loads precede the tests.
+template <int M, int TG>
+__device__ __forceinline__ bool poll_line(const ulonglong2 *src, int t, int n, unsigned want, double (&out)[M])
+{
+    unsigned pending = 0;
+#pragma unroll
+    for (int k = 0; k < M; k++)
+        if (t * M + k < n) pending |= 1u << k;
+    for (int it = 0; pending && it < kRingPolls; it++) {
+        unsigned long long a[M], b[M];
+#pragma unroll
+        for (int k = 0; k < M; k++) {
+            a[k] = b[k] = 0ull;
+            if ((pending >> k) & 1u) ld_words(src + k * TG + t, a[k], b[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < M; k++)
+            if (((pending >> k) & 1u) && unsigned(a[k] >> 32) == want && unsigned(b[k] >> 32) == want) {
+                out[k] = of_words(a[k], b[k]);
+                pending &= ~(1u << k);
+            }
+    }
+    return pending == 0;
+}
+
+// mode 0: the whole iteration; mode 1: `count` sweeps without residuals, P unchanged
+// (timing).
+template <int M, int NW>
+__global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
+    k_ring64(const __grid_constant__ Dev d, int ppb, int mode, int count)
+{
+    using Lay = RingLayout<M, NW>;
+    constexpr int TG = Lay::TG, LW = Lay::LW, CST = Lay::CST;
+    extern __shared__ double shm[];
+    __shared__ int s_fault;
+    __shared__ double s_line[2 * 8], s_tot[2 * RING_MAX_BLOCKS], s_res;
+    const int L = d.NJ - 1, n = d.sP.n;
+    const int pairs = L / 2, p0 = blockIdx.x * ppb, nl = 2 * min(ppb, pairs - p0), j0 = 2 * p0 + 1;
+    const int g = threadIdx.x / TG, t = threadIdx.x % TG, lane = t & (WARP - 1), wl = t / WARP;
+    const bool act = g < nl, odd = (g & 1) == 0;   // j0 is odd
+    const int j = j0 + g;
+    const NamedSync<NW> bar{1 + g};
+    const int nlm = 2 * ppb;
+    double *own = shm;                                  // [3][nlm][LW]
+    double *hm1 = own + size_t(3) * nlm * LW;           // [3][LW]
+    double *hm2 = hm1 + size_t(3) * LW;                 // [3][LW]
+    double *cst = hm2 + size_t(3) * LW + size_t(g) * (size_t(CST) * TG + 4 * NW);
+    double *fold = cst + size_t(CST) * TG;              // [Gtot | Htot | forward | backward][NW]
+    auto line = [&](int ver, int q) { return own + (size_t(ver) * nlm + q) * LW; };
+    auto wrap = [L](int q) { return q < 1 ? q + L : (q > L ? q - L : q); };
+    if (threadIdx.x == 0) s_fault = 0;
+
+    // operands of the line, in the chunk ownership of the solve (element e = t*M + k)
+    double fi[M], fa[M], fb[M], an[M], as[M], dv[M], c1[M], c2[M], c3[M], c4[M], v[M], su[M], sun[M];
+    if (act) {
+        const size_t base = size_t(j - 1) * LW;
+        load_factors<double, M, NW>(fi, fa, fb, d.sP.invD + base, d.sP.fa + base, d.sP.fb + base, t);
+#pragma unroll
+        for (int k = 0; k < M; k++) {
+            const int e = t * M + k;
+            const bool ok = e < n, cr = ok && e > 0 && j > 1;
+            const int c = IDX(e + 1, j), cc = cr ? IDX(e, j - 1) : 0;
+            an[k] = ok ? d.cP.AN[c] : 0.0;
+            as[k] = ok ? d.cP.AS[c] : 0.0;
+            dv[k] = ok ? d.DIVDT[c] : 0.0;
+            c1[k] = cr ? d.CNE[cc] : 0.0;
+            c2[k] = cr ? d.CSE[cc] : 0.0;
+            c3[k] = cr ? d.CNW[cc] : 0.0;
+            c4[k] = cr ? d.CSW[cc] : 0.0;
+            v[k] = ok ? d.P[c] : 0.0;
+            su[k] = 0.0;
+            line(0, g)[k * TG + t] = v[k];
+        }
+        // version -1 of a line is only read for its ghost column, which sits in element 0
+        if (t == 0) line(2, g)[0] = d.P[IDX(0, j)];
+        // the scans' constant factors (group_apply_r's products, formed once)
+        double G = 1.0;
+#pragma unroll
+        for (int k = 0; k < M; k++) {
+            G = G * fa[k];
+            cst[(2 * STAGES + 2 + k) * TG + t] = G;
+        }
+#pragma unroll
+        for (int s = 0; s < STAGES; s++) {
+            const double Gp = shfl_up(G, 1 << s);
+            cst[s * TG + t] = lane >= (1 << s) ? G : 0.0;
+            if (lane >= (1 << s)) G = G * Gp;
+        }
+        double Gx = shfl_up(G, 1);
+        cst[STAGES * TG + t] = lane == 0 ? 1.0 : Gx;
+        if (lane == WARP - 1) fold[wl] = G;
+        double H = 1.0;
+#pragma unroll
+        for (int k = M - 1; k >= 0; k--) {
+            H = H * fb[k];
+            cst[(2 * STAGES + 2 + M + k) * TG + t] = H;
+        }
+#pragma unroll
+        for (int s = 0; s < STAGES; s++) {
+            const double Hn = shfl_down(H, 1 << s);
+            cst[(STAGES + 1 + s) * TG + t] = lane + (1 << s) < WARP ? H : 0.0;
+            if (lane + (1 << s) < WARP) H = H * Hn;
+        }
+        double Hx = shfl_down(H, 1);
+        cst[(2 * STAGES + 1) * TG + t] = lane == WARP - 1 ? 1.0 : Hx;
+        if (lane == 0) fold[NW + wl] = H;
+    }
+    // scan stages whose factors are all below 2^-80 (an element's value reaches no
+    // further along the line) are left out
+    int ks = 0, hs = 0;
+    if (act) {
+        const double tiny = 0x1p-80;
+#pragma unroll
+        for (int s = 0; s < STAGES; s++) {
+            if (__any_sync(0xffffffffu, fabs(cst[s * TG + t]) > tiny)) ks = s + 1;
+            if (__any_sync(0xffffffffu, fabs(cst[(STAGES + 1 + s) * TG + t]) > tiny)) hs = s + 1;
+        }
+    }
+    // halo lines: version 0, and version -1 (ghost columns; block 0: the stored ghost row 0)
+    const int jm1 = wrap(j0 - 1), jm2 = j0 - 2;
+    for (int q = threadIdx.x; q < 3 * LW; q += blockDim.x) hm2[q] = 0.0;
+    __syncthreads();
+    for (int e = threadIdx.x; e < n; e += blockDim.x) {
+        const int w = (e % M) * TG + e / M;
+        hm1[w] = d.P[IDX(e + 1, jm1)];
+        if (j0 == 1) hm1[2 * LW + w] = d.P[IDX(e + 1, 0)];
+        if (jm2 >= 1) hm2[w] = d.P[IDX(e + 1, jm2)];
+    }
+    if (threadIdx.x == 0) {
+        if (j0 != 1) hm1[2 * LW] = d.P[IDX(0, jm1)];
+        if (jm2 >= 1) hm2[2 * LW] = d.P[IDX(0, jm2)];
+    }
+    double hal[M];   // group 0: line j0-1; the last group: line j1+1
+#pragma unroll
+    for (int k = 0; k < M; k++) hal[k] = 0.0;
+    if (act && g == 0) {
+#pragma unroll
+        for (int k = 0; k < M; k++) {
+            const int e = t * M + k;
+            if (e < n) hal[k] = d.P[IDX(e + 1, jm1)];
+        }
+    }
+    const double corner0 = d.P[IDX(0, 0)];
+    const unsigned cnt0 = d.XCNT[blockIdx.x];
+    ulonglong2 *words = reinterpret_cast<ulonglong2 *>(d.XW);
+    auto slot = [&](unsigned cnt, int q) { return words + (size_t(cnt & 1u) * L + (q - 1)) * LW; };
+    ulonglong2 *psum = words + size_t(2) * L * LW;   // [2 slots][blocks][2]
+    __syncthreads();
+
+    // source of sweep m: DIVDT minus the cross term of P^(m-1)
+    auto source = [&](int m, double (&out)[M]) {
+        const int vr = (m + 2) % 3, vg = (m + 1) % 3;
+        const double *self = line(vr, g), *row;
+        double gs = line(vg, g)[0], gr;
+        if (g >= 2) {
+            row = line(vr, g - 2);
+            gr = line(vg, g - 2)[0];
+        } else if (g == 0) {
+            row = hm2 + size_t(vr) * LW;
+            gr = hm2[size_t(vg) * LW];
+        } else if (j0 == 1) {   // line 2: the ghost row 0
+            row = hm1 + size_t(vg) * LW;
+            gr = m == 1 ? corner0 : row[0];
+        } else {
+            row = hm1 + size_t(vr) * LW;
+            gr = hm1[size_t(vg) * LW];
+        }
+#pragma unroll
+        for (int k = 0; k < M; k++) {
+            const int e = t * M + k;
+            const int w = k >= 2 ? (k - 2) * TG + t : (M >= 2 ? (k - 2 + M) * TG + t - 1 : t - 2);   // element e-2
+            const double p0 = self[k * TG + t], pm = row[k * TG + t];
+            const double q0 = e >= 2 ? self[w] : gs, qm = e >= 2 ? row[w] : gr;
+            out[k] = e < n ? pois_source(dv[k], c1[k], p0, c2[k], pm, c3[k], q0, c4[k], qm) : 0.0;
+        }
+    };
+    // the line solve of v (group_apply_r with the constant products from shared memory)
+    auto solve = [&]() {
+        double y = 0.0;
+#pragma unroll
+        for (int k = 0; k < M; k++) {
+            y = fma_rn(fa[k], y, mul_rn(fi[k], v[k]));
+            v[k] = y;
+        }
+#pragma unroll
+        for (int s = 0; s < STAGES; s++)
+            if (s < ks) y = fma_rn(cst[s * TG + t], shfl_up(y, 1 << s), y);
+        double in = shfl_up(y, 1);
+        if (lane == 0) in = 0.0;
+        if (NW > 1) {
+            if (lane == WARP - 1) fold[2 * NW + wl] = y;
+            bar();
+            double yw = 0.0;
+            for (int q = 0; q < wl; q++) yw = fma_rn(fold[q], yw, fold[2 * NW + q]);
+            in = fma_rn(cst[STAGES * TG + t], yw, in);
+        }
+#pragma unroll
+        for (int k = 0; k < M; k++) v[k] = fma_rn(cst[(2 * STAGES + 2 + k) * TG + t], in, v[k]);
+        double x = 0.0;
+#pragma unroll
+        for (int k = M - 1; k >= 0; k--) {
+            x = fma_rn(fb[k], x, v[k]);
+            v[k] = x;
+        }
+#pragma unroll
+        for (int s = 0; s < STAGES; s++)
+            if (s < hs) x = fma_rn(cst[(STAGES + 1 + s) * TG + t], shfl_down(x, 1 << s), x);
+        in = shfl_down(x, 1);
+        if (lane == WARP - 1) in = 0.0;
+        if (NW > 1) {
+            if (lane == 0) fold[3 * NW + wl] = x;
+            bar();
+            double xw = 0.0;
+            for (int q = NW - 1; q > wl; q--) xw = fma_rn(fold[NW + q], xw, fold[3 * NW + q]);
+            in = fma_rn(cst[(2 * STAGES + 1) * TG + t], xw, in);
+        }
+#pragma unroll
+        for (int k = 0; k < M; k++) v[k] = fma_rn(cst[(2 * STAGES + 2 + M + k) * TG + t], in, v[k]);
+    };
+    auto publish = [&](int m) {
+        ulonglong2 *dst = slot(cnt0 + unsigned(m), j);
+#pragma unroll
+        for (int k = 0; k < M; k++)
+            if (t * M + k < n) st_words(dst + k * TG + t, v[k], cnt0 + unsigned(m));
+    };
+    auto wait_line = [&](int q, int m) {
+        if (!poll_line<M, TG>(slot(cnt0 + unsigned(m), q), t, n, cnt0 + unsigned(m), hal)) s_fault = 1;
+    };
+
+    if (act && odd) source(1, su);
+    int m = 0, have = 0;   // sweeps done; have: group 0's halo already holds version m
+    const int per = mode ? count : d.res_every;
+    double resip = 0.0;
+    bool bad = false;
+    for (int round = 0;; round++) {
+        for (int s = 0; s < per; s++) {
+            m++;
+            const int vr = (m + 2) % 3, vw = m % 3;
+            if (act) {
+                if (odd) {
+                    if (g == 0 && m > 1 && !have) wait_line(jm1, m - 1);
+                    const double *pn = line(vr, g + 1), *ps = g == 0 ? nullptr : line(vr, g - 1);
+#pragma unroll
+                    for (int k = 0; k < M; k++) {
+                        const double lo = g == 0 ? hal[k] : ps[k * TG + t];
+                        v[k] = t * M + k < n ? pois_rhs(an[k], pn[k * TG + t], as[k], lo, su[k]) : 0.0;
+                    }
+                    solve();
+#pragma unroll
+                    for (int k = 0; k < M; k++) line(vw, g)[k * TG + t] = v[k];
+                    if (g == 0 || g == nl - 2) publish(m);
+                } else {
+                    if (g == 1 && m > 1) {
+                        double x[M];
+#pragma unroll
+                        for (int k = 0; k < M; k++) x[k] = 0.0;
+                        const unsigned want = cnt0 + unsigned(m - 1);
+                        if (!poll_line<M, TG>(slot(want, jm1), t, n, want, x)) s_fault = 1;
+#pragma unroll
+                        for (int k = 0; k < M; k++) hm1[size_t(vr) * LW + k * TG + t] = x[k];
+                        bar();
+                    }
+                    source(m, su);
+                }
+            }
+            have = 0;
+            __syncthreads();
+            if (s_fault) { bad = true; break; }   // uniform: read by every thread after the barrier
+            if (act) {
+                if (!odd) {
+                    if (g == nl - 1) wait_line(wrap(j + 1), m);
+                    const double *pn = g == nl - 1 ? nullptr : line(vw, g + 1), *ps = line(vw, g - 1);
+#pragma unroll
+                    for (int k = 0; k < M; k++) {
+                        const double hi = g == nl - 1 ? hal[k] : pn[k * TG + t];
+                        v[k] = t * M + k < n ? pois_rhs(an[k], hi, as[k], ps[k * TG + t], su[k]) : 0.0;
+                    }
+                    solve();
+#pragma unroll
+                    for (int k = 0; k < M; k++) line(vw, g)[k * TG + t] = v[k];
+                    if (g == nl - 1) publish(m);
+                } else {
+                    if (g == 0 && jm2 >= 1) {
+                        double x[M];
+#pragma unroll
+                        for (int k = 0; k < M; k++) x[k] = 0.0;
+                        const unsigned want = cnt0 + unsigned(m);
+                        if (!poll_line<M, TG>(slot(want, jm2), t, n, want, x)) s_fault = 1;
+#pragma unroll
+                        for (int k = 0; k < M; k++) hm2[size_t(vw) * LW + k * TG + t] = x[k];
+                        bar();
+                    }
+                    if (s + 1 < per) source(m + 1, su);
+                    else source(m + 1, sun);
+                }
+            }
+            __syncthreads();
+            if (s_fault) { bad = true; break; }
+        }
+        if (bad || mode) break;
+        // scaled-L1 residual of P^m with the last sweep's source
+        const int vw = m % 3;
+        double ra = 0.0, pa = 0.0;
+        if (act) {
+            double ae[M], aw[M], ap[M];
+#pragma unroll
+            for (int k = 0; k < M; k++) {
+                const int e = t * M + k, c = IDX(e + 1, j);
+                ae[k] = e < n ? d.cP.AE[c] : 0.0;
+                aw[k] = e < n ? d.cP.AW[c] : 0.0;
+                ap[k] = e < n ? d.cP.AP[c] : 0.0;
+            }
+            if (g == 0) wait_line(jm1, m);
+            const double *self = line(vw, g);
+#pragma unroll
+            for (int k = 0; k < M; k++) {
+                const int e = t * M + k;
+                if (e >= n) continue;
+                const double pe = e + 1 < n ? (k + 1 < M ? self[(k + 1) * TG + t] : self[t + 1]) : 0.0;
+                const double pw = e > 0 ? (k > 0 ? self[(k - 1) * TG + t] : self[(M - 1) * TG + t - 1]) : 0.0;
+                const double pn = g == nl - 1 ? hal[k] : line(vw, g + 1)[k * TG + t];
+                const double ps = g == 0 ? hal[k] : line(vw, g - 1)[k * TG + t];
+                pois_resid(ae[k], pe, aw[k], pw, an[k], pn, as[k], ps, su[k], ap[k], v[k], ra, pa);
+            }
+            if (odd) {
+#pragma unroll
+                for (int k = 0; k < M; k++) su[k] = sun[k];
+            }
+            line_sum2<NW>(ra, pa, fold + 2 * NW, fold + 3 * NW, t, bar);
+            if (t == 0) {
+                s_line[2 * g] = ra;
+                s_line[2 * g + 1] = pa;
+            }
+        }
+        have = 1;
+        __syncthreads();
+        const unsigned rtag = cnt0 + unsigned(m);
+        ulonglong2 *ps = psum + size_t(round & 1) * 2 * gridDim.x;
+        if (threadIdx.x == 0) {
+            pairs_sum2(s_line, nl, ra, pa);
+            st_words(ps + 2 * blockIdx.x, ra, rtag);
+            st_words(ps + 2 * blockIdx.x + 1, pa, rtag);
+        }
+        for (int q = threadIdx.x; q < 2 * (int)gridDim.x; q += blockDim.x) {
+            bool got = false;
+            for (int it = 0; !got && it < kRingPolls; it++) {
+                unsigned long long a, b;
+                ld_words(ps + q, a, b);
+                got = unsigned(a >> 32) == rtag && unsigned(b >> 32) == rtag;
+                if (got) s_tot[q] = of_words(a, b);
+            }
+            if (!got) s_fault = 1;
+        }
+        __syncthreads();
+        if (threadIdx.x < WARP) {
+            blocks_sum2([&](int q) { return s_tot[q]; }, gridDim.x, ra, pa);
+            if (threadIdx.x == 0) s_res = ra / pa;
+        }
+        __syncthreads();
+        if (s_fault) { bad = true; break; }
+        resip = s_res;
+        if (!(resip > d.resimax && m < d.nswpp)) break;
+    }
+    if (bad) {
+        if (threadIdx.x == 0) {
+            d.pctl->fault = 1;
+            d.pctl->done = 1;
+        }
+        return;
+    }
+    if (act && !mode) {
+#pragma unroll
+        for (int k = 0; k < M; k++) {
+            const int e = t * M + k;
+            if (e < n) d.P[IDX(e + 1, j)] = v[k];
+        }
+    }
+    if (threadIdx.x == 0) {
+        d.XCNT[blockIdx.x] = cnt0 + unsigned(m);
+        if (blockIdx.x == 0 && !mode) {
+            d.pctl->niter = m;
+            d.pctl->resip = resip;
+            d.pctl->capped = resip > d.resimax ? 1 : 0;
+            d.pctl->done = 1;
+        }
+    }
+}
+
+}  // namespace
+
+int ring_pairs(const fvm_ctx *c)
+{
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->p.device) != cudaSuccess || sms < 1) return 1;
+    const int room = std::min(sms, RING_MAX_BLOCKS);
+    return ((c->NJ - 1) / 2 + room - 1) / room;
+}
+
+// Ring layout of a context: pairs of lines per block so that every block has an SM of
+// its own.  d.ring_ppb (also the grouping of the residual sums in the per-colour path) is
+// set for every FP64 context; c->ring_blocks != 0 where the ring runs: the reference's
+// positional cross term, poisson_resident not 0, and blocks that fit.
+int ring_setup(fvm_ctx *c)
+{
+    c->ring_blocks = 0;
+    const int pairs = (c->NJ - 1) / 2;
+    int sms = 0;
+    FVM_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->p.device));
+    const int ppb = ring_pairs(c), nb = (pairs + ppb - 1) / ppb;
+    c->d.ring_ppb = ppb;
+    c->d.nblk_res64 = c->nblk_res64 = nb;
+    if (c->p.precision != FVM_FP64 || !c->d.dd_pos || c->p.poisson_resident == 0 || ppb > 2 || nb < 2) return FVM_OK;
+    const LineSys &s = c->d.sP;
+    int per_sm = 0;
+    cudaError_t e = cudaSuccess;
+    const bool ok = dispatch_line(s, [&](auto m, auto nw) {
+        constexpr int M_ = decltype(m)::value, NW_ = decltype(nw)::value;
+        using Lay = RingLayout<M_, NW_>;
+        auto k = k_ring64<M_, NW_>;
+        // set outside any capture, to the largest block's need, the same for every context
+        int most = 0;
+        for (int nl : {2, 4})
+            if (Lay::bytes(nl) <= 220 * 1024) most = (int)Lay::bytes(nl);
+        if ((int)Lay::bytes(2 * ppb) > most) return;
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 2 * ppb * Lay::TG, Lay::bytes(2 * ppb));
+    });
+    if (e != cudaSuccess) cudaGetLastError();
+    if (ok && e == cudaSuccess && per_sm >= 1 && nb <= sms) c->ring_blocks = nb;
+    return FVM_OK;
+}
+
+// The FP64 Poisson iteration of a context whose source term is in place (mode 0), or
+// `count` sweeps on chip (mode 1).  Cooperative: all blocks resident at once.
+int ring_launch(fvm_ctx *c, int mode, int count)
+{
+    cudaError_t e = cudaErrorInvalidValue;
+    dispatch_line(c->d.sP, [&](auto m, auto nw) {
+        constexpr int M_ = decltype(m)::value, NW_ = decltype(nw)::value;
+        using Lay = RingLayout<M_, NW_>;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(c->ring_blocks);
+        cfg.blockDim = dim3(2 * c->d.ring_ppb * Lay::TG);
+        cfg.dynamicSmemBytes = Lay::bytes(2 * c->d.ring_ppb);
+        cfg.stream = c->stream;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        e = cudaLaunchKernelEx(&cfg, k_ring64<M_, NW_>, c->d, c->d.ring_ppb, mode, count);
+    });
+    if (e != cudaSuccess) {
+        c->err = std::string("Poisson ring launch: ") + cudaGetErrorString(e);
+        return FVM_ERR_CUDA;
+    }
+    KCOUNT(c);
+    return FVM_OK;
+}
+
+}  // namespace fvm

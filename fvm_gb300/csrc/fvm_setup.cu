@@ -1,6 +1,7 @@
 // fvm_setup.cu -- one-time setup of a context: device slab, GRID/METRIC/INIT on the
 // device (FP64), the constant five-point coefficient sets of every line solve with
 // their boundary folding, and the precomputed tridiagonal factors of every line.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -74,14 +75,31 @@ void carve_coef(Bump &b, Coef &c, size_t n, int nj1)
 // Tile of the radial line family: the parameters' if given; for a MIXED context
 // whose Poisson sweeps run resident, two-warp groups once a line needs more than
 // one warp (resident sweep on 512 x 384: 1.59 us with 2 warps x 6 elements against
-// 1.86 with 4 x 3 and 1.78 with 1 x 12); else automatic (0, 0).
+// 1.86 with 4 x 3 and 1.78 with 1 x 12); for an FP64 context on the Poisson ring, as many
+// warps per line as fill the SM's four FP64 pipes with the one or two lines a block
+// solves at a time (a warp's FP64 instruction occupies its pipe for 64 cycles, so a line
+// on one warp takes M times as long as on M warps); else automatic (0, 0).
 void radial_tile(const fvm_ctx *c, int &nw, int &m)
 {
     nw = c->p.tile_r_warps;
     m = c->p.tile_r_m;
     const int n = c->NI - 1;
-    if (nw || m || c->p.precision != FVM_MIXED || !c->p.poisson_resident || n <= WARP * 4) return;
-    nw = 2;
+    if (nw || m) return;
+    if (c->p.precision == FVM_MIXED) {
+        if (!c->p.poisson_resident || n <= WARP * 4) return;
+        nw = 2;
+    } else {
+        if (!c->p.dd_positional) return;
+        nw = n <= WARP ? 1 : (n <= 2 * WARP || ring_pairs(c) > 1 ? 2 : 4);
+        if (nw == 4) {
+            m = (n + 4 * WARP - 1) / (4 * WARP);
+            return;
+        }
+        if (nw == 1) {
+            m = 1;
+            return;
+        }
+    }
     for (int mm : {1, 2, 3, 4, 6, 8})
         if (2 * WARP * mm >= n) {
             m = mm;
@@ -111,8 +129,7 @@ void carve(Bump &b, fvm_ctx *c, int nblk)
     d.RF = b.take<float>(n);
     d.DF = b.take<float>(n);
     d.PCD = b.take<float2>(9 * n);
-    // exchange words for the largest tile (32 x 4 warps x 4 elements per line)
-    d.XW = b.take<unsigned long long>(2 * size_t(c->NJ - 1) * WARP * 4 * 4);
+    d.XW = b.take<unsigned long long>(exchange_words(c));
     d.XCNT = b.take<unsigned int>(size_t(c->NJ));
     d.pctl = b.take<PCtl>(1);
     d.partial = b.take<double>(2 * size_t(nblk));
@@ -170,11 +187,9 @@ int setup_allocate(fvm_ctx *c)
     const int interior = (c->NI - 1) * (c->NJ - 1);
     c->nblk_res = (interior + 256 * RES_CELLS - 1) / (256 * RES_CELLS);   // residual kernels
     d.nblk_res = c->nblk_res;
-    c->nblk_res64 = (interior + 256 * RES64_CELLS - 1) / (256 * RES64_CELLS);   // FP64 residual (fewer)
-    d.nblk_res64 = c->nblk_res64;
     c->nblk_mres = ((c->NI - 1 + MRES_TI - 1) / MRES_TI) * ((c->NJ - 1 + MRES_TJ - 1) / MRES_TJ);
     d.nblk_mres = c->nblk_mres;
-    const int nblk_partial = std::max(c->nblk_res, c->nblk_mres);
+    const int nblk_partial = std::max({c->nblk_res, c->nblk_mres, RING_MAX_BLOCKS});
     Bump probe{nullptr};
     carve(probe, c, nblk_partial);
     c->slab_bytes = probe.off + 256;
@@ -528,7 +543,7 @@ int setup_factors(fvm_ctx *c)
         k_factor<<<(st.s->lines + 63) / 64, 64, 0, c->stream>>>(d, *st.cf, *st.s, st.circ);
         FVM_LAUNCH_CHECK(c);
     }
-    return FVM_OK;
+    return ring_setup(c);
 }
 
 int setup_grid(fvm_ctx *c)

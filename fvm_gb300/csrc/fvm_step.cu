@@ -407,8 +407,8 @@ __global__ void __launch_bounds__(128) k_pois64(const __grid_constant__ S src, i
         v[k] = 0.0;
         if (active && e < n) {
             int i = e + 1;
-            double su = dv[k] - dd_src(d, Pin, i, j);
-            v[k] = (an[k] * Pnb[IDX(i, jn)] + as[k] * Pnb[IDX(i, js)]) + su;
+            const double su = pois_src_at(d, Pin, dv[k], i, j);
+            v[k] = pois_rhs(an[k], Pnb[IDX(i, jn)], as[k], Pnb[IDX(i, js)], su);
         }
     }
     if (stop) return;
@@ -430,13 +430,15 @@ __global__ void __launch_bounds__(128) k_pois64(const __grid_constant__ S src, i
 }
 
 // Residual after an even number of iterations: P^n in P, P^(n-1) in P2.  SU of the
-// last sweep is rebuilt from P^(n-1) (with its stored ghosts).  The last block
-// publishes the count and decides convergence (iter_p.f90:50-51); inside the
-// device-side loop it also ends the loop (cond != 0).
-template <int HAS_COND, class S>
-__global__ void __launch_bounds__(256) k_pres64(const __grid_constant__ S src, cudaGraphConditionalHandle cond)
+// last sweep is rebuilt from P^(n-1) (with its stored ghosts).  A block takes the line
+// pairs of one block of the ring (fvm_ring.cu), a group of NW warps per line, so that
+// the sums are the ring's.  The last block publishes the count and decides convergence
+// (iter_p.f90:50-51); inside the device-side loop it also ends the loop (cond != 0).
+template <int M, int NW, int HAS_COND, class S>
+__global__ void __launch_bounds__(1024) k_pres64(const __grid_constant__ S src, cudaGraphConditionalHandle cond)
 {
-    __shared__ double sh[64];
+    constexpr int TG = WARP * NW;
+    __shared__ double wsum[2][1024 / WARP], lsum[2 * (1024 / WARP)];
     __shared__ bool last;
     const Dev &d = dev_of(src);
     if ((int)blockIdx.x >= d.nblk_res64) return;   // beyond this case's blocks (batch)
@@ -444,21 +446,46 @@ __global__ void __launch_bounds__(256) k_pres64(const __grid_constant__ S src, c
     batch_body_guard<HAS_COND>(d, cond);
     if (d.pctl->done) return;
     const int it = d.pctl->niter + d.res_every;
-    const int ni1 = d.NI - 1, total = ni1 * (d.NJ - 1);
+    const int p0 = blockIdx.x * d.ring_ppb, nl = 2 * min(d.ring_ppb, (d.NJ - 1) / 2 - p0);
+    const int g = threadIdx.x / TG, t = threadIdx.x % TG, j = 2 * p0 + 1 + g, n = d.NI - 1;
+    const bool act = g < nl;
     double ra = 0.0, pa = 0.0;
+    if (act) {
+        const Coef &cf = d.cP;
+        const double *P = d.P;
+        const int jn = jwrap(d, j + 1), js = jwrap(d, j - 1);
 #pragma unroll
-    for (int q = 0; q < RES64_CELLS; q++) {
-        int e = (blockIdx.x * RES64_CELLS + q) * 256 + threadIdx.x;
-        if (e < total) {
-            int i = e % ni1 + 1, j = e / ni1 + 1, c = IDX(i, j);
-            double su = d.DIVDT[c] - dd_src(d, d.P2, i, j);
-            double r = pres_at(d, d.P, su, i, j);
-            ra += fabs(r);
-            pa += fabs(d.cP.AP[c] * d.P[c]);
+        for (int k = 0; k < M; k++) {
+            const int e = t * M + k, i = e + 1;   // the ring's ownership
+            if (e < n) {
+                const int c = IDX(i, j);
+                const double su = pois_src_at(d, d.P2, d.DIVDT[c], i, j);
+                pois_resid(cf.AE[c], e + 1 < n ? P[c + 1] : 0.0, cf.AW[c], e > 0 ? P[c - 1] : 0.0, cf.AN[c],
+                           P[IDX(i, jn)], cf.AS[c], P[IDX(i, js)], su, cf.AP[c], P[c], ra, pa);
+            }
         }
     }
     griddep_launch();
-    if (!grid_sum2(d, ra, pa, sh, last, d.nblk_res64)) return;
+    if (act) {
+        line_sum2<NW>(ra, pa, wsum[0] + g * NW, wsum[1] + g * NW, t, NamedSync<NW>{1 + g});
+        if (t == 0) {
+            lsum[2 * g] = ra;
+            lsum[2 * g + 1] = pa;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        pairs_sum2(lsum, nl, ra, pa);
+        d.partial[2 * blockIdx.x] = ra;
+        d.partial[2 * blockIdx.x + 1] = pa;
+        __threadfence();
+        const unsigned nb = (unsigned)d.nblk_res64;
+        last = atomicInc(&d.pctl->ticket, nb - 1) == nb - 1;
+    }
+    __syncthreads();
+    if (!last || threadIdx.x >= WARP) return;
+    __threadfence();
+    blocks_sum2([&](int q) { return __ldcg(d.partial + q); }, d.nblk_res64, ra, pa);
     if (threadIdx.x == 0) {
         double resip = ra / pa;
         d.pctl->niter = it;
@@ -596,6 +623,7 @@ Tgt tgt_of(fvm_ctx *c)
     t.nblk_res = c->nblk_res;
     t.nblk_res64 = c->nblk_res64;
     t.nblk_mres = c->nblk_mres;
+    t.ring_ppb = c->d.ring_ppb;
     t.tr = c->d.sP;
     t.tt = c->d.sUY;
     t.mixed = c->p.precision == FVM_MIXED;
@@ -690,11 +718,16 @@ int poisson64_body(const Tgt &t, cudaGraphConditionalHandle cond, int has_cond)
         RC(launch_pois64(t, it & 1, 0, 1));
         RC(launch_pois64(t, it & 1, 1, 1));
     }
-    with_src(t, [&](const auto &src) {
-        using S = std::decay_t<decltype(src)>;
-        if (has_cond) launch_pdl(k_pres64<1, S>, dim3(t.nblk_res64, 1, t.nz), dim3(256), t.st, src, cond);
-        else launch_pdl(k_pres64<0, S>, dim3(t.nblk_res64, 1, t.nz), dim3(256), t.st, src, cond);
+    const dim3 grid(t.nblk_res64, 1, t.nz), block(2 * t.ring_ppb * WARP * t.tr.NW);
+    const bool ok = dispatch_line(t.tr, [&](auto m, auto nw) {
+        constexpr int M = decltype(m)::value, NW = decltype(nw)::value;
+        with_src(t, [&](const auto &src) {
+            using S = std::decay_t<decltype(src)>;
+            if (has_cond) launch_pdl(k_pres64<M, NW, 1, S>, grid, block, t.st, src, cond);
+            else launch_pdl(k_pres64<M, NW, 0, S>, grid, block, t.st, src, cond);
+        });
     });
+    if (!ok) return line_error(t.c);
     KCOUNT(t.c);
     FVM_LAUNCH_CHECK(t.c);
     return FVM_OK;
@@ -763,6 +796,7 @@ int sweep_pairs(const Tgt &t, int sweeps)
 {
     if (t.mixed && !t.tab.devs && t.c->res_lines)   // all sweeps in one resident launch
         return resident_sweeps(t, sweeps, 0, 0, 0u, 0, 0, 0);
+    if (!t.mixed && !t.tab.devs && t.c->ring_blocks) return ring_launch(t.c, 1, sweeps);
     for (int s = 0; s < sweeps; s++) {
         if (t.mixed) RC(mixed_sweep_pair(t, 0));
         else {
@@ -941,6 +975,7 @@ int poisson_graph_build(fvm_ctx *c)
 // bodies are launched, their kernels returning early once converged.
 long long poisson_loop_kernels(fvm_ctx *c, int niter)
 {
+    if (c->ring_blocks) return 0;   // one launch, counted when it was issued
     const int per = c->pgraph_batch;
     const bool mixed = c->p.precision == FVM_MIXED;
     long long bodies = (niter + (mixed ? 1 : 0) + per - 1) / per;
@@ -954,6 +989,7 @@ long long poisson_loop_kernels(fvm_ctx *c, int niter)
 int poisson_loop(fvm_ctx *c)
 {
     Dev &d = c->d;
+    if (c->ring_blocks) return ring_launch(c, 0, 0);
     RC(poisson_graph(c));
     if (!c->p.poisson_host_loop) {
         FVM_CUDA(c, cudaGraphLaunch(c->pgraph, c->stream));
@@ -1003,7 +1039,7 @@ int time_sweeps(fvm_ctx *c, int sweeps, double *ms_per_launch, long long *launch
     float ms = 0.f;
     FVM_CUDA(c, cudaEventElapsedTime(&ms, c->ev_a, c->ev_b));
     cudaGraphExecDestroy(ge);
-    const bool resident = c->p.precision == FVM_MIXED && c->res_lines;
+    const bool resident = c->p.precision == FVM_MIXED ? c->res_lines != 0 : c->ring_blocks != 0;
     *launches = resident ? 1LL : 2LL * sweeps;
     *ms_per_launch = ms / (2.0 * sweeps);   // per zebra colour
     c->tm.sweep_span_ms += ms;
@@ -1029,7 +1065,7 @@ int resident_fault(fvm_ctx *c)
 {
     RC(resident_reset(c));
     FVM_CUDA(c, cudaStreamSynchronize(c->stream));
-    c->err = "resident Poisson sweeps: a bounded wait for a neighbouring block ran out";
+    c->err = "on-chip Poisson sweeps: a bounded wait for a neighbouring block ran out";
     return FVM_ERR_TIMEOUT;
 }
 

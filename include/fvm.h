@@ -74,7 +74,10 @@ typedef struct fvm_params {
     /* MIXED, single context: FP32 correction sweeps of one refinement interval in
        one launch whose blocks keep their lines on chip and exchange only boundary
        lines (1, the default: lines per block chosen automatically; k >= 2, even:
-       k lines per block; 0: one launch per zebra colour).  Same results bit for bit. */
+       k lines per block; 0: one launch per zebra colour).  Same results bit for bit.
+       FP64, single context, dd_positional = 1: the whole Poisson iteration of a step
+       runs in one launch, whatever poisson_host_loop says (0: one launch per zebra
+       colour).  Same results bit for bit with the same line tile. */
     int poisson_resident;
     /* Resident sweeps: sweeps per exchange of boundary lines between blocks (0, the
        default: 2 where the layout allows it -- 4 lines per block, line groups of one
