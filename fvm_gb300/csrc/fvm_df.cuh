@@ -62,6 +62,17 @@ __device__ __forceinline__ double f2d_int(float f)
     const uint32_t lo = ex == 0u ? 0u : (m << 29);
     return __hiloint2double((int)hi, (int)lo);
 }
+// FP64 -> FP32, round to nearest even, with integer instructions where the result is a
+// normal number (the conversion instruction issues on the FP64 pipe).
+__device__ __forceinline__ float d2f_int(double x)
+{
+    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+    const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
+    if (e < 897u || e > 1149u) return (float)x;
+    const unsigned long long a = u & 0x7fffffffffffffffull;
+    const uint32_t m = (uint32_t)((a + 0x0fffffffull + ((a >> 29) & 1ull)) >> 29) - (896u << 23);
+    return __uint_as_float(m | ((uint32_t)(u >> 32) & 0x80000000u));
+}
 __device__ __forceinline__ double dd_join(dd a) { return f2d_int(a.hi) + f2d_int(a.lo); }
 
 __device__ __forceinline__ dd fast_two_sum(float a, float b)   // |a| >= |b|
