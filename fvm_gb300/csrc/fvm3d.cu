@@ -1085,39 +1085,40 @@ __global__ void k3_bcp(D3 d, int check_done)
     P[ID3(d.NI, j, k)] = (3.0 * P[ID3(d.NI - 1, j, k)] - 3.0 * P[ID3(d.NI - 2, j, k)]) + P[ID3(d.NI - 3, j, k)];
 }
 
-// Block sum of three values (warp shuffle trees, then the warps in order; thread 0
-// holds the result).
-__device__ __forceinline__ void block_sum3(double &a, double &b, double &e, double *sh)
+// Block sums of NV values (warp shuffle trees, then the warps in order; thread 0 holds
+// the results).
+template <int NV>
+__device__ __forceinline__ void block_sum(double (&v)[NV], double *sh)
 {
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_down_sync(0xffffffffu, a, o);
-        b += __shfl_down_sync(0xffffffffu, b, o);
-        e += __shfl_down_sync(0xffffffffu, e, o);
-    }
+#pragma unroll
+    for (int q = 0; q < NV; q++)
+        for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
     const int wid = threadIdx.x / WARP, lane = threadIdx.x & 31, nw = blockDim.x / WARP;
     __syncthreads();   // sh may hold an earlier round's values
-    if (lane == 0) { sh[3 * wid] = a; sh[3 * wid + 1] = b; sh[3 * wid + 2] = e; }
+    if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < NV; q++) sh[NV * wid + q] = v[q];
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double x = 0.0, y = 0.0, z = 0.0;
-        for (int w = 0; w < nw; w++) { x += sh[3 * w]; y += sh[3 * w + 1]; z += sh[3 * w + 2]; }
-        a = x;
-        b = y;
-        e = z;
-    }
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int q = 0; q < NV; q++) {
+            double x = 0.0;
+            for (int w = 0; w < nw; w++) x += sh[NV * w + q];
+            v[q] = x;
+        }
 }
 
-// Deterministic two-level sum of three values over the grid: each block's sum goes
+// Deterministic two-level sums of NV <= 4 values over the grid: each block's sums go
 // to `partial`; the last block to arrive sums the partials with all its threads
 // (a fixed strided assignment, then the block tree).  Returns true in the last
 // block, whose thread 0 holds the sums.
-__device__ bool grid_sum3(const D3 &d, double &a, double &b, double &e, double *sh, bool &last, unsigned *ticket)
+template <int NV>
+__device__ bool grid_sum(const D3 &d, double (&v)[NV], double *sh, bool &last, unsigned *ticket)
 {
-    block_sum3(a, b, e, sh);
+    block_sum<NV>(v, sh);
     if (threadIdx.x == 0) {
-        d.partial[4 * blockIdx.x] = a;
-        d.partial[4 * blockIdx.x + 1] = b;
-        d.partial[4 * blockIdx.x + 2] = e;
+#pragma unroll
+        for (int q = 0; q < NV; q++) d.partial[4 * blockIdx.x + q] = v[q];
         __threadfence();
         unsigned t = atomicInc(ticket, gridDim.x - 1);
         last = (t == gridDim.x - 1);
@@ -1125,15 +1126,12 @@ __device__ bool grid_sum3(const D3 &d, double &a, double &b, double &e, double *
     __syncthreads();
     if (!last) return false;
     __threadfence();
-    a = 0.0;
-    b = 0.0;
-    e = 0.0;
-    for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) {
-        a += ((volatile double *)d.partial)[4 * q];
-        b += ((volatile double *)d.partial)[4 * q + 1];
-        e += ((volatile double *)d.partial)[4 * q + 2];
-    }
-    block_sum3(a, b, e, sh);
+#pragma unroll
+    for (int q = 0; q < NV; q++) v[q] = 0.0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x)
+#pragma unroll
+        for (int q = 0; q < NV; q++) v[q] += ((volatile double *)d.partial)[4 * b + q];
+    block_sum<NV>(v, sh);
     return true;
 }
 
@@ -1143,11 +1141,11 @@ __device__ bool grid_sum3(const D3 &d, double &a, double &b, double &e, double *
 template <int HAS_COND>
 __global__ void __launch_bounds__(256) k3_pres(D3 d, Coef3 cf, int per, cudaGraphConditionalHandle cond)
 {
-    __shared__ double sh[3 * 8];
+    __shared__ double sh[4 * 8];
     __shared__ bool last;
     if (d.pctl->done) return;
     const int ni1 = d.NI - 1, nj1 = d.NJ - 1, total = ni1 * nj1 * (d.NK - 1);
-    double ra = 0.0, pa = 0.0, dummy = 0.0;
+    double sum[2] = {0.0, 0.0};   // |r|, |AP P|
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
         const int i = e % ni1 + 1, j = (e / ni1) % nj1 + 1, k = e / (ni1 * nj1) + 1, c = ID3(i, j, k);
         const double *P = d.P;
@@ -1155,13 +1153,13 @@ __global__ void __launch_bounds__(256) k3_pres(D3 d, Coef3 cf, int per, cudaGrap
                         cf.AN[c] * P[ID3(i, jw(d, j + 1), k)]) + cf.AS[c] * P[ID3(i, jw(d, j - 1), k)]) +
                       cf.AT[c] * P[ID3(i, j, kw(d, k + 1))]) + cf.AB[c] * P[ID3(i, j, kw(d, k - 1))]) +
                     d.SU[c]) - cf.AP[c] * P[c];
-        ra += fabs(r);
-        pa += fabs(cf.AP[c] * P[c]);
+        sum[0] += fabs(r);
+        sum[1] += fabs(cf.AP[c] * P[c]);
     }
-    if (!grid_sum3(d, ra, pa, dummy, sh, last, &d.pctl->ticket)) return;
+    if (!grid_sum<2>(d, sum, sh, last, &d.pctl->ticket)) return;
     if (threadIdx.x == 0) {
         const int it = d.pctl->niter + per;
-        const double resip = ra / pa;
+        const double resip = sum[0] / sum[1];
         d.pctl->niter = it;
         d.pctl->resip = resip;
         if (!(resip > d.resimax && it < d.nswpp)) {
@@ -1218,13 +1216,13 @@ __global__ void k3_coef_f32(D3 d)
 template <int HAS_COND>
 __global__ void __launch_bounds__(256) k3_mres(D3 d, cudaGraphConditionalHandle cond)
 {
-    __shared__ double sh[3 * 8];
+    __shared__ double sh[4 * 8];
     __shared__ bool last;
     if (d.pctl->done) return;
     const int it = d.pctl->niter;
     const Coef3 &cf = d.cf[6];
     const int ni1 = d.NI - 1, nj1 = d.NJ - 1, total = ni1 * nj1 * (d.NK - 1);
-    double ra = 0.0, pa = 0.0, dummy = 0.0;
+    double sum[2] = {0.0, 0.0};   // |r|, |AP P|
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
         const int i = e % ni1 + 1, j = (e / ni1) % nj1 + 1, k = e / (ni1 * nj1) + 1, c = ID3(i, j, k);
         const double *P = d.P;
@@ -1233,14 +1231,14 @@ __global__ void __launch_bounds__(256) k3_mres(D3 d, cudaGraphConditionalHandle 
                               cf.AN[c] * P[ID3(i, jw(d, j + 1), k)]) + cf.AS[c] * P[ID3(i, jw(d, j - 1), k)]) +
                             cf.AT[c] * P[ID3(i, j, kw(d, k + 1))]) + cf.AB[c] * P[ID3(i, j, kw(d, k - 1))]) + su) -
                          cf.AP[c] * P[c];
-        ra += fabs(r);
-        pa += fabs(cf.AP[c] * P[c]);
+        sum[0] += fabs(r);
+        sum[1] += fabs(cf.AP[c] * P[c]);
         d.RF[c] = fvm::d2f_int(r);
         d.DF[c] = 0.0f;
     }
-    if (!grid_sum3(d, ra, pa, dummy, sh, last, &d.pctl->ticket)) return;
+    if (!grid_sum<2>(d, sum, sh, last, &d.pctl->ticket)) return;
     if (threadIdx.x == 0) {
-        const double resip = ra / pa;
+        const double resip = sum[0] / sum[1];
         d.pctl->resip = resip;
         if (it > 0 && !(resip > d.resimax && it < d.nswpp)) {
             d.pctl->done = 1;
@@ -1267,13 +1265,12 @@ __device__ __forceinline__ void line_bcp(const D3 &d, int j, int k)
 // partner line (j-1, k) -- j -> j-1 maps the colour-1 lines of a plane one to one
 // onto the colour-0 lines -- and sets the BCP ghosts of both lines.
 template <int M, int NW>
-__global__ void __launch_bounds__(128) k3_line32(D3 d, LineSys s, int colour, int check_done, int apply)
+__global__ void __launch_bounds__(128) k3_line32(const __grid_constant__ D3 d, LineSys s, int colour, int check_done,
+                                                 int apply)
 {
     constexpr int TG = WARP * NW, G = 4 / NW;
     __shared__ float sm[G][TG * M + M * NW + 1];
     __shared__ float xch[G][2 * NW];
-    // the loop's done flag is loaded together with the operands below
-    const int stop = check_done ? d.pctl->done : 0;
     int gl, t, gib;
     fvm::group_of<NW>(gl, t, gib);
     int L = 0;
@@ -1282,21 +1279,39 @@ __global__ void __launch_bounds__(128) k3_line32(D3 d, LineSys s, int colour, in
     const int n = s.n, j = L % (d.NJ - 1) + 1, k = L / (d.NJ - 1) + 1;
     const int jn = jw(d, j + 1), js = jw(d, j - 1), kt = kw(d, k + 1), kb = kw(d, k - 1);
     const float *DF = d.DF;
-    float v[M];
+    // what no other sweep of the interval writes, before the wait for the preceding launch:
+    // couplings, right-hand side (the residual kernel does not trigger early) and factors
+    float v[M], an[M], as[M], at[M], ab[M], rf[M], fi[M], fa[M], fb[M];
+#pragma unroll
+    for (int q = 0; q < M; q++) {
+        const int e = q * TG + t;
+        const bool ok = active && e < n;
+        const int i = e + 1, c = ID3(i, j, k);
+        an[q] = ok ? d.ANf[c] : 0.0f;
+        as[q] = ok ? d.ANf[ID3(i, js, k)] : 0.0f;
+        at[q] = ok ? d.ATf[c] : 0.0f;
+        ab[q] = ok ? d.ATf[ID3(i, j, kb)] : 0.0f;
+        rf[q] = ok ? d.RF[c] : 0.0f;
+    }
+    const size_t base = size_t(L) * TG * M;
+    fvm::load_factors<float, M, NW>(fi, fa, fb, s.invDf + base, s.faf + base, s.fbf + base, t);
+    fvm::griddep_wait();
+    // the loop's done flag is loaded together with the operands
+    const int stop = check_done ? d.pctl->done : 0;
 #pragma unroll
     for (int q = 0; q < M; q++) {
         const int e = q * TG + t;
         v[q] = 0.0f;
         if (active && e < n) {
-            const int i = e + 1, c = ID3(i, j, k);
-            v[q] = ((d.ANf[c] * DF[ID3(i, jn, k)] + d.ANf[ID3(i, js, k)] * DF[ID3(i, js, k)]) +
-                    (d.ATf[c] * DF[ID3(i, j, kt)] + d.ATf[ID3(i, j, kb)] * DF[ID3(i, j, kb)])) + d.RF[c];
+            const int i = e + 1;
+            v[q] = ((an[q] * DF[ID3(i, jn, k)] + as[q] * DF[ID3(i, js, k)]) +
+                    (at[q] * DF[ID3(i, j, kt)] + ab[q] * DF[ID3(i, j, kb)])) + rf[q];
         }
     }
     if (stop) return;
+    fvm::griddep_launch();   // the next sweep may start its constant prologue
     fvm::to_chunks<float, M, NW>(v, sm[gib], t);
-    const size_t base = size_t(L) * TG * M;
-    fvm::group_apply<float, M, NW>(v, s.invDf + base, s.faf + base, s.fbf + base, t, xch[gib]);
+    fvm::group_apply_r<float, M, NW>(v, fi, fa, fb, t, xch[gib]);
     fvm::to_interleaved<float, M, NW>(v, sm[gib], t);
 #pragma unroll
     for (int q = 0; q < M; q++) {
@@ -1628,22 +1643,21 @@ __device__ __forceinline__ bool coef_nonneg(double lm, double mm)
 // (stress_tensor_dy.f90:486-517): result in scal[slot].
 __global__ void __launch_bounds__(256) k3_cvol(D3 d, int slot)
 {
-    __shared__ double sh[3 * 8];
+    __shared__ double sh[4 * 8];
     __shared__ bool last;
     const int ni1 = d.NI - 1, nj1 = d.NJ - 1, total = ni1 * nj1 * (d.NK - 1);
-    double lm = 0.0, mm = 0.0, inc = 0.0;
+    double sum[3] = {0.0, 0.0, 0.0};   // LM, MM and the number of points
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
         const int i = e % ni1 + 1, j = (e / ni1) % nj1 + 1, k = e / (ni1 * nj1) + 1, c = ID3(i, j, k);
         if (coef_nonneg(d.LM[c], d.MM[c])) {
-            lm += d.LM[c];
-            mm += d.MM[c];
-            inc += 1.0;
+            sum[0] += d.LM[c];
+            sum[1] += d.MM[c];
+            sum[2] += 1.0;
         }
     }
-    if (!grid_sum3(d, lm, mm, inc, sh, last, &d.pctl->ticket)) return;
+    if (!grid_sum<3>(d, sum, sh, last, &d.pctl->ticket)) return;
     if (threadIdx.x == 0) {
-        lm = lm / inc;
-        mm = mm / inc;
+        const double lm = sum[0] / sum[2], mm = sum[1] / sum[2];
         double cavg = (0.5 * lm) / mm;
         if (mm < 1e-6) cavg = 0.0;
         d.scal[slot] = cavg;
@@ -2143,7 +2157,7 @@ int line32(fvm3_ctx *c, int colour, int check_done, int apply)
     const int blocks = fvm::line_blocks(per, s.NW);
     bool ok = fvm::dispatch_line(s, [&](auto m, auto nw) {
         constexpr int M = decltype(m)::value, NW = decltype(nw)::value;
-        k3_line32<M, NW><<<blocks, 128, 0, c->stream>>>(d, s, colour, check_done, apply);
+        fvm::launch_pdl(k3_line32<M, NW>, dim3(blocks), dim3(128), c->stream, d, s, colour, check_done, apply);
     });
     if (!ok) {
         c->err = "line length above 512 cells is not supported";
