@@ -614,17 +614,15 @@ __device__ __forceinline__ bool colour_line(const D3 &d, int fam, int colour, in
         L = (j - 1) + (d.NJ - 1) * (k - 1);
         return true;
     }
-    if (fam == 1) {   // transverse (i,k): per i, (NK-1)/2 lines
-        const int h = (d.NK - 1) / 2, i = gl / h + 1;
-        if (i > d.NI - 1) return false;
-        const int k = (((i + 1) & 1) == colour ? 1 : 2) + 2 * (gl % h);
-        L = (i - 1) + (d.NI - 1) * (k - 1);
-        return true;
-    }
-    const int h = (d.NJ - 1) / 2, i = gl / h + 1;   // transverse (i,j)
+    // J lines, transverse (i,k), and K lines, transverse (i,j): neighbouring groups take
+    // neighbouring i of the colour, so that the lines of a block share their 32-byte
+    // sectors (with i slowest every element was a sector of its own, four times the
+    // bytes: 61 us a launch at 256 x 192 x 48)
+    const int h = d.NI / 2, q = gl / h + 1;   // the other index; h = ceil((NI-1)/2) lines per q
+    if (q > (fam == 1 ? d.NK : d.NJ) - 1) return false;
+    const int i = (((q + 1) & 1) == colour ? 1 : 2) + 2 * (gl % h);
     if (i > d.NI - 1) return false;
-    const int j = (((i + 1) & 1) == colour ? 1 : 2) + 2 * (gl % h);
-    L = (i - 1) + (d.NI - 1) * (j - 1);
+    L = (i - 1) + (d.NI - 1) * (q - 1);
     return true;
 }
 
@@ -1766,81 +1764,69 @@ __global__ void __launch_bounds__(128) k3_cfl(D3 d)
     }
 }
 
-// Wall force and heat-flux contributions of the two triangles of each wall face.
-__global__ void k3_wall(D3 d)
+// Wall force and heat-flux contributions of the two triangles of each wall face,
+// summed per block (fixed tree; k3_calc_final adds the blocks).  One block adding all
+// 2 (NJ-1)(NK-1) contributions took 77 us at 256 x 48 on its four FP64 pipes.
+__global__ void __launch_bounds__(128) k3_wall(D3 d)
 {
+    __shared__ double sh[5 * 4];
     const int j = blockIdx.x * blockDim.x + threadIdx.x + 1, k = blockIdx.y + 1, tri = blockIdx.z;
-    if (j > d.NJ - 1 || k > d.NK - 1) return;
-    const int i = 1, c = ID3(i, j, k);
-    int p, q, r;
-    if (tri == 0) { p = ID3(i, j, k); q = ID3(i, j + 1, k); r = ID3(i, j, k + 1); }
-    else { p = ID3(i, j + 1, k + 1); q = ID3(i, j, k + 1); r = ID3(i, j, k); }
-    const double *XG = d.XG, *YG = d.YG, *ZG = d.ZG;
-    const double A = (YG[p] * (ZG[q] - ZG[r]) + YG[q] * (ZG[r] - ZG[p])) + YG[r] * (ZG[p] - ZG[q]);
-    const double B = (ZG[p] * (XG[q] - XG[r]) + ZG[q] * (XG[r] - XG[p])) + ZG[r] * (XG[p] - XG[q]);
-    const double C = (XG[p] * (YG[q] - YG[r]) + XG[q] * (YG[r] - YG[p])) + XG[r] * (YG[p] - YG[q]);
-    double D = (XG[p] * (YG[q] * ZG[r] - YG[r] * ZG[q]) + XG[q] * (YG[r] * ZG[p] - YG[p] * ZG[r])) +
-               XG[r] * (YG[p] * ZG[q] - YG[q] * ZG[p]);
-    D = -1.0 * D;
-    const double dum = sqrt((A * A + B * B) + C * C);
-    const double dn = fabs(((A * d.X[c] + B * d.Y[c]) + C * d.Z[c]) + D) / dum;
-    const double u = d.U[c], v = d.V[c], w = d.W[c];
-    const double e1 = (v * C) / dum - (w * B) / dum, e2 = (u * C) / dum - (w * A) / dum, e3 = (u * B) / dum - (v * A) / dum;
-    double dudn = sqrt((e1 * e1 + e2 * e2) + e3 * e3);
-    dudn = dudn / dn;
-    const double area = tri == 0 ? d.AREA1[c] : d.AREA2[c];
-    const double vm = sqrt((u * u + v * v) + w * w);
-    double *o = d.wall + 8 * (size_t(tri) * d.NJ1 * (d.NK + 1) + JK(j, k));
-    o[0] = (((2.0 * d.P[c]) * area) * A) / dum;
-    o[1] = (((2.0 * d.P[c]) * area) * B) / dum;
-    o[2] = ((((2.0 / d.re) * dudn) * area) * u) / vm;
-    o[3] = ((((2.0 / d.re) * dudn) * area) * v) / vm;
-    o[4] = ((d.T[c] - d.t_wall) / dn) * area;
+    double o[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    if (j <= d.NJ - 1) {
+        const int i = 1, c = ID3(i, j, k);
+        int p, q, r;
+        if (tri == 0) { p = ID3(i, j, k); q = ID3(i, j + 1, k); r = ID3(i, j, k + 1); }
+        else { p = ID3(i, j + 1, k + 1); q = ID3(i, j, k + 1); r = ID3(i, j, k); }
+        const double *XG = d.XG, *YG = d.YG, *ZG = d.ZG;
+        const double A = (YG[p] * (ZG[q] - ZG[r]) + YG[q] * (ZG[r] - ZG[p])) + YG[r] * (ZG[p] - ZG[q]);
+        const double B = (ZG[p] * (XG[q] - XG[r]) + ZG[q] * (XG[r] - XG[p])) + ZG[r] * (XG[p] - XG[q]);
+        const double C = (XG[p] * (YG[q] - YG[r]) + XG[q] * (YG[r] - YG[p])) + XG[r] * (YG[p] - YG[q]);
+        double D = (XG[p] * (YG[q] * ZG[r] - YG[r] * ZG[q]) + XG[q] * (YG[r] * ZG[p] - YG[p] * ZG[r])) +
+                   XG[r] * (YG[p] * ZG[q] - YG[q] * ZG[p]);
+        D = -1.0 * D;
+        const double dum = sqrt((A * A + B * B) + C * C);
+        const double dn = fabs(((A * d.X[c] + B * d.Y[c]) + C * d.Z[c]) + D) / dum;
+        const double u = d.U[c], v = d.V[c], w = d.W[c];
+        const double e1 = (v * C) / dum - (w * B) / dum, e2 = (u * C) / dum - (w * A) / dum, e3 = (u * B) / dum - (v * A) / dum;
+        double dudn = sqrt((e1 * e1 + e2 * e2) + e3 * e3);
+        dudn = dudn / dn;
+        const double area = tri == 0 ? d.AREA1[c] : d.AREA2[c];
+        const double vm = sqrt((u * u + v * v) + w * w);
+        o[0] = (((2.0 * d.P[c]) * area) * A) / dum;
+        o[1] = (((2.0 * d.P[c]) * area) * B) / dum;
+        o[2] = ((((2.0 / d.re) * dudn) * area) * u) / vm;
+        o[3] = ((((2.0 / d.re) * dudn) * area) * v) / vm;
+        o[4] = ((d.T[c] - d.t_wall) / dn) * area;
+    }
+    block_sum<5>(o, sh);
+    if (threadIdx.x == 0)
+        for (int q = 0; q < 5; q++)
+            d.wall[8 * ((size_t(tri) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) + q] = o[q];
 }
 
-// Sums of the wall contributions in a fixed tree (one block: a strided partial sum
-// per thread, then the warps' shuffle trees, then the warps in order), the
-// coefficients into scal[3..16].
-__global__ void __launch_bounds__(1024) k3_calc_final(D3 d, double rtime, double sum_area)
+// Sums of k3_wall's `parts` block sums and the span average of the base pressure in a
+// fixed tree (one block of 128 threads), the coefficients into scal[3..16].
+__global__ void __launch_bounds__(128) k3_calc_final(D3 d, double rtime, double sum_area, int parts)
 {
-    __shared__ double sh[5][32];
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int nj1 = d.NJ - 1, nk1 = d.NK - 1, plane = nj1 * nk1, total = 2 * plane;
-    double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    for (int e = t; e < total; e += blockDim.x) {
-        const int tri = e / plane, r = e - tri * plane, k = r / nj1 + 1, j = r - (k - 1) * nj1 + 1;
-        const double *o = d.wall + 8 * (size_t(tri) * d.NJ1 * (d.NK + 1) + JK(j, k));
-        acc[0] = acc[0] - o[0];
-        acc[1] = acc[1] - o[1];
-        acc[2] = acc[2] + o[2];
-        acc[3] = acc[3] + o[3];
-        acc[4] = acc[4] + o[4];
-    }
+    __shared__ double sh[6 * 4];
+    double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int e = threadIdx.x; e < parts; e += blockDim.x) {
+        const double *o = d.wall + 8 * size_t(e);
 #pragma unroll
-    for (int q = 0; q < 5; q++) {
-        for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_down_sync(0xffffffffu, acc[q], o);
-        if (lane == 0) sh[q][warp] = acc[q];
-    }
-    __syncthreads();
-    if (t != 0) return;
-    double pd = 0.0, pl = 0.0, td = 0.0, tl = 0.0, snu = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
-        pd += sh[0][w];
-        pl += sh[1][w];
-        td += sh[2][w];
-        tl += sh[3][w];
-        snu += sh[4][w];
+        for (int q = 0; q < 5; q++) acc[q] += o[q];
     }
     const double *P = d.P;
-    double dumb = 0.0;
-    for (int k = 1; k <= d.NK - 1; k++) {
+    for (int k = 1 + threadIdx.x; k <= d.NK - 1; k += blockDim.x) {
         const int i = 1, j = 1;
         const double pg = 0.125 * (((((((P[ID3(i, j, k)] + P[ID3(i, j - 1, k)]) + P[ID3(i - 1, j, k)]) +
                                        P[ID3(i - 1, j - 1, k)]) + P[ID3(i, j, k + 1)]) + P[ID3(i, j - 1, k + 1)]) +
                                      P[ID3(i - 1, j, k + 1)]) + P[ID3(i - 1, j - 1, k + 1)]);
-        dumb = dumb + pg;
+        acc[5] += pg;
     }
-    dumb = dumb / (double)(d.NK - 1);
+    block_sum<6>(acc, sh);
+    if (threadIdx.x != 0) return;
+    const double pd = -acc[0], pl = -acc[1], td = acc[2], tl = acc[3], snu = acc[4];
+    const double dumb = acc[5] / (double)(d.NK - 1);
     double *s = d.scal + 3;
     s[0] = rtime;
     s[1] = __longlong_as_double((long long)*d.cflbits);
@@ -2122,8 +2108,7 @@ int line(fvm3_ctx *c, int set, const double *SU, double *phi, int colour, const 
     const int fam = set == 6 ? 0 : set % 3;
     int per;
     if (fam == 0) per = (c->NJ - 1) / 2 * (c->NK - 1);
-    else if (fam == 1) per = (c->NI - 1) * ((c->NK - 1) / 2);
-    else per = (c->NI - 1) * ((c->NJ - 1) / 2);
+    else per = (c->NI / 2) * ((fam == 1 ? c->NK : c->NJ) - 1);
     const int blocks = fvm::line_blocks(per, s.NW);
     bool ok = fvm::dispatch_line(s, [&](auto m, auto nw) {
         constexpr int M = decltype(m)::value, NW = decltype(nw)::value;
@@ -2538,8 +2523,9 @@ int calccoef(fvm3_ctx *c)   // CALCCOEF kernels; the record is read by read_coef
 {
     D3 &d = c->d;
     k3_cfl<<<dim3((c->NI - 1 + 127) / 128, c->NJ - 1, c->NK - 1), 128, 0, c->stream>>>(d);
-    k3_wall<<<dim3((c->NJ + 127) / 128, c->NK - 1, 2), 128, 0, c->stream>>>(d);
-    k3_calc_final<<<1, 1024, 0, c->stream>>>(d, c->rtime, c->sum_area);
+    const dim3 gw((c->NJ - 1 + 127) / 128, c->NK - 1, 2);
+    k3_wall<<<gw, 128, 0, c->stream>>>(d);
+    k3_calc_final<<<1, 128, 0, c->stream>>>(d, c->rtime, c->sum_area, int(gw.x * gw.y * gw.z));
     if (c->ipost && c->post) {
         k3_post_acc<<<g_lin(c), 256, 0, c->stream>>>(d, c->post);
         c->niter_pos += 1;
