@@ -2752,14 +2752,13 @@ int fvm3_upload_state(fvm3_ctx *c, const double *u, const double *v, const doubl
 {
     if (!c) return FVM_ERR_ARG;
     if (!c->grid_set) return f3::bad3(c, "fvm3_set_grid has not been called");
-    const size_t bytes = sizeof(double) * c->n;
     f3::D3 &d = c->d;
     const double *src[] = {u, v, w, p, t, nlx, nly, nlz, adv};
     double *dst[] = {d.U, d.V, d.W, d.P, d.T, d.NLX, d.NLY, d.NLZ, d.ADV};
+    F3CUDA(c, fvm::copy_arrays(dst, src, 9, c->n, cudaMemcpyHostToDevice, c->stream));
     std::vector<double *> shadowed;
     for (int k = 0; k < 9; k++) {
         if (!src[k]) continue;
-        F3CUDA(c, cudaMemcpyAsync(dst[k], src[k], bytes, cudaMemcpyHostToDevice, c->stream));
         if (c->d.dfl && dst[k] >= c->shadow_lo && dst[k] < c->shadow_hi) shadowed.push_back(dst[k]);
     }
     if (!shadowed.empty()) F3RC(f3::refresh(c, shadowed));   // double-float shadows (mixed path)
@@ -2772,12 +2771,10 @@ int fvm3_download_state(fvm3_ctx *c, double *u, double *v, double *w, double *p,
                         double *nly, double *nlz, double *adv)
 {
     if (!c) return FVM_ERR_ARG;
-    const size_t bytes = sizeof(double) * c->n;
     f3::D3 &d = c->d;
     double *dst[] = {u, v, w, p, t, nlx, nly, nlz, adv};
     const double *src[] = {d.U, d.V, d.W, d.P, d.T, d.NLX, d.NLY, d.NLZ, d.ADV};
-    for (int k = 0; k < 9; k++)
-        if (dst[k]) F3CUDA(c, cudaMemcpyAsync(dst[k], src[k], bytes, cudaMemcpyDeviceToHost, c->stream));
+    F3CUDA(c, fvm::copy_arrays(dst, src, 9, c->n, cudaMemcpyDeviceToHost, c->stream));
     F3CUDA(c, cudaStreamSynchronize(c->stream));
     return FVM_OK;
 }

@@ -170,12 +170,10 @@ int fvm_upload_state(fvm_ctx *c, const double *u, const double *v, const double 
 {
     if (!c) return FVM_ERR_ARG;
     if (!c->grid_set) return bad(c, "fvm_set_grid has not been called");
-    const size_t bytes = sizeof(double) * c->n;
     Dev &d = c->d;
     const double *src[] = {u, v, p, t, nlx, nly, adv};
     double *dst[] = {d.U, d.V, d.P, d.T, d.NLX, d.NLY, d.ADV};
-    for (int k = 0; k < 7; k++)
-        if (src[k]) FVM_CUDA(c, cudaMemcpyAsync(dst[k], src[k], bytes, cudaMemcpyHostToDevice, c->stream));
+    FVM_CUDA(c, fvm::copy_arrays(dst, src, 7, c->n, cudaMemcpyHostToDevice, c->stream));
     FVM_CUDA(c, cudaStreamSynchronize(c->stream));
     c->init_done = true;
     return FVM_OK;
@@ -185,12 +183,10 @@ int fvm_download_state(fvm_ctx *c, double *u, double *v, double *p, double *t, d
                        double *adv)
 {
     if (!c) return FVM_ERR_ARG;
-    const size_t bytes = sizeof(double) * c->n;
     Dev &d = c->d;
     double *dst[] = {u, v, p, t, nlx, nly, adv};
     const double *src[] = {d.U, d.V, d.P, d.T, d.NLX, d.NLY, d.ADV};
-    for (int k = 0; k < 7; k++)
-        if (dst[k]) FVM_CUDA(c, cudaMemcpyAsync(dst[k], src[k], bytes, cudaMemcpyDeviceToHost, c->stream));
+    FVM_CUDA(c, fvm::copy_arrays(dst, src, 7, c->n, cudaMemcpyDeviceToHost, c->stream));
     FVM_CUDA(c, cudaStreamSynchronize(c->stream));
     return FVM_OK;
 }

@@ -313,6 +313,9 @@ int resident_sweeps(const Tgt &t, int sweeps, int apply, int max_polls, unsigned
                     cudaGraphConditionalHandle cond, int has_cond, int check_done, int decide = 0);
 int resident_reset(fvm_ctx *c);
 size_t exchange_words(const fvm_ctx *c);   // 64-bit words of d.XW
+// state copies between caller buffers and the device (fvm_copy.cu)
+cudaError_t copy_arrays(double *const *dst, const double *const *src, int count, size_t n, cudaMemcpyKind kind,
+                        cudaStream_t st);
 // FP64 Poisson iteration in one launch (fvm_ring.cu)
 int ring_setup(fvm_ctx *c);
 int ring_pairs(const fvm_ctx *c);   // line pairs per block
