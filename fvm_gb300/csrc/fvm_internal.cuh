@@ -188,6 +188,7 @@ struct fvm_ctx {
     // launches), blocks, and whether the launch carries the cooperative attribute
     int res_lines = 0, res_blocks = 0;
     int res_depth = 1;   // sweeps per boundary-line exchange (1, or 2 with 4 lines per block)
+    bool res_loop = false;   // the whole mixed Poisson iteration of a step in one launch
     bool res_coop = false;
     fvm::PostState post;
     int post_suspend = 0;   // recomputation passes of the adjoint: no post-processing
@@ -311,6 +312,7 @@ int resident_setup(fvm_ctx *c);
 int resident_sweeps_on(fvm_ctx *c, const ResSys &sys, int sweeps, int apply, int check_done);
 int resident_sweeps(const Tgt &t, int sweeps, int apply, int max_polls, unsigned tag_skew,
                     cudaGraphConditionalHandle cond, int has_cond, int check_done, int decide = 0);
+int resident_loop(fvm_ctx *c);   // the whole forward iteration (c->res_loop)
 int resident_reset(fvm_ctx *c);
 size_t exchange_words(const fvm_ctx *c);   // 64-bit words of d.XW
 // state copies between caller buffers and the device (fvm_copy.cu)
@@ -536,6 +538,104 @@ __device__ __forceinline__ void group_apply_r(T (&v)[M], const T (&fi)[M], const
 #pragma unroll
         for (int k = 0; k < M; k++) v[k] = v[k] + gk[k] * xin;
     }
+}
+
+// The constant part of group_apply_r's scans, formed once for a line that is solved many
+// times: per scan stage the factor a thread multiplies (zero where group_apply_r does not
+// combine), the factors of the value carried in from the other warps, and the stages that
+// are needed: those whose factors are all at or below `tiny` (an element's value reaches
+// no further along the line) are left out.  Groups of one or two warps.
+constexpr int SCAN_STAGES = 5;
+template <typename T>
+struct ScanConst {
+    T g[SCAN_STAGES], h[SCAN_STAGES], gx, hx;
+    int stages;
+};
+template <typename T, int M>
+__device__ __forceinline__ ScanConst<T> scan_constants(const T (&fa)[M], const T (&fb)[M], int t, T tiny)
+{
+    const int lane = t & (WARP - 1);
+    ScanConst<T> c;
+    T G = T(1), H = T(1);
+    c.stages = 0;
+#pragma unroll
+    for (int k = 0; k < M; k++) G = G * fa[k];
+#pragma unroll
+    for (int k = M - 1; k >= 0; k--) H = H * fb[k];
+#pragma unroll
+    for (int s = 0; s < SCAN_STAGES; s++) {
+        const int o = 1 << s;
+        const T Gp = shfl_up(G, o), Hn = shfl_down(H, o);
+        c.g[s] = lane >= o ? G : T(0);
+        c.h[s] = lane + o < WARP ? H : T(0);
+        if (__any_sync(0xffffffffu, c.g[s] > tiny || c.g[s] < -tiny || c.h[s] > tiny || c.h[s] < -tiny)) c.stages = s + 1;
+        if (lane >= o) G = G * Gp;
+        if (lane + o < WARP) H = H * Hn;
+    }
+    const T Gx = shfl_up(G, 1), Hx = shfl_down(H, 1);
+    c.gx = lane == 0 ? T(1) : Gx;
+    c.hx = lane == WARP - 1 ? T(1) : Hx;
+    return c;
+}
+template <int K, bool UP, typename T>
+__device__ __forceinline__ T scan_values(T y, const T (&g)[SCAN_STAGES])
+{
+#pragma unroll
+    for (int s = 0; s < K; s++) y = fma_rn(g[s], UP ? shfl_up(y, 1 << s) : shfl_down(y, 1 << s), y);
+    return y;
+}
+
+// group_apply_r with those constants: the value part only, and one barrier per pass (the
+// two passes exchange through words of their own, fold[2]).  The same bits (but for the
+// left-out stages).
+template <typename T, int M, int NW, class Sync>
+__device__ __forceinline__ void group_apply_c(T (&v)[M], const T (&fi)[M], const T (&fa)[M], const T (&fb)[M],
+                                              const ScanConst<T> &c, T *fold, int t, Sync sync)
+{
+    static_assert(NW <= 2, "one or two warps per line");
+    const int lane = t & (WARP - 1), wl = t / WARP;
+    T gk[M];
+    T y = T(0), g = T(1);
+#pragma unroll
+    for (int k = 0; k < M; k++) {
+        y = fma_rn(fa[k], y, mul_rn(fi[k], v[k]));
+        v[k] = y;
+        g = g * fa[k];
+        gk[k] = g;
+    }
+    // the stage count is uniform: one branch, no test per stage on the serial chain
+    if (c.stages <= 2) y = scan_values<2, true>(y, c.g);
+    else if (c.stages == 3) y = scan_values<3, true>(y, c.g);
+    else y = scan_values<5, true>(y, c.g);
+    T in = shfl_up(y, 1);
+    if (lane == 0) in = T(0);
+    if (NW > 1) {
+        if (t == WARP - 1) fold[0] = y;
+        sync();
+        if (wl) in = fma_rn(c.gx, fold[0], in);
+    }
+#pragma unroll
+    for (int k = 0; k < M; k++) v[k] = fma_rn(gk[k], in, v[k]);
+    T x = T(0), h = T(1);
+#pragma unroll
+    for (int k = M - 1; k >= 0; k--) {
+        x = fma_rn(fb[k], x, v[k]);
+        v[k] = x;
+        h = h * fb[k];
+        gk[k] = h;
+    }
+    if (c.stages <= 2) x = scan_values<2, false>(x, c.h);
+    else if (c.stages == 3) x = scan_values<3, false>(x, c.h);
+    else x = scan_values<5, false>(x, c.h);
+    in = shfl_down(x, 1);
+    if (lane == WARP - 1) in = T(0);
+    if (NW > 1) {
+        if (t == WARP) fold[1] = x;
+        sync();
+        if (!wl) in = fma_rn(c.hx, fold[1], in);
+    }
+#pragma unroll
+    for (int k = 0; k < M; k++) v[k] = fma_rn(gk[k], in, v[k]);
 }
 
 // Load the factors of one line (chunk ownership) into registers.

@@ -43,7 +43,7 @@ void split_pcoef(fvm_ctx *c)
 // Residual of the current P (iter_p.f90:24-30, 42-44: SU = DIVDT - DD(P), then the
 // five-point residual), its scaled-L1 norm (iter_p.f90:37-50), the FP32 right-hand
 // side of the correction sweeps and the zeroed correction.  The last block decides
-// convergence.
+// convergence.  (Single contexts on the resident loop form the same residual inside it.)
 //
 // Evaluated in double-float (the terms and order of dd_src and pres_at): about
 // 2^-46 relative to |AP P| per term, far below any Poisson tolerance, on the FP32
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(256, 6) k_mres(const __grid_constant__ S src, 
 {
     constexpr int TI = MRES_TI, TJ = MRES_TJ, W = TI + 3, H = TJ + 3;
     static_assert(TI == WARP && TI * TJ == 256, "one warp per tile row");
-    __shared__ double sh[64];
+    __shared__ double sh[2 * MRES_MAX_GROUPS + 3];
     __shared__ bool last;
     __shared__ float2 ps[H][W];
     const Dev &d = dev_of(src);
@@ -120,18 +120,34 @@ __global__ void __launch_bounds__(256, 6) k_mres(const __grid_constant__ S src, 
         d.DF[c] = 0.0f;
     }
     griddep_launch();
-    double ra, pa;
-    if (!DECIDE) {
-        block_sum2f(raf, paf, ra, pa, sh);
-        if (threadIdx.x == 0) {
-            d.partial[2 * blockIdx.x] = ra;
-            d.partial[2 * blockIdx.x + 1] = pa;
-        }
-        return;
+    for (int o = 16; o > 0; o >>= 1) {
+        raf += __shfl_down_sync(0xffffffffu, raf, o);
+        paf += __shfl_down_sync(0xffffffffu, paf, o);
     }
-    if (!grid_sum2f(d, raf, paf, ra, pa, sh, last, d.nblk_mres)) return;
+    if (tx == 0) {
+        sh[ty] = (double)raf;
+        sh[TJ + ty] = (double)paf;
+    }
+    __syncthreads();
+    const int ng = (d.NJ - 1 + MRES_GROUP - 1) / MRES_GROUP;
+    if (threadIdx.x < 2 * (TJ / MRES_GROUP)) {   // the tile's two groups, two values each
+        const int value = threadIdx.x & 1, q = threadIdx.x >> 1, g = (j0 - 1) / MRES_GROUP + q;
+        if (g < ng) {
+            d.partial[2 * (g * ti + (i0 - 1) / TI) + value] = mres_lines(sh + value * TJ + q * MRES_GROUP, 1);
+            if (DECIDE) __threadfence();
+        }
+    }
+    if (!DECIDE) return;
+    __syncthreads();
     if (threadIdx.x == 0) {
-        double resip = ra / pa;
+        const unsigned nb = (unsigned)d.nblk_mres;
+        last = atomicInc(&d.pctl->ticket, nb - 1) == nb - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const double resip = mres_total(d.partial, ng, ti, sh);
+    if (threadIdx.x == 0) {
         d.pctl->resip = resip;
         if (it > 0 && !(resip > d.resimax && it < d.nswpp)) {
             d.pctl->done = 1;

@@ -301,34 +301,49 @@ __device__ __forceinline__ bool grid_sum2f(const Dev &d, float af, float bf, dou
     return grid_publish2(d, a, b, sh, last, nblk);
 }
 
-// The sums grid_publish2's last block forms, formed by any block of at least 256
-// threads from partials another kernel left: thread k < 256 adds partials k, k+256,
-// ... in increasing order, threads from 256 on contribute zero (which leaves the
-// shuffle trees' sums unchanged), then block_sum2.  Same bits as grid_publish2 with
-// 256-thread blocks.
-__device__ __forceinline__ void sum_partials256(const double *partial, int nblk, double &a, double &b, double *sh)
+// Sums of the mixed residual (sum |r|, sum |AP P|), one order for k_mres and for the
+// resident loop: 32 cells of a line in FP32 (shuffle tree), four lines of one group
+// (j = 4g+1 .. 4g+4) in order in FP64, the group's tile columns by a 16-lane tree, the
+// groups over one warp per value (lane q takes groups q, q+32, ..., then the tree).
+constexpr int MRES_GROUP = 4;          // lines per group
+constexpr int MRES_MAX_GROUPS = 128;   // 512 lines
+__device__ __forceinline__ double mres_lines(const double *w, int stride)
 {
-    a = 0.0;
-    b = 0.0;
-    if (threadIdx.x < 256) {
-        const double2 *pp = reinterpret_cast<const double2 *>(partial);
-        for (int k0 = threadIdx.x; k0 < nblk; k0 += 4 * 256) {
-            double2 x[4];
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                const int k = k0 + r * 256;
-                x[r] = k < nblk ? __ldcg(pp + k) : make_double2(0.0, 0.0);
-            }
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                if (k0 + r * 256 < nblk) {
-                    a += x[r].x;
-                    b += x[r].y;
-                }
-            }
-        }
+    return ((w[0] + w[stride]) + w[2 * stride]) + w[3 * stride];
+}
+__device__ __forceinline__ double mres_columns(double x)
+{
+    for (int o = 8; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o, 16);
+    return x;
+}
+// The last two levels from the group sums tot[2 g + value] in shared memory (visible to
+// the block), by the block's first two warps; sum|r| / sum|AP P| in *res afterwards.
+__device__ __forceinline__ void mres_ratio(const double *tot, int ng, double *ab, double *res)
+{
+    const int wid = threadIdx.x / WARP, lane = threadIdx.x & (WARP - 1);
+    if (wid < 2) {
+        double x = 0.0;
+        for (int q = lane; q < ng; q += WARP) x += tot[2 * q + wid];
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if (lane == 0) ab[wid] = x;
     }
-    block_sum2(a, b, sh);
+    __syncthreads();
+    if (threadIdx.x == 0) *res = ab[0] / ab[1];
+    __syncthreads();
+}
+// The same from the (group, column) partials k_mres left in global memory.  sh:
+// 2 MRES_MAX_GROUPS + 3 doubles; returns the ratio in every thread.
+__device__ __forceinline__ double mres_total(const double *partial, int ng, int nt, double *sh)
+{
+    const int lane = threadIdx.x & (WARP - 1), half = lane >> 4, it = lane & 15;
+    for (int g = threadIdx.x / WARP; g < ng; g += blockDim.x / WARP) {
+        const double x = mres_columns(it < nt ? __ldcg(partial + 2 * (g * nt + it) + half) : 0.0);
+        if (it == 0) sh[2 * g + half] = x;
+    }
+    __syncthreads();
+    double *ab = sh + 2 * MRES_MAX_GROUPS;
+    mres_ratio(sh, ng, ab, ab + 2);
+    return ab[2];
 }
 
 // A case's Poisson iteration has ended (converged or capped).  Inside a batch the

@@ -35,13 +35,15 @@
 // -ftz=true, as the per-colour sweeps are.
 //
 // k_pois32_resident2 (below) exchanges once per two sweeps: 4-line blocks keep an
-// 11-line window and solve the neighbours' three nearest lines again; and either
-// kernel, launched inside the forward Poisson loop, first takes the loop's
-// convergence decision from the residual kernel's block sums (resident_decide).
+// 11-line window and solve the neighbours' three nearest lines again; it also runs the
+// whole forward iteration, residuals and decisions included, in one launch.  Launched per
+// interval inside the forward Poisson loop, either kernel first takes the loop's
+// convergence decision from the residual kernel's sums (resident_decide).
 #include <type_traits>
 
 #include "fvm_internal.cuh"
 #include "fvm_ops.cuh"
+#include "fvm_df.cuh"
 
 namespace fvm {
 namespace {
@@ -61,7 +63,7 @@ __device__ __forceinline__ void st_word(unsigned long long *p, unsigned long lon
 }
 
 // Convergence decision of the forward Poisson loop at the start of a resident
-// launch (sys.decide): every block sums the block partials the residual kernel
+// launch (sys.decide): every block sums the partials the residual kernel
 // k_mres left, in that kernel's own order (the same bits in every block), and takes
 // k_mres's decision (iter_p.f90:37-50: done once the scaled residual is at the
 // tolerance or the sweeps reach the cap) with the loop's sweep count from its own
@@ -71,11 +73,7 @@ __device__ __forceinline__ void st_word(unsigned long long *p, unsigned long lon
 template <int HAS_COND>
 __device__ bool resident_decide(const Dev &d, const ResSys &sys, int S, double *sh, cudaGraphConditionalHandle cond)
 {
-    double a, b;
-    sum_partials256(d.partial, d.nblk_mres, a, b, sh);
-    if (threadIdx.x == 0) sh[0] = a / b;   // warp 0 has finished reading sh
-    __syncthreads();
-    const double resip = sh[0];
+    const double resip = mres_total(d.partial, (d.NJ - 1 + MRES_GROUP - 1) / MRES_GROUP, (d.NI - 1 + MRES_TI - 1) / MRES_TI, sh);
     const int it = (int)(d.XCNT[blockIdx.x] - sys.pctl->xbase);
     const bool stop = it > 0 && !(resip > d.resimax && it < d.nswpp);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -122,7 +120,7 @@ __global__ void __launch_bounds__(ResLayout<M, NW>::MAXT, 1)
     constexpr int TG = Lay::TG, LW = Lay::LW;
     extern __shared__ float shm[];
     __shared__ int s_fault, s_stop;
-    __shared__ double s_sum[64];
+    __shared__ double s_sum[2 * MRES_MAX_GROUPS + 3];
     float *lines = shm;
     const int g = threadIdx.x / TG, t = threadIdx.x % TG;
     float *xch = shm + size_t(B + 1) * LW + size_t(g) * 2 * NW;
@@ -268,6 +266,27 @@ __global__ void __launch_bounds__(ResLayout<M, NW>::MAXT, 1)
 // every block publishes its two even lines once per pair and polls four lines at
 // the start of the next, so one exchange serves two sweeps.  Tags and slots as in
 // k_pois32_resident, counted per pair.
+//
+// LOOP: the whole forward iteration of a step in one launch.  The block also keeps the
+// FP64 pressure of its lines and of lines j0-2, j0-1 and j0+4 (what the residual of
+// its lines reads: rows j, j+-1 and the positional cross term's j-2) with their
+// double-float split, and each interval
+//   - forms the residual of its four lines in double-float, k_mres's terms in k_mres's
+//     order, publishes the four lines (FP32) and its sums, polls the five other lines of
+//     its window and every block's sums, and takes the decision (all blocks add the same
+//     values in the same order);
+//   - runs the sweeps;
+//   - adds the corrections to its pressure, publishes the three lines that neighbours
+//     need and adds theirs to its copies, so these stay the owners' bits.
+// Ghost columns and the ghost row 0 hold the stored values in the first interval and
+// BCP's of the current pressure afterwards.  The line words of an interval alternate
+// between two slots of their own; a slot is rewritten two intervals later, after a
+// decision that every reader has contributed to.
+//
+// Bound: the serial chain of the four half-sweeps of a pair, each a line solve (two scans
+// over two warps) between block barriers, and one exchange (0.41 us one way).  The solve
+// keeps its scans' constant products in registers (group_apply_c): half the shuffles, and
+// only the stages that reach (3 of 5 on 384-cell lines with 6 elements a thread).
 template <int M, int NW>
 struct ResLayout2 {
     static constexpr int B = 4;
@@ -276,36 +295,61 @@ struct ResLayout2 {
     static constexpr int NL = B + 7;   // window rows
     static constexpr int NG = B + 5;   // line groups (rows 1 .. B+5)
     static constexpr int NT = NG * TG;
-    static size_t bytes() { return sizeof(float) * (size_t(NL) * LW + size_t(NG) * 2 * NW); }
+    // Row of group gi.  A warp's quarter of the SM is its index mod 4: rows in group order
+    // put every odd row of a two-warp layout on two quarters and every even row on the
+    // other two; these orders spread the rows of each half-sweep over all four (512 x 384:
+    // 1.39 -> 1.26 us per sweep; one-warp rows unchanged).
+    __device__ static constexpr int row(int gi)
+    {
+        return int(((NW == 1 ? 0x864297531ull : 0x982756431ull) >> (4 * gi)) & 15u);
+    }
+    static constexpr size_t sweep_floats() { return (size_t(NL) * LW + size_t(NG) * 2 + 3) & ~size_t(3); }
+    // LOOP: pressure of 7 lines (FP64), its split and that of the ghost row 0, the own
+    // lines' residual
+    static constexpr int PL = 7;
+    static size_t bytes(int n, bool loop)
+    {
+        size_t b = sizeof(float) * sweep_floats();
+        if (loop) b += sizeof(double) * size_t(PL) * (n + 1) + sizeof(float2) * size_t(PL + 1) * (n + 1) + sizeof(float) * size_t(B) * LW;
+        return b;
+    }
 };
 
-template <int M, int NW, int HAS_COND>
+// Line words of the loop behind the sweeps' two slots: final corrections, residuals.
+__device__ __forceinline__ unsigned long long *loop_words(const Dev &d, int what, int slot, int L, int LW)
+{
+    return d.XW + size_t(2 + 2 * what + slot) * L * LW;
+}
+
+template <int M, int NW, int HAS_COND, int LOOP>
 __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
     k_pois32_resident2(const __grid_constant__ Dev d, const __grid_constant__ ResSys sys, int S, int apply,
                        int check_done, int max_polls, unsigned tag_skew, cudaGraphConditionalHandle cond)
 {
     using Lay = ResLayout2<M, NW>;
-    constexpr int TG = Lay::TG, LW = Lay::LW, B = Lay::B, NL = Lay::NL;
+    constexpr int TG = Lay::TG, LW = Lay::LW, B = Lay::B, NL = Lay::NL, PL = Lay::PL;
+    static_assert(B == MRES_GROUP, "a block's lines are one group of the residual sums");
     extern __shared__ float shm[];
     __shared__ int s_fault, s_stop;
-    __shared__ double s_sum[64];
+    __shared__ double s_sum[2 * MRES_MAX_GROUPS + 3], s_w[LOOP ? 2 * B * 16 : 1];
     float *rows = shm;
     const int gi = threadIdx.x / TG, t = threadIdx.x % TG;
-    const int w = gi + 1;   // the window row this group solves
-    float *xch = shm + size_t(NL) * LW + size_t(gi) * 2 * NW;
+    const int w = Lay::row(gi);   // the window row this group solves
+    float *fold = shm + size_t(NL) * LW + 2 * gi;
     const NamedSync<NW> bar{1 + gi};
     const int L = d.NJ - 1;
     const int j0 = blockIdx.x * B + 1;
     auto wrap = [L](int j) { return j < 1 ? j + L : (j > L ? j - L : j); };
     const int j = wrap(j0 - 3 + w);
     const int n = d.sP.n;
+    const bool own = w >= 3 && w <= B + 2;   // the block's own lines
     if (threadIdx.x == 0) {
         s_fault = 0;
         s_stop = check_done ? sys.pctl->done : 0;
     }
     __syncthreads();
     if (s_stop) return;
-    if (sys.decide && resident_decide<HAS_COND>(d, sys, S, s_sum, cond)) return;
+    if (!LOOP && sys.decide && resident_decide<HAS_COND>(d, sys, S, s_sum, cond)) return;
 
     const size_t base = size_t(j - 1) * LW;
     float fi[M], fa[M], fb[M], an[M], as[M], rf[M], v[M];
@@ -317,18 +361,43 @@ __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
         const int c = IDX(e + 1, j);
         an[k] = ok ? sys.ANf[c] : 0.0f;
         as[k] = ok ? sys.ASf[c] : 0.0f;
-        rf[k] = ok ? sys.RF[c] : 0.0f;
+        rf[k] = !LOOP && ok ? sys.RF[c] : 0.0f;
         v[k] = 0.0f;
     }
-    for (int q = threadIdx.x; q < NL * LW; q += Lay::NT) rows[q] = 0.0f;   // the correction starts from zero
+    const ScanConst<float> sc = scan_constants<float, M>(fa, fb, t, 0x1p-60f);
     const unsigned cnt0 = d.XCNT[blockIdx.x];
     const bool odd = (w & 1) != 0;
     // the outer even rows, each polled by the group next to it
     const int hrow = w == 1 ? 0 : (w == 3 ? 2 : (w == B + 3 ? B + 4 : (w == B + 5 ? B + 6 : -1)));
     const int hline = hrow >= 0 ? wrap(j0 - 3 + hrow) : 0;
     const bool publish = !odd && w >= 4 && w <= B + 2;
-    __syncthreads();
 
+    // poll the words of line q (chunk ownership) until they carry the tag
+    auto poll = [&](const unsigned long long *src, unsigned want, auto &&take) {
+        unsigned pending = 0;
+#pragma unroll
+        for (int k = 0; k < M; k++)
+            if (t * M + k < n) pending |= 1u << k;
+        for (int it = 0; pending && it < max_polls; it++) {
+            unsigned long long wd[M];
+#pragma unroll
+            for (int k = 0; k < M; k++) wd[k] = ((pending >> k) & 1u) ? ld_word(src + k * TG + t) : 0ull;
+#pragma unroll
+            for (int k = 0; k < M; k++) {
+                if (((pending >> k) & 1u) && unsigned(wd[k] >> 32) == want) {
+                    take(k, __uint_as_float(unsigned(wd[k])));
+                    pending &= ~(1u << k);
+                }
+            }
+        }
+        if (pending) s_fault = 1;
+    };
+    auto post = [&](unsigned long long *dst, unsigned tag32) {
+        const unsigned long long tag = (unsigned long long)tag32 << 32;
+#pragma unroll
+        for (int k = 0; k < M; k++)
+            if (t * M + k < n) st_word(dst + k * TG + t, tag | __float_as_uint(v[k]));
+    };
     auto solve = [&]() {
 #pragma unroll
         for (int k = 0; k < M; k++) {
@@ -336,57 +405,203 @@ __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
             const float xn = rows[(w + 1) * LW + k * TG + t];
             v[k] = t * M + k < n ? pois32_rhs(an[k], xn, as[k], xs, rf[k]) : 0.0f;
         }
-        group_apply_r<float, M, NW>(v, fi, fa, fb, t, xch, bar);
+        group_apply_c<float, M, NW>(v, fi, fa, fb, sc, fold, t, bar);
 #pragma unroll
         for (int k = 0; k < M; k++) rows[w * LW + k * TG + t] = v[k];
     };
+    // S sweeps from a zero correction; false (in every thread) when a wait ran out
+    auto sweeps = [&](unsigned cnt) {
+        for (int q = threadIdx.x; q < NL * LW; q += Lay::NT) rows[q] = 0.0f;
+        __syncthreads();
+        for (int sw = 1; sw <= S; sw += 2) {   // sweeps sw and sw+1
+            if (sw > 1 && hrow >= 0)
+                poll(d.XW + (size_t(((sw - 1) >> 1) & 1) * L + (hline - 1)) * LW, cnt + unsigned(sw - 1) + tag_skew,
+                     [&](int k, float x) { rows[hrow * LW + k * TG + t] = x; });
+            __syncthreads();
+            if (s_fault) return false;   // uniform: read by every thread after the barrier
+            if (odd) solve();                                  // sweep sw, odd rows 1 .. B+5
+            __syncthreads();
+            if (!odd) solve();                                 // sweep sw, even rows 2 .. B+4
+            __syncthreads();
+            if (odd && w >= 3 && w <= B + 3) solve();          // sweep sw+1, odd rows 3 .. B+3
+            __syncthreads();
+            if (publish) {                                     // sweep sw+1, the block's even lines
+                solve();
+                post(d.XW + (size_t(((sw + 1) >> 1) & 1) * L + (j - 1)) * LW, cnt + unsigned(sw + 1));
+            }
+            __syncthreads();
+        }
+        return true;
+    };
 
-    int sw = 1;
-    for (; sw <= S; sw += 2) {   // sweeps sw and sw+1
-        if (sw > 1 && hrow >= 0) {
-            const unsigned want = cnt0 + unsigned(sw - 1) + tag_skew;
-            const unsigned long long *src = d.XW + (size_t(((sw - 1) >> 1) & 1) * L + (hline - 1)) * LW;
-            unsigned pending = 0;
+    if constexpr (LOOP) {
+        const int PW = n + 1, nt = (n + WARP - 1) / WARP, nb = gridDim.x;
+        double *P = reinterpret_cast<double *>(shm + Lay::sweep_floats());   // [PL][PW]: lines j0-2 .. j0+4, columns 0 .. n
+        float2 *ps = reinterpret_cast<float2 *>(P + size_t(PL) * PW);        // [PL + 1][PW]: split, and ghost row 0
+        float *rfs = reinterpret_cast<float *>(ps + size_t(PL + 1) * PW);    // [B][LW]: own residual, words as in rows
+        double *s_ab = s_sum + 2 * MRES_MAX_GROUPS;
+        const int pl = w - 1;   // P line of the group (rows 1 .. 7)
+        unsigned long long *psum = d.XW + size_t(6) * L * LW;
+        auto split = [](double x) {
+            const dd q = dd_split(x);
+            return make_float2(q.hi, q.lo);
+        };
+        if (pl < PL) {
 #pragma unroll
-            for (int k = 0; k < M; k++)
-                if (t * M + k < n) pending |= 1u << k;
-            for (int it = 0; pending && it < max_polls; it++) {
-                unsigned long long wd[M];
+            for (int k = 0; k < M; k++) {
+                const int e = t * M + k;
+                if (e < n) {
+                    const double x = d.P[IDX(e + 1, j)];
+                    P[pl * PW + e + 1] = x;
+                    ps[pl * PW + e + 1] = split(x);
+                }
+            }
+            if (t == 0) ps[pl * PW] = split(d.P[IDX(0, j)]);
+        } else if (pl == PL && j0 == 1) {
+            for (int i = t; i < PW; i += TG) ps[PL * PW + i] = split(d.P[IDX(i, 0)]);
+        }
+        __syncthreads();
+        const int wid = threadIdx.x / WARP, lane = threadIdx.x & (WARP - 1);
+        unsigned cnt = cnt0;
+        int it = 0;
+        double resip = 0.0;
+        bool bad = false;
+        for (int round = 0;; round++) {
+            // residual of the own lines: one warp per line and 32 cells
+            for (int task = wid; task < B * nt; task += Lay::NT / WARP) {
+                const int q = task & (B - 1), col = task / B, i = col * WARP + lane + 1, jq = j0 + q;
+                const bool inside = i <= n, has_cross = inside && i > 1 && jq > 1;
+                const int c = inside ? IDX(i, jq) : 0, cc = has_cross ? IDX(i - 1, jq - 1) : 0;
+                float2 cf[9];
 #pragma unroll
-                for (int k = 0; k < M; k++) wd[k] = ((pending >> k) & 1u) ? ld_word(src + k * TG + t) : 0ull;
+                for (int k = 0; k < 9; k++) {
+                    const bool ok = k < 5 ? inside : has_cross;
+                    cf[k] = ok ? d.PCD[size_t(k) * d.n + (k < 5 ? c : cc)] : make_float2(0.0f, 0.0f);
+                }
+                float raf = 0.0f, paf = 0.0f;
+                if (inside) {
+                    const double divdt = d.DIVDT[c];
+                    const float2 *r0 = ps + (q + 2) * PW, *rm = r0 - 2 * PW;
+                    if (q == 1 && j0 == 1) rm = ps + PL * PW;   // line 2: the ghost row
+                    auto at = [](float2 x) { return dd(x.x, x.y); };
+                    auto co = [&](int k) { return at(cf[k]); };
+                    dd cross = dd(0.0f, 0.0f);
+                    if (has_cross)
+                        cross = ((co(5) * at(r0[i]) + co(6) * at(rm[i])) + co(7) * at(r0[i - 2])) + co(8) * at(rm[i - 2]);
+                    const dd su = dd_split(divdt) - cross;
+                    const dd app = co(4) * at(r0[i]);
+                    const dd pe = i < n ? at(r0[i + 1]) : dd(0.0f, 0.0f);   // AE(NI-1) = 0
+                    const dd r = ((((co(0) * pe + co(1) * at(r0[i - 1])) + co(2) * at(r0[PW + i])) + co(3) * at((r0 - PW)[i])) + su) - app;
+                    raf = fabsf(r.hi);
+                    paf = fabsf(app.hi);
+                    const int e = i - 1;
+                    rfs[q * LW + (e % M) * TG + e / M] = r.hi;
+                }
+                for (int o = 16; o > 0; o >>= 1) {
+                    raf += __shfl_down_sync(0xffffffffu, raf, o);
+                    paf += __shfl_down_sync(0xffffffffu, paf, o);
+                }
+                if (lane == 0) {
+                    s_w[q * 16 + col] = (double)raf;
+                    s_w[(B + q) * 16 + col] = (double)paf;
+                }
+            }
+            __syncthreads();
+            const unsigned rtag = cnt + 1u;
+            unsigned long long *rw = loop_words(d, 1, round & 1, L, LW);
+            unsigned long long *pw = psum + size_t(round & 1) * 4 * nb;
+            if (own) {
+#pragma unroll
+                for (int k = 0; k < M; k++) v[k] = t * M + k < n ? rfs[(w - 3) * LW + k * TG + t] : 0.0f;
+                post(rw + size_t(j - 1) * LW, rtag);
+#pragma unroll
+                for (int k = 0; k < M; k++) rf[k] = v[k];
+            }
+            if (wid == Lay::NT / WARP - 1) {   // the last group's last warp: the block's sums
+                const int half = lane >> 4, col = lane & 15;
+                const double x = mres_columns(col < nt ? mres_lines(s_w + half * B * 16 + col, 16) : 0.0);
+                if (col == 0) {
+                    const unsigned long long b = (unsigned long long)__double_as_longlong(x), tag = (unsigned long long)rtag << 32;
+                    st_word(pw + 4 * blockIdx.x + 2 * half, tag | (b & 0xffffffffull));
+                    st_word(pw + 4 * blockIdx.x + 2 * half + 1, tag | (b >> 32));
+                }
+            }
+            if (!own)
+                poll(rw + size_t(j - 1) * LW, rtag, [&](int k, float x) { rf[k] = x; });
+            else
+                for (int q = (w - 3) * TG + t; q < 2 * nb; q += B * TG) {
+                    bool got = false;
+                    for (int i = 0; !got && i < max_polls; i++) {
+                        const unsigned long long a = ld_word(pw + 2 * q), b = ld_word(pw + 2 * q + 1);
+                        got = unsigned(a >> 32) == rtag && unsigned(b >> 32) == rtag;
+                        if (got) s_sum[q] = __hiloint2double((int)(unsigned)b, (int)(unsigned)a);
+                    }
+                    if (!got) s_fault = 1;
+                }
+            __syncthreads();
+            mres_ratio(s_sum, nb, s_ab, s_ab + 2);
+            if (s_fault) { bad = true; break; }
+            resip = s_ab[2];
+            if (it > 0 && !(resip > d.resimax && it < d.nswpp)) break;
+            if (!sweeps(cnt)) { bad = true; break; }
+            cnt += unsigned(S);
+            it += S;
+            // corrections: own lines, and the neighbours' three
+            unsigned long long *fw = loop_words(d, 0, round & 1, L, LW);
+            if (own && w != 4) post(fw + size_t(j - 1) * LW, cnt);
+            if (w <= 2 || w == B + 3)
+                poll(fw + size_t(j - 1) * LW, cnt, [&](int k, float x) { v[k] = x; });
+            if (pl < PL) {
 #pragma unroll
                 for (int k = 0; k < M; k++) {
-                    if (((pending >> k) & 1u) && unsigned(wd[k] >> 32) == want) {
-                        rows[hrow * LW + k * TG + t] = __uint_as_float(unsigned(wd[k]));
-                        pending &= ~(1u << k);
+                    const int e = t * M + k;
+                    if (e < n) {
+                        const double x = P[pl * PW + e + 1] + f2d_int(v[k]);
+                        P[pl * PW + e + 1] = x;
+                        const float2 q = split(x);
+                        ps[pl * PW + e + 1] = q;
+                        if (e == 0) ps[pl * PW] = q;
+                        if (j0 == 1 && w == 2) {   // line NJ-1: the ghost row 0
+                            ps[PL * PW + e + 1] = q;
+                            if (e == 0) ps[PL * PW] = q;
+                        }
                     }
                 }
             }
-            if (pending) s_fault = 1;
+            __syncthreads();
+            if (s_fault) { bad = true; break; }
         }
-        __syncthreads();
-        if (s_fault) break;   // uniform: read by every thread after the barrier
-        if (odd) solve();                                  // sweep sw, odd rows 1 .. B+5
-        __syncthreads();
-        if (!odd) solve();                                 // sweep sw, even rows 2 .. B+4
-        __syncthreads();
-        if (odd && w >= 3 && w <= B + 3) solve();          // sweep sw+1, odd rows 3 .. B+3
-        __syncthreads();
-        if (publish) {                                     // sweep sw+1, the block's even lines
-            solve();
-            unsigned long long *dst = d.XW + (size_t(((sw + 1) >> 1) & 1) * L + (j - 1)) * LW;
-            const unsigned long long tag = (unsigned long long)(cnt0 + unsigned(sw + 1)) << 32;
+        if (bad) {   // a wait ran out: end the loop, leave P alone
+            if (threadIdx.x == 0) {
+                d.pctl->fault = 1;
+                d.pctl->done = 1;
+            }
+            return;
+        }
+        if (own) {
 #pragma unroll
-            for (int k = 0; k < M; k++)
-                if (t * M + k < n) st_word(dst + k * TG + t, tag | __float_as_uint(v[k]));
+            for (int k = 0; k < M; k++) {
+                const int e = t * M + k;
+                if (e < n) d.P[IDX(e + 1, j)] = P[pl * PW + e + 1];
+            }
         }
-        __syncthreads();
+        if (threadIdx.x == 0) {
+            d.XCNT[blockIdx.x] = cnt + 2u;   // past the last residual's tag
+            if (blockIdx.x == 0) {
+                d.pctl->niter = it;
+                d.pctl->resip = resip;
+                d.pctl->capped = resip > d.resimax ? 1 : 0;
+                d.pctl->done = 1;
+            }
+        }
+        return;
     }
 
+    const bool ok = sweeps(cnt0);
     // the next residual launch (programmatic) may start its coefficient prologue;
     // it reads P only after its dependency wait, i.e. after this grid has finished
     griddep_launch();
-    if (sw <= S) {   // a wait ran out: end the loop, leave P alone
+    if (!ok) {   // a wait ran out: end the loop, leave P alone
         if (threadIdx.x == 0) {
             sys.pctl->fault = 1;
             sys.pctl->done = 1;
@@ -394,7 +609,7 @@ __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
         }
         return;
     }
-    if (w >= 3 && w <= B + 2) {   // the block's own lines
+    if (own) {
 #pragma unroll
         for (int k = 0; k < M; k++) {
             const int e = t * M + k;
@@ -415,7 +630,7 @@ __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
     if (threadIdx.x == 0) d.XCNT[blockIdx.x] = cnt0 + unsigned(S);
 }
 
-template <int M, int NW, int HAS_COND>
+template <int M, int NW, int HAS_COND, int LOOP>
 cudaError_t launch_resident2(const fvm_ctx *c, const ResSys &sys, cudaStream_t st, int S, int apply, int check_done,
                              int max_polls, unsigned skew, cudaGraphConditionalHandle cond)
 {
@@ -423,14 +638,14 @@ cudaError_t launch_resident2(const fvm_ctx *c, const ResSys &sys, cudaStream_t s
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(c->res_blocks);
     cfg.blockDim = dim3(Lay::NT);
-    cfg.dynamicSmemBytes = Lay::bytes();
+    cfg.dynamicSmemBytes = Lay::bytes(c->d.sP.n, LOOP != 0);
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = c->res_coop ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k_pois32_resident2<M, NW, HAS_COND>, c->d, sys, S, apply, check_done, max_polls,
+    return cudaLaunchKernelEx(&cfg, k_pois32_resident2<M, NW, HAS_COND, LOOP>, c->d, sys, S, apply, check_done, max_polls,
                               skew, cond);
 }
 
@@ -513,21 +728,30 @@ int resident_setup(fvm_ctx *c)
     // two sweeps per exchange where the window fits: 4 lines per block, line groups
     // of one or two warps, at least three blocks around the ring, all co-resident
     c->res_depth = 1;
+    c->res_loop = false;
     if (c->res_lines == 4 && c->p.resident_depth != 1 && c->res_blocks >= 3) {
         cudaError_t e = cudaSuccess;
         dispatch_line(s, [&](auto m, auto nw) {
             constexpr int M_ = decltype(m)::value, NW_ = decltype(nw)::value;
             if constexpr (NW_ <= 2) {
                 using Lay = ResLayout2<M_, NW_>;
-                auto k0 = k_pois32_resident2<M_, NW_, 0>;
-                auto k1 = k_pois32_resident2<M_, NW_, 1>;
-                int per_sm = 0;
-                e = cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::bytes());
+                auto k0 = k_pois32_resident2<M_, NW_, 0, 0>;
+                auto k1 = k_pois32_resident2<M_, NW_, 1, 0>;
+                auto kl = k_pois32_resident2<M_, NW_, 0, 1>;
+                const int n = WARP * NW_ * M_, most = (int)Lay::bytes(n, false), most_l = (int)Lay::bytes(n, true);
+                int per_sm = 0, per_sm_l = 0;
+                e = cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+                if (e == cudaSuccess) e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+                if (e == cudaSuccess) e = cudaFuncSetAttribute(kl, cudaFuncAttributeMaxDynamicSharedMemorySize, most_l);
                 if (e == cudaSuccess)
-                    e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lay::bytes());
+                    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k1, Lay::NT, Lay::bytes(s.n, false));
                 if (e == cudaSuccess)
-                    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k1, Lay::NT, Lay::bytes());
+                    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_l, kl, Lay::NT, Lay::bytes(s.n, true));
                 if (e == cudaSuccess && c->res_blocks <= per_sm * sms) c->res_depth = 2;
+                // the whole iteration in one launch: the reference's positional cross term,
+                // an even interval
+                c->res_loop = c->res_depth == 2 && c->d.dd_pos && c->d.refine_sweeps % 2 == 0 &&
+                              c->res_blocks <= per_sm_l * sms;
             }
         });
         if (e != cudaSuccess) cudaGetLastError();
@@ -558,8 +782,8 @@ int launch_sys(fvm_ctx *c, const ResSys &sys, cudaStream_t st, int sweeps, int a
         constexpr int M_ = decltype(m)::value, NW_ = decltype(nw)::value;
         if constexpr (NW_ <= 2) {
             if (pairs) {
-                if (has_cond) e = launch_resident2<M_, NW_, 1>(c, sys, st, sweeps, apply, check_done, polls, tag_skew, cond);
-                else e = launch_resident2<M_, NW_, 0>(c, sys, st, sweeps, apply, check_done, polls, tag_skew, cond);
+                if (has_cond) e = launch_resident2<M_, NW_, 1, 0>(c, sys, st, sweeps, apply, check_done, polls, tag_skew, cond);
+                else e = launch_resident2<M_, NW_, 0, 0>(c, sys, st, sweeps, apply, check_done, polls, tag_skew, cond);
                 return;
             }
         }
@@ -590,6 +814,24 @@ int resident_sweeps(const Tgt &t, int sweeps, int apply, int max_polls, unsigned
     return launch_sys(t.c, sys, t.st, sweeps, apply, max_polls, tag_skew, cond, has_cond, check_done);
 }
 
+// The whole forward iteration of a step whose source is in place.
+int resident_loop(fvm_ctx *c)
+{
+    cudaError_t e = cudaErrorInvalidValue;
+    const ResSys sys = forward_sys(c);
+    dispatch_line(c->d.sP, [&](auto m, auto nw) {
+        constexpr int M_ = decltype(m)::value, NW_ = decltype(nw)::value;
+        if constexpr (NW_ <= 2)
+            e = launch_resident2<M_, NW_, 0, 1>(c, sys, c->stream, c->d.refine_sweeps, 0, 0, kResidentPolls, 0u, 0);
+    });
+    if (e != cudaSuccess) {
+        c->err = std::string("resident Poisson loop launch: ") + cudaGetErrorString(e);
+        return FVM_ERR_CUDA;
+    }
+    KCOUNT(c);
+    return FVM_OK;
+}
+
 // The same sweeps on another system of the context's line tile (the adjoint's
 // transposed Poisson equation); no graph condition, default wait bound.
 int resident_sweeps_on(fvm_ctx *c, const ResSys &sys, int sweeps, int apply, int check_done)
@@ -598,12 +840,13 @@ int resident_sweeps_on(fvm_ctx *c, const ResSys &sys, int sweeps, int apply, int
 }
 
 // Exchange words of a context: two slots of every line in the largest tile (32 x 4
-// warps x 4 elements), one word per FP32 value or two per FP64 value, and the FP64
-// ring's two slots of block sums.
+// warps x 4 elements) -- FP32, one word per value: sweeps, final corrections and
+// residuals of the resident loop; FP64: two words per value of the ring -- and two slots
+// of block sums.
 size_t exchange_words(const fvm_ctx *c)
 {
     const size_t line = 2 * size_t(c->NJ - 1) * WARP * 4 * 4;
-    return c->p.precision == FVM_MIXED ? line : 2 * line + 2 * 4 * size_t(RING_MAX_BLOCKS);
+    return (c->p.precision == FVM_MIXED ? 3 : 2) * line + 2 * 4 * size_t(RING_MAX_BLOCKS);
 }
 
 // After a wait ran out: the blocks' sweep counts may disagree, so clear the

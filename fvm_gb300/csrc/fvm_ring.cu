@@ -119,15 +119,18 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
     __shared__ double s_line[2 * 8], s_tot[2 * RING_MAX_BLOCKS], s_res;
     const int L = d.NJ - 1, n = d.sP.n;
     const int pairs = L / 2, p0 = blockIdx.x * ppb, nl = 2 * min(ppb, pairs - p0), j0 = 2 * p0 + 1;
-    const int g = threadIdx.x / TG, t = threadIdx.x % TG, lane = t & (WARP - 1), wl = t / WARP;
+    // group gi takes line j0 + g, the block's odd lines first: a warp's quarter of the SM is
+    // its index mod 4, and the lines solved at a time then cover all four
+    const int gi = threadIdx.x / TG, g = gi < ppb ? 2 * gi : 2 * (gi - ppb) + 1;
+    const int t = threadIdx.x % TG, lane = t & (WARP - 1), wl = t / WARP;
     const bool act = g < nl, odd = (g & 1) == 0;   // j0 is odd
     const int j = j0 + g;
-    const NamedSync<NW> bar{1 + g};
+    const NamedSync<NW> bar{1 + gi};
     const int nlm = 2 * ppb;
     double *own = shm;                                  // [3][nlm][LW]
     double *hm1 = own + size_t(3) * nlm * LW;           // [3][LW]
     double *hm2 = hm1 + size_t(3) * LW;                 // [3][LW]
-    double *cst = hm2 + size_t(3) * LW + size_t(g) * (size_t(CST) * TG + 4 * NW);
+    double *cst = hm2 + size_t(3) * LW + size_t(gi) * (size_t(CST) * TG + 4 * NW);
     double *fold = cst + size_t(CST) * TG;              // [Gtot | Htot | forward | backward][NW]
     auto line = [&](int ver, int q) { return own + (size_t(ver) * nlm + q) * LW; };
     auto wrap = [L](int q) { return q < 1 ? q + L : (q > L ? q - L : q); };

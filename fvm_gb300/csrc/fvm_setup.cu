@@ -189,7 +189,9 @@ int setup_allocate(fvm_ctx *c)
     d.nblk_res = c->nblk_res;
     c->nblk_mres = ((c->NI - 1 + MRES_TI - 1) / MRES_TI) * ((c->NJ - 1 + MRES_TJ - 1) / MRES_TJ);
     d.nblk_mres = c->nblk_mres;
-    const int nblk_partial = std::max({c->nblk_res, c->nblk_mres, RING_MAX_BLOCKS});
+    // block sums of the residual kernels; k_mres leaves one per four lines and 32 cells
+    const int nblk_partial = std::max({c->nblk_res, ((c->NJ + 2) / 4) * ((c->NI - 1 + MRES_TI - 1) / MRES_TI),
+                                       (int)RING_MAX_BLOCKS});
     Bump probe{nullptr};
     carve(probe, c, nblk_partial);
     c->slab_bytes = probe.off + 256;

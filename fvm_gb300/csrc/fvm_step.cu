@@ -975,7 +975,7 @@ int poisson_graph_build(fvm_ctx *c)
 // bodies are launched, their kernels returning early once converged.
 long long poisson_loop_kernels(fvm_ctx *c, int niter)
 {
-    if (c->ring_blocks) return 0;   // one launch, counted when it was issued
+    if (c->ring_blocks || c->res_loop) return 0;   // one launch, counted when it was issued
     const int per = c->pgraph_batch;
     const bool mixed = c->p.precision == FVM_MIXED;
     long long bodies = (niter + (mixed ? 1 : 0) + per - 1) / per;
@@ -990,6 +990,7 @@ int poisson_loop(fvm_ctx *c)
 {
     Dev &d = c->d;
     if (c->ring_blocks) return ring_launch(c, 0, 0);
+    if (c->res_loop) return resident_loop(c);
     RC(poisson_graph(c));
     if (!c->p.poisson_host_loop) {
         FVM_CUDA(c, cudaGraphLaunch(c->pgraph, c->stream));

@@ -75,6 +75,9 @@ typedef struct fvm_params {
        one launch whose blocks keep their lines on chip and exchange only boundary
        lines (1, the default: lines per block chosen automatically; k >= 2, even:
        k lines per block; 0: one launch per zebra colour).  Same results bit for bit.
+       With two sweeps per exchange (resident_depth), dd_positional = 1 and an even
+       refine_sweeps the whole Poisson iteration of a step, residuals included, is one
+       launch, whatever poisson_host_loop says.
        FP64, single context, dd_positional = 1: the whole Poisson iteration of a step
        runs in one launch, whatever poisson_host_loop says (0: one launch per zebra
        colour).  Same results bit for bit with the same line tile. */
