@@ -57,7 +57,7 @@ struct Adj {
 namespace {
 
 // ---------------------------------------------------------------------------------
-// Geometry of the drag formula (calccoef.f90:50-98 as in k_calc_rows): wall-normal
+// Geometry of the drag formula (calccoef.f90:50-98 as in k_wall_geom): wall-normal
 // distance DN1 and normal angle TH2 of the first cell of column j.
 // ---------------------------------------------------------------------------------
 __device__ void wall_normal(const Dev &d, int j, double &DN1, double &TH2)

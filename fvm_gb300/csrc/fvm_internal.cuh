@@ -123,7 +123,7 @@ struct Dev {
     // reductions
     PCtl *pctl;
     double *partial;               // per-block partial sums (2 per block)
-    double *coefrow;               // per-j CALCCOEF contributions (6 per j)
+    double *WALLG;                 // geometry of the wall forces (k_wall_geom, 5 per j)
     unsigned long long *cflbits;
     double *scal;                  // small scalars: [0]=sum_area
     // line systems and coefficients
@@ -252,6 +252,7 @@ int setup_factors(fvm_ctx *c);
 void split_pcoef(fvm_ctx *c);   // double-float planes of the pressure coefficients (d.PCD)
 int setup_controls(fvm_ctx *c, double omega, const double *blow);
 int setup_grid(fvm_ctx *c);
+int setup_wall_geom(fvm_ctx *c);
 int setup_init(fvm_ctx *c, const double *du, const double *dv);
 int run_begin_step(fvm_ctx *c);
 int run_contra_vel(fvm_ctx *c);

@@ -133,7 +133,7 @@ void carve(Bump &b, fvm_ctx *c, int nblk)
     d.XCNT = b.take<unsigned int>(size_t(c->NJ));
     d.pctl = b.take<PCtl>(1);
     d.partial = b.take<double>(2 * size_t(nblk));
-    d.coefrow = b.take<double>(8 * size_t(nj1));
+    d.WALLG = b.take<double>(5 * size_t(nj1));
     d.cflbits = b.take<unsigned long long>(1);
     d.scal = b.take<double>(16);
     carve_coef(b, d.cP, n, nj1);
@@ -354,6 +354,42 @@ __global__ void k_area(Dev d)
     d.scal[0] = sum;
 }
 
+// Geometry of the wall forces (calccoef.f90:58-98) per wall cell j: distance DN1 and the
+// sine and cosine of the normal angle TH2 and of THETA, five values at WALLG + 5 j.
+__global__ void k_wall_geom(Dev d)
+{
+    int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
+    if (j > d.NJ - 1) return;
+    const int c = IDX(1, j);
+    const double X = d.X[c], Y = d.Y[c];
+    const double xa = d.XG[IDX(1, j)], ya = d.YG[IDX(1, j)], xb = d.XG[IDX(1, j + 1)], yb = d.YG[IDX(1, j + 1)];
+    double L1 = sqrt((X - xa) * (X - xa) + (Y - ya) * (Y - ya));
+    double L2 = sqrt((X - xb) * (X - xb) + (Y - yb) * (Y - yb));
+    double L3 = sqrt((xb - xa) * (xb - xa) + (yb - ya) * (yb - ya));
+    double TH1 = acos((((L1 * L1) + (L2 * L2)) - (L3 * L3)) / ((2.0 * L1) * L2));
+    double DN1 = ((L1 * L2) / L3) * sin(TH1);
+    double LA = (yb - ya) / (xb - xa);
+    double LB = ya - LA * xa;
+    double LA_ = -1.0 / LA;
+    double LB_ = Y - LA_ * X;
+    double X1 = (LB_ - LB) / (LA - LA_);
+    double Y1 = (LA * (LB_ - LB)) / (LA - LA_) + LB;
+    double DN2 = sqrt((Y - Y1) * (Y - Y1) + (X - X1) * (X - X1));
+    double TH2 = atan((Y - Y1) / (X - X1));
+    double sg = asin((Y - Y1) / DN2);
+    if (TH2 >= 0.0 && sg > 0.0) TH2 = TH2;
+    else if (TH2 < 0.0 && sg > 0.0) TH2 = d.pi + TH2;
+    else if (TH2 >= 0.0 && sg <= 0.0) TH2 = d.pi + TH2;
+    else if (TH2 < 0.0 && sg < 0.0) TH2 = 2.0 * d.pi + TH2;
+    const double th = d.THETA[c];
+    double *o = d.WALLG + 5 * j;
+    o[0] = DN1;
+    o[1] = sin(TH2);
+    o[2] = cos(TH2);
+    o[3] = sin(th);
+    o[4] = cos(th);
+}
+
 __global__ void k_wall_values(Dev d)
 {
     int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -548,6 +584,14 @@ int setup_factors(fvm_ctx *c)
     return ring_setup(c);
 }
 
+// d.WALLG from the current X, Y, XG, YG and THETA.
+int setup_wall_geom(fvm_ctx *c)
+{
+    k_wall_geom<<<(c->NJ - 1 + 63) / 64, 64, 0, c->stream>>>(c->d);
+    FVM_LAUNCH_CHECK(c);
+    return FVM_OK;
+}
+
 int setup_grid(fvm_ctx *c)
 {
     Dev &d = c->d;
@@ -564,7 +608,9 @@ int setup_grid(fvm_ctx *c)
     k_area<<<1, 1, 0, st>>>(d);
     k_wall_values<<<(c->NJ + 1 + 127) / 128, 128, 0, st>>>(d);
     FVM_LAUNCH_CHECK(c);
-    int rc = build_line_sets(c);
+    int rc = setup_wall_geom(c);
+    if (rc) return rc;
+    rc = build_line_sets(c);
     if (rc) return rc;
     // Jacobian check (metric.f90:120 prints cells with |J| < 1e-15): reject the grid
     std::vector<double> dj(c->n);

@@ -499,47 +499,10 @@ __global__ void __launch_bounds__(1024) k_pres64(const __grid_constant__ S src, 
 }
 
 // ---------------------------------------------------------------------------------
-// CALCCOEF (calccoef.f90:9-120): per-j wall contributions, CFL maximum, then a
-// single-thread fixed-order sum (the reference's J order).
+// CALCCOEF (calccoef.f90:9-120): CFL maximum (k_cfl), then the wall contributions per j
+// and their fixed-order sums in one block.  The wall geometry (k_wall_geom) is formed with
+// the grid: its square roots and inverse trigonometric functions took 16 us a step.
 // ---------------------------------------------------------------------------------
-template <class S>
-__global__ void k_calc_rows(const __grid_constant__ S src)
-{
-    const Dev &d = dev_of(src);
-    int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    if (j > d.NJ - 1) return;
-    const int c = IDX(1, j);
-    const double X = d.X[c], Y = d.Y[c];
-    const double xa = d.XG[IDX(1, j)], ya = d.YG[IDX(1, j)], xb = d.XG[IDX(1, j + 1)], yb = d.YG[IDX(1, j + 1)];
-    double L1 = sqrt((X - xa) * (X - xa) + (Y - ya) * (Y - ya));
-    double L2 = sqrt((X - xb) * (X - xb) + (Y - yb) * (Y - yb));
-    double L3 = sqrt((xb - xa) * (xb - xa) + (yb - ya) * (yb - ya));
-    double TH1 = acos((((L1 * L1) + (L2 * L2)) - (L3 * L3)) / ((2.0 * L1) * L2));
-    double DN1 = ((L1 * L2) / L3) * sin(TH1);
-    double LA = (yb - ya) / (xb - xa);
-    double LB = ya - LA * xa;
-    double LA_ = -1.0 / LA;
-    double LB_ = Y - LA_ * X;
-    double X1 = (LB_ - LB) / (LA - LA_);
-    double Y1 = (LA * (LB_ - LB)) / (LA - LA_) + LB;
-    double DN2 = sqrt((Y - Y1) * (Y - Y1) + (X - X1) * (X - X1));
-    double TH2 = atan((Y - Y1) / (X - X1));
-    double sg = asin((Y - Y1) / DN2);
-    if (TH2 >= 0.0 && sg > 0.0) TH2 = TH2;
-    else if (TH2 < 0.0 && sg > 0.0) TH2 = d.pi + TH2;
-    else if (TH2 >= 0.0 && sg <= 0.0) TH2 = d.pi + TH2;
-    else if (TH2 < 0.0 && sg < 0.0) TH2 = 2.0 * d.pi + TH2;
-    double dudn = ((d.U[c] * sin(TH2) - d.V[c] * cos(TH2)) - d.vel_rot) / DN1;
-    double dtdn = (d.T[c] - d.t_wall) / DN1;
-    double th = d.THETA[c], ar = d.AREA[c], p = d.P[c];
-    double *row = d.coefrow + 8 * j;
-    row[0] = ((2.0 * p) * ar) * cos(th);
-    row[1] = ((2.0 * p) * ar) * sin(th);
-    row[2] = (((2.0 / d.re) * dudn) * ar) * sin(th);
-    row[3] = (((2.0 / d.re) * dudn) * ar) * cos(th);
-    row[4] = dtdn * ar;
-}
-
 template <class S>
 __global__ void k_cfl(const __grid_constant__ S src)
 {
@@ -557,22 +520,37 @@ __global__ void k_cfl(const __grid_constant__ S src)
 }
 
 template <class S>
-__global__ void k_calc_final(const __grid_constant__ S src, double rtime, fvm_coeffs *out)
+__global__ void __launch_bounds__(512) k_calc_final(const __grid_constant__ S src, double rtime, fvm_coeffs *out)
 {
+    __shared__ double rows[5][512];
     const Dev &d = dev_of(src);
     if (d.bctl) {   // batch: the case's device time, one record per step and case
         rtime = *d.btime;
         out = d.bhist + (size_t)d.bctl->step * d.bctl->ncases + d.case_id;
     }
+    for (int j = 1 + (int)threadIdx.x; j <= d.NJ - 1; j += blockDim.x) {
+        const int c = IDX(1, j);
+        const double *g = d.WALLG + 5 * j;
+        const double dn = g[0], st = g[3], ct = g[4];
+        const double dudn = ((d.U[c] * g[1] - d.V[c] * g[2]) - d.vel_rot) / dn;
+        const double dtdn = (d.T[c] - d.t_wall) / dn;
+        const double ar = d.AREA[c], p = d.P[c];
+        rows[0][j - 1] = ((2.0 * p) * ar) * ct;
+        rows[1][j - 1] = ((2.0 * p) * ar) * st;
+        rows[2][j - 1] = (((2.0 / d.re) * dudn) * ar) * st;
+        rows[3][j - 1] = (((2.0 / d.re) * dudn) * ar) * ct;
+        rows[4][j - 1] = dtdn * ar;
+    }
+    __syncthreads();
+    if (threadIdx.x >= WARP) return;
     // one warp: each lane sums every 32nd row, then a fixed shuffle tree
     double pd = 0.0, pl = 0.0, td = 0.0, tl = 0.0, nu = 0.0;
-    for (int j = 1 + (int)threadIdx.x; j <= d.NJ - 1; j += 32) {
-        const double *row = d.coefrow + 8 * j;
-        pd = pd - row[0];
-        pl = pl - row[1];
-        td = td + row[2];
-        tl = tl - row[3];
-        nu = nu + row[4];
+    for (int j = (int)threadIdx.x; j < d.NJ - 1; j += 32) {
+        pd = pd - rows[0][j];
+        pl = pl - rows[1][j];
+        td = td + rows[2][j];
+        tl = tl - rows[3][j];
+        nu = nu + rows[4][j];
     }
     for (int o = 16; o > 0; o >>= 1) {
         pd += __shfl_down_sync(0xffffffffu, pd, o);
@@ -636,6 +614,8 @@ Tgt tgt_of(fvm_ctx *c)
 
 namespace {
 
+// threads of k_calc_final: one wall cell each, whole warps (NJ-1 <= 512)
+inline int calc_threads(const Tgt &t) { return (t.NJ - 1 + WARP - 1) / WARP * WARP; }
 inline dim3 interior_grid(const Tgt &t) { return dim3((t.NI - 1 + 127) / 128, t.NJ - 1, t.nz); }
 
 #define RC(x)                 \
@@ -784,9 +764,8 @@ int step_after_poisson(const Tgt &t, double rtime, fvm_coeffs *dout)
     LAUNCH_S(t, k_bcp_ghosts, dim3((t.NI + t.NJ + 127) / 128, 1, t.nz), 128);
     LAUNCH_S(t, k_grad, interior_grid(t), 128, +1.0, 1);
     if (t.thermal) RC(predictor_sweeps(t, FVM_FIELD_T));
-    LAUNCH_S(t, k_calc_rows, dim3((t.NJ + 127) / 128, 1, t.nz), 128);
     LAUNCH_S(t, k_cfl, interior_grid(t), 128);
-    LAUNCH_S(t, k_calc_final, dim3(1, 1, t.nz), 32, rtime, dout);
+    LAUNCH_S(t, k_calc_final, dim3(1, 1, t.nz), calc_threads(t), rtime, dout);
     return FVM_OK;
 }
 
@@ -1142,9 +1121,8 @@ int run_calccoef(fvm_ctx *c, fvm_coeffs *out)
 {
     Tgt t = tgt_of(c);
     fvm_coeffs *dout = coef_slot(c);
-    LAUNCH_S(t, k_calc_rows, dim3((t.NJ + 127) / 128, 1, 1), 128);
     LAUNCH_S(t, k_cfl, interior_grid(t), 128);
-    LAUNCH_S(t, k_calc_final, dim3(1, 1, 1), 32, c->rtime, dout);
+    LAUNCH_S(t, k_calc_final, dim3(1, 1, 1), calc_threads(t), c->rtime, dout);
     const double cl_prev = c->last.cl;   // CL_NM1 (calccoef.f90:109)
     fvm_coeffs co;
     RC(calccoef_copy(c, dout, &co));
