@@ -285,12 +285,12 @@ int run_adjoint(fvm_ctx *c, int window, int ckpt, double *J, double *dJ_domega, 
 int run_adjoint_vjp(fvm_ctx *c, double *const *lam, double *dctrl);
 void adj_destroy(fvm_ctx *c);
 int theta_pairs(const Tgt &t, int field, int sweeps);
-int predictor_sweeps(const Tgt &t, int field);
+int predictor_sweeps(const Tgt &t, int field, int fields);
 // mixed precision (fvm_mixed.cu)
 int mixed_poisson_body(const Tgt &t, cudaGraphConditionalHandle cond, int has_cond);
 int mixed_sweep_pair(const Tgt &t, int apply);
-int mixed_predictor_radial(const Tgt &t, int field, int colour, int refresh);
-int mixed_predictor_theta(const Tgt &t, int field, int colour, int ghosts);
+int mixed_predictor_radial(const Tgt &t, int field, int fields, int colour, int refresh);
+int mixed_predictor_theta(const Tgt &t, int field, int fields, int colour, int ghosts);
 // line-resident FP32 sweeps (fvm_resident.cu).  The correction system a launch
 // solves: line factors (in the layout of the context's radial tile) and couplings,
 // the FP32 right-hand side and correction, the FP64 field the correction is added

@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(128) k_rad_dc(const __grid_constant__ S src, i
     __shared__ float xch[G][2 * NW];
     const Dev &d = dev_of(src);
     if ((int)blockIdx.x * G >= (d.NJ - 1) / 2) return;   // beyond this case's lines (batch)
-    const PredLine L = pred_line(d, field, 0);
+    const PredLine L = pred_line(d, field + (int)blockIdx.y, 0);
     const LineSys &s = L.s;
     const Coef &cf = L.cf;
     const double *SU = L.SU, *wallF = L.wallF, *farF = L.farF;
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(128) k_theta_dc(const __grid_constant__ S src,
     __shared__ float xch[G][2 * NW];
     const Dev &d = dev_of(src);
     if (2 * (int)blockIdx.x * G + 1 + colour > d.NI - 1) return;   // beyond this case's lines (batch)
-    const PredLine L = pred_line(d, field, 1);
+    const PredLine L = pred_line(d, field + (int)blockIdx.y, 1);
     const LineSys &s = L.s;
     const Coef &cf = L.cf;
     const double *SU = L.SU, *wallF = L.wallF, *farF = L.farF;
@@ -421,14 +421,14 @@ __global__ void __launch_bounds__(128) k_theta_dc(const __grid_constant__ S src,
     }
 }
 
-int mixed_predictor_radial(const Tgt &t, int field, int colour, int refresh)
+int mixed_predictor_radial(const Tgt &t, int field, int fields, int colour, int refresh)
 {
     const int blocks = line_blocks((t.NJ - 1) / 2, t.tr.NW);
     bool ok = dispatch_line(t.tr, [&](auto m, auto nw) {
         with_src(t, [&](const auto &src) {
             using S = std::decay_t<decltype(src)>;
             k_rad_dc<decltype(m)::value, decltype(nw)::value, S>
-                <<<dim3(blocks, 1, t.nz), 128, 0, t.st>>>(src, field, colour, refresh);
+                <<<dim3(blocks, fields, t.nz), 128, 0, t.st>>>(src, field, colour, refresh);
         });
     });
     if (!ok) {
@@ -440,14 +440,14 @@ int mixed_predictor_radial(const Tgt &t, int field, int colour, int refresh)
     return FVM_OK;
 }
 
-int mixed_predictor_theta(const Tgt &t, int field, int colour, int ghosts)
+int mixed_predictor_theta(const Tgt &t, int field, int fields, int colour, int ghosts)
 {
     const int blocks = line_blocks((t.NI - 1 + 1 - colour) / 2, t.tt.NW);
     bool ok = dispatch_line(t.tt, [&](auto m, auto nw) {
         with_src(t, [&](const auto &src) {
             using S = std::decay_t<decltype(src)>;
             k_theta_dc<decltype(m)::value, decltype(nw)::value, S>
-                <<<dim3(blocks, 1, t.nz), 128, 0, t.st>>>(src, field, colour, ghosts);
+                <<<dim3(blocks, fields, t.nz), 128, 0, t.st>>>(src, field, colour, ghosts);
         });
     });
     if (!ok) {

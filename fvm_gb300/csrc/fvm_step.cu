@@ -159,10 +159,13 @@ __global__ void k_af_su1(Dev d, int field)
 // BCU folding; the cross term of ITER_T is built from V when v_cross is set (the
 // reference's iter_T.f90:89-95), else from the field itself.
 template <class S>
-__global__ void k_af_su2(const __grid_constant__ S src, int field, int v_cross)
+__global__ void k_af_su2(const __grid_constant__ S src, int field, int fields, int v_cross)
 {
     const Dev &d = dev_of(src);
-    INTERIOR_IJ
+    const int nx = gridDim.x / fields;   // blocks along i; the fields side by side
+    field += blockIdx.x / nx;
+    const int i = (blockIdx.x % nx) * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1;
+    if (i > d.NI - 1 || j > d.NJ - 1) return;
     int c = IDX(i, j);
     FieldRefs f = field_refs(d, field);
     const double *xfield = (field == FVM_FIELD_T && v_cross) ? d.V : f.phi;
@@ -270,7 +273,7 @@ __global__ void __launch_bounds__(128) k_radial(const __grid_constant__ S src, i
     __shared__ double xch[G][2 * NW];
     const Dev &d = dev_of(src);
     if ((int)blockIdx.x * G >= (d.NJ - 1) / 2) return;   // beyond this case's lines (batch)
-    const PredLine L = pred_line(d, field, 0);
+    const PredLine L = pred_line(d, field + (int)blockIdx.y, 0);
     const LineSys &s = L.s;
     const Coef &cf = L.cf;
     const double *SU = L.SU, *wallF = L.wallF, *farF = L.farF;
@@ -319,7 +322,7 @@ __global__ void __launch_bounds__(128) k_theta(const __grid_constant__ S src, in
     __shared__ double xch[G][2 * NW];
     const Dev &d = dev_of(src);
     if (2 * (int)blockIdx.x * G + 1 + colour > d.NI - 1) return;   // beyond this case's lines (batch)
-    const PredLine L = pred_line(d, field, 1);
+    const PredLine L = pred_line(d, field + (int)blockIdx.y, 1);
     const LineSys &s = L.s;
     const Coef &cf = L.cf;
     const double *SU = L.SU, *wallF = L.wallF, *farF = L.farF;
@@ -642,14 +645,14 @@ int line_error(fvm_ctx *c)
     return FVM_ERR_ARG;
 }
 
-int launch_radial(const Tgt &t, int field, int colour, int refresh)
+int launch_radial(const Tgt &t, int field, int fields, int colour, int refresh)
 {
     const int blocks = line_blocks((t.NJ - 1) / 2, t.tr.NW);
     bool ok = dispatch_line(t.tr, [&](auto m, auto nw) {
         with_src(t, [&](const auto &src) {
             using S = std::decay_t<decltype(src)>;
             k_radial<decltype(m)::value, decltype(nw)::value, BCK_DIRICHLET, S>
-                <<<dim3(blocks, 1, t.nz), 128, 0, t.st>>>(src, field, colour, refresh);
+                <<<dim3(blocks, fields, t.nz), 128, 0, t.st>>>(src, field, colour, refresh);
         });
     });
     if (!ok) return line_error(t.c);
@@ -658,14 +661,14 @@ int launch_radial(const Tgt &t, int field, int colour, int refresh)
     return FVM_OK;
 }
 
-int launch_theta(const Tgt &t, int field, int colour, int ghosts)
+int launch_theta(const Tgt &t, int field, int fields, int colour, int ghosts)
 {
     const int blocks = line_blocks((t.NI - 1 + 1 - colour) / 2, t.tt.NW);
     bool ok = dispatch_line(t.tt, [&](auto m, auto nw) {
         with_src(t, [&](const auto &src) {
             using S = std::decay_t<decltype(src)>;
             k_theta<decltype(m)::value, decltype(nw)::value, S>
-                <<<dim3(blocks, 1, t.nz), 128, 0, t.st>>>(src, field, colour, ghosts);
+                <<<dim3(blocks, fields, t.nz), 128, 0, t.st>>>(src, field, colour, ghosts);
         });
     });
     if (!ok) return line_error(t.c);
@@ -715,20 +718,24 @@ int poisson64_body(const Tgt &t, cudaGraphConditionalHandle cond, int has_cond)
 
 }  // namespace
 
-// The predictor of one field after its first-factor SU is in place.
-int predictor_sweeps(const Tgt &t, int field)
+// The predictor of `fields` fields (U and V together, or one) after their first-factor
+// SU is in place; they do not read each other.  Together they fill more of the GPU and
+// save five launches a step (32 x 24: 297 -> 265 us, 4 mixed steps at 128 x 96 3121 -> 2940 us).
+int predictor_sweeps(const Tgt &t, int field, int fields)
 {
     const bool tk = field == FVM_FIELD_T;
     // sweep 1 (radial lines), ghosts refreshed from the pre-sweep field (BCU)
     for (int colour = 0; colour < 2; colour++) {
-        if (t.mixed) RC(mixed_predictor_radial(t, field, colour, colour == 0));
-        else RC(launch_radial(t, field, colour, colour == 0));
+        if (t.mixed) RC(mixed_predictor_radial(t, field, fields, colour, colour == 0));
+        else RC(launch_radial(t, field, fields, colour, colour == 0));
     }
     // second factor right-hand side from the first-sweep field
-    LAUNCH_S(t, k_af_su2, interior_grid(t), 128, field, (tk && t.iter_t_bug) ? 1 : 0);
+    dim3 g2 = interior_grid(t);
+    g2.x *= fields;
+    LAUNCH_S(t, k_af_su2, g2, 128, field, fields, (tk && t.iter_t_bug) ? 1 : 0);
     for (int colour = 0; colour < 2; colour++) {
-        if (t.mixed) RC(mixed_predictor_theta(t, field, colour, tk ? 1 : 0));
-        else RC(launch_theta(t, field, colour, tk ? 1 : 0));
+        if (t.mixed) RC(mixed_predictor_theta(t, field, fields, colour, tk ? 1 : 0));
+        else RC(launch_theta(t, field, fields, colour, tk ? 1 : 0));
     }
     return FVM_OK;
 }
@@ -742,8 +749,7 @@ int step_before_poisson(const Tgt &t)
     LAUNCH_S(t, k_farfield_step, dim3((t.NJ + 127) / 128, 1, t.nz), 128);
     LAUNCH_S(t, k_contra_vel, interior_grid(t), 128, 0);
     LAUNCH_S(t, k_explicit, interior_grid(t), 128, t.thermal);
-    RC(predictor_sweeps(t, FVM_FIELD_U));
-    RC(predictor_sweeps(t, FVM_FIELD_V));
+    RC(predictor_sweeps(t, FVM_FIELD_U, 2));
     LAUNCH_S(t, k_grad, interior_grid(t), 128, -1.0, 0);
     LAUNCH_S(t, k_contra_vel, interior_grid(t), 128, 1);
     return FVM_OK;
@@ -763,7 +769,7 @@ int step_after_poisson(const Tgt &t, double rtime, fvm_coeffs *dout)
 {
     LAUNCH_S(t, k_bcp_ghosts, dim3((t.NI + t.NJ + 127) / 128, 1, t.nz), 128);
     LAUNCH_S(t, k_grad, interior_grid(t), 128, +1.0, 1);
-    if (t.thermal) RC(predictor_sweeps(t, FVM_FIELD_T));
+    if (t.thermal) RC(predictor_sweeps(t, FVM_FIELD_T, 1));
     LAUNCH_S(t, k_cfl, interior_grid(t), 128);
     LAUNCH_S(t, k_calc_final, dim3(1, 1, t.nz), calc_threads(t), rtime, dout);
     return FVM_OK;
@@ -791,8 +797,8 @@ int theta_pairs(const Tgt &t, int field, int sweeps)
 {
     for (int s = 0; s < sweeps; s++)
         for (int colour = 0; colour < 2; colour++) {
-            if (t.mixed) RC(mixed_predictor_theta(t, field, colour, 0));
-            else RC(launch_theta(t, field, colour, 0));
+            if (t.mixed) RC(mixed_predictor_theta(t, field, 1, colour, 0));
+            else RC(launch_theta(t, field, 1, colour, 0));
         }
     return FVM_OK;
 }
@@ -851,7 +857,7 @@ int run_iter_u(fvm_ctx *c, int field)
     k_af_su1<<<interior_grid(tgt_of(c)), 128, 0, c->stream>>>(c->d, field);
     KCOUNT(c);
     FVM_LAUNCH_CHECK(c);
-    return predictor_sweeps(tgt_of(c), field);
+    return predictor_sweeps(tgt_of(c), field, 1);
 }
 
 int run_remove_grad(fvm_ctx *c)
@@ -1114,7 +1120,7 @@ int run_iter_t(fvm_ctx *c)
     k_af_su1<<<interior_grid(tgt_of(c)), 128, 0, c->stream>>>(c->d, FVM_FIELD_T);
     KCOUNT(c);
     FVM_LAUNCH_CHECK(c);
-    return predictor_sweeps(tgt_of(c), FVM_FIELD_T);
+    return predictor_sweeps(tgt_of(c), FVM_FIELD_T, 1);
 }
 
 int run_calccoef(fvm_ctx *c, fvm_coeffs *out)
