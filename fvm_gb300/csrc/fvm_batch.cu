@@ -32,6 +32,8 @@ struct fvm_batch {
     Dev *d_devs = nullptr;            // device table of the cases' views
     BatchCtl *d_bctl = nullptr;
     double *d_time = nullptr;         // per-case simulated time
+    int *d_cases = nullptr;           // case lists of the cluster launches
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     fvm_coeffs *d_hist = nullptr;     // records [step * ncases + case]
     fvm_coeffs *h_hist = nullptr;     // pinned copy
     int hist_cap = 0;                 // steps of record capacity
@@ -148,9 +150,50 @@ void drop_graph(fvm_batch *b)
     b->graph = nullptr;
 }
 
-// Capture one time step of every case: the launches before the Poisson loop, a
-// while-conditional node whose body holds `groups` residual intervals of the
-// batched Poisson iteration, and the launches after it.
+// The mixed Poisson iteration with one cluster per case, captured on the batch's streams:
+// cases whose blocks fit an SM twice in one launch, the larger ones in another beside it,
+// each from the most to the fewest cells so that the last to finish are small.  Returns
+// false (nothing captured) when a case has no cluster form.
+bool cluster_plan(fvm_batch *b, std::vector<int> (&cls)[2], size_t (&smem)[2])
+{
+    for (int k = 0; k < b->ncases; k++) {
+        const size_t n = fvm::cluster_bytes(b->cases[k], b->t.tr);
+        if (!n) return false;
+        const int q = fvm::cluster_two_per_sm(n) ? 1 : 0;
+        cls[q].push_back(k);
+        smem[q] = std::max(smem[q], n);
+    }
+    for (auto &v : cls)
+        std::stable_sort(v.begin(), v.end(), [b](int x, int y) { return b->cases[x]->n > b->cases[y]->n; });
+    return true;
+}
+
+int cluster_capture(fvm_batch *b, const std::vector<int> (&cls)[2], const size_t (&smem)[2])
+{
+    fvm_ctx *sh = &b->shell;
+    cudaStream_t st[2] = {sh->stream, sh->stream};
+    if (!cls[0].empty() && !cls[1].empty()) {
+        st[1] = b->st2;
+        FVM_CUDA(sh, cudaEventRecord(b->ev_fork, sh->stream));
+        FVM_CUDA(sh, cudaStreamWaitEvent(b->st2, b->ev_fork, 0));
+    }
+    int at = 0;
+    for (int q = 0; q < 2; q++) {
+        if (cls[q].empty()) continue;
+        const int rc = fvm::cluster_launch(b->t, st[q], b->d_cases + at, (int)cls[q].size(), smem[q]);
+        if (rc) return rc;
+        at += (int)cls[q].size();
+    }
+    if (st[1] != st[0]) {
+        FVM_CUDA(sh, cudaEventRecord(b->ev_join, b->st2));
+        FVM_CUDA(sh, cudaStreamWaitEvent(sh->stream, b->ev_join, 0));
+    }
+    return FVM_OK;
+}
+
+// Capture one time step of every case: the launches before the Poisson loop, the
+// iteration (cluster_capture, or a while-conditional node whose body holds `groups`
+// residual intervals of the batched iteration), and the launches after it.
 int build_graph(fvm_batch *b)
 {
     if (b->graph) return FVM_OK;
@@ -160,6 +203,14 @@ int build_graph(fvm_batch *b)
     const int groups = b->cases[0]->p.poisson_groups > 0 ? b->cases[0]->p.poisson_groups : (32 + per - 1) / per;
     cudaStream_t st = sh->stream;
     cudaGraph_t g = nullptr;
+    std::vector<int> cls[2];
+    size_t smem[2] = {0, 0};
+    const bool clusters = cluster_plan(b, cls, smem);
+    if (clusters) {
+        std::vector<int> list(cls[0]);
+        list.insert(list.end(), cls[1].begin(), cls[1].end());
+        FVM_CUDA(sh, cudaMemcpy(b->d_cases, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice));
+    }
     FVM_CUDA(sh, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     sh->capturing = true;
     sh->pgraph_kernels = 0;
@@ -167,7 +218,9 @@ int build_graph(fvm_batch *b)
     const int before = sh->pgraph_kernels;
     cudaError_t e = cudaSuccess;
     cudaGraphConditionalHandle h{};
-    if (rc == FVM_OK) {
+    if (rc == FVM_OK && clusters) {
+        rc = cluster_capture(b, cls, smem);
+    } else if (rc == FVM_OK) {
         cudaStreamCaptureStatus cs;
         cudaGraph_t cg = nullptr;
         const cudaGraphNode_t *deps = nullptr;
@@ -194,7 +247,7 @@ int build_graph(fvm_batch *b)
             if (e2 != cudaSuccess && rc == FVM_OK) e = e2;
         }
     }
-    const int body = sh->pgraph_kernels - before;
+    const int body = clusters ? 0 : sh->pgraph_kernels - before;
     if (rc == FVM_OK && e == cudaSuccess) rc = fvm::step_after_poisson(t, 0.0, nullptr);
     if (rc == FVM_OK && e == cudaSuccess) rc = fvm::launch_batch_tick(t, b->d_bctl);
     sh->capturing = false;
@@ -308,6 +361,9 @@ int fvm_batch_create(int ncases, const fvm_params *params, fvm_batch **out)
     if (e == cudaSuccess) e = cudaMalloc(&b->d_devs, sizeof(Dev) * ncases);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_bctl, sizeof(BatchCtl));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_time, sizeof(double) * ncases);
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_cases, sizeof(int) * ncases);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming);
     if (e != cudaSuccess) {
         fvm_batch_destroy(b);
         return FVM_ERR_CUDA;
@@ -340,6 +396,9 @@ int fvm_batch_destroy(fvm_batch *b)
     if (b->d_devs) cudaFree(b->d_devs);
     if (b->d_bctl) cudaFree(b->d_bctl);
     if (b->d_time) cudaFree(b->d_time);
+    if (b->d_cases) cudaFree(b->d_cases);
+    if (b->ev_fork) cudaEventDestroy(b->ev_fork);
+    if (b->ev_join) cudaEventDestroy(b->ev_join);
     if (b->d_hist) cudaFree(b->d_hist);
     if (b->h_hist) cudaFreeHost(b->h_hist);
     if (b->shell.ev_a) cudaEventDestroy(b->shell.ev_a);

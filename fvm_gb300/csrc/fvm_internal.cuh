@@ -316,6 +316,10 @@ int resident_sweeps(const Tgt &t, int sweeps, int apply, int max_polls, unsigned
 int resident_loop(fvm_ctx *c);   // the whole forward iteration (c->res_loop)
 int resident_reset(fvm_ctx *c);
 size_t exchange_words(const fvm_ctx *c);   // 64-bit words of d.XW
+// mixed Poisson iteration of a batch, one cluster per case (fvm_cluster.cu)
+size_t cluster_bytes(const fvm_ctx *c, const LineSys &tile);
+bool cluster_two_per_sm(size_t bytes);
+int cluster_launch(const Tgt &t, cudaStream_t st, const int *cases, int count, size_t smem);
 // state copies between caller buffers and the device (fvm_copy.cu)
 cudaError_t copy_arrays(double *const *dst, const double *const *src, int count, size_t n, cudaMemcpyKind kind,
                         cudaStream_t st);
