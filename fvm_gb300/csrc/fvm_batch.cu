@@ -151,15 +151,14 @@ void drop_graph(fvm_batch *b)
 }
 
 // The mixed Poisson iteration with one cluster per case, captured on the batch's streams:
-// cases whose blocks fit an SM twice in one launch, the larger ones in another beside it,
-// each from the most to the fewest cells so that the last to finish are small.  Returns
+// cases of 16 blocks in one launch, those of 8 in another beside it, each from the most to the fewest cells so that the last to finish are small.  Returns
 // false (nothing captured) when a case has no cluster form.
 bool cluster_plan(fvm_batch *b, std::vector<int> (&cls)[2], size_t (&smem)[2])
 {
     for (int k = 0; k < b->ncases; k++) {
         const size_t n = fvm::cluster_bytes(b->cases[k], b->t.tr);
         if (!n) return false;
-        const int q = fvm::cluster_two_per_sm(n) ? 1 : 0;
+        const int q = fvm::cluster_blocks(b->cases[k]) == 16 ? 0 : 1;
         cls[q].push_back(k);
         smem[q] = std::max(smem[q], n);
     }
@@ -180,7 +179,7 @@ int cluster_capture(fvm_batch *b, const std::vector<int> (&cls)[2], const size_t
     int at = 0;
     for (int q = 0; q < 2; q++) {
         if (cls[q].empty()) continue;
-        const int rc = fvm::cluster_launch(b->t, st[q], b->d_cases + at, (int)cls[q].size(), smem[q]);
+        const int rc = fvm::cluster_launch(b->t, st[q], b->d_cases + at, (int)cls[q].size(), q == 0 ? 16 : 8, smem[q]);
         if (rc) return rc;
         at += (int)cls[q].size();
     }

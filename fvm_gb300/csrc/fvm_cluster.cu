@@ -5,7 +5,7 @@
 // The batched path launched one grid over all cases per zebra colour (two per sweep), and
 // each launch read every operand from L2 again: 7.4 us a launch for 64 cases, most of it
 // launch latency and dependent L2 round trips.  The cases are independent, so here a
-// cluster of CLUSTER blocks keeps one case's FP32 factors, couplings, residual and
+// cluster of 8 or 16 blocks keeps one case's FP32 factors, couplings, residual and
 // correction in shared memory for the whole iteration; boundary lines and residual sums
 // travel through distributed shared memory, and the only waits are the cluster's own
 // hardware barriers (about 480 cycles with 512 threads).  Clusters need not run at the
@@ -20,7 +20,7 @@
 // is k_pois32's, so the results are the per-colour path's bit for bit.
 //
 // Operands sit in shared memory rather than in registers so that two blocks of 512 threads
-// fit an SM for cases of up to 128 lines (the south coupling of a line is the north coupling
+// fit an SM for up to 16 lines of 192 cells a block (the south coupling of a line is the north coupling
 // of the line below: the operator is symmetric): one block's barrier hides behind the
 // other's solves.
 #include <cooperative_groups.h>
@@ -37,13 +37,13 @@ namespace cg = cooperative_groups;
 namespace fvm {
 namespace {
 
-constexpr int CLUSTER = 8;      // blocks per case (the portable maximum)
 constexpr int CT = 512;         // threads per block
 constexpr size_t CLUSTER_SMEM = 220 * 1024;
-constexpr size_t CLUSTER_SMEM_TWO = 112 * 1024;   // two blocks per SM
 
-// Lines per block of a case of L lines.
-inline __host__ __device__ int cluster_lines(int L) { return 4 * (((L + 3) / 4 + CLUSTER - 1) / CLUSTER); }
+// Blocks per case of L lines -- 16 (the most a cluster takes) where 8 would own more than
+// 16 lines each and no longer fit an SM twice -- and lines per block.
+inline __host__ __device__ int cluster_size(int L) { return L > 128 ? 16 : 8; }
+inline __host__ __device__ int cluster_lines(int L) { return 4 * (((L + 3) / 4 + cluster_size(L) - 1) / cluster_size(L)); }
 
 // Shared memory of a block: an (nl + 1 lines), fi, fa, fb, rf, x (nl lines each), two halo
 // lines; sums; the split pressure of lines j0-2 .. j0+nl and of the ghost row 0.
@@ -97,6 +97,8 @@ __global__ void __launch_bounds__(CT, 2) k_cluster32(DevTable tab, const int *ca
             an[size_t(q) * LW + k * TG + t] = e < n ? d.cP.ANf[IDX(e + 1, jn)] : 0.0f;
         }
         if (q == nl) break;
+#pragma unroll
+        for (int k = 0; k < M; k++) rf[size_t(q) * LW + k * TG + t] = 0.0f;   // the padding stays zero
         const size_t base = size_t(j0 + q - 1) * LW;
 #pragma unroll
         for (int k = 0; k < M; k++) {
@@ -170,7 +172,7 @@ __global__ void __launch_bounds__(CT, 2) k_cluster32(DevTable tab, const int *ca
             const int half = lane >> 4, col = lane & 15;
             const double v = mres_columns(col < nt ? mres_lines(s_w + size_t(half * per + 4 * q) * 16 + col, 16) : 0.0);
             if (col == 0)
-                for (int r = 0; r < CLUSTER; r++)
+                for (int r = 0; r < (int)gridDim.x; r++)
                     *cluster.map_shared_rank(s_tot + 2 * ((j0 - 1) / MRES_GROUP + q) + half, r) = v;
         }
         cluster_barrier();
@@ -180,20 +182,19 @@ __global__ void __launch_bounds__(CT, 2) k_cluster32(DevTable tab, const int *ca
         for (int half = 0; half < 2 * S; half++) {   // colour 0: the odd lines q = 0, 2, ...
             const int colour = half & 1;
             for (int q = 2 * g + colour; q < nl; q += 2 * G) {
-                const float *xs = q > 0 ? x + size_t(q - 1) * LW : lo, *xn = q + 1 < nl ? x + size_t(q + 1) * LW : hi;
+                const int o = q * LW + t;
+                const float *xs = q > 0 ? x + o - LW : lo + t, *xn = q + 1 < nl ? x + o + LW : hi + t;
                 float v[M], fi[M], fa[M], fb[M];
 #pragma unroll
-                for (int k = 0; k < M; k++) {
-                    const int w = k * TG + t;
-                    const size_t o = size_t(q) * LW + w;
-                    v[k] = t * M + k < n ? pois32_rhs(an[o + LW], xn[w], an[o], xs[w], rf[o]) : 0.0f;
-                    fi[k] = sfi[o];
-                    fa[k] = sfa[o];
-                    fb[k] = sfb[o];
+                for (int k = 0; k < M; k++) {   // padding: zero couplings, residual and factors
+                    v[k] = pois32_rhs(an[o + LW + k * TG], xn[k * TG], an[o + k * TG], xs[k * TG], rf[o + k * TG]);
+                    fi[k] = sfi[o + k * TG];
+                    fa[k] = sfa[o + k * TG];
+                    fb[k] = sfb[o + k * TG];
                 }
                 group_apply_r<float, M, NW>(v, fi, fa, fb, t, xch[g], bar);
 #pragma unroll
-                for (int k = 0; k < M; k++) x[size_t(q) * LW + k * TG + t] = v[k];
+                for (int k = 0; k < M; k++) x[o + k * TG] = v[k];
                 if (q == 0)
 #pragma unroll
                     for (int k = 0; k < M; k++) hi_prev[k * TG + t] = v[k];
@@ -242,26 +243,27 @@ size_t cluster_bytes(const fvm_ctx *c, const LineSys &tile)
     return b <= CLUSTER_SMEM ? b : 0;
 }
 
-// Whether two blocks with that much shared memory fit an SM.
-bool cluster_two_per_sm(size_t bytes) { return bytes <= CLUSTER_SMEM_TWO; }
+int cluster_blocks(const fvm_ctx *c) { return cluster_size(c->NJ - 1); }
 
-// The iteration of the `count` cases listed in device memory, `smem` bytes a block.
-int cluster_launch(const Tgt &t, cudaStream_t st, const int *cases, int count, size_t smem)
+// The iteration of the `count` cases listed in device memory, `blocks` blocks a case with
+// `smem` bytes each.
+int cluster_launch(const Tgt &t, cudaStream_t st, const int *cases, int count, int blocks, size_t smem)
 {
     cudaError_t e = cudaErrorInvalidValue;
     dispatch_line(t.tr, [&](auto m, auto nw) {
         constexpr int M_ = decltype(m)::value, NW_ = decltype(nw)::value;
         auto k = k_cluster32<M_, NW_>;
         e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLUSTER_SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(CLUSTER, 1, count);
+        cfg.gridDim = dim3(blocks, 1, count);
         cfg.blockDim = dim3(CT);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = st;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = CLUSTER;
+        at[0].val.clusterDim.x = blocks;
         at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;

@@ -14,8 +14,8 @@ pytestmark = pytest.mark.gpu
 BATCHES = [
     ([(4, 5), (8, 6), (12, 20)], (1, 1, 1, 1)),                  # one to three blocks of four lines
     ([(32, 24), (36, 30), (100, 17)], (1, 1, 4, 1)),             # 36: two lines in no block's way; 100: 13 groups
-    ([(64, 48), (132, 90), (256, 64)], (2, 2, 4, 2)),            # blocks of 8, 20 and 32 lines
-    ([(64, 48), (240, 192), (96, 33)], (2, 3, 4, 2)),            # one and two blocks per SM
+    ([(64, 48), (132, 90), (256, 64)], (2, 2, 4, 2)),            # blocks of 8, 12 and 16 lines
+    ([(64, 48), (240, 192), (96, 33)], (2, 3, 4, 2)),            # clusters of 8 and of 16 blocks
     ([(128, 100), (64, 128)], (4, 1, 4, 1)),
     ([(64, 190), (80, 150)], (1, 6, 1, 3)),
     ([(512, 380), (64, 40)], (1, 12, 4, 4)),                     # too large for a block: per-colour kernels
