@@ -1113,10 +1113,18 @@ int adj_poisson_graph(fvm_ctx *c)
 int adj_poisson(fvm_ctx *c)
 {
     fvm_adj *A = c->adj;
-    ARC(adj_poisson_graph(c));
-    k_adj_pctl_reset<<<1, 1, 0, c->stream>>>(A->a);
-    const long max_launches = (long)c->d.nswpp / A->pgraph_iters + 2;
-    for (long l = 0;; l++) {
+    const Adj &a = A->a;
+    const bool ring = c->ring_blocks != 0;   // FP64: the whole iteration in one launch
+    if (!ring) ARC(adj_poisson_graph(c));
+    k_adj_pctl_reset<<<1, 1, 0, c->stream>>>(a);
+    if (ring) {
+        ARC(ring_launch_adjoint(c, RingSys{a.sPT.invD, a.sPT.fa, a.sPT.fb, a.cPT.AN, a.cPT.AS, a.cPT.AE, a.cPT.AW, a.cPT.AP, a.g,
+                                           a.mu, a.pctl, 4}));
+        FVM_CUDA(c, cudaMemcpyAsync(A->h_pctl, a.pctl, sizeof(PCtl), cudaMemcpyDeviceToHost, c->stream));
+        FVM_CUDA(c, cudaStreamSynchronize(c->stream));
+    }
+    const long max_launches = ring ? 0 : (long)c->d.nswpp / A->pgraph_iters + 2;
+    for (long l = 0; !ring; l++) {
         if (l >= max_launches) {
             c->err = "adjoint Poisson iteration did not report completion within the sweep cap";
             return FVM_ERR_TIMEOUT;
@@ -1131,7 +1139,7 @@ int adj_poisson(fvm_ctx *c)
         ARC(resident_reset(c));
         FVM_CUDA(c, cudaMemsetAsync(&A->a.pctl->fault, 0, sizeof(int), c->stream));
         FVM_CUDA(c, cudaStreamSynchronize(c->stream));
-        c->err = "adjoint Poisson: a bounded wait of the resident sweeps ran out";
+        c->err = "adjoint Poisson: a bounded wait of the on-chip sweeps ran out";
         return FVM_ERR_TIMEOUT;
     }
     if (!std::isfinite(A->h_pctl->resip)) {

@@ -326,7 +326,16 @@ cudaError_t copy_arrays(double *const *dst, const double *const *src, int count,
 // FP64 Poisson iteration in one launch (fvm_ring.cu)
 int ring_setup(fvm_ctx *c);
 int ring_pairs(const fvm_ctx *c);   // line pairs per block
+// the line system, residual coefficients, source, unknown and control of a ring launch,
+// sweeps per residual
+struct RingSys {
+    const double *invD, *fa, *fb, *AN, *AS, *AE, *AW, *AP, *SRC;
+    double *X;
+    PCtl *pctl;
+    int per;
+};
 int ring_launch(fvm_ctx *c, int mode, int count);
+int ring_launch_adjoint(fvm_ctx *c, const RingSys &sys);
 }  // namespace fvm
 
 // ---------------------------------------------------------------------------------

@@ -31,6 +31,11 @@
 // the same decision.  Every wait is bounded; one that runs out sets the fault flag, the
 // pressure is left alone and the host reports FVM_ERR_TIMEOUT.
 //
+// ADJ: the transposed equation of the adjoint, (A^T + G^T DD^T) mu = g (fvm_adjoint.cu).
+// Its lagged cross term at (i,j) reads mu^(n-1) at rows j and j+2 (wrapped), columns i and
+// i+2, at i = 1 column 2 as well, and no ghosts; the residual takes the cross term of
+// the current mu.  So the halo lines are j1+1 and j1+2 instead of j0-1 and j0-2.
+//
 // Bound: FP64.  A warp's FP64 instruction holds its quarter of the SM's FP64 pipe for 64
 // cycles (measured: a dependent chain of DFMAs, and the same chain beside three others
 // on the quarter, run at 67 and 259 cycles a step), so a line costs 64 cycles times the FP64
@@ -58,7 +63,7 @@ template <int M, int NW>
 struct RingLayout {
     static constexpr int TG = WARP * NW, LW = TG * M;
     static constexpr int CST = 2 * (STAGES + 1) + 2 * M;   // per-thread scan constants
-    // lines (3 versions), the halo lines j0-1 and j0-2 (3 versions each), per line the
+    // lines (3 versions), two halo lines of the cross term (3 versions each), per line the
     // scan constants, the warps' total products and the fold buffers
     static size_t doubles(int nl) { return size_t(3) * (nl + 2) * LW + size_t(nl) * (size_t(CST) * TG + 4 * NW); }
     static size_t bytes(int nl) { return sizeof(double) * doubles(nl); }
@@ -108,9 +113,9 @@ __device__ __forceinline__ bool poll_line(const ulonglong2 *src, int t, int n, u
 
 // mode 0: the whole iteration; mode 1: `count` sweeps without residuals, P unchanged
 // (timing).
-template <int M, int NW>
+template <int M, int NW, int ADJ>
 __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
-    k_ring64(const __grid_constant__ Dev d, int ppb, int mode, int count)
+    k_ring64(const __grid_constant__ Dev d, const __grid_constant__ RingSys sys, int ppb, int mode, int count)
 {
     using Lay = RingLayout<M, NW>;
     constexpr int TG = Lay::TG, LW = Lay::LW, CST = Lay::CST;
@@ -137,28 +142,43 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
     if (threadIdx.x == 0) s_fault = 0;
 
     // operands of the line, in the chunk ownership of the solve (element e = t*M + k)
-    double fi[M], fa[M], fb[M], an[M], as[M], dv[M], c1[M], c2[M], c3[M], c4[M], v[M], su[M], sun[M];
+    double fi[M], fa[M], fb[M], an[M], as[M], dv[M], c1[M], c2[M], c3[M], c4[M], v[M], su[M], sun[M], w5 = 0.0, w6 = 0.0;
     if (act) {
         const size_t base = size_t(j - 1) * LW;
-        load_factors<double, M, NW>(fi, fa, fb, d.sP.invD + base, d.sP.fa + base, d.sP.fb + base, t);
+        load_factors<double, M, NW>(fi, fa, fb, sys.invD + base, sys.fa + base, sys.fb + base, t);
 #pragma unroll
         for (int k = 0; k < M; k++) {
             const int e = t * M + k;
-            const bool ok = e < n, cr = ok && e > 0 && j > 1;
-            const int c = IDX(e + 1, j), cc = cr ? IDX(e, j - 1) : 0;
-            an[k] = ok ? d.cP.AN[c] : 0.0;
-            as[k] = ok ? d.cP.AS[c] : 0.0;
-            dv[k] = ok ? d.DIVDT[c] : 0.0;
-            c1[k] = cr ? d.CNE[cc] : 0.0;
-            c2[k] = cr ? d.CSE[cc] : 0.0;
-            c3[k] = cr ? d.CNW[cc] : 0.0;
-            c4[k] = cr ? d.CSW[cc] : 0.0;
-            v[k] = ok ? d.P[c] : 0.0;
+            const bool ok = e < n;
+            const int c = IDX(e + 1, j);
+            an[k] = ok ? sys.AN[c] : 0.0;
+            as[k] = ok ? sys.AS[c] : 0.0;
+            dv[k] = ok ? sys.SRC[c] : 0.0;
+            if (ADJ) {   // weights at (i-1, j-1), (i-1, y), (i+1, j-1), (i+1, y), y = j+1 or, from line NJ-1, 1
+                const int y = j == L ? 1 : j + 1;
+                const bool up = ok && j != L - 1, dn = ok && j > 1, we = e > 0, ea = e + 2 < n;
+                c1[k] = dn && we ? d.CNE[IDX(e, j - 1)] : 0.0;
+                c2[k] = up && we ? d.CSE[IDX(e, y)] : 0.0;
+                c3[k] = dn && ea ? d.CNW[IDX(e + 2, j - 1)] : 0.0;
+                c4[k] = up && ea ? d.CSW[IDX(e + 2, y)] : 0.0;
+                if (e == 0) {   // the wall ghost's share of cell 1: column 2
+                    w5 = dn && n > 1 ? d.CNW[IDX(1, j - 1)] : 0.0;
+                    w6 = up && n > 1 ? d.CSW[IDX(1, y)] : 0.0;
+                }
+            } else {
+                const bool cr = ok && e > 0 && j > 1;
+                const int cc = cr ? IDX(e, j - 1) : 0;
+                c1[k] = cr ? d.CNE[cc] : 0.0;
+                c2[k] = cr ? d.CSE[cc] : 0.0;
+                c3[k] = cr ? d.CNW[cc] : 0.0;
+                c4[k] = cr ? d.CSW[cc] : 0.0;
+            }
+            v[k] = ok ? sys.X[c] : 0.0;
             su[k] = 0.0;
             line(0, g)[k * TG + t] = v[k];
         }
         // version -1 of a line is only read for its ghost column, which sits in element 0
-        if (t == 0) line(2, g)[0] = d.P[IDX(0, j)];
+        if (!ADJ && t == 0) line(2, g)[0] = sys.X[IDX(0, j)];
         // the scans' constant factors (group_apply_r's products, formed once)
         double G = 1.0;
 #pragma unroll
@@ -202,20 +222,24 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
             if (__any_sync(0xffffffffu, fabs(cst[(STAGES + 1 + s) * TG + t]) > tiny)) hs = s + 1;
         }
     }
-    // halo lines: version 0, and version -1 (ghost columns; block 0: the stored ghost row 0)
-    const int jm1 = wrap(j0 - 1), jm2 = j0 - 2;
+    // halo lines: version 0, and version -1 (ghost columns; block 0: the stored ghost row 0).
+    // hm1: line j0-1 (ADJ: j1+2, even), hm2: line j0-2 (ADJ: j1+1, odd)
+    const int jm1 = wrap(j0 - 1), j1 = j0 + nl - 1;
+    const int je = ADJ ? wrap(j1 + 2) : jm1, jo = ADJ ? wrap(j1 + 1) : j0 - 2;
     for (int q = threadIdx.x; q < 3 * LW; q += blockDim.x) hm2[q] = 0.0;
     __syncthreads();
     for (int e = threadIdx.x; e < n; e += blockDim.x) {
         const int w = (e % M) * TG + e / M;
-        hm1[w] = d.P[IDX(e + 1, jm1)];
-        if (j0 == 1) hm1[2 * LW + w] = d.P[IDX(e + 1, 0)];
-        if (jm2 >= 1) hm2[w] = d.P[IDX(e + 1, jm2)];
+        hm1[w] = sys.X[IDX(e + 1, je)];
+        if (!ADJ && j0 == 1) hm1[2 * LW + w] = sys.X[IDX(e + 1, 0)];
+        if (jo >= 1) hm2[w] = sys.X[IDX(e + 1, jo)];
     }
-    if (threadIdx.x == 0) {
-        if (j0 != 1) hm1[2 * LW] = d.P[IDX(0, jm1)];
-        if (jm2 >= 1) hm2[2 * LW] = d.P[IDX(0, jm2)];
+    if (!ADJ && threadIdx.x == 0) {
+        if (j0 != 1) hm1[2 * LW] = sys.X[IDX(0, jm1)];
+        if (jo >= 1) hm2[2 * LW] = sys.X[IDX(0, jo)];
     }
+    // groups that poll the halo lines of the cross term for themselves
+    const int ge = ADJ ? nl - 1 : 1, go = ADJ ? nl - 2 : 0;
     double hal[M];   // group 0: line j0-1; the last group: line j1+1
 #pragma unroll
     for (int k = 0; k < M; k++) hal[k] = 0.0;
@@ -223,19 +247,37 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
 #pragma unroll
         for (int k = 0; k < M; k++) {
             const int e = t * M + k;
-            if (e < n) hal[k] = d.P[IDX(e + 1, jm1)];
+            if (e < n) hal[k] = sys.X[IDX(e + 1, jm1)];
         }
     }
-    const double corner0 = d.P[IDX(0, 0)];
+    const double corner0 = ADJ ? 0.0 : sys.X[IDX(0, 0)];
     const unsigned cnt0 = d.XCNT[blockIdx.x];
     ulonglong2 *words = reinterpret_cast<ulonglong2 *>(d.XW);
     auto slot = [&](unsigned cnt, int q) { return words + (size_t(cnt & 1u) * L + (q - 1)) * LW; };
     ulonglong2 *psum = words + size_t(2) * L * LW;   // [2 slots][blocks][2]
     __syncthreads();
 
-    // source of sweep m: DIVDT minus the cross term of P^(m-1)
+    // source of sweep m: DIVDT (g) minus the cross term of P^(m-1) (mu^(m-1))
     auto source = [&](int m, double (&out)[M]) {
         const int vr = (m + 2) % 3, vg = (m + 1) % 3;
+        if (ADJ) {
+            const double *self = line(vr, g);
+            const double *row = g + 2 < nl ? line(vr, g + 2) : (odd ? hm2 : hm1) + size_t(vr) * LW;
+#pragma unroll
+            for (int k = 0; k < M; k++) {
+                const int e = t * M + k;
+                const int w = k + 2 < M ? (k + 2) * TG + t : (M >= 2 ? (k + 2 - M) * TG + t + 1 : t + 2);   // element e+2
+                const double p0 = self[k * TG + t], pp = row[k * TG + t];
+                const double q0 = e + 2 < n ? self[w] : 0.0, qp = e + 2 < n ? row[w] : 0.0;
+                double x = e < n ? pois_source(dv[k], c1[k], p0, c2[k], pp, c3[k], q0, c4[k], qp) : 0.0;
+                if (e == 0 && n > 1) {
+                    const int w1 = M >= 2 ? TG : 1;   // element 1
+                    x = fma_rn(-w6, row[w1], fma_rn(-w5, self[w1], x));
+                }
+                out[k] = x;
+            }
+            return;
+        }
         const double *self = line(vr, g), *row;
         double gs = line(vg, g)[0], gr;
         if (g >= 2) {
@@ -315,7 +357,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
 
     if (act && odd) source(1, su);
     int m = 0, have = 0;   // sweeps done; have: group 0's halo already holds version m
-    const int per = mode ? count : d.res_every;
+    const int per = mode ? count : sys.per;
     double resip = 0.0;
     bool bad = false;
     for (int round = 0;; round++) {
@@ -334,19 +376,23 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
                     solve();
 #pragma unroll
                     for (int k = 0; k < M; k++) line(vw, g)[k * TG + t] = v[k];
-                    if (g == 0 || g == nl - 2) publish(m);
+                    if (g == 0 || (!ADJ && g == nl - 2)) publish(m);
                 } else {
-                    if (g == 1 && m > 1) {
+                    if (ADJ && have) {
+                        // the residual has formed this sweep's source
+                    } else {
+                    if (g == ge && m > 1) {
                         double x[M];
 #pragma unroll
                         for (int k = 0; k < M; k++) x[k] = 0.0;
                         const unsigned want = cnt0 + unsigned(m - 1);
-                        if (!poll_line<M, TG>(slot(want, jm1), t, n, want, x)) s_fault = 1;
+                        if (!poll_line<M, TG>(slot(want, je), t, n, want, x)) s_fault = 1;
 #pragma unroll
                         for (int k = 0; k < M; k++) hm1[size_t(vr) * LW + k * TG + t] = x[k];
                         bar();
                     }
                     source(m, su);
+                    }
                 }
             }
             have = 0;
@@ -364,14 +410,14 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
                     solve();
 #pragma unroll
                     for (int k = 0; k < M; k++) line(vw, g)[k * TG + t] = v[k];
-                    if (g == nl - 1) publish(m);
+                    if (g == nl - 1 || (ADJ && g == 1)) publish(m);
                 } else {
-                    if (g == 0 && jm2 >= 1) {
+                    if (g == go && jo >= 1) {
                         double x[M];
 #pragma unroll
                         for (int k = 0; k < M; k++) x[k] = 0.0;
                         const unsigned want = cnt0 + unsigned(m);
-                        if (!poll_line<M, TG>(slot(want, jm2), t, n, want, x)) s_fault = 1;
+                        if (!poll_line<M, TG>(slot(want, jo), t, n, want, x)) s_fault = 1;
 #pragma unroll
                         for (int k = 0; k < M; k++) hm2[size_t(vw) * LW + k * TG + t] = x[k];
                         bar();
@@ -384,17 +430,35 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
             if (s_fault) { bad = true; break; }
         }
         if (bad || mode) break;
-        // scaled-L1 residual of P^m with the last sweep's source
+        // scaled-L1 residual of P^m with the last sweep's source (of mu^m with its own)
         const int vw = m % 3;
         double ra = 0.0, pa = 0.0;
         if (act) {
+            if (ADJ) {
+                if (odd) {
+#pragma unroll
+                    for (int k = 0; k < M; k++) su[k] = sun[k];
+                } else {
+                    if (g == ge) {
+                        double x[M];
+#pragma unroll
+                        for (int k = 0; k < M; k++) x[k] = 0.0;
+                        const unsigned want = cnt0 + unsigned(m);
+                        if (!poll_line<M, TG>(slot(want, je), t, n, want, x)) s_fault = 1;
+#pragma unroll
+                        for (int k = 0; k < M; k++) hm1[size_t(vw) * LW + k * TG + t] = x[k];
+                        bar();
+                    }
+                    source(m + 1, su);
+                }
+            }
             double ae[M], aw[M], ap[M];
 #pragma unroll
             for (int k = 0; k < M; k++) {
                 const int e = t * M + k, c = IDX(e + 1, j);
-                ae[k] = e < n ? d.cP.AE[c] : 0.0;
-                aw[k] = e < n ? d.cP.AW[c] : 0.0;
-                ap[k] = e < n ? d.cP.AP[c] : 0.0;
+                ae[k] = e < n ? sys.AE[c] : 0.0;
+                aw[k] = e < n ? sys.AW[c] : 0.0;
+                ap[k] = e < n ? sys.AP[c] : 0.0;
             }
             if (g == 0) wait_line(jm1, m);
             const double *self = line(vw, g);
@@ -408,7 +472,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
                 const double ps = g == 0 ? hal[k] : line(vw, g - 1)[k * TG + t];
                 pois_resid(ae[k], pe, aw[k], pw, an[k], pn, as[k], ps, su[k], ap[k], v[k], ra, pa);
             }
-            if (odd) {
+            if (!ADJ && odd) {
 #pragma unroll
                 for (int k = 0; k < M; k++) su[k] = sun[k];
             }
@@ -440,7 +504,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
         __syncthreads();
         if (threadIdx.x < WARP) {
             blocks_sum2([&](int q) { return s_tot[q]; }, gridDim.x, ra, pa);
-            if (threadIdx.x == 0) s_res = ra / pa;
+            if (threadIdx.x == 0) s_res = ADJ && !(pa > 0.0) ? 0.0 : ra / pa;
         }
         __syncthreads();
         if (s_fault) { bad = true; break; }
@@ -449,8 +513,8 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
     }
     if (bad) {
         if (threadIdx.x == 0) {
-            d.pctl->fault = 1;
-            d.pctl->done = 1;
+            sys.pctl->fault = 1;
+            sys.pctl->done = 1;
         }
         return;
     }
@@ -458,16 +522,16 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
 #pragma unroll
         for (int k = 0; k < M; k++) {
             const int e = t * M + k;
-            if (e < n) d.P[IDX(e + 1, j)] = v[k];
+            if (e < n) sys.X[IDX(e + 1, j)] = v[k];
         }
     }
     if (threadIdx.x == 0) {
         d.XCNT[blockIdx.x] = cnt0 + unsigned(m);
         if (blockIdx.x == 0 && !mode) {
-            d.pctl->niter = m;
-            d.pctl->resip = resip;
-            d.pctl->capped = resip > d.resimax ? 1 : 0;
-            d.pctl->done = 1;
+            sys.pctl->niter = m;
+            sys.pctl->resip = resip;
+            sys.pctl->capped = resip > d.resimax ? 1 : 0;
+            sys.pctl->done = 1;
         }
     }
 }
@@ -502,13 +566,15 @@ int ring_setup(fvm_ctx *c)
     const bool ok = dispatch_line(s, [&](auto m, auto nw) {
         constexpr int M_ = decltype(m)::value, NW_ = decltype(nw)::value;
         using Lay = RingLayout<M_, NW_>;
-        auto k = k_ring64<M_, NW_>;
+        auto k = k_ring64<M_, NW_, 0>;
+        auto ka = k_ring64<M_, NW_, 1>;
         // set outside any capture, to the largest block's need, the same for every context
         int most = 0;
         for (int nl : {2, 4})
             if (Lay::bytes(nl) <= 220 * 1024) most = (int)Lay::bytes(nl);
         if ((int)Lay::bytes(2 * ppb) > most) return;
         e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(ka, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         if (e == cudaSuccess)
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 2 * ppb * Lay::TG, Lay::bytes(2 * ppb));
     });
@@ -517,9 +583,9 @@ int ring_setup(fvm_ctx *c)
     return FVM_OK;
 }
 
-// The FP64 Poisson iteration of a context whose source term is in place (mode 0), or
-// `count` sweeps on chip (mode 1).  Cooperative: all blocks resident at once.
-int ring_launch(fvm_ctx *c, int mode, int count)
+namespace {
+template <int ADJ>
+int launch(fvm_ctx *c, const RingSys &sys, int mode, int count)
 {
     cudaError_t e = cudaErrorInvalidValue;
     dispatch_line(c->d.sP, [&](auto m, auto nw) {
@@ -535,7 +601,7 @@ int ring_launch(fvm_ctx *c, int mode, int count)
         at[0].val.cooperative = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, k_ring64<M_, NW_>, c->d, c->d.ring_ppb, mode, count);
+        e = cudaLaunchKernelEx(&cfg, k_ring64<M_, NW_, ADJ>, c->d, sys, c->d.ring_ppb, mode, count);
     });
     if (e != cudaSuccess) {
         c->err = std::string("Poisson ring launch: ") + cudaGetErrorString(e);
@@ -544,5 +610,18 @@ int ring_launch(fvm_ctx *c, int mode, int count)
     KCOUNT(c);
     return FVM_OK;
 }
+}  // namespace
+
+// The FP64 Poisson iteration of a context whose source term is in place (mode 0), or
+// `count` sweeps on chip (mode 1).  Cooperative: all blocks resident at once.
+int ring_launch(fvm_ctx *c, int mode, int count)
+{
+    const Dev &d = c->d;
+    return launch<0>(c, RingSys{d.sP.invD, d.sP.fa, d.sP.fb, d.cP.AN, d.cP.AS, d.cP.AE, d.cP.AW, d.cP.AP, d.DIVDT, d.P, d.pctl,
+                                d.res_every}, mode, count);
+}
+
+// The adjoint's transposed equation, its factors in the layout of the radial tile.
+int ring_launch_adjoint(fvm_ctx *c, const RingSys &sys) { return launch<1>(c, sys, 0, 0); }
 
 }  // namespace fvm
