@@ -48,6 +48,7 @@ struct Adj {
     double *lomega;                          // [0]: rotation adjoint through the drag formula
     double *DCU, *DCV, *DCP;                 // dCd/dU(1,j), dCd/dV(1,j), dCd/dP(1,j)
     double *DCW;                             // [0]: dCd/d(omega) through the drag formula
+    double *ST0, *CT0;                       // sine and cosine of THETA(0,j)
     Coef cPT, cXT, cYT;                      // transposed coefficient sets (Poisson, first, second factor)
     LineSys sPT, sXT, sYT;                   // their line factors
     PCtl *pctl;                              // adjoint Poisson iteration control
@@ -90,6 +91,8 @@ __global__ void k_adj_dragcoef(Dev d, Adj a)
 {
     int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
     if (j > d.NJ - 1) return;
+    a.ST0[j] = sin(d.THETA[IDX(0, j)]);
+    a.CT0[j] = cos(d.THETA[IDX(0, j)]);
     double DN1, TH2;
     wall_normal(d, j, DN1, TH2);
     const int c = IDX(1, j);
@@ -801,22 +804,20 @@ __global__ void k_adj_pctl_reset(Adj a)
 
 // Controls from the wall-value adjoints: UFW = -omega sin th + b cos th,
 // VFW = omega cos th + b sin th (th = THETA(0,j)); out[0] = dJ/domega,
-// out[j] = dJ/db_j (j = 1..NJ-1).
-__global__ void k_adj_controls(Dev d, Adj a, double *out)
+// out[j] = dJ/db_j (j = 1..NJ-1).  One block, the rotation's sum in a fixed tree (one
+// thread forming it took 189 us at 128 wall cells).
+__global__ void __launch_bounds__(512) k_adj_controls(Dev d, Adj a, double *out)
 {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j > d.NJ - 1) return;
-    if (j == 0) {
-        double s = a.lomega[0];
-        for (int k = 1; k <= d.NJ - 1; k++) {
-            const double th = d.THETA[IDX(0, k)];
-            s += -sin(th) * a.lUFW[k] + cos(th) * a.lVFW[k];
-        }
-        out[0] = s;
-        return;
+    __shared__ double sh[64];
+    const int j = threadIdx.x + 1;
+    double s = 0.0, none = 0.0;
+    if (j <= d.NJ - 1) {
+        const double st = a.ST0[j], ct = a.CT0[j], u = a.lUFW[j], v = a.lVFW[j];
+        s = -st * u + ct * v;
+        out[j] = (ct * u + st * v) + a.lblow[j];
     }
-    const double th = d.THETA[IDX(0, j)];
-    out[j] = (cos(th) * a.lUFW[j] + sin(th) * a.lVFW[j]) + a.lblow[j];
+    block_sum2(s, none, sh);
+    if (threadIdx.x == 0) out[0] = a.lomega[0] + s;
 }
 
 }  // namespace
@@ -832,6 +833,7 @@ struct fvm_adj {
     double *ckpt = nullptr;              // checkpoints: nckpt x 7 full arrays
     double *base = nullptr;              // U, V before every step of a segment: seg x 2 full arrays
     double *fin = nullptr;               // state at the end of the window: 7 full arrays
+    double *one = nullptr;               // U, V before the step of run_adjoint_vjp
     int nckpt = 0, nseg_steps = 0;
     cudaGraphExec_t pgraph = nullptr;    // adjoint Poisson loop body
     int pgraph_iters = 0;
@@ -978,7 +980,7 @@ int adj_setup(fvm_ctx *c)
         return (6 * cnt + 2 * s.lines) * sizeof(double) + 16 * 256;
     };
     // per transposed set: AP, AE, AW, AN, AS (FP64) and ANf, ASf (FP32)
-    size_t bytes = (30 * n + 10 * nj1 + 16) * sizeof(double) + 3 * (6 * n * sizeof(double) + 8 * 256) +
+    size_t bytes = (30 * n + 12 * nj1 + 16) * sizeof(double) + 3 * (6 * n * sizeof(double) + 8 * 256) +
                    sys_bytes(d.sP) + sys_bytes(d.sUX) + sys_bytes(d.sUY) + 64 * 256 + sizeof(PCtl) +
                    2 * size_t(c->nblk_res) * sizeof(double);
     cudaError_t e = cudaMalloc(&A->slab, bytes);
@@ -1002,7 +1004,7 @@ int adj_setup(fvm_ctx *c)
                        &a.lSe, &a.lSeV, &a.lPf, &a.g, &a.mu, &a.XD, &a.lUh, &a.lVh, &a.lSU, &a.lSUV, &a.lFE,
                        &a.lFW, &a.lFN, &a.lFS};
     for (auto q : full) *q = take(n);
-    double **perj[] = {&a.lUFW, &a.lVFW, &a.lFFU, &a.lFFV, &a.lblow, &a.DCU, &a.DCV, &a.DCP};
+    double **perj[] = {&a.lUFW, &a.lVFW, &a.lFFU, &a.lFFV, &a.lblow, &a.DCU, &a.DCV, &a.DCP, &a.ST0, &a.CT0};
     for (auto q : perj) *q = take(nj1);
     a.lomega = take(2);
     a.DCW = take(2);
@@ -1283,7 +1285,7 @@ int adj_zero(fvm_ctx *c)
 int adj_controls(fvm_ctx *c, double *dJ_domega, double *dJ_dblow)
 {
     fvm_adj *A = c->adj;
-    k_adj_controls<<<(c->NJ + 127) / 128, 128, 0, c->stream>>>(c->d, A->a, A->ctrl);
+    k_adj_controls<<<1, 512, 0, c->stream>>>(c->d, A->a, A->ctrl);   // NJ-1 <= 512
     FVM_LAUNCH_CHECK(c);
     std::vector<double> h(c->NJ + 1);
     FVM_CUDA(c, cudaMemcpyAsync(h.data(), A->ctrl, sizeof(double) * c->NJ, cudaMemcpyDeviceToHost, c->stream));
@@ -1393,8 +1395,8 @@ int run_adjoint_vjp(fvm_ctx *c, double *const *lam, double *dctrl)
     const Adj &a = A->a;
     const size_t n = c->n, bytes = sizeof(double) * n;
     if (!A->fin) FVM_CUDA(c, cudaMalloc(&A->fin, sizeof(double) * 7 * n));
-    double *ub = nullptr;
-    FVM_CUDA(c, cudaMalloc(&ub, 2 * bytes));
+    if (!A->one) FVM_CUDA(c, cudaMalloc(&A->one, 2 * bytes));
+    double *ub = A->one;
     int rc = FVM_OK;
     do {
         if ((rc = state_copy(c, A->fin, true))) break;
@@ -1415,7 +1417,6 @@ int run_adjoint_vjp(fvm_ctx *c, double *const *lam, double *dctrl)
         rc = state_copy(c, A->fin, false);
     } while (false);
     cudaStreamSynchronize(c->stream);
-    cudaFree(ub);
     return rc;
 }
 
@@ -1428,6 +1429,7 @@ void adj_destroy(fvm_ctx *c)
     if (A->ckpt) cudaFree(A->ckpt);
     if (A->base) cudaFree(A->base);
     if (A->fin) cudaFree(A->fin);
+    if (A->one) cudaFree(A->one);
     if (A->h_pctl) cudaFreeHost(A->h_pctl);
     delete A;
     c->adj = nullptr;
