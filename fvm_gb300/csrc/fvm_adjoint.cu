@@ -49,6 +49,10 @@ struct Adj {
     double *DCU, *DCV, *DCP;                 // dCd/dU(1,j), dCd/dV(1,j), dCd/dP(1,j)
     double *DCW;                             // [0]: dCd/d(omega) through the drag formula
     double *ST0, *CT0;                       // sine and cosine of THETA(0,j)
+    // nine split planes of the transposed equation's residual for the one-launch mixed
+    // iteration: AE, AW, AN, AS, AP, then the cross weights of (i,j), (i,j+2), (i+2,j),
+    // (i+2,j+2) -- at i = 1, whose first two vanish, those of (2,j) and (2,j+2) there
+    float2 *PC;
     Coef cPT, cXT, cYT;                      // transposed coefficient sets (Poisson, first, second factor)
     LineSys sPT, sXT, sYT;                   // their line factors
     PCtl *pctl;                              // adjoint Poisson iteration control
@@ -793,6 +797,29 @@ __global__ void k_adj_coef_f32(Dev d, Coef cf)
     cf.ASf[c] = (float)cf.AS[c];
 }
 
+// Adj::PC (positional cross term; the terms of xd_at gathered per cell).
+__global__ void k_adj_planes(Dev d, Adj a)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1, n = d.NI - 1, L = d.NJ - 1;
+    if (i > n || j > L) return;
+    const int c = IDX(i, j), y = j == L ? 1 : j + 1;   // line NJ-1 reads line 2 through the ghost row
+    const bool up = j != L - 1, dn = j > 1, ea = i + 2 <= n;
+    double w[4] = {0.0, 0.0, dn && ea ? d.CNW[IDX(i + 1, j - 1)] : 0.0, up && ea ? d.CSW[IDX(i + 1, y)] : 0.0};
+    if (i > 1) {
+        w[0] = dn ? d.CNE[IDX(i - 1, j - 1)] : 0.0;
+        w[1] = up ? d.CSE[IDX(i - 1, y)] : 0.0;
+    } else if (n > 1) {   // the wall ghost's share
+        w[0] = dn ? d.CNW[IDX(1, j - 1)] : 0.0;
+        w[1] = up ? d.CSW[IDX(1, y)] : 0.0;
+    }
+    const double v[9] = {a.cPT.AE[c], a.cPT.AW[c], a.cPT.AN[c], a.cPT.AS[c], a.cPT.AP[c], w[0], w[1], w[2], w[3]};
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        const dd q = dd_split(v[k]);
+        a.PC[size_t(k) * d.n + c] = make_float2(q.hi, q.lo);
+    }
+}
+
 __global__ void k_adj_pctl_reset(Adj a)
 {
     a.pctl->niter = 0;
@@ -980,7 +1007,7 @@ int adj_setup(fvm_ctx *c)
         return (6 * cnt + 2 * s.lines) * sizeof(double) + 16 * 256;
     };
     // per transposed set: AP, AE, AW, AN, AS (FP64) and ANf, ASf (FP32)
-    size_t bytes = (30 * n + 12 * nj1 + 16) * sizeof(double) + 3 * (6 * n * sizeof(double) + 8 * 256) +
+    size_t bytes = ((c->res_loop ? 39 : 30) * n + 12 * nj1 + 16) * sizeof(double) + 3 * (6 * n * sizeof(double) + 8 * 256) +
                    sys_bytes(d.sP) + sys_bytes(d.sUX) + sys_bytes(d.sUY) + 64 * 256 + sizeof(PCtl) +
                    2 * size_t(c->nblk_res) * sizeof(double);
     cudaError_t e = cudaMalloc(&A->slab, bytes);
@@ -1006,6 +1033,7 @@ int adj_setup(fvm_ctx *c)
     for (auto q : full) *q = take(n);
     double **perj[] = {&a.lUFW, &a.lVFW, &a.lFFU, &a.lFFV, &a.lblow, &a.DCU, &a.DCV, &a.DCP, &a.ST0, &a.CT0};
     for (auto q : perj) *q = take(nj1);
+    a.PC = c->res_loop ? reinterpret_cast<float2 *>(take(9 * n)) : nullptr;
     a.lomega = take(2);
     a.DCW = take(2);
     A->ctrl = take(nj1);
@@ -1035,6 +1063,7 @@ int adj_setup(fvm_ctx *c)
     k_adj_factor<<<(a.sXT.lines + 63) / 64, 64, 0, c->stream>>>(d, a.cXT, a.sXT, 0);
     k_adj_factor<<<(a.sYT.lines + 63) / 64, 64, 0, c->stream>>>(d, a.cYT, a.sYT, 1);
     k_adj_dragcoef<<<(c->NJ + 127) / 128, 128, 0, c->stream>>>(d, a);
+    if (a.PC) k_adj_planes<<<igrid(c), 128, 0, c->stream>>>(d, a);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
@@ -1046,6 +1075,13 @@ int adj_setup(fvm_ctx *c)
     }
     c->adj = A;
     return FVM_OK;
+}
+
+// The transposed Poisson correction of the mixed path.
+ResSys adj_sys(const fvm_ctx *c)
+{
+    const Adj &a = c->adj->a;
+    return ResSys{a.sPT.invDf, a.sPT.faf, a.sPT.fbf, a.cPT.ANf, a.cPT.ASf, c->d.RF, c->d.DF, a.mu, a.pctl, 0, 0, a.PC, a.g};
 }
 
 // Adjoint Poisson loop body: `groups` x (res_every x [cross term, colour 0,
@@ -1064,7 +1100,7 @@ int adj_poisson_graph(fvm_ctx *c)
     bool ok = true;
     // the transposed FP32 correction: in the forward solve's resident kernel when the
     // context uses it (its transposed factors share the forward tile), else per colour
-    const ResSys sys{a.sPT.invDf, a.sPT.faf, a.sPT.fbf, a.cPT.ANf, a.cPT.ASf, d.RF, d.DF, a.mu, a.pctl, 0};
+    const ResSys sys = adj_sys(c);
     for (int q = 0; q < groups && ok && mixed && c->res_lines; q++) {
         k_adj_mres<<<c->nblk_res, 256, 0, c->stream>>>(d, a, c->p.resimax, c->d.nswpp);
         int rc = resident_sweeps_on(c, sys, per, 1, 1);
@@ -1116,11 +1152,12 @@ int adj_poisson(fvm_ctx *c)
 {
     fvm_adj *A = c->adj;
     const Adj &a = A->a;
-    const bool ring = c->ring_blocks != 0;   // FP64: the whole iteration in one launch
+    const bool ring = c->ring_blocks != 0 || a.PC;   // the whole iteration in one launch
     if (!ring) ARC(adj_poisson_graph(c));
     k_adj_pctl_reset<<<1, 1, 0, c->stream>>>(a);
     if (ring) {
-        ARC(ring_launch_adjoint(c, RingSys{a.sPT.invD, a.sPT.fa, a.sPT.fb, a.cPT.AN, a.cPT.AS, a.cPT.AE, a.cPT.AW, a.cPT.AP, a.g,
+        if (a.PC) ARC(resident_loop_adjoint(c, adj_sys(c)));
+        else ARC(ring_launch_adjoint(c, RingSys{a.sPT.invD, a.sPT.fa, a.sPT.fb, a.cPT.AN, a.cPT.AS, a.cPT.AE, a.cPT.AW, a.cPT.AP, a.g,
                                            a.mu, a.pctl, 4}));
         FVM_CUDA(c, cudaMemcpyAsync(A->h_pctl, a.pctl, sizeof(PCtl), cudaMemcpyDeviceToHost, c->stream));
         FVM_CUDA(c, cudaStreamSynchronize(c->stream));

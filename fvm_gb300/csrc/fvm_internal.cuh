@@ -307,6 +307,9 @@ struct ResSys {
     // 1: the launch first sums the block partials the forward residual kernel left
     // and takes the loop's convergence decision (forward Poisson loop only)
     int decide;
+    // the whole iteration in one launch: split planes of the residual's coefficients, source
+    const float2 *PC;
+    const double *SRC;
 };
 int resident_setup(fvm_ctx *c);
 // the same launch on another system (the adjoint's transposed Poisson equation)
@@ -314,6 +317,7 @@ int resident_sweeps_on(fvm_ctx *c, const ResSys &sys, int sweeps, int apply, int
 int resident_sweeps(const Tgt &t, int sweeps, int apply, int max_polls, unsigned tag_skew,
                     cudaGraphConditionalHandle cond, int has_cond, int check_done, int decide = 0);
 int resident_loop(fvm_ctx *c);   // the whole forward iteration (c->res_loop)
+int resident_loop_adjoint(fvm_ctx *c, const ResSys &sys);   // the same of the transposed equation
 int resident_reset(fvm_ctx *c);
 size_t exchange_words(const fvm_ctx *c);   // 64-bit words of d.XW
 // mixed Poisson iteration of a batch, one cluster per case (fvm_cluster.cu)

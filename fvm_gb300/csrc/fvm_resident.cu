@@ -283,6 +283,10 @@ __global__ void __launch_bounds__(ResLayout<M, NW>::MAXT, 1)
 // between two slots of their own; a slot is rewritten two intervals later, after a
 // decision that every reader has contributed to.
 //
+// LOOP = 2: the adjoint's transposed equation (fvm_adjoint.cu).  Its cross term reads rows j
+// and j+2, columns i and i+2 (at i = 1 column 2) and no ghosts, so the pressure-like
+// unknown is kept for lines j0-1 .. j0+5.
+//
 // Bound: the serial chain of the four half-sweeps of a pair, each a line solve (two scans
 // over two warps) between block barriers, and one exchange (0.41 us one way).  The solve
 // keeps its scans' constant products in registers (group_apply_c): half the shuffles, and
@@ -440,25 +444,26 @@ __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
         float2 *ps = reinterpret_cast<float2 *>(P + size_t(PL) * PW);        // [PL + 1][PW]: split, and ghost row 0
         float *rfs = reinterpret_cast<float *>(ps + size_t(PL + 1) * PW);    // [B][LW]: own residual, words as in rows
         double *s_ab = s_sum + 2 * MRES_MAX_GROUPS;
-        const int pl = w - 1;   // P line of the group (rows 1 .. 7)
+        constexpr int ADJ = LOOP == 2 ? 1 : 0;
+        const int pl = w - 1 - ADJ;   // P line of the group (rows 1 .. 7; ADJ: 2 .. 8)
         unsigned long long *psum = d.XW + size_t(6) * L * LW;
         auto split = [](double x) {
             const dd q = dd_split(x);
             return make_float2(q.hi, q.lo);
         };
-        if (pl < PL) {
+        if (pl >= 0 && pl < PL) {
 #pragma unroll
             for (int k = 0; k < M; k++) {
                 const int e = t * M + k;
                 if (e < n) {
-                    const double x = d.P[IDX(e + 1, j)];
+                    const double x = sys.X[IDX(e + 1, j)];
                     P[pl * PW + e + 1] = x;
                     ps[pl * PW + e + 1] = split(x);
                 }
             }
-            if (t == 0) ps[pl * PW] = split(d.P[IDX(0, j)]);
-        } else if (pl == PL && j0 == 1) {
-            for (int i = t; i < PW; i += TG) ps[PL * PW + i] = split(d.P[IDX(i, 0)]);
+            if (t == 0) ps[pl * PW] = split(sys.X[IDX(0, j)]);
+        } else if (!ADJ && pl == PL && j0 == 1) {
+            for (int i = t; i < PW; i += TG) ps[PL * PW + i] = split(sys.X[IDX(i, 0)]);
         }
         __syncthreads();
         const int wid = threadIdx.x / WARP, lane = threadIdx.x & (WARP - 1);
@@ -470,17 +475,33 @@ __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
             // residual of the own lines: one warp per line and 32 cells
             for (int task = wid; task < B * nt; task += Lay::NT / WARP) {
                 const int q = task & (B - 1), col = task / B, i = col * WARP + lane + 1, jq = j0 + q;
-                const bool inside = i <= n, has_cross = inside && i > 1 && jq > 1;
-                const int c = inside ? IDX(i, jq) : 0, cc = has_cross ? IDX(i - 1, jq - 1) : 0;
+                const bool inside = i <= n, has_cross = ADJ ? inside : inside && i > 1 && jq > 1;
+                const int c = inside ? IDX(i, jq) : 0, cc = ADJ ? c : (has_cross ? IDX(i - 1, jq - 1) : 0);
                 float2 cf[9];
 #pragma unroll
                 for (int k = 0; k < 9; k++) {
                     const bool ok = k < 5 ? inside : has_cross;
-                    cf[k] = ok ? d.PCD[size_t(k) * d.n + (k < 5 ? c : cc)] : make_float2(0.0f, 0.0f);
+                    cf[k] = ok ? sys.PC[size_t(k) * d.n + (k < 5 ? c : cc)] : make_float2(0.0f, 0.0f);
                 }
                 float raf = 0.0f, paf = 0.0f;
-                if (inside) {
-                    const double divdt = d.DIVDT[c];
+                if (ADJ && inside) {
+                    const float2 *r0 = ps + (q + 1) * PW, *rp = r0 + 2 * PW, none = make_float2(0.0f, 0.0f);
+                    auto at = [](float2 x) { return dd(x.x, x.y); };
+                    auto co = [&](int k) { return at(cf[k]); };
+                    const int i1 = i == 1 ? 2 : i;   // the planes of cell 1 hold its column-2 weights
+                    const bool in1 = i1 <= n, in2 = i + 2 <= n;
+                    const dd cross = ((co(5) * at(in1 ? r0[i1] : none) + co(6) * at(in1 ? rp[i1] : none)) +
+                                      co(7) * at(in2 ? r0[i + 2] : none)) + co(8) * at(in2 ? rp[i + 2] : none);
+                    const dd app = co(4) * at(r0[i]);
+                    const dd am = (((app - co(0) * at(i < n ? r0[i + 1] : none)) - co(1) * at(r0[i - 1])) - co(2) * at(r0[PW + i])) -
+                                  co(3) * at((r0 - PW)[i]);
+                    const dd r = (dd_split(sys.SRC[c]) - cross) - am;
+                    raf = fabsf(r.hi);
+                    paf = fabsf(app.hi);
+                    const int e = i - 1;
+                    rfs[q * LW + (e % M) * TG + e / M] = r.hi;
+                } else if (inside) {
+                    const double divdt = sys.SRC[c];
                     const float2 *r0 = ps + (q + 2) * PW, *rm = r0 - 2 * PW;
                     if (q == 1 && j0 == 1) rm = ps + PL * PW;   // line 2: the ghost row
                     auto at = [](float2 x) { return dd(x.x, x.y); };
@@ -541,17 +562,17 @@ __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
             __syncthreads();
             mres_ratio(s_sum, nb, s_ab, s_ab + 2);
             if (s_fault) { bad = true; break; }
-            resip = s_ab[2];
+            resip = ADJ && !(s_ab[1] > 0.0) ? 0.0 : s_ab[2];
             if (it > 0 && !(resip > d.resimax && it < d.nswpp)) break;
             if (!sweeps(cnt)) { bad = true; break; }
             cnt += unsigned(S);
             it += S;
             // corrections: own lines, and the neighbours' three
             unsigned long long *fw = loop_words(d, 0, round & 1, L, LW);
-            if (own && w != 4) post(fw + size_t(j - 1) * LW, cnt);
-            if (w <= 2 || w == B + 3)
+            if (own && w != (ADJ ? 5 : 4)) post(fw + size_t(j - 1) * LW, cnt);
+            if (pl >= 0 && pl < PL && !own)
                 poll(fw + size_t(j - 1) * LW, cnt, [&](int k, float x) { v[k] = x; });
-            if (pl < PL) {
+            if (pl >= 0 && pl < PL) {
 #pragma unroll
                 for (int k = 0; k < M; k++) {
                     const int e = t * M + k;
@@ -560,8 +581,8 @@ __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
                         P[pl * PW + e + 1] = x;
                         const float2 q = split(x);
                         ps[pl * PW + e + 1] = q;
-                        if (e == 0) ps[pl * PW] = q;
-                        if (j0 == 1 && w == 2) {   // line NJ-1: the ghost row 0
+                        if (!ADJ && e == 0) ps[pl * PW] = q;
+                        if (!ADJ && j0 == 1 && w == 2) {   // line NJ-1: the ghost row 0
                             ps[PL * PW + e + 1] = q;
                             if (e == 0) ps[PL * PW] = q;
                         }
@@ -573,8 +594,8 @@ __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
         }
         if (bad) {   // a wait ran out: end the loop, leave P alone
             if (threadIdx.x == 0) {
-                d.pctl->fault = 1;
-                d.pctl->done = 1;
+                sys.pctl->fault = 1;
+                sys.pctl->done = 1;
             }
             return;
         }
@@ -582,16 +603,16 @@ __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
 #pragma unroll
             for (int k = 0; k < M; k++) {
                 const int e = t * M + k;
-                if (e < n) d.P[IDX(e + 1, j)] = P[pl * PW + e + 1];
+                if (e < n) sys.X[IDX(e + 1, j)] = P[pl * PW + e + 1];
             }
         }
         if (threadIdx.x == 0) {
             d.XCNT[blockIdx.x] = cnt + 2u;   // past the last residual's tag
             if (blockIdx.x == 0) {
-                d.pctl->niter = it;
-                d.pctl->resip = resip;
-                d.pctl->capped = resip > d.resimax ? 1 : 0;
-                d.pctl->done = 1;
+                sys.pctl->niter = it;
+                sys.pctl->resip = resip;
+                sys.pctl->capped = resip > d.resimax ? 1 : 0;
+                sys.pctl->done = 1;
             }
         }
         return;
@@ -738,11 +759,13 @@ int resident_setup(fvm_ctx *c)
                 auto k0 = k_pois32_resident2<M_, NW_, 0, 0>;
                 auto k1 = k_pois32_resident2<M_, NW_, 1, 0>;
                 auto kl = k_pois32_resident2<M_, NW_, 0, 1>;
+                auto ka = k_pois32_resident2<M_, NW_, 0, 2>;
                 const int n = WARP * NW_ * M_, most = (int)Lay::bytes(n, false), most_l = (int)Lay::bytes(n, true);
                 int per_sm = 0, per_sm_l = 0;
                 e = cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
                 if (e == cudaSuccess) e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
                 if (e == cudaSuccess) e = cudaFuncSetAttribute(kl, cudaFuncAttributeMaxDynamicSharedMemorySize, most_l);
+                if (e == cudaSuccess) e = cudaFuncSetAttribute(ka, cudaFuncAttributeMaxDynamicSharedMemorySize, most_l);
                 if (e == cudaSuccess)
                     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k1, Lay::NT, Lay::bytes(s.n, false));
                 if (e == cudaSuccess)
@@ -769,7 +792,7 @@ namespace {
 ResSys forward_sys(const fvm_ctx *c)
 {
     const Dev &d = c->d;
-    return ResSys{d.sP.invDf, d.sP.faf, d.sP.fbf, d.cP.ANf, d.cP.ASf, d.RF, d.DF, d.P, d.pctl, 1, 0};
+    return ResSys{d.sP.invDf, d.sP.faf, d.sP.fbf, d.cP.ANf, d.cP.ASf, d.RF, d.DF, d.P, d.pctl, 1, 0, d.PCD, d.DIVDT};
 }
 
 int launch_sys(fvm_ctx *c, const ResSys &sys, cudaStream_t st, int sweeps, int apply, int max_polls,
@@ -814,15 +837,15 @@ int resident_sweeps(const Tgt &t, int sweeps, int apply, int max_polls, unsigned
     return launch_sys(t.c, sys, t.st, sweeps, apply, max_polls, tag_skew, cond, has_cond, check_done);
 }
 
-// The whole forward iteration of a step whose source is in place.
-int resident_loop(fvm_ctx *c)
+namespace {
+template <int LOOP>
+int launch_loop(fvm_ctx *c, const ResSys &sys)
 {
     cudaError_t e = cudaErrorInvalidValue;
-    const ResSys sys = forward_sys(c);
     dispatch_line(c->d.sP, [&](auto m, auto nw) {
         constexpr int M_ = decltype(m)::value, NW_ = decltype(nw)::value;
         if constexpr (NW_ <= 2)
-            e = launch_resident2<M_, NW_, 0, 1>(c, sys, c->stream, c->d.refine_sweeps, 0, 0, kResidentPolls, 0u, 0);
+            e = launch_resident2<M_, NW_, 0, LOOP>(c, sys, c->stream, c->d.refine_sweeps, 0, 0, kResidentPolls, 0u, 0);
     });
     if (e != cudaSuccess) {
         c->err = std::string("resident Poisson loop launch: ") + cudaGetErrorString(e);
@@ -831,6 +854,12 @@ int resident_loop(fvm_ctx *c)
     KCOUNT(c);
     return FVM_OK;
 }
+}  // namespace
+
+// The whole iteration whose source is in place: the forward pressure, and another system
+// of the context's line tile with the transposed cross term.
+int resident_loop(fvm_ctx *c) { return launch_loop<1>(c, forward_sys(c)); }
+int resident_loop_adjoint(fvm_ctx *c, const ResSys &sys) { return launch_loop<2>(c, sys); }
 
 // The same sweeps on another system of the context's line tile (the adjoint's
 // transposed Poisson equation); no graph condition, default wait bound.

@@ -70,3 +70,29 @@ def test_loop_and_adjoint_share_the_exchange_words():
         ctx.adjoint_vjp(lam)
         ctx.step(2)
     assert np.array_equal(a.get("P"), b.get("P")) and np.array_equal(a.get("U"), b.get("U"))
+
+
+# theta lines, radial cells, tile, sweeps per interval, cap, tolerance of the iteration
+ADJOINT = [(12, 5, (1, 1), 2, 6, 0.0), (40, 64, (2, 1), 4, 12, 0.0), (100, 97, (1, 4), 6, 18, 0.0),
+           (64, 380, (1, 12), 8, 16, 0.0), (512, 510, (2, 8), 2, 4, 0.0), (64, 48, (1, 2), 4, 400, 1e-3)]
+
+
+@pytest.mark.parametrize("n_theta,n_r,tile,refine,cap,resimax", ADJOINT)
+def test_transposed_loop_equals_per_colour_kernels(n_theta, n_r, tile, refine, cap, resimax):
+    """The transposed iteration in one launch: the cross term is summed in another order
+    (1e-14 of it), which moves an FP32 residual by 2^-24 at most now and then: below 1e-6
+    of each array, at the same interval of the iteration."""
+    case = make_case(n_theta=n_theta, n_r=n_r, skew=0.3, vel_rot=0.2, nswpp=cap, resimax=resimax)
+    names = ("U", "V", "P", "NLX", "NLY")
+    out = []
+    for resident in (1, 0):
+        ctx = make_gpu(case, precision=capi.MIXED, refine_sweeps=refine, poisson_resident=resident, tile_r_warps=tile[0],
+                       tile_r_m=tile[1])
+        ctx.step(2)
+        rng = np.random.default_rng(11)
+        out.append(ctx.adjoint_vjp({nm: rng.standard_normal(ctx.get("U").shape) for nm in names}))
+        ctx.close()
+    (x, wx, bx), (y, wy, by) = out
+    for nm in names:
+        assert np.isfinite(x[nm]).all() and np.linalg.norm(x[nm] - y[nm]) <= 1e-6 * np.linalg.norm(y[nm]), nm
+    assert abs(wx - wy) <= 1e-6 * max(abs(wy), 1.0) and np.linalg.norm(bx - by) <= 1e-6 * np.linalg.norm(by)
