@@ -48,7 +48,6 @@ struct Adj {
     double *lomega;                          // [0]: rotation adjoint through the drag formula
     double *DCU, *DCV, *DCP;                 // dCd/dU(1,j), dCd/dV(1,j), dCd/dP(1,j)
     double *DCW;                             // [0]: dCd/d(omega) through the drag formula
-    double *ST0, *CT0;                       // sine and cosine of THETA(0,j)
     // nine split planes of the transposed equation's residual for the one-launch mixed
     // iteration: AE, AW, AN, AS, AP, then the cross weights of (i,j), (i,j+2), (i+2,j),
     // (i+2,j+2) -- at i = 1, whose first two vanish, those of (2,j) and (2,j+2) there
@@ -95,8 +94,6 @@ __global__ void k_adj_dragcoef(Dev d, Adj a)
 {
     int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
     if (j > d.NJ - 1) return;
-    a.ST0[j] = sin(d.THETA[IDX(0, j)]);
-    a.CT0[j] = cos(d.THETA[IDX(0, j)]);
     double DN1, TH2;
     wall_normal(d, j, DN1, TH2);
     const int c = IDX(1, j);
@@ -836,11 +833,12 @@ __global__ void k_adj_pctl_reset(Adj a)
 __global__ void __launch_bounds__(512) k_adj_controls(Dev d, Adj a, double *out)
 {
     __shared__ double sh[64];
-    const int j = threadIdx.x + 1;
     double s = 0.0, none = 0.0;
-    if (j <= d.NJ - 1) {
-        const double st = a.ST0[j], ct = a.CT0[j], u = a.lUFW[j], v = a.lVFW[j];
-        s = -st * u + ct * v;
+    for (int j = threadIdx.x + 1; j <= d.NJ - 1; j += 512) {
+        double st, ct;
+        sincos(d.THETA[IDX(0, j)], &st, &ct);
+        const double u = a.lUFW[j], v = a.lVFW[j];
+        s += -st * u + ct * v;
         out[j] = (ct * u + st * v) + a.lblow[j];
     }
     block_sum2(s, none, sh);
@@ -1007,7 +1005,7 @@ int adj_setup(fvm_ctx *c)
         return (6 * cnt + 2 * s.lines) * sizeof(double) + 16 * 256;
     };
     // per transposed set: AP, AE, AW, AN, AS (FP64) and ANf, ASf (FP32)
-    size_t bytes = ((c->res_loop ? 39 : 30) * n + 12 * nj1 + 16) * sizeof(double) + 3 * (6 * n * sizeof(double) + 8 * 256) +
+    size_t bytes = ((c->res_loop ? 39 : 30) * n + 10 * nj1 + 16) * sizeof(double) + 3 * (6 * n * sizeof(double) + 8 * 256) +
                    sys_bytes(d.sP) + sys_bytes(d.sUX) + sys_bytes(d.sUY) + 64 * 256 + sizeof(PCtl) +
                    2 * size_t(c->nblk_res) * sizeof(double);
     cudaError_t e = cudaMalloc(&A->slab, bytes);
@@ -1031,7 +1029,7 @@ int adj_setup(fvm_ctx *c)
                        &a.lSe, &a.lSeV, &a.lPf, &a.g, &a.mu, &a.XD, &a.lUh, &a.lVh, &a.lSU, &a.lSUV, &a.lFE,
                        &a.lFW, &a.lFN, &a.lFS};
     for (auto q : full) *q = take(n);
-    double **perj[] = {&a.lUFW, &a.lVFW, &a.lFFU, &a.lFFV, &a.lblow, &a.DCU, &a.DCV, &a.DCP, &a.ST0, &a.CT0};
+    double **perj[] = {&a.lUFW, &a.lVFW, &a.lFFU, &a.lFFV, &a.lblow, &a.DCU, &a.DCV, &a.DCP};
     for (auto q : perj) *q = take(nj1);
     a.PC = c->res_loop ? reinterpret_cast<float2 *>(take(9 * n)) : nullptr;
     a.lomega = take(2);
@@ -1322,7 +1320,7 @@ int adj_zero(fvm_ctx *c)
 int adj_controls(fvm_ctx *c, double *dJ_domega, double *dJ_dblow)
 {
     fvm_adj *A = c->adj;
-    k_adj_controls<<<1, 512, 0, c->stream>>>(c->d, A->a, A->ctrl);   // NJ-1 <= 512
+    k_adj_controls<<<1, 512, 0, c->stream>>>(c->d, A->a, A->ctrl);
     FVM_LAUNCH_CHECK(c);
     std::vector<double> h(c->NJ + 1);
     FVM_CUDA(c, cudaMemcpyAsync(h.data(), A->ctrl, sizeof(double) * c->NJ, cudaMemcpyDeviceToHost, c->stream));
