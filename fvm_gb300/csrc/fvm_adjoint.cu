@@ -39,7 +39,7 @@ struct Adj {
     double *lUn, *lVn;                       // accumulators of the adjoint of U^n, V^n (full arrays)
     double *lW, *lWV;                        // interior scratch (ghost-map transposes)
     double *lSc, *lScV, *lSe, *lSeV;         // S_U/S_V adjoints of the correction and of the explicit phase
-    double *lPf, *g, *mu, *XD;               // Poisson adjoint: source, solution, lagged cross term
+    double *g, *mu, *XD;                     // Poisson adjoint: source, solution, lagged cross term
     double *lUh, *lVh;                       // adjoint of u-hat, v-hat (full arrays)
     double *lSU, *lSUV;                      // predictor right-hand side adjoints
     double *lFE, *lFW, *lFN, *lFS;           // face flux adjoints (UE, UW, VN, VS)
@@ -59,6 +59,15 @@ struct Adj {
 };
 
 namespace {
+
+// One array per velocity component.  The transposed operators of U and V are independent of
+// each other and share a launch, the component along z (y for line kernels): a launch of
+// one component fills a fraction of the chip and lasts as long (per step of 128 x 96:
+// 48 launches fewer, the transposed step 1190 -> 960 us).
+struct Two {
+    double *u, *v;
+    __device__ double *operator[](int k) const { return k ? v : u; }
+};
 
 // ---------------------------------------------------------------------------------
 // Geometry of the drag formula (calccoef.f90:50-98 as in k_wall_geom): wall-normal
@@ -125,10 +134,11 @@ __global__ void k_adj_coef_t(Dev d, Coef src, Coef dst)
 // Dirichlet ghost map of BCU/BCV as ghost_dirichlet writes it from the interior
 // values w: phi(0,j) = -w(1,j) + 2 wallF(j), phi(NI,j) = -w(NI-1,j) + 2 farF(j),
 // phi(i,0) = w(i,NJ-1), phi(i,NJ) = w(i,1), corners from the cells (1|NI-1, 1|NJ-1).
-// Folds the adjoint of the whole array lphi into the interior adjoint out (added),
-// the wall / far-field value adjoints, and clears lphi's ghosts.
-__global__ void k_adj_gd(Dev d, double *lphi, double *out, double *lwall, double *lfar, int overwrite)
+// Folds the adjoint of the whole array lphi into the interior adjoint out and the
+// wall / far-field value adjoints (added).
+__global__ void k_adj_gd(Dev d, Two phi, Two outs, Two walls, Two fars)
 {
+    double *lphi = phi[blockIdx.z], *out = outs[blockIdx.z], *lwall = walls[blockIdx.z], *lfar = fars[blockIdx.z];
     int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1;
     const int NI = d.NI, NJ = d.NJ;
     if (i > NI - 1 || j > NJ - 1) return;
@@ -149,12 +159,13 @@ __global__ void k_adj_gd(Dev d, double *lphi, double *out, double *lwall, double
         s -= g;
         lfar[j] += 2.0 * g;
     }
-    out[IDX(i, j)] = overwrite ? s : out[IDX(i, j)] + s;
+    out[IDX(i, j)] = s;
 }
 
 // Clear the ghost cells of a full array (after their adjoint has been folded).
-__global__ void k_adj_clear_ghosts(Dev d, double *a)
+__global__ void k_adj_clear_ghosts(Dev d, Two arr)
 {
+    double *a = arr[blockIdx.z];
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int NI = d.NI, NJ = d.NJ;
     if (t <= NJ) {
@@ -301,8 +312,10 @@ __device__ __forceinline__ void cross_scatter(const Dev &d, const double *K, dou
 
 // Second-factor right-hand side transposed (iter_u.f90:86-99 as k_af_su2):
 // SU2 = RJDT phi + cross(JYE, phi) + 2 awall wallF (i=1) + 2 afar farF (i=NI-1).
-__global__ void k_adj_su2(Dev d, const double *lsu, double *lphi, double *lwall, double *lfar)
+__global__ void k_adj_su2(Dev d, Two su, Two phi, Two walls, Two fars)
 {
+    const double *lsu = su[blockIdx.z];
+    double *lphi = phi[blockIdx.z], *lwall = walls[blockIdx.z], *lfar = fars[blockIdx.z];
     int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1;
     if (i > d.NI - 1 || j > d.NJ - 1) return;
     const int c = IDX(i, j);
@@ -321,55 +334,56 @@ __global__ void k_adj_su2(Dev d, const double *lsu, double *lphi, double *lwall,
 //   DIF = D-weighted differences + the cross term of cell (i-1,j-1) (positional)
 // lnl: adjoint of the NL computed in this step (in: from the next step, where it is
 // NL_nm1; out: the adjoint of this step's NL_nm1 input).  Scatters into lphi (the
-// adjoint of phi_n, full array), the flux adjoints, lS (S adjoint), wall/far values.
-__global__ void k_adj_explicit(Dev d, Adj a, const double *phin, const double *lsu, double *lnl, double *lphi,
-                               double *lS, double *lwall, double *lfar)
+// adjoint of phi_n, full array), the S adjoint, wall/far values; the flux adjoints are
+// the two components' sums, so one thread takes both components of its cell.
+__global__ void k_adj_explicit(Dev d, Adj a, const double *un, const double *vn)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1;
     if (i > d.NI - 1 || j > d.NJ - 1) return;
-    const int c = IDX(i, j);
-    const double L = lsu[c];
-    const double rek = d.re;
-    // right-hand side assembly
-    atomicAdd(&lphi[c], d.RJDT[c] * L);
-    const double lnew = lnl[c] - (3.0 * rek) * L;   // adjoint of this step's NL
-    lnl[c] = rek * L;                                // adjoint of NL_nm1 (the previous step's NL)
-    lS[c] += (2.0 * rek) * L;
-    cross_scatter(d, d.JXE, lphi, i, j, L);
-    if (i == 1) lwall[j] += (2.0 * d.cUX.awall[j]) * L;
-    if (i == d.NI - 1) lfar[j] += (2.0 * d.cUX.afar[j]) * L;
-    // DIF (orthogonal part and the cross term)
-    {
-        const int e = IDX(i + 1, j), w = IDX(i - 1, j), nn = IDX(i, j + 1), s = IDX(i, j - 1);
-        atomicAdd(&lphi[e], d.DE[c] * L);
-        atomicAdd(&lphi[w], d.DW[c] * L);
-        atomicAdd(&lphi[nn], d.DN[c] * L);
-        atomicAdd(&lphi[s], d.DS[c] * L);
-        atomicAdd(&lphi[c], -(((d.DE[c] + d.DW[c]) + d.DN[c]) + d.DS[c]) * L);
+    const int c = IDX(i, j), e = IDX(i + 1, j), w = IDX(i - 1, j), nn = IDX(i, j + 1), s = IDX(i, j - 1);
+    const double rek = d.re, de = d.DE[c], dw = d.DW[c], dn = d.DN[c], ds = d.DS[c];
+    const double ue = d.UE[c], uw = d.UW[c], vnf = d.VN[c], vsf = d.VS[c], rj = d.RJDT[c];
+    double fe = 0.0, fw = 0.0, fn = 0.0, fs = 0.0;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const double *phin = k ? vn : un;
+        double *lphi = k ? a.lVn : a.lUn, *lnl = k ? a.lNLY : a.lNLX, *lS = k ? a.lSeV : a.lSe;
+        const double L = (k ? a.lSUV : a.lSU)[c];
+        // right-hand side assembly
+        const double lnew = lnl[c] - (3.0 * rek) * L;   // adjoint of this step's NL
+        lnl[c] = rek * L;                                // adjoint of NL_nm1 (the previous step's NL)
+        lS[c] += (2.0 * rek) * L;
+        cross_scatter(d, d.JXE, lphi, i, j, L);
+        if (i == 1) (k ? a.lVFW : a.lUFW)[j] += (2.0 * d.cUX.awall[j]) * L;
+        if (i == d.NI - 1) (k ? a.lFFV : a.lFFU)[j] += (2.0 * d.cUX.afar[j]) * L;
         if (!d.dd_pos) cross_scatter(d, d.JQ12, lphi, i, j, L);
         else if (i > 1 && j > 1) cross_scatter(d, d.JQ12, lphi, i - 1, j - 1, L);
-    }
-    // NL (nl.f90:21-27): 0.5*UE(p_c+p_e) - 0.5*UW(p_c+p_w) + 0.5*VN(p_c+p_n) - 0.5*VS(p_c+p_s)
-    {
-        const int e = IDX(i + 1, j), w = IDX(i - 1, j), nn = IDX(i, j + 1), s = IDX(i, j - 1);
+        // DIF (orthogonal part) and NL (nl.f90:21-27): 0.5*UE(p_c+p_e) - 0.5*UW(p_c+p_w)
+        // + 0.5*VN(p_c+p_n) - 0.5*VS(p_c+p_s)
         const double h = 0.5 * lnew;
-        atomicAdd(&lphi[c], h * (((d.UE[c] - d.UW[c]) + d.VN[c]) - d.VS[c]));
-        atomicAdd(&lphi[e], h * d.UE[c]);
-        atomicAdd(&lphi[w], -h * d.UW[c]);
-        atomicAdd(&lphi[nn], h * d.VN[c]);
-        atomicAdd(&lphi[s], -h * d.VS[c]);
+        atomicAdd(&lphi[c], (rj * L - (((de + dw) + dn) + ds) * L) + h * (((ue - uw) + vnf) - vsf));
+        atomicAdd(&lphi[e], de * L + h * ue);
+        atomicAdd(&lphi[w], dw * L - h * uw);
+        atomicAdd(&lphi[nn], dn * L + h * vnf);
+        atomicAdd(&lphi[s], ds * L - h * vsf);
         const double pc = phin[c];
-        a.lFE[c] += h * (pc + phin[e]);
-        a.lFW[c] -= h * (pc + phin[w]);
-        a.lFN[c] += h * (pc + phin[nn]);
-        a.lFS[c] -= h * (pc + phin[s]);
+        fe += h * (pc + phin[e]);
+        fw -= h * (pc + phin[w]);
+        fn += h * (pc + phin[nn]);
+        fs -= h * (pc + phin[s]);
     }
+    a.lFE[c] = fe;
+    a.lFW[c] = fw;
+    a.lFN[c] = fn;
+    a.lFS[c] = fs;
 }
 
 // Far-field values transposed (bcu.f90:27-32 as k_farfield_step): outflow columns
 // f(j) = 0.5(q_NI + q_NI-1) - dt*uin*(a (q_NI - q_NI-1) + b dq), inflow constant.
-__global__ void k_adj_farfield(Dev d, const double *lfar, double *lq)
+__global__ void k_adj_farfield(Dev d, Two fars, Two qs)
 {
+    const double *lfar = fars[blockIdx.z];
+    double *lq = qs[blockIdx.z];
     int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
     if (j > d.NJ - 1) return;
     const int NI = d.NI;
@@ -391,8 +405,10 @@ __global__ void k_adj_farfield(Dev d, const double *lfar, double *lq)
 // Dirichlet ghosts of the pre-sweep field (refresh_row_ghosts with BCK_DIRICHLET),
 // i.e. k_adj_gd applied to the ghost part only, folded into the pre-sweep
 // interior accumulator.
-__global__ void k_adj_refresh(Dev d, double *lphi, double *lpre, double *lwall, double *lfar)
+__global__ void k_adj_refresh(Dev d, Two phi, Two pre, Two walls, Two fars)
 {
+    const double *lphi = phi[blockIdx.z];
+    double *lpre = pre[blockIdx.z], *lwall = walls[blockIdx.z], *lfar = fars[blockIdx.z];
     int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1;
     const int NI = d.NI, NJ = d.NJ;
     if (i > NI - 1 || j > NJ - 1) return;
@@ -417,8 +433,9 @@ __global__ void k_adj_refresh(Dev d, double *lphi, double *lpre, double *lwall, 
 }
 
 // out_int += in_int (interior), then in cleared (full array).
-__global__ void k_adj_add_interior(Dev d, double *out, double *in)
+__global__ void k_adj_add_interior(Dev d, Two outs, Two ins)
 {
+    double *out = outs[blockIdx.z], *in = ins[blockIdx.z];
     int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1;
     if (i > d.NI - 1 || j > d.NJ - 1) return;
     out[IDX(i, j)] += in[IDX(i, j)];
@@ -445,8 +462,9 @@ __global__ void k_adj_grad(Dev d, Adj a, const double *lw, const double *lwv, do
 // forward coupling coefficients, and the line's own adjoint is cleared.
 // ---------------------------------------------------------------------------------
 template <int M, int NW>
-__global__ void __launch_bounds__(128) k_adj_line_r(Dev d, LineSys s, Coef cf, double *lam, double *lrhs, int colour)
+__global__ void __launch_bounds__(128) k_adj_line_r(Dev d, LineSys s, Coef cf, Two lams, Two rhs, int colour)
 {
+    double *lam = lams[blockIdx.y], *lrhs = rhs[blockIdx.y];
     constexpr int TG = WARP * NW, G = 4 / NW;
     __shared__ double sm[G][TG * M + M * NW + 1];
     __shared__ double xch[G][2 * NW];
@@ -480,8 +498,9 @@ __global__ void __launch_bounds__(128) k_adj_line_r(Dev d, LineSys s, Coef cf, d
 }
 
 template <int M, int NW>
-__global__ void __launch_bounds__(128) k_adj_line_t(Dev d, LineSys s, Coef cf, double *lam, double *lrhs, int colour)
+__global__ void __launch_bounds__(128) k_adj_line_t(Dev d, LineSys s, Coef cf, Two lams, Two rhs, int colour)
 {
+    double *lam = lams[blockIdx.y], *lrhs = rhs[blockIdx.y];
     constexpr int TG = WARP * NW, G = 4 / NW;
     __shared__ double sm[G][TG * M + M * NW + 1];
     __shared__ double xch[G][2 * NW];
@@ -858,7 +877,6 @@ struct fvm_adj {
     double *ckpt = nullptr;              // checkpoints: nckpt x 7 full arrays
     double *base = nullptr;              // U, V before every step of a segment: seg x 2 full arrays
     double *fin = nullptr;               // state at the end of the window: 7 full arrays
-    double *one = nullptr;               // U, V before the step of run_adjoint_vjp
     int nckpt = 0, nseg_steps = 0;
     cudaGraphExec_t pgraph = nullptr;    // adjoint Poisson loop body
     int pgraph_iters = 0;
@@ -1025,14 +1043,16 @@ int adj_setup(fvm_ctx *c)
         return r;
     };
     Adj &a = A->a;
-    double **full[] = {&a.lU, &a.lV, &a.lP, &a.lNLX, &a.lNLY, &a.lUn, &a.lVn, &a.lW, &a.lWV, &a.lSc, &a.lScV,
-                       &a.lSe, &a.lSeV, &a.lPf, &a.g, &a.mu, &a.XD, &a.lUh, &a.lVh, &a.lSU, &a.lSUV, &a.lFE,
-                       &a.lFW, &a.lFN, &a.lFS};
+    // in the order in which adj_clear zeroes groups of them
+    double **full[] = {&a.lU, &a.lV, &a.lUn, &a.lVn, &a.lP, &a.lNLX, &a.lNLY, &a.mu, &a.lUh, &a.lVh, &a.lSe, &a.lSeV,
+                       &a.lSU, &a.lSUV, &a.lW, &a.lWV, &a.lSc, &a.lScV, &a.g, &a.XD, &a.lFE, &a.lFW, &a.lFN, &a.lFS};
     for (auto q : full) *q = take(n);
-    double **perj[] = {&a.lUFW, &a.lVFW, &a.lFFU, &a.lFFV, &a.lblow, &a.DCU, &a.DCV, &a.DCP};
+    double **perj[] = {&a.lFFU, &a.lFFV, &a.lUFW, &a.lVFW, &a.lblow};
     for (auto q : perj) *q = take(nj1);
-    a.PC = c->res_loop ? reinterpret_cast<float2 *>(take(9 * n)) : nullptr;
     a.lomega = take(2);
+    double **drag[] = {&a.DCU, &a.DCV, &a.DCP};
+    for (auto q : drag) *q = take(nj1);
+    a.PC = c->res_loop ? reinterpret_cast<float2 *>(take(9 * n)) : nullptr;
     a.DCW = take(2);
     A->ctrl = take(nj1);
     carve_coef_t(p, a.cPT, n);
@@ -1186,12 +1206,12 @@ int adj_poisson(fvm_ctx *c)
     return FVM_OK;
 }
 
-int line_r(fvm_ctx *c, const LineSys &sT, const Coef &cf, double *lam, double *lrhs, int colour)
+int line_r(fvm_ctx *c, const LineSys &sT, const Coef &cf, Two lam, Two lrhs, int colour)
 {
     const int blocks = line_blocks((c->NJ - 1) / 2, sT.NW);
     bool ok = dispatch_line(sT, [&](auto m, auto nw) {
         k_adj_line_r<decltype(m)::value, decltype(nw)::value>
-            <<<blocks, 128, 0, c->stream>>>(c->d, sT, cf, lam, lrhs, colour);
+            <<<dim3(blocks, 2), 128, 0, c->stream>>>(c->d, sT, cf, lam, lrhs, colour);
     });
     if (!ok) {
         c->err = "unsupported line length";
@@ -1201,12 +1221,12 @@ int line_r(fvm_ctx *c, const LineSys &sT, const Coef &cf, double *lam, double *l
     return FVM_OK;
 }
 
-int line_t(fvm_ctx *c, const LineSys &sT, const Coef &cf, double *lam, double *lrhs, int colour)
+int line_t(fvm_ctx *c, const LineSys &sT, const Coef &cf, Two lam, Two lrhs, int colour)
 {
     const int blocks = line_blocks((c->NI - 1 + 1 - colour) / 2, sT.NW);
     bool ok = dispatch_line(sT, [&](auto m, auto nw) {
         k_adj_line_t<decltype(m)::value, decltype(nw)::value>
-            <<<blocks, 128, 0, c->stream>>>(c->d, sT, cf, lam, lrhs, colour);
+            <<<dim3(blocks, 2), 128, 0, c->stream>>>(c->d, sT, cf, lam, lrhs, colour);
     });
     if (!ok) {
         c->err = "unsupported line length";
@@ -1216,105 +1236,95 @@ int line_t(fvm_ctx *c, const LineSys &sT, const Coef &cf, double *lam, double *l
     return FVM_OK;
 }
 
-// The predictor of one velocity component transposed: lam holds the adjoint of
+// Zero the arrays from `first` to `last` of the slab, neighbours in adj_setup's order.
+int adj_clear(fvm_ctx *c, double *first, double *last, size_t len)
+{
+    FVM_CUDA(c, cudaMemsetAsync(first, 0, (last + len - first) * sizeof(double), c->stream));
+    return FVM_OK;
+}
+
+// The predictors of the velocity components transposed: lam holds the adjoint of
 // u** (interior, ghosts zero) on entry; on exit lsu holds the adjoint of the
 // first-factor right-hand side and lpre has gained the adjoint of the pre-sweep
 // field (u^n as the sweeps' initial iterate and the source of their ghost rows).
-int adj_predictor(fvm_ctx *c, double *lam, double *lsu, double *lpre, double *lwall, double *lfar)
+int adj_predictor(fvm_ctx *c, Two lam, Two lsu, Two lpre, Two lwall, Two lfar)
 {
     fvm_adj *A = c->adj;
     const Adj &a = A->a;
     const Dev &d = c->d;
-    const size_t bytes = sizeof(double) * c->n;
-    FVM_CUDA(c, cudaMemsetAsync(lsu, 0, bytes, c->stream));
+    dim3 G = igrid(c);
+    G.z = 2;
+    ARC(adj_clear(c, lsu.u, lsu.v, c->n));
     ARC(line_t(c, a.sYT, d.cUY, lam, lsu, 1));
     ARC(line_t(c, a.sYT, d.cUY, lam, lsu, 0));
-    k_adj_su2<<<igrid(c), 128, 0, c->stream>>>(d, lsu, lam, lwall, lfar);
-    k_adj_refresh<<<igrid(c), 128, 0, c->stream>>>(d, lam, lpre, lwall, lfar);
-    k_adj_clear_ghosts<<<(std::max(c->NI, c->NJ) + 1 + 127) / 128, 128, 0, c->stream>>>(d, lam);
-    FVM_CUDA(c, cudaMemsetAsync(lsu, 0, bytes, c->stream));
+    k_adj_su2<<<G, 128, 0, c->stream>>>(d, lsu, lam, lwall, lfar);
+    k_adj_refresh<<<G, 128, 0, c->stream>>>(d, lam, lpre, lwall, lfar);
+    k_adj_clear_ghosts<<<dim3((std::max(c->NI, c->NJ) + 1 + 127) / 128, 1, 2), 128, 0, c->stream>>>(d, lam);
+    ARC(adj_clear(c, lsu.u, lsu.v, c->n));
     ARC(line_r(c, a.sXT, d.cUX, lam, lsu, 1));
     ARC(line_r(c, a.sXT, d.cUX, lam, lsu, 0));
-    k_adj_add_interior<<<igrid(c), 128, 0, c->stream>>>(d, lpre, lam);
+    k_adj_add_interior<<<G, 128, 0, c->stream>>>(d, lpre, lam);
     FVM_LAUNCH_CHECK(c);
     return FVM_OK;
 }
 
 // One step reversed.  On entry a.lU, lV, lP, lNLX, lNLY hold the adjoint of the
-// state after the step; ubase/vbase the U, V of the state before it (full arrays).
+// state after the step, on return that of the state before it; ubase/vbase the U, V of
+// the state before it (full arrays; d.U, d.V themselves or a copy that they are set to).
 // drag_scale: weight of this step's drag coefficient in the objective.
 int adj_step(fvm_ctx *c, const double *ubase, const double *vbase, double drag_scale)
 {
     fvm_adj *A = c->adj;
-    const Adj &a = A->a;
+    Adj &a = A->a;
     Dev &d = c->d;
     cudaStream_t st = c->stream;
-    const size_t bytes = sizeof(double) * c->n, jb = sizeof(double) * (c->NJ + 1);
-    const dim3 G = igrid(c);
+    const size_t n = c->n, bytes = sizeof(double) * n;
+    const dim3 G = igrid(c), G2(G.x, G.y, 2);
     const int rows = (c->NJ + 127) / 128;
-    FVM_CUDA(c, cudaMemsetAsync(a.lFFU, 0, jb, st));
-    FVM_CUDA(c, cudaMemsetAsync(a.lFFV, 0, jb, st));
+    const Two lW{a.lW, a.lWV}, wall{a.lUFW, a.lVFW}, far{a.lFFU, a.lFFV}, lam{a.lU, a.lV}, base{a.lUn, a.lVn};
+    ARC(adj_clear(c, a.lFFU, a.lFFV, c->NJ + 1));
     // CALCCOEF of the state after the step
     if (drag_scale != 0.0) k_adj_drag<<<rows, 128, 0, st>>>(d, a, drag_scale);
     // correction and BCU/BCV (Main.f90:97-107)
-    k_adj_gd<<<G, 128, 0, st>>>(d, a.lU, a.lW, a.lUFW, a.lFFU, 1);
-    k_adj_gd<<<G, 128, 0, st>>>(d, a.lV, a.lWV, a.lVFW, a.lFFV, 1);
-    FVM_CUDA(c, cudaMemsetAsync(a.lUh, 0, bytes, st));
-    FVM_CUDA(c, cudaMemsetAsync(a.lVh, 0, bytes, st));
+    k_adj_gd<<<G2, 128, 0, st>>>(d, lam, lW, wall, far);
+    ARC(adj_clear(c, a.lUh, a.lSeV, n));   // lUh, lVh, lSe, lSeV
     k_adj_correct<<<G, 128, 0, st>>>(d, a);
-    FVM_CUDA(c, cudaMemcpyAsync(a.lPf, a.lP, bytes, cudaMemcpyDeviceToDevice, st));
-    k_adj_psource<<<G, 128, 0, st>>>(d, a.lSc, a.lScV, a.lPf);
-    k_adj_gfull<<<G, 128, 0, st>>>(d, a.lPf, a.g);
+    // lP becomes the full-array adjoint of the pressure
+    k_adj_psource<<<G, 128, 0, st>>>(d, a.lSc, a.lScV, a.lP);
+    k_adj_gfull<<<G, 128, 0, st>>>(d, a.lP, a.g);
     FVM_LAUNCH_CHECK(c);
     // ITER_P (converged) and its source DIV/dt
     ARC(adj_poisson(c));
     k_adj_div<<<G, 128, 0, st>>>(d, a);
     k_adj_flux<<<G, 128, 0, st>>>(d, a, a.lFE, a.lFW, a.lFN, a.lFS, a.lUh, a.lVh);
     // u^ = u** - dt S/J with BCU/BCV (Main.f90:80-87)
-    k_adj_gd<<<G, 128, 0, st>>>(d, a.lUh, a.lW, a.lUFW, a.lFFU, 1);
-    k_adj_gd<<<G, 128, 0, st>>>(d, a.lVh, a.lWV, a.lVFW, a.lFFV, 1);
-    FVM_CUDA(c, cudaMemsetAsync(a.lSe, 0, bytes, st));
-    FVM_CUDA(c, cudaMemsetAsync(a.lSeV, 0, bytes, st));
-    FVM_CUDA(c, cudaMemsetAsync(a.lU, 0, bytes, st));
-    FVM_CUDA(c, cudaMemsetAsync(a.lV, 0, bytes, st));
+    k_adj_gd<<<G2, 128, 0, st>>>(d, Two{a.lUh, a.lVh}, lW, wall, far);
+    ARC(adj_clear(c, std::min(a.lU, a.lUn), std::max(a.lV, a.lVn), n));   // both pairs
     k_adj_grad<<<G, 128, 0, st>>>(d, a, a.lW, a.lWV, a.lU, a.lV);
     FVM_LAUNCH_CHECK(c);
     // predictors (ITER_U, ITER_V)
-    FVM_CUDA(c, cudaMemsetAsync(a.lUn, 0, bytes, st));
-    FVM_CUDA(c, cudaMemsetAsync(a.lVn, 0, bytes, st));
-    ARC(adj_predictor(c, a.lU, a.lSU, a.lUn, a.lUFW, a.lFFU));
-    ARC(adj_predictor(c, a.lV, a.lSUV, a.lVn, a.lVFW, a.lFFV));
+    ARC(adj_predictor(c, lam, Two{a.lSU, a.lSUV}, base, wall, far));
     // explicit phase at the base point: fluxes of u^n
-    FVM_CUDA(c, cudaMemcpyAsync(d.U, ubase, bytes, cudaMemcpyDeviceToDevice, st));
-    FVM_CUDA(c, cudaMemcpyAsync(d.V, vbase, bytes, cudaMemcpyDeviceToDevice, st));
+    if (ubase != d.U) FVM_CUDA(c, cudaMemcpyAsync(d.U, ubase, bytes, cudaMemcpyDeviceToDevice, st));
+    if (vbase != d.V) FVM_CUDA(c, cudaMemcpyAsync(d.V, vbase, bytes, cudaMemcpyDeviceToDevice, st));
     run_contra_vel(c);
-    FVM_CUDA(c, cudaMemsetAsync(a.lFE, 0, bytes, st));
-    FVM_CUDA(c, cudaMemsetAsync(a.lFW, 0, bytes, st));
-    FVM_CUDA(c, cudaMemsetAsync(a.lFN, 0, bytes, st));
-    FVM_CUDA(c, cudaMemsetAsync(a.lFS, 0, bytes, st));
-    k_adj_explicit<<<G, 128, 0, st>>>(d, a, ubase, a.lSU, a.lNLX, a.lUn, a.lSe, a.lUFW, a.lFFU);
-    k_adj_explicit<<<G, 128, 0, st>>>(d, a, vbase, a.lSUV, a.lNLY, a.lVn, a.lSeV, a.lVFW, a.lFFV);
-    FVM_CUDA(c, cudaMemsetAsync(a.lP, 0, bytes, st));
+    k_adj_explicit<<<G, 128, 0, st>>>(d, a, ubase, vbase);
+    ARC(adj_clear(c, a.lP, a.lP, n));
     k_adj_psource<<<G, 128, 0, st>>>(d, a.lSe, a.lSeV, a.lP);
     k_adj_flux<<<G, 128, 0, st>>>(d, a, a.lFE, a.lFW, a.lFN, a.lFS, a.lUn, a.lVn);
-    k_adj_farfield<<<rows, 128, 0, st>>>(d, a.lFFU, a.lUn);
-    k_adj_farfield<<<rows, 128, 0, st>>>(d, a.lFFV, a.lVn);
+    k_adj_farfield<<<dim3(rows, 1, 2), 128, 0, st>>>(d, far, base);
     FVM_LAUNCH_CHECK(c);
-    FVM_CUDA(c, cudaMemcpyAsync(a.lU, a.lUn, bytes, cudaMemcpyDeviceToDevice, st));
-    FVM_CUDA(c, cudaMemcpyAsync(a.lV, a.lVn, bytes, cudaMemcpyDeviceToDevice, st));
+    std::swap(a.lU, a.lUn);
+    std::swap(a.lV, a.lVn);
     return FVM_OK;
 }
 
+// Adjoint of the state after the last step, the Poisson adjoint's start, control sums.
 int adj_zero(fvm_ctx *c)
 {
     const Adj &a = c->adj->a;
-    const size_t bytes = sizeof(double) * c->n, jb = sizeof(double) * (c->NJ + 1);
-    double *full[] = {a.lU, a.lV, a.lP, a.lNLX, a.lNLY, a.mu};
-    for (double *p : full) FVM_CUDA(c, cudaMemsetAsync(p, 0, bytes, c->stream));
-    double *perj[] = {a.lUFW, a.lVFW, a.lblow};
-    for (double *p : perj) FVM_CUDA(c, cudaMemsetAsync(p, 0, jb, c->stream));
-    FVM_CUDA(c, cudaMemsetAsync(a.lomega, 0, 2 * sizeof(double), c->stream));
-    return FVM_OK;
+    ARC(adj_clear(c, std::min(a.lU, a.lUn), a.mu, c->n));   // lU, lV, lUn, lVn, lP, lNLX, lNLY, mu
+    return adj_clear(c, a.lUFW, a.lomega, 2);               // lUFW, lVFW, lblow, lomega
 }
 
 int adj_controls(fvm_ctx *c, double *dJ_domega, double *dJ_dblow)
@@ -1428,29 +1438,18 @@ int run_adjoint_vjp(fvm_ctx *c, double *const *lam, double *dctrl)
     ARC(adj_setup(c));
     fvm_adj *A = c->adj;
     const Adj &a = A->a;
-    const size_t n = c->n, bytes = sizeof(double) * n;
-    if (!A->fin) FVM_CUDA(c, cudaMalloc(&A->fin, sizeof(double) * 7 * n));
-    if (!A->one) FVM_CUDA(c, cudaMalloc(&A->one, 2 * bytes));
-    double *ub = A->one;
-    int rc = FVM_OK;
-    do {
-        if ((rc = state_copy(c, A->fin, true))) break;
-        if ((rc = adj_zero(c))) break;
-        if (cudaMemcpyAsync(ub, c->d.U, bytes, cudaMemcpyDeviceToDevice, c->stream) ||
-            cudaMemcpyAsync(ub + n, c->d.V, bytes, cudaMemcpyDeviceToDevice, c->stream)) { rc = FVM_ERR_CUDA; break; }
-        double *dst[] = {a.lU, a.lV, a.lP, a.lNLX, a.lNLY};
-        for (int k = 0; k < 5 && !rc; k++)
-            if (cudaMemcpyAsync(dst[k], lam[k], bytes, cudaMemcpyHostToDevice, c->stream)) rc = FVM_ERR_CUDA;
-        if (rc) break;
-        // the step's own forward values (fluxes of u^n) are recomputed inside
-        if ((rc = adj_step(c, ub, ub + n, 0.0))) break;
-        for (int k = 0; k < 5 && !rc; k++)
-            if (cudaMemcpyAsync(lam[k], dst[k], bytes, cudaMemcpyDeviceToHost, c->stream)) rc = FVM_ERR_CUDA;
-        if (rc) break;
-        rc = adj_controls(c, dctrl, dctrl ? dctrl + 1 : nullptr);
-        if (rc) break;
-        rc = state_copy(c, A->fin, false);
-    } while (false);
+    const size_t bytes = sizeof(double) * c->n;
+    int rc = adj_zero(c);
+    double *dst[] = {a.lU, a.lV, a.lP, a.lNLX, a.lNLY};
+    for (int k = 0; k < 5 && !rc; k++)
+        if (cudaMemcpyAsync(dst[k], lam[k], bytes, cudaMemcpyHostToDevice, c->stream)) rc = FVM_ERR_CUDA;
+    // the step's own forward values (fluxes of u^n) are recomputed inside; nothing else of
+    // the state is written
+    if (!rc) rc = adj_step(c, c->d.U, c->d.V, 0.0);
+    const double *out[] = {a.lU, a.lV, a.lP, a.lNLX, a.lNLY};
+    for (int k = 0; k < 5 && !rc; k++)
+        if (cudaMemcpyAsync(lam[k], out[k], bytes, cudaMemcpyDeviceToHost, c->stream)) rc = FVM_ERR_CUDA;
+    if (!rc) rc = adj_controls(c, dctrl, dctrl ? dctrl + 1 : nullptr);
     cudaStreamSynchronize(c->stream);
     return rc;
 }
@@ -1464,7 +1463,6 @@ void adj_destroy(fvm_ctx *c)
     if (A->ckpt) cudaFree(A->ckpt);
     if (A->base) cudaFree(A->base);
     if (A->fin) cudaFree(A->fin);
-    if (A->one) cudaFree(A->one);
     if (A->h_pctl) cudaFreeHost(A->h_pctl);
     delete A;
     c->adj = nullptr;
