@@ -111,6 +111,18 @@ struct D3 {
     double *wall;           // 8 per (j,k) and triangle
 };
 
+// The fields of one launch of a predictor kernel: up to four with the same coefficient set
+// (U, V, W), each with its own arrays.
+struct Fields {
+    struct F {
+        double *phi, *SU;                             // the field, its sweep's right-hand side
+        const double *phin, *ina, *inb, *inc, *ind;   // k3_af_rhs
+        const double *ff;                             // far-field values
+        int kind;                                     // 0 U, 1 V or W, 2 T
+    } f[4];
+    int n;
+};
+
 #define ID3(i, j, k) ((i) + d.NI1 * ((j) + d.NJ1 * (k)))
 #define JK(j, k) ((j) + d.NJ1 * (k))
 
@@ -676,55 +688,120 @@ __device__ __forceinline__ void couple_coefs(const Coef3 &cf, const double *&c1,
     c4 = FAM == 2 ? cf.AS : cf.AB;
 }
 
+// Right-hand side of cell c of a line: the four transverse couplings and the source as
+// fused multiply-adds.
+template <class T>
+__device__ __forceinline__ T line_rhs(const D3 &d, const double *c1, const double *c2, const double *c3, const double *c4,
+                                      const double *phi, const double *SU, const LineGeo &g, int c)
+{
+    return fma(lds<T>(d, c1, c), lds<T>(d, phi, c + g.o1),
+               fma(lds<T>(d, c2, c), lds<T>(d, phi, c + g.o2),
+                   fma(lds<T>(d, c3, c), lds<T>(d, phi, c + g.o3),
+                       fma(lds<T>(d, c4, c), lds<T>(d, phi, c + g.o4), ld<T>(SU[c])))));
+}
+
 // T: double (FP64 path, every set) or dd (mixed path, the predictor sets 0..5, whose
 // couplings and phi are read through their shadows and factors from sd; phi is
 // stored with its shadow, so the second colour reads the first colour's values).
-template <int M, int NW, int FAM, class T = double>
-__global__ void __launch_bounds__(128) k3_line(D3 d, LineSys s, Coef3 cf, const double *SU, double *phi, int colour,
+// I lines; neighbouring blocks take the fields of one group of lines, which share its
+// coefficients through L2.
+template <int M, int NW, class T = double>
+__global__ void __launch_bounds__(128) k3_line(D3 d, LineSys s, Coef3 cf, const __grid_constant__ Fields S, int colour,
                                                const PCtl *stop, LineDD sd)
 {
     constexpr int TG = WARP * NW, G = 4 / NW;
     __shared__ T sm[G][TG * M + M * NW + 1];
     __shared__ T xch[G][2 * NW];
     const int ended = stop ? stop->done : 0;   // the Poisson loop has ended (tested after the loads)
-    int gl, t, gib;
-    fvm::group_of<NW>(gl, t, gib);
+    const int gib = threadIdx.x / TG, t = threadIdx.x % TG, gl = int(blockIdx.x) / S.n * G + gib;
+    const Fields::F &f = S.f[int(blockIdx.x) % S.n];
+    double *phi = f.phi;
     int L = 0;
-    const bool active = colour_line(d, FAM, colour, gl, L);
+    const bool active = colour_line(d, 0, colour, gl, L);
     if (!active) L = 0;
     const int n = s.n;
-    const LineGeo g = line_geo<FAM>(d, L);
+    const LineGeo g = line_geo<0>(d, L);
     const double *c1, *c2, *c3, *c4;
-    couple_coefs<FAM>(cf, c1, c2, c3, c4);
+    couple_coefs<0>(cf, c1, c2, c3, c4);
     T v[M];
 #pragma unroll
     for (int q = 0; q < M; q++) {
         const int e = q * TG + t;
-        v[q] = T(0);
-        if (active && e < n) {
-            const int c = g.base + e * g.stride;
-            // the four transverse couplings and the source as fused multiply-adds
-            v[q] = fma(lds<T>(d, c1, c), lds<T>(d, phi, c + g.o1),
-                       fma(lds<T>(d, c2, c), lds<T>(d, phi, c + g.o2),
-                           fma(lds<T>(d, c3, c), lds<T>(d, phi, c + g.o3),
-                               fma(lds<T>(d, c4, c), lds<T>(d, phi, c + g.o4), ld<T>(SU[c])))));
-        }
+        v[q] = active && e < n ? line_rhs<T>(d, c1, c2, c3, c4, phi, f.SU, g, g.base + e) : T(0);
     }
     if (ended) return;
     fvm::to_chunks<T, M, NW>(v, sm[gib], t);
     const size_t base = size_t(L) * TG * M;
-    if constexpr (std::is_same<T, double>::value) {
+    if constexpr (std::is_same<T, double>::value)
         fvm::group_apply<double, M, NW>(v, s.invD + base, s.fa + base, s.fb + base, t, xch[gib]);
-        if (FAM != 0) fvm::group_cyclic_fix<double, M, NW>(v, s.z + base, s.cv[L], s.sinv[L], n, t, xch[gib]);
-    } else {
-        fvm::group_apply<dd, M, NW>(v, sd.invD + base, sd.fa + base, sd.fb + base, t, xch[gib]);
-        if (FAM != 0) fvm::group_cyclic_fix<dd, M, NW>(v, sd.z + base, sd.cv[L], sd.sinv[L], n, t, xch[gib]);
-    }
+    else fvm::group_apply<dd, M, NW>(v, sd.invD + base, sd.fa + base, sd.fb + base, t, xch[gib]);
     fvm::to_interleaved<T, M, NW>(v, sm[gib], t);
 #pragma unroll
     for (int q = 0; q < M; q++) {
         const int e = q * TG + t;
-        if (active && e < n) sts(d, phi, g.base + e * g.stride, v[q]);
+        if (active && e < n) sts(d, phi, g.base + e, v[q]);
+    }
+}
+
+// J lines (FAM 1) and K lines (FAM 2), cyclic.  A block takes JK_LINES lines of a colour,
+// neighbours in i, and loads and stores them with its threads across the lines (4 rows
+// of 8 cells a warp); the elements go through shared memory to the groups that solve
+// them.  With the threads along a line every element of a load lay in a row of its own
+// and the load took 32 passes of the L1 tags.  One colour of one component at 256 x 192 x 48,
+// mixed: J lines 53 -> 36 us, K lines 50 -> 49 us.
+constexpr int JK_LINES = 8, JK_THREADS = 256;
+
+template <int M, int NW, int FAM, class T>
+__global__ void __launch_bounds__(JK_THREADS) k3_line_jk(D3 d, LineSys s, Coef3 cf, const __grid_constant__ Fields S,
+                                                         int colour, LineDD sd)
+{
+    constexpr int TG = WARP * NW, G = JK_THREADS / TG, ROWS = JK_THREADS / JK_LINES;
+    // element e of a line in word e + e / M: the chunks of neighbouring threads start an odd
+    // number of words apart; lines 2 words (mod 16) apart, which keeps the row-wise
+    // accesses (8 lines x 2 elements) on 16 different words
+    constexpr int LEN = TG * (M + 1), LP = LEN + (18 - LEN % 16) % 16;
+    __shared__ T tile[JK_LINES * LP];
+    __shared__ T xch[G][2 * NW];
+    const int gl0 = int(blockIdx.x) / S.n * JK_LINES;
+    const Fields::F &f = S.f[int(blockIdx.x) % S.n];
+    double *phi = f.phi;
+    const int n = s.n, l = threadIdx.x % JK_LINES, row = threadIdx.x / JK_LINES;
+    int L = 0;
+    const bool active = colour_line(d, FAM, colour, gl0 + l, L);
+    const LineGeo g = line_geo<FAM>(d, active ? L : 0);
+    const double *c1, *c2, *c3, *c4;
+    couple_coefs<FAM>(cf, c1, c2, c3, c4);
+    if (active) {
+#pragma unroll 2
+        for (int e = row; e < n; e += ROWS)
+            tile[l * LP + e + e / M] = line_rhs<T>(d, c1, c2, c3, c4, phi, f.SU, g, g.base + e * g.stride);
+    }
+    __syncthreads();
+    const int gib = threadIdx.x / TG, t = threadIdx.x % TG;
+#pragma unroll 1
+    for (int q = gib; q < JK_LINES; q += G) {   // JK_LINES / G rounds, the same in every group
+        int Lq = 0;
+        const bool own = colour_line(d, FAM, colour, gl0 + q, Lq);
+        if (!own) Lq = 0;
+        T v[M];
+        T *x = tile + q * LP + t * (M + 1);
+#pragma unroll
+        for (int k = 0; k < M; k++) v[k] = own && t * M + k < n ? x[k] : T(0);
+        const size_t base = size_t(Lq) * TG * M;
+        if constexpr (std::is_same<T, double>::value) {
+            fvm::group_apply<double, M, NW>(v, s.invD + base, s.fa + base, s.fb + base, t, xch[gib]);
+            fvm::group_cyclic_fix<double, M, NW>(v, s.z + base, s.cv[Lq], s.sinv[Lq], n, t, xch[gib]);
+        } else {
+            fvm::group_apply<dd, M, NW>(v, sd.invD + base, sd.fa + base, sd.fb + base, t, xch[gib]);
+            fvm::group_cyclic_fix<dd, M, NW>(v, sd.z + base, sd.cv[Lq], sd.sinv[Lq], n, t, xch[gib]);
+        }
+#pragma unroll
+        for (int k = 0; k < M; k++) x[k] = v[k];
+    }
+    __syncthreads();
+    if (active) {
+#pragma unroll 2
+        for (int e = row; e < n; e += ROWS) sts(d, phi, g.base + e * g.stride, tile[l * LP + e + e / M]);
     }
 }
 
@@ -952,8 +1029,11 @@ __global__ void k3_farfield(D3 d)
 // Threads [0, nin): the two I ghosts of the interior line (j, k); the others: cell i
 // of a ghost row (j in {0, NJ} or k in {0, NK}; the K-plane rows first).  Mixed
 // path: the ghosts' shadows too.
-__global__ void k3_bcu(D3 d, double *phi, const double *ff, int kind)
+__global__ void k3_bcu(D3 d, const __grid_constant__ Fields S)
 {
+    double *phi = S.f[blockIdx.y].phi;
+    const double *ff = S.f[blockIdx.y].ff;
+    const int kind = S.f[blockIdx.y].kind;
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const int nj1 = d.NJ - 1, nk1 = d.NK - 1;
     const long long nin = (long long)nj1 * nk1;
@@ -997,11 +1077,13 @@ __global__ void k3_bcu(D3 d, double *phi, const double *ff, int kind)
 // T: double (FP64 path) or dd (mixed path, where 2 Re J / dt is J times the
 // precomputed 2 Re / dt instead of a division per cell).
 template <class T>
-__global__ void k3_af_rhs(D3 d, Coef3 cf, int split, int kind, const double *phi, const double *phin,
-                          const double *ina, const double *inb, const double *inc, const double *ind,
-                          const double *ff)
+__global__ void k3_af_rhs(D3 d, Coef3 cf, int split, const __grid_constant__ Fields S)
 {
-    CELL3(1, d.NI - 1, 1, d.NJ - 1, 1, d.NK - 1)
+    const Fields::F &q = S.f[int(blockIdx.x) % S.n];
+    const double *phi = q.phi, *phin = q.phin, *ina = q.ina, *inb = q.inb, *inc = q.inc, *ind = q.ind, *ff = q.ff;
+    const int kind = q.kind, i = int(blockIdx.x) / S.n * int(blockDim.x) + int(threadIdx.x) + 1;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1, k = blockIdx.z + 1;
+    if (i > d.NI - 1 || j > d.NJ - 1) return;
     const int c = ID3(i, j, k);
     const double *J = d.DJAC;
     const T cr = cross_w<T>(d, d.CWA[split], 1 + split, phi, c, i);
@@ -1022,7 +1104,7 @@ __global__ void k3_af_rhs(D3 d, Coef3 cf, int split, int kind, const double *phi
     const double uf = kind == 2 ? d.t_wall : 0.0;
     if (i == 1) su = su + scale2(ld<T>(cf.awall[JK(j, k)]), 2.0f) * ld<T>(uf);
     if (i == d.NI - 1) su = su + scale2(ld<T>(cf.afar[JK(j, k)]), 2.0f) * ld<T>(ff[JK(j, k)]);
-    d.SU[c] = to_d(su);
+    q.SU[c] = to_d(su);
 }
 
 // u += sign * dt * S / J (main.f90:84-86, 104-106).  The update of the state is
@@ -2101,30 +2183,27 @@ int refresh_constants(fvm3_ctx *c)
     return refresh(c, a);
 }
 
-int line(fvm3_ctx *c, int set, const double *SU, double *phi, int colour, const PCtl *stop = nullptr)
+// One colour of a line sweep of the fields S (which share set `set`).
+int line(fvm3_ctx *c, int set, const Fields &S, int colour, const PCtl *stop = nullptr)
 {
     const D3 &d = c->d;
     const LineSys &s = d.sys[set];
     const int fam = set == 6 ? 0 : set % 3;
-    int per;
-    if (fam == 0) per = (c->NJ - 1) / 2 * (c->NK - 1);
-    else per = (c->NI / 2) * ((fam == 1 ? c->NK : c->NJ) - 1);
-    const int blocks = fvm::line_blocks(per, s.NW);
+    const bool dfl = d.dfl && set < 6;   // predictor sets of the mixed path: double-float
     bool ok = fvm::dispatch_line(s, [&](auto m, auto nw) {
         constexpr int M = decltype(m)::value, NW = decltype(nw)::value;
-        const LineDD none{};
-        if (d.dfl && set < 6) {   // predictor sets of the mixed path: double-float
-            const LineDD &sd = d.sysd[set];
-            if (fam == 0) k3_line<M, NW, 0, dd><<<blocks, 128, 0, c->stream>>>(d, s, d.cf[set], SU, phi, colour, stop, sd);
-            else if (fam == 1) k3_line<M, NW, 1, dd><<<blocks, 128, 0, c->stream>>>(d, s, d.cf[set], SU, phi, colour, stop, sd);
-            else k3_line<M, NW, 2, dd><<<blocks, 128, 0, c->stream>>>(d, s, d.cf[set], SU, phi, colour, stop, sd);
-        } else if (fam == 0) {
-            k3_line<M, NW, 0><<<blocks, 128, 0, c->stream>>>(d, s, d.cf[set], SU, phi, colour, stop, none);
-        } else if (fam == 1) {
-            k3_line<M, NW, 1><<<blocks, 128, 0, c->stream>>>(d, s, d.cf[set], SU, phi, colour, stop, none);
-        } else {
-            k3_line<M, NW, 2><<<blocks, 128, 0, c->stream>>>(d, s, d.cf[set], SU, phi, colour, stop, none);
+        const LineDD sd = dfl ? d.sysd[set] : LineDD{};
+        if (fam == 0) {
+            const unsigned blocks = unsigned(S.n) * fvm::line_blocks((c->NJ - 1) / 2 * (c->NK - 1), s.NW);
+            if (dfl) k3_line<M, NW, dd><<<blocks, 128, 0, c->stream>>>(d, s, d.cf[set], S, colour, stop, sd);
+            else k3_line<M, NW><<<blocks, 128, 0, c->stream>>>(d, s, d.cf[set], S, colour, stop, sd);
+            return;
         }
+        const int per = (c->NI / 2) * ((fam == 1 ? c->NK : c->NJ) - 1);
+        const unsigned blocks = unsigned(S.n) * ((per + JK_LINES - 1) / JK_LINES);
+        auto go = [&](auto kernel) { kernel<<<blocks, JK_THREADS, 0, c->stream>>>(d, s, d.cf[set], S, colour, sd); };
+        if (dfl) go(fam == 1 ? k3_line_jk<M, NW, 1, dd> : k3_line_jk<M, NW, 2, dd>);
+        else go(fam == 1 ? k3_line_jk<M, NW, 1, double> : k3_line_jk<M, NW, 2, double>);
     });
     if (!ok) {
         c->err = "line length above 512 cells is not supported";
@@ -2222,34 +2301,44 @@ static inline bool dfloat(const fvm3_ctx *c) { return c->p.precision == FVM_MIXE
         else K<double><<<(grid), (block), 0, (c)->stream>>>(__VA_ARGS__);         \
     } while (0)
 
-int bcu(fvm3_ctx *c, double *phi, const double *ff, int kind);
+// BCU/BCT of the fields S (phi, ff, kind) with their periodic copies.
+int bcu(fvm3_ctx *c, const Fields &S)
+{
+    const long long nt = (long long)(c->NJ - 1) * (c->NK - 1) +
+                         (2LL * (c->NJ + 1) + 2LL * (c->NK - 1)) * (c->NI + 1);
+    k3_bcu<<<dim3((unsigned)((nt + 255) / 256), S.n), 256, 0, c->stream>>>(c->d, S);
+    F3CHECK(c);
+    return FVM_OK;
+}
 
-// One predictor sweep set (three AF sweeps) of a field: kind 0 U, 1 V or W, 2 T.
-int predictor(fvm3_ctx *c, int kind, double *phi, const double *phin, const double *ina, const double *inb,
-              const double *inc, const double *ind, const double *ff)
+// One predictor sweep set (three AF sweeps) of the fields S, which share their coefficient
+// set: independent of each other, they go in the same launches.
+int predictor(fvm3_ctx *c, const Fields &S)
 {
     D3 &d = c->d;
-    const int base = kind == 2 ? 3 : 0;
-    // the field's shadow: refreshed once; later the line solves write the interior
+    const int base = S.f[0].kind == 2 ? 3 : 0;
+    // the fields' shadows: refreshed once; later the line solves write the interior
     // shadows and k3_bcu the ghosts'
-    F3RC(refresh(c, {phi}));
+    if (S.n == 3) F3RC(refresh(c, {S.f[0].phi, S.f[1].phi, S.f[2].phi}));
+    else F3RC(refresh(c, {S.f[0].phi}));
+    dim3 G = g_int(c);
+    G.x *= S.n;
     for (int split = 0; split < 3; split++) {
-        F3_LAUNCH(c, k3_af_rhs, g_int(c), B_INT, d, d.cf[base + split], split, kind, phi, phin, ina, inb, inc, ind,
-                  ff);
-        F3RC(bcu(c, phi, ff, kind));
-        F3RC(line(c, base + split, d.SU, phi, 0));
-        F3RC(line(c, base + split, d.SU, phi, 1));
+        F3_LAUNCH(c, k3_af_rhs, G, B_INT, d, d.cf[base + split], split, S);
+        F3RC(bcu(c, S));
+        F3RC(line(c, base + split, S, 0));
+        F3RC(line(c, base + split, S, 1));
     }
     return FVM_OK;
 }
 
-int bcu(fvm3_ctx *c, double *phi, const double *ff, int kind)
+Fields poisson_field(const D3 &d, double *phi)
 {
-    const long long nt = (long long)(c->NJ - 1) * (c->NK - 1) +
-                         (2LL * (c->NJ + 1) + 2LL * (c->NK - 1)) * (c->NI + 1);
-    k3_bcu<<<(unsigned)((nt + 255) / 256), 256, 0, c->stream>>>(c->d, phi, ff, kind);
-    F3CHECK(c);
-    return FVM_OK;
+    Fields S{};
+    S.f[0].phi = phi;
+    S.f[0].SU = d.SU;
+    S.n = 1;
+    return S;
 }
 
 // The Poisson loop body: `groups` x (res_every x [source, BCP, sweep], residual).
@@ -2298,13 +2387,14 @@ int poisson_graph(fvm3_ctx *c)
         }
         if (rc == FVM_OK) rc = halo(c, {d.P});
     }
+    const Fields pf = poisson_field(d, d.P);
     for (int q = 0; q < groups && rc == FVM_OK && !mixed; q++) {
         for (int it = 0; it < per && rc == FVM_OK; it++) {
             k3_psu<<<g_int(c), B_INT, 0, c->stream>>>(d);
             k3_bcp<<<dim3((c->NJ + 127) / 128, c->NK + 1), 128, 0, c->stream>>>(d, 1);
             rc = halo(c, {d.P});
-            if (rc == FVM_OK) rc = line(c, 6, d.SU, d.P, 0, d.pctl);
-            if (rc == FVM_OK) rc = line(c, 6, d.SU, d.P, 1, d.pctl);
+            if (rc == FVM_OK) rc = line(c, 6, pf, 0, d.pctl);
+            if (rc == FVM_OK) rc = line(c, 6, pf, 1, d.pctl);
         }
         if (dev_loop) k3_pres<1><<<d.nblk, 256, 0, c->stream>>>(d, d.cf[6], per, h);
         else k3_pres<0><<<d.nblk, 256, 0, c->stream>>>(d, d.cf[6], per, h);
@@ -2369,6 +2459,19 @@ int sep_filter(fvm3_ctx *c, int mode)
     return FVM_OK;
 }
 
+// The velocity components.  Their right-hand sides are kept in SU and in U2, U3: contravariant
+// velocities, formed anew before each use of theirs (contra_vel).
+Fields velocity(const fvm3_ctx *c)
+{
+    const D3 &d = c->d;
+    Fields S{};
+    S.f[0] = {d.U, d.SU, d.U_N, d.NLX, d.NLX_NM1, d.DIFX, d.S_U, d.FFU, 0};
+    S.f[1] = {d.V, d.U2, d.V_N, d.NLY, d.NLY_NM1, d.DIFY, d.S_V, d.FFV, 1};
+    S.f[2] = {d.W, d.U3, d.W_N, d.NLZ, d.NLZ_NM1, d.DIFZ, d.S_W, d.FFW, 1};
+    S.n = 3;
+    return S;
+}
+
 int sgs(fvm3_ctx *c)
 {
     D3 &d = c->d;
@@ -2382,10 +2485,13 @@ int sgs(fvm3_ctx *c)
                           d.DTD[1], d.DTD[2]}));
     F3_LAUNCH(c, k3_mag, g_lin(c), 256, d);
     F3RC(sep_filter(c, SEP_HATS));
-    F3RC(bcu(c, d.UH, d.FFU, 0));
-    F3RC(bcu(c, d.VH, d.FFV, 1));
-    F3RC(bcu(c, d.WH, d.FFW, 1));
-    F3RC(bcu(c, d.TH, d.FFT, 2));
+    Fields hats = velocity(c);
+    double *const H[4] = {d.UH, d.VH, d.WH, d.TH};
+    for (int q = 0; q < 4; q++) hats.f[q].phi = H[q];
+    hats.f[3].ff = d.FFT;
+    hats.f[3].kind = 2;
+    hats.n = 4;
+    F3RC(bcu(c, hats));
     F3RC(refresh(c, {d.UH, d.VH, d.WH, d.TH}));
     F3RC(sep_filter(c, SEP_VEL));
     F3_LAUNCH(c, k3_germano, g_int(c), B_INT, d, 1);
@@ -2468,20 +2574,14 @@ int p_source(fvm3_ctx *c)   // P_SOURCE(P)
 
 int iter_u(fvm3_ctx *c, int comp)   // ITER_U of U (0), V (1) or W (2), main.f90:81-88
 {
-    D3 &d = c->d;
-    if (comp == 0) return predictor(c, 0, d.U, d.U_N, d.NLX, d.NLX_NM1, d.DIFX, d.S_U, d.FFU);
-    if (comp == 1) return predictor(c, 1, d.V, d.V_N, d.NLY, d.NLY_NM1, d.DIFY, d.S_V, d.FFV);
-    return predictor(c, 1, d.W, d.W_N, d.NLZ, d.NLZ_NM1, d.DIFZ, d.S_W, d.FFW);
+    Fields S = velocity(c);
+    S.f[0] = S.f[comp];
+    S.f[0].SU = c->d.SU;
+    S.n = 1;
+    return predictor(c, S);
 }
 
-int bcu_all(fvm3_ctx *c)   // BCU of U, V, W
-{
-    D3 &d = c->d;
-    F3RC(bcu(c, d.U, d.FFU, 0));
-    F3RC(bcu(c, d.V, d.FFV, 1));
-    F3RC(bcu(c, d.W, d.FFW, 1));
-    return FVM_OK;
-}
+int bcu_all(fvm3_ctx *c) { return bcu(c, velocity(c)); }   // BCU of U, V, W
 
 int remove_grad(fvm3_ctx *c)   // main.f90:90-97: u -= dt S/J, BCU
 {
@@ -2515,8 +2615,11 @@ int iter_t(fvm3_ctx *c)   // main.f90:143-145: ITER_T, BCT
 {
     D3 &d = c->d;
     if (!d.thermal) return FVM_OK;
-    F3RC(predictor(c, 2, d.T, d.T_N, d.ADV, d.ADV_NM1, d.DIFT, nullptr, d.FFT));
-    return bcu(c, d.T, d.FFT, 2);
+    Fields S{};
+    S.f[0] = {d.T, d.SU, d.T_N, d.ADV, d.ADV_NM1, d.DIFT, nullptr, d.FFT, 2};
+    S.n = 1;
+    F3RC(predictor(c, S));
+    return bcu(c, S);
 }
 
 int calccoef(fvm3_ctx *c)   // CALCCOEF kernels; the record is read by read_coeffs
@@ -2542,7 +2645,7 @@ int step(fvm3_ctx *c)
     if (c->p.use_les) F3RC(sgs(c));
     F3RC(dif_all(c));
     F3RC(p_source(c));
-    for (int comp = 0; comp < 3; comp++) F3RC(iter_u(c, comp));
+    F3RC(predictor(c, velocity(c)));   // ITER_U of U, V, W
     F3RC(remove_grad(c));
     F3RC(iter_p(c));
     F3RC(correct(c));
@@ -3006,13 +3109,14 @@ int fvm3_time_sweeps(fvm3_ctx *c, int sweeps, double *ms_per_sweep)
     F3CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     int rc = FVM_OK;
     const bool mixed = c->p.precision == FVM_MIXED;
+    const f3::Fields pf = f3::poisson_field(d, d.DIVDT);
     for (int s = 0; s < sweeps && rc == FVM_OK; s++) {
         if (mixed) {
             rc = f3::line32(c, 0, 0, 0);
             if (rc == FVM_OK) rc = f3::line32(c, 1, 0, 0);
         } else {
-            rc = f3::line(c, 6, d.SU, d.DIVDT, 0);
-            if (rc == FVM_OK) rc = f3::line(c, 6, d.SU, d.DIVDT, 1);
+            rc = f3::line(c, 6, pf, 0);
+            if (rc == FVM_OK) rc = f3::line(c, 6, pf, 1);
         }
     }
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
