@@ -743,43 +743,51 @@ __global__ void __launch_bounds__(128) k3_line(D3 d, LineSys s, Coef3 cf, const 
     }
 }
 
-// J lines (FAM 1) and K lines (FAM 2), cyclic.  A block takes JK_LINES lines of a colour,
-// neighbours in i, and loads and stores them with its threads across the lines (4 rows
-// of 8 cells a warp); the elements go through shared memory to the groups that solve
+// J lines (FAM 1) and K lines (FAM 2), cyclic.  A block takes jk_lines lines of a colour,
+// neighbours in i, and loads and stores them with its threads across the lines (rows of
+// 8 or 16 cells); the elements go through shared memory to the groups that solve
 // them.  With the threads along a line every element of a load lay in a row of its own
 // and the load took 32 passes of the L1 tags.  One colour of one component at 256 x 192 x 48,
-// mixed: J lines 53 -> 36 us, K lines 50 -> 49 us.
-constexpr int JK_LINES = 8, JK_THREADS = 256;
+// mixed: J lines (4 elements x 2 warps) 53 -> 32 us, K lines (2 x 1) 50 -> 35 us.
+// Bound: latency, with DRAM at about half its rate; what helps is warps on the chip.  LINES
+// 8, four blocks per SM while the registers hold the chunk (J lines, three components:
+// 97 us without the bound, 86 with four, 96 with six).  LINES 16, five blocks, for short
+// chunks of one warp on grids with blocks for every place (K lines, three components: 110 us
+// with 8 lines, 95 with 16; at 64 x 48 x 16, 288 such blocks, 6.5 us with 8 and 9.0 with
+// 16).  Factors loaded before the wait for the tile cost more in warps than they hide.
+constexpr int JK_THREADS = 256;
+__host__ __device__ constexpr int jk_blocks(int M, int LINES) { return LINES == 16 ? 5 : (M <= 4 ? 4 : 1); }
 
-template <int M, int NW, int FAM, class T>
-__global__ void __launch_bounds__(JK_THREADS) k3_line_jk(D3 d, LineSys s, Coef3 cf, const __grid_constant__ Fields S,
+template <int M, int NW, int FAM, int LINES, class T>
+__global__ void __launch_bounds__(JK_THREADS, jk_blocks(M, LINES)) k3_line_jk(D3 d, LineSys s, Coef3 cf, const __grid_constant__ Fields S,
                                                          int colour, LineDD sd)
 {
-    constexpr int TG = WARP * NW, G = JK_THREADS / TG, ROWS = JK_THREADS / JK_LINES;
+    constexpr int TG = WARP * NW, G = JK_THREADS / TG, ROWS = JK_THREADS / LINES;
+    constexpr int UNROLL = LINES == 16 ? 1 : 2;
     // element e of a line in word e + e / M: the chunks of neighbouring threads start an odd
-    // number of words apart; lines 2 words (mod 16) apart, which keeps the row-wise
-    // accesses (8 lines x 2 elements) on 16 different words
-    constexpr int LEN = TG * (M + 1), LP = LEN + (18 - LEN % 16) % 16;
-    __shared__ T tile[JK_LINES * LP];
+    // number of words apart; lines 16 / LINES words (mod 16) apart, which keeps the row-wise
+    // accesses (neighbouring lines, neighbouring elements) on 16 different words
+    constexpr int LEN = TG * (M + 1), LP = LEN + (16 + 16 / LINES - LEN % 16) % 16;
+    __shared__ T tile[LINES * LP];
     __shared__ T xch[G][2 * NW];
-    const int gl0 = int(blockIdx.x) / S.n * JK_LINES;
+    const int gl0 = int(blockIdx.x) / S.n * LINES;
     const Fields::F &f = S.f[int(blockIdx.x) % S.n];
     double *phi = f.phi;
-    const int n = s.n, l = threadIdx.x % JK_LINES, row = threadIdx.x / JK_LINES;
+    const int n = s.n, l = threadIdx.x % LINES, row = threadIdx.x / LINES;
     int L = 0;
     const bool active = colour_line(d, FAM, colour, gl0 + l, L);
     const LineGeo g = line_geo<FAM>(d, active ? L : 0);
     const double *c1, *c2, *c3, *c4;
     couple_coefs<FAM>(cf, c1, c2, c3, c4);
     if (active) {
-#pragma unroll 2
+#pragma unroll UNROLL
         for (int e = row; e < n; e += ROWS)
             tile[l * LP + e + e / M] = line_rhs<T>(d, c1, c2, c3, c4, phi, f.SU, g, g.base + e * g.stride);
     }
     __syncthreads();
     const int gib = threadIdx.x / TG, t = threadIdx.x % TG;
 #pragma unroll 1
-    for (int q = gib; q < JK_LINES; q += G) {   // JK_LINES / G rounds, the same in every group
+    for (int q = gib; q < LINES; q += G) {   // LINES / G rounds, the same in every group
         int Lq = 0;
         const bool own = colour_line(d, FAM, colour, gl0 + q, Lq);
         if (!own) Lq = 0;
@@ -800,7 +808,7 @@ __global__ void __launch_bounds__(JK_THREADS) k3_line_jk(D3 d, LineSys s, Coef3 
     }
     __syncthreads();
     if (active) {
-#pragma unroll 2
+#pragma unroll UNROLL
         for (int e = row; e < n; e += ROWS) sts(d, phi, g.base + e * g.stride, tile[l * LP + e + e / M]);
     }
 }
@@ -1345,7 +1353,7 @@ __device__ __forceinline__ void line_bcp(const D3 &d, int j, int k)
 // partner line (j-1, k) -- j -> j-1 maps the colour-1 lines of a plane one to one
 // onto the colour-0 lines -- and sets the BCP ghosts of both lines.
 template <int M, int NW>
-__global__ void __launch_bounds__(128) k3_line32(const __grid_constant__ D3 d, LineSys s, int colour, int check_done,
+__global__ void __launch_bounds__(128, 6) k3_line32(const __grid_constant__ D3 d, LineSys s, int colour, int check_done,
                                                  int apply)
 {
     constexpr int TG = WARP * NW, G = 4 / NW;
@@ -2200,10 +2208,17 @@ int line(fvm3_ctx *c, int set, const Fields &S, int colour, const PCtl *stop = n
             return;
         }
         const int per = (c->NI / 2) * ((fam == 1 ? c->NK : c->NJ) - 1);
-        const unsigned blocks = unsigned(S.n) * ((per + JK_LINES - 1) / JK_LINES);
-        auto go = [&](auto kernel) { kernel<<<blocks, JK_THREADS, 0, c->stream>>>(d, s, d.cf[set], S, colour, sd); };
-        if (dfl) go(fam == 1 ? k3_line_jk<M, NW, 1, dd> : k3_line_jk<M, NW, 2, dd>);
-        else go(fam == 1 ? k3_line_jk<M, NW, 1, double> : k3_line_jk<M, NW, 2, double>);
+        auto go = [&](auto lines) {
+            constexpr int LINES = decltype(lines)::value;
+            const unsigned blocks = unsigned(S.n) * ((per + LINES - 1) / LINES);
+            auto launch = [&](auto kernel) { kernel<<<blocks, JK_THREADS, 0, c->stream>>>(d, s, d.cf[set], S, colour, sd); };
+            if (dfl) launch(fam == 1 ? k3_line_jk<M, NW, 1, LINES, dd> : k3_line_jk<M, NW, 2, LINES, dd>);
+            else launch(fam == 1 ? k3_line_jk<M, NW, 1, LINES, double> : k3_line_jk<M, NW, 2, LINES, double>);
+        };
+        if constexpr (NW == 1 && M <= 3) {
+            if ((long long)S.n * per >= 16LL * 5 * 152) return go(std::integral_constant<int, 16>());
+        }
+        go(std::integral_constant<int, 8>());
     });
     if (!ok) {
         c->err = "line length above 512 cells is not supported";

@@ -13,7 +13,7 @@ from tests.helpers import rel_l2
 pytestmark = pytest.mark.gpu
 
 # theta cells, radial cells, span cells
-GRIDS = [(8, 7, 8), (10, 9, 12), (34, 13, 30), (66, 20, 34), (130, 11, 10), (258, 7, 8), (12, 8, 130), (10, 130, 8)]
+GRIDS = [(8, 7, 8), (10, 9, 12), (34, 13, 30), (66, 20, 34), (66, 130, 96), (130, 11, 10), (258, 7, 8), (12, 8, 130), (10, 130, 8)]
 FIELDS = ("U", "V", "W", "P", "T")
 
 
