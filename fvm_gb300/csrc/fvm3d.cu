@@ -1037,7 +1037,10 @@ __global__ void k3_farfield(D3 d)
 // Threads [0, nin): the two I ghosts of the interior line (j, k); the others: cell i
 // of a ghost row (j in {0, NJ} or k in {0, NK}; the K-plane rows first).  Mixed
 // path: the ghosts' shadows too.
-__global__ void k3_bcu(D3 d, const __grid_constant__ Fields S)
+// P: the pressure instead (bcp.f90:24-34): P(0) = P(1), P(NI) the cubic extrapolation; `stop`:
+// part of the Poisson loop, nothing once it has ended.
+template <bool P = false>
+__global__ void k3_bcu(D3 d, const __grid_constant__ Fields S, const PCtl *stop)
 {
     double *phi = S.f[blockIdx.y].phi;
     const double *ff = S.f[blockIdx.y].ff;
@@ -1047,20 +1050,26 @@ __global__ void k3_bcu(D3 d, const __grid_constant__ Fields S)
     const long long nin = (long long)nj1 * nk1;
     const long long nrow = 2LL * (d.NJ + 1) + 2LL * nk1;
     if (t >= nin + nrow * d.NI1) return;
+    if (P && stop && stop->done) return;
     const double uf = kind == 2 ? d.t_wall : 0.0;
     auto put = [&](int c, double v) {
         phi[c] = v;
-        if (d.dfl) {
+        if (!P && d.dfl) {
             const dd s = fvm::dd_split(v);
             shadow(d, phi)[c] = make_float2(s.hi, s.lo);
         }
+    };
+    auto wall = [&](int j, int k) { return P ? phi[ID3(1, j, k)] : (-phi[ID3(1, j, k)]) + 2.0 * uf; };
+    auto far = [&](int j, int k) {
+        if (P) return (3.0 * phi[ID3(d.NI - 1, j, k)] - 3.0 * phi[ID3(d.NI - 2, j, k)]) + phi[ID3(d.NI - 3, j, k)];
+        return (-phi[ID3(d.NI - 1, j, k)]) + 2.0 * ff[JK(j, k)];
     };
     int i, j, k;
     if (t < nin) {
         j = (int)(t % nj1) + 1;
         k = (int)(t / nj1) + 1;
-        put(ID3(0, j, k), (-phi[ID3(1, j, k)]) + 2.0 * uf);
-        put(ID3(d.NI, j, k), (-phi[ID3(d.NI - 1, j, k)]) + 2.0 * ff[JK(j, k)]);
+        put(ID3(0, j, k), wall(j, k));
+        put(ID3(d.NI, j, k), far(j, k));
         return;
     }
     const long long q = t - nin;
@@ -1075,8 +1084,8 @@ __global__ void k3_bcu(D3 d, const __grid_constant__ Fields S)
         k = r2 % nk1 + 1;
     }
     const int js = jw(d, j), ks = kw(d, k), c = ID3(i, j, k);
-    if (i == 0) put(c, (-phi[ID3(1, js, ks)]) + 2.0 * uf);
-    else if (i == d.NI) put(c, (-phi[ID3(d.NI - 1, js, ks)]) + 2.0 * ff[JK(js, ks)]);
+    if (i == 0) put(c, wall(js, ks));
+    else if (i == d.NI) put(c, far(js, ks));
     else put(c, phi[ID3(i, js, ks)]);
 }
 
@@ -1159,18 +1168,6 @@ __global__ void k3_psu(D3 d)
     const int c = ID3(i, j, k);
     if (d.pctl->done) return;
     d.SU[c] = d.DIVDT[c] - cross12(d, d.P, i, j, k);
-}
-
-// BCP ghosts (bcp.f90:24-34): P(0) = P(1), P(NI) cubic extrapolation (periodic
-// copy follows).  check_done: part of the Poisson loop.
-__global__ void k3_bcp(D3 d, int check_done)
-{
-    const int j = blockIdx.x * blockDim.x + threadIdx.x + 1, k = blockIdx.y;
-    if (j > d.NJ - 1 || k > d.NK) return;
-    if (check_done && d.pctl->done) return;
-    double *P = d.P;
-    P[ID3(0, j, k)] = P[ID3(1, j, k)];
-    P[ID3(d.NI, j, k)] = (3.0 * P[ID3(d.NI - 1, j, k)] - 3.0 * P[ID3(d.NI - 2, j, k)]) + P[ID3(d.NI - 3, j, k)];
 }
 
 // Block sums of NV values (warp shuffle trees, then the warps in order; thread 0 holds
@@ -2122,7 +2119,11 @@ void carve(Bump &b, fvm3_ctx *c)
     float **f32[] = {&d.RF, &d.DF, &d.ANf, &d.ATf};
     for (auto p : f32) *p = reinterpret_cast<float *>(b.take((n + 1) / 2));
     d.FB = b.take(24 * n);
-    d.nblk = 8 * 152;   // residual and reduction kernels: 8 blocks of 256 threads per SM
+    // residual and reduction kernels: 8 blocks of 256 threads per SM, no more than there are
+    // cells for (idle blocks' sums and tickets took half of a launch at 64 x 48 x 16; the
+    // zeros they added change no bit)
+    const long long cells = (long long)(c->NI - 1) * (c->NJ - 1) * (c->NK - 1);
+    d.nblk = (int)std::min<long long>(8 * 152, (cells + 255) / 256);
     d.partial = b.take(4 * size_t(d.nblk));
     d.pctl = reinterpret_cast<PCtl *>(b.take(8));
     d.scal = b.take(32);
@@ -2316,12 +2317,34 @@ static inline bool dfloat(const fvm3_ctx *c) { return c->p.precision == FVM_MIXE
         else K<double><<<(grid), (block), 0, (c)->stream>>>(__VA_ARGS__);         \
     } while (0)
 
-// BCU/BCT of the fields S (phi, ff, kind) with their periodic copies.
-int bcu(fvm3_ctx *c, const Fields &S)
+Fields poisson_field(const D3 &d, double *phi)
+{
+    Fields S{};
+    S.f[0].phi = phi;
+    S.f[0].SU = d.SU;
+    S.n = 1;
+    return S;
+}
+
+dim3 bcu_grid(const fvm3_ctx *c, int fields)
 {
     const long long nt = (long long)(c->NJ - 1) * (c->NK - 1) +
                          (2LL * (c->NJ + 1) + 2LL * (c->NK - 1)) * (c->NI + 1);
-    k3_bcu<<<dim3((unsigned)((nt + 255) / 256), S.n), 256, 0, c->stream>>>(c->d, S);
+    return dim3((unsigned)((nt + 255) / 256), fields);
+}
+
+// BCU/BCT of the fields S (phi, ff, kind) with their periodic copies.
+int bcu(fvm3_ctx *c, const Fields &S)
+{
+    k3_bcu<><<<bcu_grid(c, S.n), 256, 0, c->stream>>>(c->d, S, nullptr);
+    F3CHECK(c);
+    return FVM_OK;
+}
+
+// BCP with the periodic copy of P (stop: part of the Poisson loop).
+int bcp(fvm3_ctx *c, const PCtl *stop)
+{
+    k3_bcu<true><<<bcu_grid(c, 1), 256, 0, c->stream>>>(c->d, poisson_field(c->d, c->d.P), stop);
     F3CHECK(c);
     return FVM_OK;
 }
@@ -2345,15 +2368,6 @@ int predictor(fvm3_ctx *c, const Fields &S)
         F3RC(line(c, base + split, S, 1));
     }
     return FVM_OK;
-}
-
-Fields poisson_field(const D3 &d, double *phi)
-{
-    Fields S{};
-    S.f[0].phi = phi;
-    S.f[0].SU = d.SU;
-    S.n = 1;
-    return S;
 }
 
 // The Poisson loop body: `groups` x (res_every x [source, BCP, sweep], residual).
@@ -2406,8 +2420,7 @@ int poisson_graph(fvm3_ctx *c)
     for (int q = 0; q < groups && rc == FVM_OK && !mixed; q++) {
         for (int it = 0; it < per && rc == FVM_OK; it++) {
             k3_psu<<<g_int(c), B_INT, 0, c->stream>>>(d);
-            k3_bcp<<<dim3((c->NJ + 127) / 128, c->NK + 1), 128, 0, c->stream>>>(d, 1);
-            rc = halo(c, {d.P});
+            rc = bcp(c, d.pctl);
             if (rc == FVM_OK) rc = line(c, 6, pf, 0, d.pctl);
             if (rc == FVM_OK) rc = line(c, 6, pf, 1, d.pctl);
         }
@@ -2607,12 +2620,9 @@ int remove_grad(fvm3_ctx *c)   // main.f90:90-97: u -= dt S/J, BCU
 
 int iter_p(fvm3_ctx *c)   // main.f90:99-104: CONTRA_VEL, ITER_P, BCP
 {
-    D3 &d = c->d;
     F3RC(contra_vel(c, 1));
     F3RC(poisson(c));
-    k3_bcp<<<dim3((c->NJ + 127) / 128, c->NK + 1), 128, 0, c->stream>>>(d, 0);
-    F3RC(halo(c, {d.P}));
-    return FVM_OK;
+    return bcp(c, nullptr);
 }
 
 int correct(fvm3_ctx *c)   // main.f90:106-140: P_SOURCE, u += dt S/J, reference pressure, BCU
