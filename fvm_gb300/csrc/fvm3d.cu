@@ -101,7 +101,7 @@ struct D3 {
     // (the Poisson operator is symmetric: AS(j) = AN(j-1) and AB(k) = AT(k-1), the
     // south and bottom couplings are read as the neighbours' north and top ones)
     float *RF, *DF, *ANf, *ATf;
-    // SGS model: two banks of 12 arrays for the separable test filters
+    // SGS model: the banks of 12 arrays of the separable test filters (mixed path: one)
     double *FB;
     // reductions
     PCtl *pctl;
@@ -1552,11 +1552,17 @@ __global__ void k3_filter(D3 d, const double *in, double *out)
 
 // ---------------------------------------------------------------------------------
 // The test filter (test_filter.f90:13-21) applied separably: the [1,2,1]^3/64 box
-// filter is the product of three [1,2,1] passes, I, J, then K with the 1/64, so
-// the 22 filters of a step (the filtered velocity and temperature, the Germano
-// products, the heat-flux products) read each input three times instead of 27.
-// Bank b, array q at FB + (12 b + q) n.  The result is the reference's 27-point
-// sum up to rounding (the terms are added in another order).
+// filter is the product of three [1,2,1] passes, I, J, then K with the 1/64.  The 22
+// filters of a step (the filtered velocity and temperature, the Germano products, the
+// heat-flux products) take the I pass in the launch that forms their inputs.  Mixed path: the
+// J pass too, and the K pass where the result is used, so that an array of the bank is
+// written once and read once (six passes over it before: 693 us of a step at 256 x 192
+// x 48, now 245 and 43 more in the kernels that use them).  FP64 path: J and K are
+// passes of their own, for which the DRAM time of a pass hides its FP64 instructions; the
+// fused forms, which repeat rows, are bound by those (192 x 160 x 32, the filters and
+// the kernels that use them: 811 us fused, 752 like this).  Bank b, array q at FB + (12 b + q) n;
+// the mixed path has bank 0 only.  The result is the reference's 27-point sum up to
+// rounding (the terms are added in another order).
 // ---------------------------------------------------------------------------------
 __device__ __forceinline__ double *fbank(const D3 &d, int b, int q) { return d.FB + (size_t(12 * b + q)) * d.n; }
 // Bank elements hold doubles in the FP64 path and (hi, lo) pairs in the mixed path.
@@ -1575,40 +1581,96 @@ __device__ __forceinline__ void bank_st(const D3 &d, int b, int q, int c, dd v)
 {
     reinterpret_cast<float2 *>(fbank(d, b, q))[c] = make_float2(v.hi, v.lo);
 }
-
-enum { SEP_HATS = 0, SEP_VEL = 1, SEP_HEAT = 2 };
-
-// Filter inputs over the whole array into bank 0: U, V, W, T (SEP_HATS); the
-// velocity products uu, vv, ww, uv, uw, vw and MAG*S11, S22, S33, S12, S13, S23
-// (SEP_VEL, stress_tensor_dy.f90:266-483); uT, vT, wT and MAG*dT/dx_q (SEP_HEAT,
-// stress_tensor_dy.f90:590-680).
 template <class T>
-__global__ void k3_prod(D3 d, int mode)
+__device__ __forceinline__ T sep3(T a, T b, T c) { return (a + scale2(b, 2.0f)) + c; }
+// The filtered array q at an interior cell (mixed path: the K pass on the way).
+template <class T>
+__device__ __forceinline__ T filtered(const D3 &d, int q, int c)
 {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= d.n) return;
-    const T u = lds<T>(d, d.U, c), v = lds<T>(d, d.V, c), w = lds<T>(d, d.W, c), t = lds<T>(d, d.T, c);
-    if (mode == SEP_HATS) {
-        bank_st(d, 0, 0, c, u);
-        bank_st(d, 0, 1, c, v);
-        bank_st(d, 0, 2, c, w);
-        bank_st(d, 0, 3, c, t);
-    } else if (mode == SEP_VEL) {
+    const int o = d.NI1 * d.NJ1;
+    if constexpr (std::is_same<T, double>::value) return bank_ld<T>(d, 0, q, c);
+    else return scale2(sep3(bank_ld<T>(d, 0, q, c - o), bank_ld<T>(d, 0, q, c), bank_ld<T>(d, 0, q, c + o)), 1.0f / 64.0f);
+}
+
+// What is filtered: U, V, W, T (SEP_HATS); the velocity products uu, vv, ww, uv, uw, vw
+// and MAG*S11, S22, S33, S12, S13, S23 (SEP_VEL, stress_tensor_dy.f90:266-483); uT, vT,
+// wT and MAG*dT/dx_q (SEP_HEAT, stress_tensor_dy.f90:590-680).
+enum { SEP_HATS = 0, SEP_VEL = 1, SEP_HEAT = 2 };
+constexpr int sep_arrays(int mode) { return mode == SEP_HATS ? 4 : (mode == SEP_VEL ? 12 : 6); }
+
+template <class T, int MODE>
+__device__ __forceinline__ void sep_inputs(const D3 &d, int c, T (&x)[sep_arrays(MODE)])
+{
+    const T u = lds<T>(d, d.U, c), v = lds<T>(d, d.V, c), w = lds<T>(d, d.W, c);
+    if constexpr (MODE == SEP_HATS) {
+        x[0] = u;
+        x[1] = v;
+        x[2] = w;
+        x[3] = lds<T>(d, d.T, c);
+    } else if constexpr (MODE == SEP_VEL) {
         const T mg = lds<T>(d, d.MAG, c);
         const T uv[3] = {u, v, w};
 #pragma unroll
         for (int q = 0; q < 6; q++) {
             const int a = q < 3 ? q : (q == 5 ? 1 : 0), b = q < 3 ? q : (q == 3 ? 1 : 2);
-            bank_st(d, 0, q, c, uv[a] * uv[b]);
-            bank_st(d, 0, 6 + q, c, mg * lds<T>(d, d.L[3 * a + b], c));
+            x[q] = uv[a] * uv[b];
+            x[6 + q] = mg * lds<T>(d, d.L[3 * a + b], c);
         }
     } else {
-        const T mg = lds<T>(d, d.MAG, c);
-        bank_st(d, 0, 0, c, u * t);
-        bank_st(d, 0, 1, c, v * t);
-        bank_st(d, 0, 2, c, w * t);
+        const T t = lds<T>(d, d.T, c), mg = lds<T>(d, d.MAG, c);
+        x[0] = u * t;
+        x[1] = v * t;
+        x[2] = w * t;
 #pragma unroll
-        for (int q = 0; q < 3; q++) bank_st(d, 0, 3 + q, c, mg * lds<T>(d, d.DTD[q], c));
+        for (int q = 0; q < 3; q++) x[3 + q] = mg * lds<T>(d, d.DTD[q], c);
+    }
+}
+
+__device__ __forceinline__ double lane_up(double v) { return __shfl_up_sync(0xffffffffu, v, 1); }
+__device__ __forceinline__ double lane_down(double v) { return __shfl_down_sync(0xffffffffu, v, 1); }
+__device__ __forceinline__ dd lane_up(dd v) { return dd(__shfl_up_sync(0xffffffffu, v.hi, 1), __shfl_up_sync(0xffffffffu, v.lo, 1)); }
+__device__ __forceinline__ dd lane_down(dd v)
+{
+    return dd(__shfl_down_sync(0xffffffffu, v.hi, 1), __shfl_down_sync(0xffffffffu, v.lo, 1));
+}
+
+// The I and J passes of the inputs of MODE on every plane k, into bank 0.  A warp takes 32
+// cells along i (30 results: the neighbours come by shuffle) and walks ROWS rows along j,
+// keeping the last two rows' I sums in registers.  ROWS 0: the I pass of one row.
+// Bound: DRAM (SEP_VEL at 256 x 192 x 48, mixed: 114 us with 8 rows; with its own launch for
+// the inputs and the two passes about 220).
+template <class T, int MODE, int ROWS>
+__global__ void __launch_bounds__(128) k3_filter_ij(D3 d)
+{
+    constexpr int NQ = sep_arrays(MODE);
+    const int lane = threadIdx.x & 31, i = blockIdx.x * 30 + lane, k = blockIdx.z;
+    const int w = blockIdx.y * 4 + threadIdx.x / 32, j0 = ROWS ? w * ROWS + 1 : w;
+    if (j0 > (ROWS ? d.NJ - 1 : d.NJ)) return;
+    const bool in = i <= d.NI, out = lane >= 1 && lane <= 30 && i <= d.NI - 1;
+    T a[NQ], b[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; q++) a[q] = b[q] = T(0);
+#pragma unroll 2
+    for (int r = 0; r < (ROWS ? ROWS + 2 : 1); r++) {
+        const int j = ROWS ? j0 - 1 + r : j0;
+        if (j > d.NJ) break;
+        T x[NQ];
+        if (in) sep_inputs<T, MODE>(d, ID3(i, j, k), x);
+        else {
+#pragma unroll
+            for (int q = 0; q < NQ; q++) x[q] = T(0);
+        }
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+            const T y = sep3(lane_up(x[q]), x[q], lane_down(x[q]));
+            if (ROWS == 0) {
+                if (out) bank_st(d, 0, q, ID3(i, j, k), y);
+            } else if (r >= 2 && out) {
+                bank_st(d, 0, q, ID3(i, j - 1, k), sep3(a[q], b[q], y));
+            }
+            a[q] = b[q];
+            b[q] = y;
+        }
     }
 }
 
@@ -1616,31 +1678,39 @@ struct Out4 {
     double *p[4];
 };
 
-// One [1,2,1] pass over nq arrays from bank src to bank dst: dir 0 (I) for
-// i = 1..NI-1 on every (j, k); dir 1 (J) for j = 1..NJ-1 on every k; dir 2 (K) on
-// the interior, with the 1/64, into bank dst or, when out.p[0] is set, into out.p[q].
-template <class T>
+// FP64 path: one [1,2,1] pass over nq arrays from bank src to bank dst: dir 1 (J) for
+// j = 1..NJ-1 on every k; dir 2 (K) on the interior, with the 1/64, into bank dst or, when
+// out.p[0] is set, into out.p[q].
 __global__ void k3_sep(D3 d, int src, int dst, int nq, int dir, Out4 out)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y + (dir == 0 ? 0 : 1);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int k = blockIdx.z + (dir == 2 ? 1 : 0);
-    if (i > d.NI - 1 || j > (dir == 0 ? d.NJ : d.NJ - 1) || k > (dir == 2 ? d.NK - 1 : d.NK)) return;
-    const int c = ID3(i, j, k), o = dir == 0 ? 1 : (dir == 1 ? d.NI1 : d.NI1 * d.NJ1);
+    if (i > d.NI - 1 || j > d.NJ - 1 || k > (dir == 2 ? d.NK - 1 : d.NK)) return;
+    const int c = ID3(i, j, k), o = dir == 1 ? d.NI1 : d.NI1 * d.NJ1;
     for (int q = 0; q < nq; q++) {
-        const T r = (bank_ld<T>(d, src, q, c - o) + scale2(bank_ld<T>(d, src, q, c), 2.0f)) + bank_ld<T>(d, src, q, c + o);
-        if (dir != 2) bank_st(d, dst, q, c, r);
-        else if (out.p[0]) out.p[q][c] = to_d(scale2(r, 1.0f / 64.0f));
-        else bank_st(d, dst, q, c, scale2(r, 1.0f / 64.0f));
+        const double *s = fbank(d, src, q);
+        const double r = sep3(s[c - o], s[c], s[c + o]);
+        if (dir != 2) fbank(d, dst, q)[c] = r;
+        else (out.p[0] ? out.p[q] : fbank(d, dst, q))[c] = r * (1.0 / 64.0);
     }
 }
 
+// Mixed path: the filtered velocity and temperature.
+__global__ void k3_hats(D3 d)
+{
+    CELL3(1, d.NI - 1, 1, d.NJ - 1, 1, d.NK - 1)
+    const int c = ID3(i, j, k);
+    double *out[4] = {d.UH, d.VH, d.WH, d.TH};
+#pragma unroll
+    for (int q = 0; q < 4; q++) out[q][c] = to_d(filtered<dd>(d, q, c));
+}
+
 // Germano terms of the six velocity components (11, 22, 33, 12, 13, 23) from the
-// filtered products in bank b, accumulated into LM and MM in that order with the
+// filtered products in the bank, accumulated into LM and MM in that order with the
 // off-diagonal ones weighted 2; the strain rate of the filtered velocity and its
 // magnitude once per cell (MAGH is kept for the heat flux).
 template <class T>
-__global__ void __launch_bounds__(128, 6) k3_germano(D3 d, int b)
+__global__ void __launch_bounds__(128, 6) k3_germano(D3 d)
 {
     CELL3(1, d.NI - 1, 1, d.NJ - 1, 1, d.NK - 1)
     const int c = ID3(i, j, k);
@@ -1654,8 +1724,8 @@ __global__ void __launch_bounds__(128, 6) k3_germano(D3 d, int b)
 #pragma unroll
     for (int q = 0; q < 6; q++) {
         const int a = q < 3 ? q : (q == 5 ? 1 : 0), bb = q < 3 ? q : (q == 3 ? 1 : 2);
-        const T l = (-bank_ld<T>(d, b, q, c)) + lds<T>(d, uh[a], c) * lds<T>(d, uh[bb], c);
-        const T dout = bank_ld<T>(d, b, 6 + q, c);
+        const T l = (-filtered<T>(d, q, c)) + lds<T>(d, uh[a], c) * lds<T>(d, uh[bb], c);
+        const T dout = filtered<T>(d, 6 + q, c);
         // fac = 0.5 on the diagonal, 0.25 off it: hs = S / fac, m = ((4 magh) fac) hs
         const float fac = a == bb ? 0.5f : 0.25f;
         const T hs = scale2(S[3 * a + bb], 1.0f / fac);
@@ -1677,9 +1747,9 @@ __global__ void __launch_bounds__(128, 6) k3_germano(D3 d, int b)
 }
 
 // Temperature terms P_q, R_q of the three heat-flux components from the filtered
-// products in bank b, accumulated into LM and MM.
+// products in the bank, accumulated into LM and MM.
 template <class T>
-__global__ void k3_germano_t(D3 d, int b)
+__global__ void k3_germano_t(D3 d)
 {
     CELL3(1, d.NI - 1, 1, d.NJ - 1, 1, d.NK - 1)
     const int c = ID3(i, j, k);
@@ -1689,8 +1759,8 @@ __global__ void k3_germano_t(D3 d, int b)
     T lm, mm;
 #pragma unroll
     for (int q = 0; q < 3; q++) {
-        const T l = (-bank_ld<T>(d, b, q, c)) + lds<T>(d, uh[q], c) * lds<T>(d, d.TH, c);
-        const T dout = bank_ld<T>(d, b, 3 + q, c);
+        const T l = (-filtered<T>(d, q, c)) + lds<T>(d, uh[q], c) * lds<T>(d, d.TH, c);
+        const T dout = filtered<T>(d, 3 + q, c);
         const T g = (dxi<T>(d, M1[q], d.TH, i, j, k) + deta<T>(d, M2[q], d.TH, i, j, k)) +
                     dzeta<T>(d, M3[q], d.TH, i, j, k);
         T m = scale2(scale2(magh, 4.0f), 0.5f) * g;
@@ -2118,7 +2188,7 @@ void carve(Bump &b, fvm3_ctx *c)
     }
     float **f32[] = {&d.RF, &d.DF, &d.ANf, &d.ATf};
     for (auto p : f32) *p = reinterpret_cast<float *>(b.take((n + 1) / 2));
-    d.FB = b.take(24 * n);
+    d.FB = b.take((c->p.precision == FVM_MIXED ? 12 : 24) * n);
     // residual and reduction kernels: 8 blocks of 256 threads per SM, no more than there are
     // cells for (idle blocks' sums and tickets took half of a launch at 64 x 48 x 16; the
     // zeros they added change no bit)
@@ -2470,19 +2540,31 @@ int poisson(fvm3_ctx *c)
     return FVM_OK;
 }
 
-// The separable test filter of the inputs of `mode` (SEP_HATS: into UH, VH, WH,
-// TH; otherwise into bank 1).
-int sep_filter(fvm3_ctx *c, int mode)
+// The test filter of MODE's inputs as far as its passes are launches of their own (SEP_HATS:
+// into UH, VH, WH, TH).
+template <int MODE>
+int filter(fvm3_ctx *c)
 {
-    D3 &d = c->d;
-    const int nq = mode == SEP_HATS ? 4 : (mode == SEP_VEL ? 12 : 6);
-    Out4 none{}, hats{};
-    if (mode == SEP_HATS) hats = Out4{{d.UH, d.VH, d.WH, d.TH}};
-    F3_LAUNCH(c, k3_prod, g_lin(c), 256, d, mode);
-    const dim3 gi((c->NI - 1 + 31) / 32, (c->NJ + 1 + 3) / 4, c->NK + 1), gj((c->NI - 1 + 31) / 32, (c->NJ - 1 + 3) / 4, c->NK + 1);
-    F3_LAUNCH(c, k3_sep, gi, B_INT, d, 0, 1, nq, 0, none);
-    F3_LAUNCH(c, k3_sep, gj, B_INT, d, 1, 0, nq, 1, none);
-    F3_LAUNCH(c, k3_sep, g_int(c), B_INT, d, 0, 1, nq, 2, mode == SEP_HATS ? hats : none);
+    const D3 &d = c->d;
+    const unsigned ti = (c->NI - 1 + 29) / 30;
+    if (dfloat(c)) {
+        // longer walks read fewer rows twice; short ones where the warps would not fill the
+        // chip (SEP_VEL at 64 x 48 x 16: 11.0 us with 4 rows)
+        const bool lng = (long long)ti * ((c->NJ - 1 + 7) / 8) * (c->NK + 1) >= 16 * 152;
+        const dim3 grid(ti, (c->NJ - 1 + (lng ? 31 : 15)) / (lng ? 32 : 16), c->NK + 1);
+        if (lng) k3_filter_ij<dd, MODE, 8><<<grid, 128, 0, c->stream>>>(d);
+        else k3_filter_ij<dd, MODE, 4><<<grid, 128, 0, c->stream>>>(d);
+        if (MODE == SEP_HATS) k3_hats<<<g_int(c), B_INT, 0, c->stream>>>(d);
+    } else {
+        Out4 out{};
+        if (MODE == SEP_HATS) out = Out4{{d.UH, d.VH, d.WH, d.TH}};
+        const int nq = sep_arrays(MODE);
+        dim3 gj = g_int(c);
+        gj.z = c->NK + 1;
+        k3_filter_ij<double, MODE, 0><<<dim3(ti, (c->NJ + 1 + 3) / 4, c->NK + 1), 128, 0, c->stream>>>(d);
+        k3_sep<<<gj, B_INT, 0, c->stream>>>(d, 0, 1, nq, 1, Out4{});
+        k3_sep<<<g_int(c), B_INT, 0, c->stream>>>(d, 1, 0, nq, 2, out);
+    }
     F3CHECK(c);
     return FVM_OK;
 }
@@ -2512,7 +2594,7 @@ int sgs(fvm3_ctx *c)
     F3RC(halo_shadows(c, {d.L[0], d.L[1], d.L[2], d.L[3], d.L[4], d.L[5], d.L[6], d.L[7], d.L[8], d.DTD[0],
                           d.DTD[1], d.DTD[2]}));
     F3_LAUNCH(c, k3_mag, g_lin(c), 256, d);
-    F3RC(sep_filter(c, SEP_HATS));
+    F3RC(filter<SEP_HATS>(c));
     Fields hats = velocity(c);
     double *const H[4] = {d.UH, d.VH, d.WH, d.TH};
     for (int q = 0; q < 4; q++) hats.f[q].phi = H[q];
@@ -2521,15 +2603,15 @@ int sgs(fvm3_ctx *c)
     hats.n = 4;
     F3RC(bcu(c, hats));
     F3RC(refresh(c, {d.UH, d.VH, d.WH, d.TH}));
-    F3RC(sep_filter(c, SEP_VEL));
-    F3_LAUNCH(c, k3_germano, g_int(c), B_INT, d, 1);
+    F3RC(filter<SEP_VEL>(c));
+    F3_LAUNCH(c, k3_germano, g_int(c), B_INT, d);
     if (d.les_zavg) k3_czavg<<<dim3((c->NI - 1 + 127) / 128, c->NJ - 1), 128, 0, st>>>(d);
     else k3_cvol<<<d.nblk, 256, 0, st>>>(d, 0);
     k3_eddy<<<g_lin(c), 256, 0, st>>>(d, 0, d.EV);
     F3_LAUNCH(c, k3_sgs, g_int(c), B_INT, d);
     if (d.thermal) {
-        F3RC(sep_filter(c, SEP_HEAT));
-        F3_LAUNCH(c, k3_germano_t, g_int(c), B_INT, d, 1);
+        F3RC(filter<SEP_HEAT>(c));
+        F3_LAUNCH(c, k3_germano_t, g_int(c), B_INT, d);
         if (d.les_zavg) k3_czavg<<<dim3((c->NI - 1 + 127) / 128, c->NJ - 1), 128, 0, st>>>(d);
         else k3_cvol<<<d.nblk, 256, 0, st>>>(d, 1);
         k3_eddy<<<g_lin(c), 256, 0, st>>>(d, 1, d.EC);
