@@ -2044,6 +2044,8 @@ struct fvm3_ctx {
     fvm::PCtl *h_pctl = nullptr;
     cudaGraphExec_t pgraph = nullptr;
     int pgraph_iters = 0;
+    cudaGraphExec_t sgraph[2] = {};   // fvm3_step's launches before and after the Poisson loop
+    long long steps = 0;              // taken by fvm3_step
     fvm3_coeffs last{};
     cudaEvent_t ev_a = nullptr, ev_b = nullptr;
     // post-processing: 17 sum arrays on the device, allocated on first use
@@ -2640,15 +2642,25 @@ int read_coeffs(fvm3_ctx *c, fvm3_coeffs *out)
 }
 
 // The routines of the time loop (main.f90:33-147), one host function per call point.
-int begin_step(fvm3_ctx *c)   // main.f90:37-44, the far-field values of BCU/BCT from the step-n fields
+int begin_fields(fvm3_ctx *c)   // main.f90:37-44, the far-field values of BCU/BCT from the step-n fields
 {
     D3 &d = c->d;
-    c->niter_time += 1;
-    c->rtime = c->rtime + d.dt;
     k3_begin<<<g_lin(c), 256, 0, c->stream>>>(d);
     k3_farfield<<<dim3((c->NJ + 127) / 128, c->NK - 1), 128, 0, c->stream>>>(d);
     F3CHECK(c);
     return refresh(c, {d.U_N, d.V_N, d.W_N, d.T_N});
+}
+
+void tick(fvm3_ctx *c)
+{
+    c->niter_time += 1;
+    c->rtime = c->rtime + c->d.dt;
+}
+
+int begin_step(fvm3_ctx *c)
+{
+    tick(c);
+    return begin_fields(c);
 }
 
 int contra_vel(fvm3_ctx *c, int with_div)   // CONTRA_VEL; with_div: the Poisson source too
@@ -2729,12 +2741,21 @@ int iter_t(fvm3_ctx *c)   // main.f90:143-145: ITER_T, BCT
     return bcu(c, S);
 }
 
-int calccoef(fvm3_ctx *c)   // CALCCOEF kernels; the record is read by read_coeffs
+dim3 wall_grid(const fvm3_ctx *c) { return dim3((c->NJ - 1 + 127) / 128, c->NK - 1, 2); }
+
+int calc_sums(fvm3_ctx *c)
 {
     D3 &d = c->d;
     k3_cfl<<<dim3((c->NI - 1 + 127) / 128, c->NJ - 1, c->NK - 1), 128, 0, c->stream>>>(d);
-    const dim3 gw((c->NJ - 1 + 127) / 128, c->NK - 1, 2);
-    k3_wall<<<gw, 128, 0, c->stream>>>(d);
+    k3_wall<<<wall_grid(c), 128, 0, c->stream>>>(d);
+    F3CHECK(c);
+    return FVM_OK;
+}
+
+int calc_record(fvm3_ctx *c)
+{
+    D3 &d = c->d;
+    const dim3 gw = wall_grid(c);
     k3_calc_final<<<1, 128, 0, c->stream>>>(d, c->rtime, c->sum_area, int(gw.x * gw.y * gw.z));
     if (c->ipost && c->post) {
         k3_post_acc<<<g_lin(c), 256, 0, c->stream>>>(d, c->post);
@@ -2744,20 +2765,62 @@ int calccoef(fvm3_ctx *c)   // CALCCOEF kernels; the record is read by read_coef
     return FVM_OK;
 }
 
+int calccoef(fvm3_ctx *c)   // CALCCOEF kernels; the record is read by read_coeffs
+{
+    F3RC(calc_sums(c));
+    return calc_record(c);
+}
+
+// Part k of a step: its launches as one graph from the context's second step on (their
+// arguments do not change while it lives; a graph costs about a step of a small grid to
+// build, which a single step would not earn back).  One launch from the host reads more than
+// a kilobyte of arguments and takes longer than a kernel of a small grid: 64 x 48 x 16, two
+// steps: 1655 -> 1364 us.  Without a graph (no memory for it) the launches are made.
+template <class Body>
+int part(fvm3_ctx *c, int k, Body body)
+{
+    if (c->steps == 0) return body();
+    if (!c->sgraph[k]) {
+        cudaGraph_t g = nullptr;
+        F3CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+        const int rc = body();
+        const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+        if (rc == FVM_OK && e == cudaSuccess && cudaGraphInstantiate(&c->sgraph[k], g, 0) != cudaSuccess) c->sgraph[k] = nullptr;
+        if (g) cudaGraphDestroy(g);
+        F3RC(rc);
+        if (!c->sgraph[k]) {
+            cudaGetLastError();
+            return body();
+        }
+    }
+    F3CUDA(c, cudaGraphLaunch(c->sgraph[k], c->stream));
+    return FVM_OK;
+}
+
 int step(fvm3_ctx *c)
 {
-    F3RC(begin_step(c));
-    F3RC(contra_vel(c, 0));
-    F3RC(nl_all(c));
-    if (c->p.use_les) F3RC(sgs(c));
-    F3RC(dif_all(c));
-    F3RC(p_source(c));
-    F3RC(predictor(c, velocity(c)));   // ITER_U of U, V, W
-    F3RC(remove_grad(c));
-    F3RC(iter_p(c));
-    F3RC(correct(c));
-    F3RC(iter_t(c));
-    return calccoef(c);
+    tick(c);
+    F3RC(part(c, 0, [c] {
+        F3RC(begin_fields(c));
+        F3RC(contra_vel(c, 0));
+        F3RC(nl_all(c));
+        if (c->p.use_les) F3RC(sgs(c));
+        F3RC(dif_all(c));
+        F3RC(p_source(c));
+        F3RC(predictor(c, velocity(c)));   // ITER_U of U, V, W
+        F3RC(remove_grad(c));
+        return contra_vel(c, 1);
+    }));
+    F3RC(poisson(c));
+    F3RC(part(c, 1, [c] {
+        F3RC(bcp(c, nullptr));
+        F3RC(correct(c));
+        F3RC(iter_t(c));
+        return calc_sums(c);
+    }));
+    F3RC(calc_record(c));
+    c->steps++;
+    return FVM_OK;
 }
 
 double *array_by_name(fvm3_ctx *c, const char *name)
@@ -2869,6 +2932,8 @@ int fvm3_destroy(fvm3_ctx *c)
     if (!c) return FVM_ERR_ARG;
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->pgraph) cudaGraphExecDestroy(c->pgraph);
+    for (cudaGraphExec_t g : c->sgraph)
+        if (g) cudaGraphExecDestroy(g);
     if (c->slab) cudaFree(c->slab);
     if (c->post) cudaFree(c->post);
     if (c->h_pctl) cudaFreeHost(c->h_pctl);
