@@ -106,6 +106,7 @@ int fvm_create(const fvm_params *p, fvm_ctx **out)
     cudaError_t e = cudaSetDevice(p->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMallocHost(&c->h_pctl, sizeof(fvm::PCtl));
+    if (e == cudaSuccess) e = cudaMallocHost(&c->h_coef, sizeof(fvm_coeffs));
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev_a);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev_b);
     if (e != cudaSuccess) {
@@ -130,8 +131,10 @@ int fvm_destroy(fvm_ctx *c)
     fvm::adj_destroy(c);
     fvm::post_free(c);
     if (c->pgraph) cudaGraphExecDestroy(c->pgraph);
+    fvm::step_graphs_free(c);
     if (c->slab) cudaFree(c->slab);
     if (c->h_pctl) cudaFreeHost(c->h_pctl);
+    if (c->h_coef) cudaFreeHost(c->h_coef);
     if (c->ev_a) cudaEventDestroy(c->ev_a);
     if (c->ev_b) cudaEventDestroy(c->ev_b);
     if (c->stream) cudaStreamDestroy(c->stream);

@@ -180,6 +180,13 @@ struct fvm_ctx {
     // instrumentation
     cudaEvent_t ev_a = nullptr, ev_b = nullptr;   // span around the first sweep group of a replay
     int pgraph_kernels = 0;                       // kernel nodes in the Poisson graph
+    // run_step's launches before and after the Poisson loop (step_part), their kernels, and the
+    // view of the context that the last step's launches had
+    cudaGraphExec_t sgraph[2] = {};
+    int sgraph_kernels[2] = {};
+    fvm::Dev step_view{};
+    bool step_seen = false, step_same = false;
+    fvm_coeffs *h_coef = nullptr;                 // pinned: CALCCOEF's record, written by its kernel
     int span_launches = 0;                        // sweep kernels inside the span
     bool capturing = false;
     fvm_timing tm{};
@@ -278,6 +285,7 @@ int run_resident_wait_test(fvm_ctx *c, int max_polls);
 int step_before_poisson(const Tgt &t);
 int poisson_bodies(const Tgt &t, cudaGraphConditionalHandle cond, int has_cond, int groups);
 int step_after_poisson(const Tgt &t, double rtime, fvm_coeffs *dout);
+void step_graphs_free(fvm_ctx *c);
 int sweep_pairs(const Tgt &t, int sweeps);
 int launch_batch_tick(const Tgt &t, BatchCtl *b);
 // discrete adjoint (fvm_adjoint.cu)

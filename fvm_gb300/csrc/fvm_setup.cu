@@ -422,6 +422,7 @@ int setup_controls(fvm_ctx *c, double omega, const double *blow)
     FVM_LAUNCH_CHECK(c);
     if (c->pgraph) cudaGraphExecDestroy(c->pgraph);
     c->pgraph = nullptr;
+    step_graphs_free(c);
     return FVM_OK;
 }
 

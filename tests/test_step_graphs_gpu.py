@@ -1,0 +1,48 @@
+"""A step's launches as graphs from a context's second step on: the same bits and the same
+kernel count as the launches, through changes of the controls and of the grid."""
+import numpy as np
+import pytest
+
+from fvm_gb300 import capi
+from tests.helpers import make_case, make_gpu
+
+pytestmark = pytest.mark.gpu
+
+NAMES = ("U", "V", "P", "T", "NLX", "ADV")
+
+
+@pytest.mark.parametrize("precision", [capi.FP64, capi.MIXED], ids=["fp64", "mixed"])
+def test_graph_steps_equal_launched_steps(precision):
+    case = make_case(n_theta=24, n_r=17, skew=0.3, vel_rot=0.2, nswpp=16, resimax=0.0)
+    kw = dict(precision=precision, refine_sweeps=4)
+    a, b = make_gpu(case, **kw), make_gpu(case, **kw)
+    recs = []
+    for omega in (0.2, 0.2, 0.7):
+        a.set_controls(omega)
+        for _ in range(3):
+            b.set_controls(omega)   # the context has changed: this step launches
+            recs.append((a.step(1), b.step(1)))
+    for x, y in recs:
+        for k in ("time", "cd", "cl", "nu", "resid", "sweeps"):
+            assert x[k] == y[k], k
+    # a new grid on a context whose graphs exist
+    other = make_case(n_theta=24, n_r=17, skew=0.1, vel_rot=0.2, nswpp=16, resimax=0.0)
+    a.set_grid(other["g"].xg, other["g"].yg)
+    b.set_grid(other["g"].xg, other["g"].yg)
+    for _ in range(3):
+        b.set_controls(0.7)
+        x, y = a.step(1), b.step(1)
+        assert x["cd"] == y["cd"] and x["resid"] == y["resid"]
+    for nm in NAMES:
+        assert np.isfinite(a.get(nm)).all() and np.array_equal(a.get(nm), b.get(nm)), nm
+
+
+def test_kernels_of_a_graph_are_counted():
+    case = make_case(n_theta=24, n_r=17, skew=0.3, vel_rot=0.2, nswpp=16, resimax=0.0)
+    ctx = make_gpu(case, precision=capi.FP64)
+    counts = []
+    for _ in range(4):
+        ctx.timing_reset()
+        ctx.step(1)
+        counts.append(ctx.timing()["kernel_launches"])
+    assert len(set(counts)) == 1 and counts[0] > 8, counts
