@@ -744,6 +744,34 @@ inline bool dispatch_line(const LineSys &s, F &&f)
     }
 }
 
+// The launches of `body` as graph `g` (captured at the first call; `kernels`: what KCOUNT
+// counted in it).  Without a graph (no memory for it) the launches are made.
+template <class Body>
+int graph_part(fvm_ctx *c, cudaGraphExec_t &g, int &kernels, Body body)
+{
+    if (!g) {
+        cudaGraph_t t = nullptr;
+        FVM_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+        const int before = c->pgraph_kernels;
+        c->capturing = true;
+        const int rc = body();
+        c->capturing = false;
+        kernels = c->pgraph_kernels - before;
+        c->pgraph_kernels = before;
+        const cudaError_t e = cudaStreamEndCapture(c->stream, &t);
+        if (rc == FVM_OK && e == cudaSuccess && cudaGraphInstantiate(&g, t, 0) != cudaSuccess) g = nullptr;
+        if (t) cudaGraphDestroy(t);
+        if (rc) return rc;
+        if (!g) {
+            cudaGetLastError();
+            return body();
+        }
+    }
+    FVM_CUDA(c, cudaGraphLaunch(g, c->stream));
+    c->tm.kernel_launches += kernels;
+    return FVM_OK;
+}
+
 // Launch with programmatic stream serialization (captured into graphs as
 // programmatic edges): the kernel may begin while the preceding kernel drains.
 template <typename... KArgs, typename... Args>

@@ -1069,33 +1069,12 @@ int resident_fault(fvm_ctx *c)
 // last one left it (the launches carry it by value; whatever changes it -- a grid,
 // controls -- takes the step after it through the launches again).  A first step is not
 // worth a graph, which costs about as much to build.  Direct launches: 269 us for a step at
-// 32 x 24 FP64 against 221, 2940 us for four at 128 x 96 mixed against 2834.  Without a
-// graph (no memory for it) the launches are made.
+// 32 x 24 FP64 against 221, 2940 us for four at 128 x 96 mixed against 2834.
 template <class Body>
 int step_part(fvm_ctx *c, int k, Body body)
 {
     if (!c->step_same || c->capturing) return body();
-    if (!c->sgraph[k]) {
-        cudaGraph_t g = nullptr;
-        FVM_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-        const int before = c->pgraph_kernels;   // what KCOUNT counts into meanwhile
-        c->capturing = true;
-        const int rc = body();
-        c->capturing = false;
-        c->sgraph_kernels[k] = c->pgraph_kernels - before;
-        c->pgraph_kernels = before;
-        const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
-        if (rc == FVM_OK && e == cudaSuccess && cudaGraphInstantiate(&c->sgraph[k], g, 0) != cudaSuccess) c->sgraph[k] = nullptr;
-        if (g) cudaGraphDestroy(g);
-        RC(rc);
-        if (!c->sgraph[k]) {
-            cudaGetLastError();
-            return body();
-        }
-    }
-    FVM_CUDA(c, cudaGraphLaunch(c->sgraph[k], c->stream));
-    c->tm.kernel_launches += c->sgraph_kernels[k];
-    return FVM_OK;
+    return graph_part(c, c->sgraph[k], c->sgraph_kernels[k], body);
 }
 
 }  // namespace

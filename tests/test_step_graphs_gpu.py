@@ -46,3 +46,31 @@ def test_kernels_of_a_graph_are_counted():
         ctx.step(1)
         counts.append(ctx.timing()["kernel_launches"])
     assert len(set(counts)) == 1 and counts[0] > 8, counts
+
+
+@pytest.mark.parametrize("precision", [capi.FP64, capi.MIXED], ids=["fp64", "mixed"])
+def test_transposed_steps_repeat_themselves(precision):
+    """Launched and replayed transposed steps, before and after a change of the controls; the
+    scatters add in any order: 1e-12 of each array."""
+    case = make_case(n_theta=24, n_r=17, skew=0.3, vel_rot=0.2, nswpp=32, resimax=0.0)
+    kw = dict(precision=precision, refine_sweeps=4)
+    ctx = make_gpu(case, **kw)
+    ctx.step(1)
+    state = {nm: ctx.get(nm) for nm in ("U", "V", "P", "T", "NLX", "NLY", "ADV")}
+    names = ("U", "V", "P", "NLX", "NLY")
+    rng = np.random.default_rng(5)
+    lam = {nm: rng.standard_normal(state["U"].shape) for nm in names}
+    for omega in (0.2, 0.6):
+        ctx.set_controls(omega)
+        fresh = make_gpu(case, **kw)
+        fresh.set_controls(omega)
+        for nm, a in state.items():
+            fresh.set(nm, a)
+        want = fresh.adjoint_vjp(lam)
+        for _ in range(6):
+            got = ctx.adjoint_vjp(lam)
+            for nm in names:
+                assert np.linalg.norm(got[0][nm] - want[0][nm]) <= 1e-12 * np.linalg.norm(want[0][nm]), nm
+            assert abs(got[1] - want[1]) <= 1e-12 * max(1.0, abs(want[1]))
+        for nm, a in state.items():
+            assert np.array_equal(ctx.get(nm), a), nm
