@@ -177,6 +177,8 @@ struct Arrs {
 __global__ void k3_halo(D3 d, Arrs A)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
+    fvm::griddep_wait();
+    fvm::griddep_launch();
     if (i > d.NI) return;
     if (r <= d.NK) {
         const int k = r, ks = kw(d, k);
@@ -1165,9 +1167,9 @@ __global__ void k3_grad(D3 d, double sign)
 __global__ void k3_psu(D3 d)
 {
     CELL3(1, d.NI - 1, 1, d.NJ - 1, 1, d.NK - 1)
-    const int c = ID3(i, j, k);
-    if (d.pctl->done) return;
-    d.SU[c] = d.DIVDT[c] - cross12(d, d.P, i, j, k);
+    const int c = ID3(i, j, k), ended = d.pctl->done;   // tested after the loads
+    const double su = d.DIVDT[c] - cross12(d, d.P, i, j, k);
+    if (!ended) d.SU[c] = su;
 }
 
 // Block sums of NV values (warp shuffle trees, then the warps in order; thread 0 holds
@@ -1303,6 +1305,8 @@ __global__ void __launch_bounds__(256) k3_mres(D3 d, cudaGraphConditionalHandle 
 {
     __shared__ double sh[4 * 8];
     __shared__ bool last;
+    fvm::griddep_wait();
+    fvm::griddep_launch();
     if (d.pctl->done) return;
     const int it = d.pctl->niter;
     const Coef3 &cf = d.cf[6];
@@ -1364,9 +1368,9 @@ __global__ void __launch_bounds__(128, 6) k3_line32(const __grid_constant__ D3 d
     const int n = s.n, j = L % (d.NJ - 1) + 1, k = L / (d.NJ - 1) + 1;
     const int jn = jw(d, j + 1), js = jw(d, j - 1), kt = kw(d, k + 1), kb = kw(d, k - 1);
     const float *DF = d.DF;
-    // what no other sweep of the interval writes, before the wait for the preceding launch:
-    // couplings, right-hand side (the residual kernel does not trigger early) and factors
-    float v[M], an[M], as[M], at[M], ab[M], rf[M], fi[M], fa[M], fb[M];
+    // what no launch of a step writes, before the wait for the preceding launch: couplings and
+    // factors
+    float v[M], an[M], as[M], at[M], ab[M], fi[M], fa[M], fb[M];
 #pragma unroll
     for (int q = 0; q < M; q++) {
         const int e = q * TG + t;
@@ -1376,7 +1380,6 @@ __global__ void __launch_bounds__(128, 6) k3_line32(const __grid_constant__ D3 d
         as[q] = ok ? d.ANf[ID3(i, js, k)] : 0.0f;
         at[q] = ok ? d.ATf[c] : 0.0f;
         ab[q] = ok ? d.ATf[ID3(i, j, kb)] : 0.0f;
-        rf[q] = ok ? d.RF[c] : 0.0f;
     }
     const size_t base = size_t(L) * TG * M;
     fvm::load_factors<float, M, NW>(fi, fa, fb, s.invDf + base, s.faf + base, s.fbf + base, t);
@@ -1390,7 +1393,7 @@ __global__ void __launch_bounds__(128, 6) k3_line32(const __grid_constant__ D3 d
         if (active && e < n) {
             const int i = e + 1;
             v[q] = ((an[q] * DF[ID3(i, jn, k)] + as[q] * DF[ID3(i, js, k)]) +
-                    (at[q] * DF[ID3(i, j, kt)] + ab[q] * DF[ID3(i, j, kb)])) + rf[q];
+                    (at[q] * DF[ID3(i, j, kt)] + ab[q] * DF[ID3(i, j, kb)])) + d.RF[ID3(i, j, k)];
         }
     }
     if (stop) return;
@@ -2210,12 +2213,15 @@ const dim3 B_INT(32, 4, 1);
 inline dim3 g_full3(const fvm3_ctx *c) { return dim3((c->NI + 1 + 127) / 128, c->NJ + 1, c->NK + 1); }
 inline int g_lin(const fvm3_ctx *c) { return (c->n + 255) / 256; }
 
-int halo(fvm3_ctx *c, std::initializer_list<double *> arrs)
+// in_loop: part of the Poisson loop, launched while its predecessor finishes.
+int halo(fvm3_ctx *c, std::initializer_list<double *> arrs, bool in_loop = false)
 {
     Arrs A{};
     A.n = 0;
     for (double *a : arrs) A.a[A.n++] = a;
-    k3_halo<<<dim3((c->NI + 1 + 127) / 128, c->NK + 1 + c->NJ + 1), 128, 0, c->stream>>>(c->d, A);
+    const dim3 grid((c->NI + 1 + 127) / 128, c->NK + 1 + c->NJ + 1);
+    if (in_loop) fvm::launch_pdl(k3_halo, grid, dim3(128), c->stream, c->d, A);
+    else k3_halo<<<grid, 128, 0, c->stream>>>(c->d, A);
     F3CHECK(c);
     return FVM_OK;
 }
@@ -2277,7 +2283,7 @@ int line(fvm3_ctx *c, int set, const Fields &S, int colour, const PCtl *stop = n
         if (fam == 0) {
             const unsigned blocks = unsigned(S.n) * fvm::line_blocks((c->NJ - 1) / 2 * (c->NK - 1), s.NW);
             if (dfl) k3_line<M, NW, dd><<<blocks, 128, 0, c->stream>>>(d, s, d.cf[set], S, colour, stop, sd);
-            else k3_line<M, NW><<<blocks, 128, 0, c->stream>>>(d, s, d.cf[set], S, colour, stop, sd);
+            else k3_line<M, NW, double><<<blocks, 128, 0, c->stream>>>(d, s, d.cf[set], S, colour, stop, sd);
             return;
         }
         const int per = (c->NI / 2) * ((fam == 1 ? c->NK : c->NJ) - 1);
@@ -2480,13 +2486,12 @@ int poisson_graph(fvm3_ctx *c)
     int rc = FVM_OK;
     for (int q = 0; q < groups && rc == FVM_OK && mixed; q++) {
         // residual (ends the loop), FP32 correction sweeps, P += dP, ghosts
-        if (dev_loop) k3_mres<1><<<d.nblk, 256, 0, c->stream>>>(d, h);
-        else k3_mres<0><<<d.nblk, 256, 0, c->stream>>>(d, h);
+        fvm::launch_pdl(dev_loop ? k3_mres<1> : k3_mres<0>, dim3(d.nblk), dim3(256), c->stream, d, h);
         for (int it = 0; it < per && rc == FVM_OK; it++) {
             rc = line32(c, 0, 1, 0);
             if (rc == FVM_OK) rc = line32(c, 1, 1, it == per - 1);   // the last one adds dP and the BCP ghosts
         }
-        if (rc == FVM_OK) rc = halo(c, {d.P});
+        if (rc == FVM_OK) rc = halo(c, {d.P}, true);
     }
     const Fields pf = poisson_field(d, d.P);
     for (int q = 0; q < groups && rc == FVM_OK && !mixed; q++) {
