@@ -662,6 +662,8 @@ def run_les3d_bench(args):
     pk = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(pk):
         peaks = json.load(open(pk))
+    clk = ClockSampler(local)
+    clk.open()
     res = {}
     parts = {"all": (("mixed", capi.MIXED), ("fp64", capi.FP64)), "mixed": (("mixed", capi.MIXED),),
              "fp64": (("fp64", capi.FP64),)}[args.parts]
@@ -673,9 +675,7 @@ def run_les3d_bench(args):
         print(f"les3d {name}: {args.warmup} warm-up steps {time.perf_counter() - t0:.1f} s", file=sys.stderr,
               flush=True)
         dist.barrier()
-        clk = ClockSampler(local) if name == "mixed" else None
-        if clk:
-            clk.start()
+        clk.begin()
         ms, sweeps = 0.0, []
         for _ in range(args.steps):
             flush.fill_(1.0)
@@ -688,17 +688,18 @@ def run_les3d_bench(args):
             b.synchronize()
             ms += a.elapsed_time(b)
             sweeps.append(c["sweeps"])
-        clocks = clk.stop() if clk else None
+        clk.end()
         dist.barrier()
         ms = dist.max_over_ranks(ms, device="cuda")
         sweep_ms = ctx.time_sweeps(50)
         fields = {nm: ctx.get(nm) for nm in ("U", "V", "W", "P", "T")}
-        res[name] = dict(ms=ms, sweeps=sweeps, clocks=clocks, cd=c["cd"], resid=c["resid"], sweep_ms=sweep_ms,
+        res[name] = dict(ms=ms, sweeps=sweeps, cd=c["cd"], resid=c["resid"], sweep_ms=sweep_ms,
                          fields=fields, u_max=float(np.abs(fields["U"]).max()))
         print(f"les3d {name}: {ms / args.steps:.1f} ms/step, sweeps {sweeps}, sweep pair {sweep_ms * 1e3:.1f} us",
               file=sys.stderr, flush=True)
         ctx.close()
     if args.parts != "all":   # profiling runs: one precision only
+        clk.close()
         if rank == 0:
             nm = parts[0][0]
             print(json.dumps({"metric": METRIC, "workload": w["name"], "parts": nm,
