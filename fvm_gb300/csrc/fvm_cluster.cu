@@ -22,7 +22,9 @@
 // Operands sit in shared memory rather than in registers so that two blocks of 512 threads
 // fit an SM for up to 16 lines of 192 cells a block (the south coupling of a line is the north coupling
 // of the line below: the operator is symmetric): one block's barrier hides behind the
-// other's solves.
+// other's solves (operands in registers, one block per SM: 8 % slower).  Measured: 64 ragged
+// cases of 64..256 x 48..192 cells, two steps of 512 sweeps with their transfers, 44.9 -> 27.2
+// ms; 64 cases, 2048 sweeps, 35.4 -> 24.4 ms a step.
 #include <cooperative_groups.h>
 
 #include <algorithm>

@@ -44,8 +44,8 @@
 // exchange, 0.41 us one way through L2, twice a sweep.  The products of the constant
 // factors that the line solve's scans carry are formed once per launch and kept in
 // shared memory: per sweep only the value part of the scans is left.
-// Measured (step with 512 or 2048 sweeps, residual every 8): 128 x 96 FP64 7.51 -> 2.27 ms
-// (14.3 -> 3.9 us per sweep), 512 x 384 39.6 -> 16.6 ms (18 -> 7.6 us; 196,608 cells x 11
+// Measured (step with 512 or 2048 sweeps, residual every 8): 128 x 96 FP64 7.48 -> 2.17 ms
+// (14.3 -> 3.9 us per sweep), 512 x 384 39.8 -> 16.1 ms (18 -> 7.6 us; 196,608 cells x 11
 // instructions at the chip's 0.63 T/s: 3.4 us).
 #include <algorithm>
 #include <type_traits>
