@@ -151,8 +151,9 @@ void drop_graph(fvm_batch *b)
 }
 
 // The mixed Poisson iteration with one cluster per case, captured on the batch's streams:
-// cases of 16 blocks in one launch, those of 8 in another beside it, each from the most to the fewest cells so that the last to finish are small.  Returns
-// false (nothing captured) when a case has no cluster form.
+// cases of 16 blocks in one launch, those of 8 in another beside it, each from the most to
+// the fewest cells so that the last to finish are small.  Returns false (nothing captured)
+// when a case has no cluster form.
 bool cluster_plan(fvm_batch *b, std::vector<int> (&cls)[2], size_t (&smem)[2])
 {
     for (int k = 0; k < b->ncases; k++) {
