@@ -177,8 +177,6 @@ struct Arrs {
 __global__ void k3_halo(D3 d, Arrs A)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
-    fvm::griddep_wait();
-    fvm::griddep_launch();
     if (i > d.NI) return;
     if (r <= d.NK) {
         const int k = r, ks = kw(d, k);
@@ -892,15 +890,30 @@ __device__ __forceinline__ T nl3(const D3 &d, const double *in, int c, int i, in
                   0.5f);
 }
 
-// The 12 edge neighbours of a cell: (+-1,+-1,0), (+-1,0,+-1), (0,+-1,+-1) in the
-// order (+,+), (+,-), (-,+), (-,-) of each pair.
-__device__ __forceinline__ int edge_off(const D3 &d, int e)
+// Steps from a cell to its neighbours along J and K: as stored, ghosts included, or ...
+struct Steps {
+    int jp, jm, kp, km;
+};
+__device__ __forceinline__ Steps stored_steps(const D3 &d)
 {
     const int sj = d.NI1, sk = d.NI1 * d.NJ1;
-    const int a = (e & 2) ? -1 : 1, b = (e & 1) ? -1 : 1;
-    if (e < 4) return a + b * sj;
-    if (e < 8) return a + b * sk;
-    return a * sj + b * sk;
+    return {sj, -sj, sk, -sk};
+}
+// ... through the periodic wrap.
+__device__ __forceinline__ Steps wrapped_steps(const D3 &d, int j, int k)
+{
+    const int sj = d.NI1, sk = d.NI1 * d.NJ1;
+    return {(jw(d, j + 1) - j) * sj, (jw(d, j - 1) - j) * sj, (kw(d, k + 1) - k) * sk, (kw(d, k - 1) - k) * sk};
+}
+
+// The 12 edge neighbours of a cell: (+-1,+-1,0), (+-1,0,+-1), (0,+-1,+-1) in the
+// order (+,+), (+,-), (-,+), (-,-) of each pair.
+__device__ __forceinline__ int edge_off(const Steps &o, int e)
+{
+    const bool a = (e & 2) == 0, b = (e & 1) == 0;
+    if (e < 4) return (a ? 1 : -1) + (b ? o.jp : o.jm);
+    if (e < 8) return (a ? 1 : -1) + (b ? o.kp : o.km);
+    return (a ? o.jp : o.jm) + (b ? o.kp : o.km);
 }
 
 // A twelve-term cross derivative (dif_diagonal.f90:13-32, iter_u.f90:61-84) is
@@ -914,7 +927,7 @@ __device__ __forceinline__ int edge_off(const D3 &d, int e)
 // far field, which leaves the (i,j) pair of CW, CWA[0] and CWA[1] and nothing of CWA[2] --
 // 36 of the 48 weights' loads and FMAs saved, the same bits.
 template <class T = double>
-__device__ __forceinline__ T cross_w(const D3 &d, double *const *W, int set, const double *f, int c, int i)
+__device__ __forceinline__ T cross_w(const D3 &d, double *const *W, int set, const double *f, int c, int i, const Steps &o)
 {
     const int pairs = d.cwp[set * d.NI1 + i];
     T s = T(0);
@@ -922,8 +935,13 @@ __device__ __forceinline__ T cross_w(const D3 &d, double *const *W, int set, con
     for (int p = 0; p < 3; p++)
         if (pairs & (1 << p))
 #pragma unroll
-            for (int e = 4 * p; e < 4 * p + 4; e++) s = fma(lds<T>(d, W[e], c), lds<T>(d, f, c + edge_off(d, e)), s);
+            for (int e = 4 * p; e < 4 * p + 4; e++) s = fma(lds<T>(d, W[e], c), lds<T>(d, f, c + edge_off(o, e)), s);
     return s;
+}
+template <class T = double>
+__device__ __forceinline__ T cross_w(const D3 &d, double *const *W, int set, const double *f, int c, int i)
+{
+    return cross_w<T>(d, W, set, f, c, i, stored_steps(d));
 }
 
 // DIF_DIAGONAL with the J*Q weights
@@ -1300,8 +1318,11 @@ __global__ void k3_coef_f32(D3 d)
     d.ATf[c] = (float)cf.AT[c];
 }
 
+// Bound: FP64 issue (73 us of 93 at 256 x 192 x 48).  Five blocks: what the compiler takes
+// by itself (40 registers, six blocks) orders the loads worse, 20.5 against 21.3 ms for two
+// steps.
 template <int HAS_COND>
-__global__ void __launch_bounds__(256) k3_mres(D3 d, cudaGraphConditionalHandle cond)
+__global__ void __launch_bounds__(256, 5) k3_mres(D3 d, cudaGraphConditionalHandle cond)
 {
     __shared__ double sh[4 * 8];
     __shared__ bool last;
@@ -1315,10 +1336,12 @@ __global__ void __launch_bounds__(256) k3_mres(D3 d, cudaGraphConditionalHandle 
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
         const int i = e % ni1 + 1, j = (e / ni1) % nj1 + 1, k = e / (ni1 * nj1) + 1, c = ID3(i, j, k);
         const double *P = d.P;
-        const double su = d.DIVDT[c] - cross12(d, P, i, j, k);
-        const double r = ((((((cf.AE[c] * P[ID3(i + 1, j, k)] + cf.AW[c] * P[ID3(i - 1, j, k)]) +
-                              cf.AN[c] * P[ID3(i, jw(d, j + 1), k)]) + cf.AS[c] * P[ID3(i, jw(d, j - 1), k)]) +
-                            cf.AT[c] * P[ID3(i, j, kw(d, k + 1))]) + cf.AB[c] * P[ID3(i, j, kw(d, k - 1))]) + su) -
+        // the cross term of the first interval reads the J and K ghosts as stored; then they
+        // would be copies of the wrapped cells, which are read instead (no copy per interval)
+        const Steps o = wrapped_steps(d, j, k);
+        const double su = d.DIVDT[c] - cross_w<double>(d, d.CW, 0, P, c, i, it == 0 ? stored_steps(d) : o);
+        const double r = ((((((cf.AE[c] * P[c + 1] + cf.AW[c] * P[c - 1]) + cf.AN[c] * P[c + o.jp]) + cf.AS[c] * P[c + o.jm]) +
+                            cf.AT[c] * P[c + o.kp]) + cf.AB[c] * P[c + o.km]) + su) -
                          cf.AP[c] * P[c];
         sum[0] += fabs(r);
         sum[1] += fabs(cf.AP[c] * P[c]);
@@ -2213,15 +2236,12 @@ const dim3 B_INT(32, 4, 1);
 inline dim3 g_full3(const fvm3_ctx *c) { return dim3((c->NI + 1 + 127) / 128, c->NJ + 1, c->NK + 1); }
 inline int g_lin(const fvm3_ctx *c) { return (c->n + 255) / 256; }
 
-// in_loop: part of the Poisson loop, launched while its predecessor finishes.
-int halo(fvm3_ctx *c, std::initializer_list<double *> arrs, bool in_loop = false)
+int halo(fvm3_ctx *c, std::initializer_list<double *> arrs)
 {
     Arrs A{};
     A.n = 0;
     for (double *a : arrs) A.a[A.n++] = a;
-    const dim3 grid((c->NI + 1 + 127) / 128, c->NK + 1 + c->NJ + 1);
-    if (in_loop) fvm::launch_pdl(k3_halo, grid, dim3(128), c->stream, c->d, A);
-    else k3_halo<<<grid, 128, 0, c->stream>>>(c->d, A);
+    k3_halo<<<dim3((c->NI + 1 + 127) / 128, c->NK + 1 + c->NJ + 1), 128, 0, c->stream>>>(c->d, A);
     F3CHECK(c);
     return FVM_OK;
 }
@@ -2485,13 +2505,12 @@ int poisson_graph(fvm3_ctx *c)
     }
     int rc = FVM_OK;
     for (int q = 0; q < groups && rc == FVM_OK && mixed; q++) {
-        // residual (ends the loop), FP32 correction sweeps, P += dP, ghosts
+        // residual (ends the loop), FP32 correction sweeps, P += dP, I ghosts
         fvm::launch_pdl(dev_loop ? k3_mres<1> : k3_mres<0>, dim3(d.nblk), dim3(256), c->stream, d, h);
         for (int it = 0; it < per && rc == FVM_OK; it++) {
             rc = line32(c, 0, 1, 0);
             if (rc == FVM_OK) rc = line32(c, 1, 1, it == per - 1);   // the last one adds dP and the BCP ghosts
         }
-        if (rc == FVM_OK) rc = halo(c, {d.P}, true);
     }
     const Fields pf = poisson_field(d, d.P);
     for (int q = 0; q < groups && rc == FVM_OK && !mixed; q++) {
