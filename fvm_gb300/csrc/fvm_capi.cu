@@ -210,10 +210,12 @@ int fvm_set_array(fvm_ctx *c, const char *name, const double *in)
     double *a = fvm::array_by_name(c, name);
     if (!a) return bad(c, "unknown array name");
     FVM_CUDA(c, cudaMemcpyAsync(a, in, sizeof(double) * c->n, cudaMemcpyHostToDevice, c->stream));
-    for (const double *g : {c->d.X, c->d.Y, c->d.XG, c->d.YG, c->d.THETA})   // what the wall forces are formed from
+    // what the wall forces and the adjoint's drag sensitivities are formed from
+    for (const double *g : {c->d.X, c->d.Y, c->d.XG, c->d.YG, c->d.THETA, c->d.AREA})
         if (a == g && c->grid_set) {
             const int rc = fvm::setup_wall_geom(c);
             if (rc) return rc;
+            fvm::adj_destroy(c);
         }
     FVM_CUDA(c, cudaStreamSynchronize(c->stream));
     return FVM_OK;

@@ -562,9 +562,12 @@ static int build_line_sets(fvm_ctx *c)
 
 // Line tiles from the parameters (0: automatic) and the factors of every line
 // family in the tile's layout.  Called at setup and again when the tile changes.
+// The adjoint keeps transposed coefficients and factors of its own, in the tile it was
+// made with: it is dropped and made anew at its next use.
 int setup_factors(fvm_ctx *c)
 {
     Dev &d = c->d;
+    adj_destroy(c);
     auto tile = [](LineSys &s, int nw, int m) {
         s.NW = nw > 0 ? nw : group_warps(s.n);
         s.M = m > 0 ? m : (s.n + WARP * s.NW - 1) / (WARP * s.NW);
