@@ -320,6 +320,7 @@ struct ResSys {
     const double *SRC;
 };
 int resident_setup(fvm_ctx *c);
+int resident_retile(fvm_ctx *c);   // resident_setup of a context whose radial tile has changed
 // the same launch on another system (the adjoint's transposed Poisson equation)
 int resident_sweeps_on(fvm_ctx *c, const ResSys &sys, int sweeps, int apply, int check_done);
 int resident_sweeps(const Tgt &t, int sweeps, int apply, int max_polls, unsigned tag_skew,

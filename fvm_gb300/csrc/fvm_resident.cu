@@ -705,7 +705,8 @@ constexpr int kResidentPolls = 1 << 21;
 int resident_setup(fvm_ctx *c)
 {
     c->res_lines = c->res_blocks = 0;
-    c->res_coop = false;
+    c->res_depth = 1;
+    c->res_loop = c->res_coop = false;
     const int want = c->p.poisson_resident;
     if (c->p.precision != FVM_MIXED || want == 0) return FVM_OK;
     const LineSys &s = c->d.sP;
@@ -751,8 +752,6 @@ int resident_setup(fvm_ctx *c)
     }
     // two sweeps per exchange where the window fits: 4 lines per block, line groups
     // of one or two warps, at least three blocks around the ring, all co-resident
-    c->res_depth = 1;
-    c->res_loop = false;
     if (c->res_lines == 4 && c->p.resident_depth != 1 && c->res_blocks >= 3) {
         cudaError_t e = cudaSuccess;
         dispatch_line(s, [&](auto m, auto nw) {
@@ -879,6 +878,21 @@ size_t exchange_words(const fvm_ctx *c)
 {
     const size_t line = 2 * size_t(c->NJ - 1) * WARP * 4 * 4;
     return (c->p.precision == FVM_MIXED ? 3 : 2) * line + 2 * 4 * size_t(RING_MAX_BLOCKS);
+}
+
+// The layout for a radial tile set after the context was created.  A layout that the
+// parameters ask for and the new tile does not allow is given up (one sweep per exchange, or
+// the per-colour kernels): the tile is the batch's, which runs none of them.  The exchange
+// words have another layout and the blocks' counts may be of another number of blocks.
+int resident_retile(fvm_ctx *c)
+{
+    const std::string err = c->err;
+    const int rc = resident_setup(c);
+    if (rc == FVM_ERR_ARG) c->err = err;
+    else if (rc) return rc;
+    if (c->pgraph) cudaGraphExecDestroy(c->pgraph);
+    c->pgraph = nullptr;
+    return resident_reset(c);
 }
 
 // After a wait ran out: the blocks' sweep counts may disagree, so clear the

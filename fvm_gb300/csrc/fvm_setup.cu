@@ -563,11 +563,13 @@ static int build_line_sets(fvm_ctx *c)
 // Line tiles from the parameters (0: automatic) and the factors of every line
 // family in the tile's layout.  Called at setup and again when the tile changes.
 // The adjoint keeps transposed coefficients and factors of its own, in the tile it was
-// made with: it is dropped and made anew at its next use.
+// made with: it is dropped and made anew at its next use.  With another radial tile the
+// layout of the on-chip Poisson sweeps is chosen again.
 int setup_factors(fvm_ctx *c)
 {
     Dev &d = c->d;
     adj_destroy(c);
+    const int old_nw = d.sP.NW, old_m = d.sP.M;
     auto tile = [](LineSys &s, int nw, int m) {
         s.NW = nw > 0 ? nw : group_warps(s.n);
         s.M = m > 0 ? m : (s.n + WARP * s.NW - 1) / (WARP * s.NW);
@@ -584,6 +586,10 @@ int setup_factors(fvm_ctx *c)
     for (auto &st : sets) {
         k_factor<<<(st.s->lines + 63) / 64, 64, 0, c->stream>>>(d, *st.cf, *st.s, st.circ);
         FVM_LAUNCH_CHECK(c);
+    }
+    if (d.sP.NW != old_nw || d.sP.M != old_m) {
+        const int rc = resident_retile(c);
+        if (rc) return rc;
     }
     return ring_setup(c);
 }
