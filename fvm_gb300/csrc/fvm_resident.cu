@@ -289,8 +289,7 @@ __global__ void __launch_bounds__(ResLayout<M, NW>::MAXT, 1)
 //
 // Bound: the serial chain of the four half-sweeps of a pair, each a line solve (two scans
 // over two warps) between block barriers, and one exchange (0.41 us one way).  The solve
-// keeps its scans' constant products in registers (group_apply_c): half the shuffles, and
-// only the stages that reach (3 of 5 on 384-cell lines with 6 elements a thread).
+// keeps its scans' constant products in registers (group_apply_c): half the shuffles.
 // Measured against one launch per interval (with the steps around it): 512 x 384, two steps of
 // 2048 sweeps 8.95 -> 6.59 ms; 128 x 96, four steps of 512 4.22 -> 3.17 ms; the transposed step
 // at 128 x 96 1.77 -> 1.19 ms.
@@ -371,7 +370,7 @@ __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
         rf[k] = !LOOP && ok ? sys.RF[c] : 0.0f;
         v[k] = 0.0f;
     }
-    const ScanConst<float> sc = scan_constants<float, M>(fa, fb, t, 0x1p-60f);
+    const ScanConst<float> sc = scan_constants<float, M>(fa, fb, t);
     const unsigned cnt0 = d.XCNT[blockIdx.x];
     const bool odd = (w & 1) != 0;
     // the outer even rows, each polled by the group next to it
