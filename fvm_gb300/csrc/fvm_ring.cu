@@ -16,7 +16,11 @@
 // operand) and reads rows j and j-2, columns i and i-2, of P^(n-1); ghost column 0 and
 // ghost row 0 hold values one BCP older, so they are P^(n-2)(1,j) and P^(n-2)(i,NJ-1).
 // A line's pressure is therefore kept in three versions.  Every operation is k_pois64's
-// and k_pres64's in the same rounding order: both paths give the same bits.
+// and k_pres64's in the same rounding order, but for scan stages whose factors are all at
+// most 2^-80, which are left out (3 to 7 % of a step): both paths give the same bits unless
+// a value lies 2^27 or more below another on its line, where they differ by at most 2^-80 of
+// the larger one a solve and, through later roundings, by units in the last place of the
+// largest.  A line with a value that is not finite is not finite throughout, as there.
 //
 // A block with lines j0 .. j1 needs from others: line j0-1 (even, version n-1: coupling
 // of j0, cross term of j0+1), line j0-2 (odd, version n-1: cross term of j0) and line
@@ -120,7 +124,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
     using Lay = RingLayout<M, NW>;
     constexpr int TG = Lay::TG, LW = Lay::LW, CST = Lay::CST;
     extern __shared__ double shm[];
-    __shared__ int s_fault;
+    __shared__ int s_fault, s_nf;
     __shared__ double s_line[2 * 8], s_tot[2 * RING_MAX_BLOCKS], s_res;
     const int L = d.NJ - 1, n = d.sP.n;
     const int pairs = L / 2, p0 = blockIdx.x * ppb, nl = 2 * min(ppb, pairs - p0), j0 = 2 * p0 + 1;
@@ -139,7 +143,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
     double *fold = cst + size_t(CST) * TG;              // [Gtot | Htot | forward | backward][NW]
     auto line = [&](int ver, int q) { return own + (size_t(ver) * nlm + q) * LW; };
     auto wrap = [L](int q) { return q < 1 ? q + L : (q > L ? q - L : q); };
-    if (threadIdx.x == 0) s_fault = 0;
+    if (threadIdx.x == 0) s_fault = s_nf = 0;
 
     // operands of the line, in the chunk ownership of the solve (element e = t*M + k)
     double fi[M], fa[M], fb[M], an[M], as[M], dv[M], c1[M], c2[M], c3[M], c4[M], v[M], su[M], sun[M], w5 = 0.0, w6 = 0.0;
@@ -211,8 +215,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
         cst[(2 * STAGES + 1) * TG + t] = lane == WARP - 1 ? 1.0 : Hx;
         if (lane == 0) fold[NW + wl] = H;
     }
-    // scan stages whose factors are all below 2^-80 (an element's value reaches no
-    // further along the line) are left out
+    // scan stages whose factors are all at most 2^-80 are left out
     int ks = 0, hs = 0;
     if (act) {
         const double tiny = 0x1p-80;
@@ -504,7 +507,10 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
         __syncthreads();
         if (threadIdx.x < WARP) {
             blocks_sum2([&](int q) { return s_tot[q]; }, gridDim.x, ra, pa);
-            if (threadIdx.x == 0) s_res = ADJ && !(pa > 0.0) ? 0.0 : ra / pa;
+            if (threadIdx.x == 0) {
+                s_res = ADJ && !(pa > 0.0) ? 0.0 : ra / pa;
+                s_nf = !(isfinite(ra) && isfinite(pa));
+            }
         }
         __syncthreads();
         if (s_fault) { bad = true; break; }
@@ -519,6 +525,22 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
         return;
     }
     if (act && !mode) {
+        // a value that is not finite fills its line, as in a solve with every stage
+        if (s_nf) {
+            bool nf = false;
+#pragma unroll
+            for (int k = 0; k < M; k++) nf = nf || (t * M + k < n && !isfinite(v[k]));
+            nf = __any_sync(0xffffffffu, nf);
+            if (NW > 1) {
+                if (lane == 0) fold[2 * NW + wl] = nf ? 1.0 : 0.0;
+                bar();
+#pragma unroll
+                for (int q = 0; q < NW; q++) nf = nf || fold[2 * NW + q] != 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < M; k++)
+                if (nf) v[k] = __longlong_as_double(0x7ff8000000000000ll);
+        }
 #pragma unroll
         for (int k = 0; k < M; k++) {
             const int e = t * M + k;

@@ -80,7 +80,10 @@ typedef struct fvm_params {
        launch, whatever poisson_host_loop says.
        FP64, single context, dd_positional = 1: the whole Poisson iteration of a step
        runs in one launch, whatever poisson_host_loop says (0: one launch per zebra
-       colour).  Same results bit for bit with the same line tile. */
+       colour).  It leaves out contributions of at most 2^-80 of the value that they come
+       from on the same line: with the same line tile the same results bit for bit
+       where no value lies 2^27 or more below another on its line, else equal to
+       rounding of the largest. */
     int poisson_resident;
     /* Resident sweeps: sweeps per exchange of boundary lines between blocks (0, the
        default: 2 where the layout allows it -- 4 lines per block, line groups of one
