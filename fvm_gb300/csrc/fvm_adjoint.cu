@@ -1172,6 +1172,25 @@ int adj_poisson_graph(fvm_ctx *c)
     return FVM_OK;
 }
 
+// The transposed iteration in one launch (max_polls, skewed: 0, or a check of its waits).
+int adj_one_launch(fvm_ctx *c, int max_polls, int skewed)
+{
+    const Adj &a = c->adj->a;
+    if (a.PC) return resident_loop_adjoint(c, adj_sys(c), max_polls, skewed);
+    return ring_launch_adjoint(c, RingSys{a.sPT.invD, a.sPT.fa, a.sPT.fb, a.cPT.AN, a.cPT.AS, a.cPT.AE, a.cPT.AW, a.cPT.AP, a.g,
+                                          a.mu, a.pctl, 4}, max_polls, skewed);
+}
+
+// A bounded wait of the on-chip sweeps ran out: clear the exchange state.
+int adj_fault(fvm_ctx *c)
+{
+    ARC(resident_reset(c));
+    FVM_CUDA(c, cudaMemsetAsync(&c->adj->a.pctl->fault, 0, sizeof(int), c->stream));
+    FVM_CUDA(c, cudaStreamSynchronize(c->stream));
+    c->err = "adjoint Poisson: a bounded wait of the on-chip sweeps ran out";
+    return FVM_ERR_TIMEOUT;
+}
+
 int adj_poisson(fvm_ctx *c)
 {
     fvm_adj *A = c->adj;
@@ -1180,9 +1199,7 @@ int adj_poisson(fvm_ctx *c)
     if (!ring) ARC(adj_poisson_graph(c));
     k_adj_pctl_reset<<<1, 1, 0, c->stream>>>(a);
     if (ring) {
-        if (a.PC) ARC(resident_loop_adjoint(c, adj_sys(c)));
-        else ARC(ring_launch_adjoint(c, RingSys{a.sPT.invD, a.sPT.fa, a.sPT.fb, a.cPT.AN, a.cPT.AS, a.cPT.AE, a.cPT.AW, a.cPT.AP, a.g,
-                                           a.mu, a.pctl, 4}));
+        ARC(adj_one_launch(c, 0, 0));
         FVM_CUDA(c, cudaMemcpyAsync(A->h_pctl, a.pctl, sizeof(PCtl), cudaMemcpyDeviceToHost, c->stream));
         FVM_CUDA(c, cudaStreamSynchronize(c->stream));
     }
@@ -1198,13 +1215,7 @@ int adj_poisson(fvm_ctx *c)
         if (A->h_pctl->done) break;
     }
     A->adj_sweeps += A->h_pctl->niter;
-    if (A->h_pctl->fault) {   // a bounded wait of the resident sweeps ran out
-        ARC(resident_reset(c));
-        FVM_CUDA(c, cudaMemsetAsync(&A->a.pctl->fault, 0, sizeof(int), c->stream));
-        FVM_CUDA(c, cudaStreamSynchronize(c->stream));
-        c->err = "adjoint Poisson: a bounded wait of the on-chip sweeps ran out";
-        return FVM_ERR_TIMEOUT;
-    }
+    if (A->h_pctl->fault) return adj_fault(c);
     if (!std::isfinite(A->h_pctl->resip)) {
         c->err = "non-finite adjoint Poisson residual";
         return FVM_ERR_NAN;
@@ -1485,6 +1496,22 @@ int run_adjoint_vjp(fvm_ctx *c, double *const *lam, double *dctrl)
     if (!rc) rc = adj_controls(c, dctrl, dctrl ? dctrl + 1 : nullptr);
     cudaStreamSynchronize(c->stream);
     return rc;
+}
+
+// The transposed form of run_loop_wait_test.
+int run_adjoint_wait_test(fvm_ctx *c, int wait, int max_polls)
+{
+    ARC(adj_setup(c));
+    fvm_adj *A = c->adj;
+    k_adj_pctl_reset<<<1, 1, 0, c->stream>>>(A->a);
+    ARC(adj_one_launch(c, max_polls, wait));
+    FVM_CUDA(c, cudaMemcpyAsync(A->h_pctl, A->a.pctl, sizeof(PCtl), cudaMemcpyDeviceToHost, c->stream));
+    FVM_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (!A->h_pctl->fault) {
+        c->err = "a wait that cannot be satisfied did not report";
+        return FVM_ERR_CUDA;
+    }
+    return adj_fault(c);
 }
 
 void adj_destroy(fvm_ctx *c)

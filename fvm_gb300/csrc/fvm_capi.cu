@@ -343,6 +343,14 @@ int fvm_resident_wait_test(fvm_ctx *c, int max_polls)
     return fvm::run_resident_wait_test(c, max_polls);
 }
 
+int fvm_loop_wait_test(fvm_ctx *c, int transposed, int wait, int max_polls)
+{
+    READY();
+    if (wait < 1 || wait > fvm::WAIT_LAST) return bad(c, "wait must be in 1 .. 4");
+    if (max_polls < 1 || max_polls > (1 << 24)) return bad(c, "max_polls must be in 1 .. 2^24");
+    return fvm::run_loop_wait_test(c, transposed != 0, wait, max_polls);
+}
+
 int fvm_resident_info(fvm_ctx *c, int *lines_per_block, int *blocks, int *sweeps_per_exchange)
 {
     READY();

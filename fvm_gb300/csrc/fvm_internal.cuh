@@ -51,6 +51,25 @@ struct Coef {
     double *afar = nullptr;    // raw AE(NI-1,j) before folding (per j)
 };
 
+// Waits of the one-launch Poisson iterations by what they wait for, numbered as in
+// fvm_loop_wait_test, and their bound; a check of the bounded waits adds WAIT_SKEW to the tags of
+// one kind (0 otherwise), which no block publishes.  FP64 ring: lines of the odd and of the even half-sweep, lines and block
+// sums of the residual.  Mixed loop: lines of the sweeps, corrections, lines and sums of
+// the residual.
+enum { WAIT_ODD = 1, WAIT_EVEN = 2, WAIT_RES = 3, WAIT_SUMS = 4, WAIT_SWEEP = 1, WAIT_CORR = 2, WAIT_LAST = 4 };
+constexpr unsigned WAIT_SKEW = 0x40000000u;
+struct Waits {
+    int max_polls = 0;
+    unsigned skew[WAIT_LAST] = {};
+};
+inline Waits waits_of(int max_polls, int skewed)   // skewed: one of WAIT_*, or 0
+{
+    Waits w;
+    w.max_polls = max_polls;
+    if (skewed) w.skew[skewed - 1] = WAIT_SKEW;
+    return w;
+}
+
 // Device control block of the Poisson iteration.
 struct PCtl {
     int niter;          // sweeps done in the current ITER_P
@@ -281,6 +300,7 @@ int run_step(fvm_ctx *c, int nsteps, fvm_coeffs *out);
 double *array_by_name(fvm_ctx *c, const char *name);
 int run_time_sweeps(fvm_ctx *c, int sweeps, double *ms_per_launch, long long *launches);
 int run_resident_wait_test(fvm_ctx *c, int max_polls);
+int run_loop_wait_test(fvm_ctx *c, int transposed, int wait, int max_polls);
 // launch sequences shared by single contexts and batches (fvm_step.cu)
 int step_before_poisson(const Tgt &t);
 int poisson_bodies(const Tgt &t, cudaGraphConditionalHandle cond, int has_cond, int groups);
@@ -292,6 +312,7 @@ int launch_batch_tick(const Tgt &t, BatchCtl *b);
 int run_adjoint(fvm_ctx *c, int window, int ckpt, double *J, double *dJ_domega, double *dJ_dblow);
 int run_adjoint_vjp(fvm_ctx *c, double *const *lam, double *dctrl);
 void adj_destroy(fvm_ctx *c);
+int run_adjoint_wait_test(fvm_ctx *c, int wait, int max_polls);
 int theta_pairs(const Tgt &t, int field, int sweeps);
 int predictor_sweeps(const Tgt &t, int field, int fields);
 // mixed precision (fvm_mixed.cu)
@@ -325,8 +346,9 @@ int resident_retile(fvm_ctx *c);   // resident_setup of a context whose radial t
 int resident_sweeps_on(fvm_ctx *c, const ResSys &sys, int sweeps, int apply, int check_done);
 int resident_sweeps(const Tgt &t, int sweeps, int apply, int max_polls, unsigned tag_skew,
                     cudaGraphConditionalHandle cond, int has_cond, int check_done, int decide = 0);
-int resident_loop(fvm_ctx *c);   // the whole forward iteration (c->res_loop)
-int resident_loop_adjoint(fvm_ctx *c, const ResSys &sys);   // the same of the transposed equation
+// the whole forward iteration (c->res_loop), and the same of the transposed equation
+int resident_loop(fvm_ctx *c, int max_polls = 0, int skewed = 0);
+int resident_loop_adjoint(fvm_ctx *c, const ResSys &sys, int max_polls = 0, int skewed = 0);
 int resident_reset(fvm_ctx *c);
 size_t exchange_words(const fvm_ctx *c);   // 64-bit words of d.XW
 // mixed Poisson iteration of a batch, one cluster per case (fvm_cluster.cu)
@@ -347,8 +369,8 @@ struct RingSys {
     PCtl *pctl;
     int per;
 };
-int ring_launch(fvm_ctx *c, int mode, int count);
-int ring_launch_adjoint(fvm_ctx *c, const RingSys &sys);
+int ring_launch(fvm_ctx *c, int mode, int count, int max_polls = 0, int skewed = 0);
+int ring_launch_adjoint(fvm_ctx *c, const RingSys &sys, int max_polls = 0, int skewed = 0);
 }  // namespace fvm
 
 // ---------------------------------------------------------------------------------

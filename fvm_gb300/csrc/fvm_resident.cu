@@ -330,7 +330,7 @@ __device__ __forceinline__ unsigned long long *loop_words(const Dev &d, int what
 template <int M, int NW, int HAS_COND, int LOOP>
 __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
     k_pois32_resident2(const __grid_constant__ Dev d, const __grid_constant__ ResSys sys, int S, int apply,
-                       int check_done, int max_polls, unsigned tag_skew, cudaGraphConditionalHandle cond)
+                       int check_done, const __grid_constant__ Waits waits, cudaGraphConditionalHandle cond)
 {
     using Lay = ResLayout2<M, NW>;
     constexpr int TG = Lay::TG, LW = Lay::LW, B = Lay::B, NL = Lay::NL, PL = Lay::PL;
@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
 #pragma unroll
         for (int k = 0; k < M; k++)
             if (t * M + k < n) pending |= 1u << k;
-        for (int it = 0; pending && it < max_polls; it++) {
+        for (int it = 0; pending && it < waits.max_polls; it++) {
             unsigned long long wd[M];
 #pragma unroll
             for (int k = 0; k < M; k++) wd[k] = ((pending >> k) & 1u) ? ld_word(src + k * TG + t) : 0ull;
@@ -421,7 +421,8 @@ __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
         __syncthreads();
         for (int sw = 1; sw <= S; sw += 2) {   // sweeps sw and sw+1
             if (sw > 1 && hrow >= 0)
-                poll(d.XW + (size_t(((sw - 1) >> 1) & 1) * L + (hline - 1)) * LW, cnt + unsigned(sw - 1) + tag_skew,
+                poll(d.XW + (size_t(((sw - 1) >> 1) & 1) * L + (hline - 1)) * LW,
+                     cnt + unsigned(sw - 1) + waits.skew[WAIT_SWEEP - 1],
                      [&](int k, float x) { rows[hrow * LW + k * TG + t] = x; });
             __syncthreads();
             if (s_fault) return false;   // uniform: read by every thread after the barrier
@@ -550,13 +551,14 @@ __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
                 }
             }
             if (!own)
-                poll(rw + size_t(j - 1) * LW, rtag, [&](int k, float x) { rf[k] = x; });
+                poll(rw + size_t(j - 1) * LW, rtag + waits.skew[WAIT_RES - 1], [&](int k, float x) { rf[k] = x; });
             else
                 for (int q = (w - 3) * TG + t; q < 2 * nb; q += B * TG) {
                     bool got = false;
-                    for (int i = 0; !got && i < max_polls; i++) {
+                    const unsigned want = rtag + waits.skew[WAIT_SUMS - 1];
+                    for (int i = 0; !got && i < waits.max_polls; i++) {
                         const unsigned long long a = ld_word(pw + 2 * q), b = ld_word(pw + 2 * q + 1);
-                        got = unsigned(a >> 32) == rtag && unsigned(b >> 32) == rtag;
+                        got = unsigned(a >> 32) == want && unsigned(b >> 32) == want;
                         if (got) s_sum[q] = __hiloint2double((int)(unsigned)b, (int)(unsigned)a);
                     }
                     if (!got) s_fault = 1;
@@ -573,7 +575,7 @@ __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
             unsigned long long *fw = loop_words(d, 0, round & 1, L, LW);
             if (own && w != (ADJ ? 5 : 4)) post(fw + size_t(j - 1) * LW, cnt);
             if (pl >= 0 && pl < PL && !own)
-                poll(fw + size_t(j - 1) * LW, cnt, [&](int k, float x) { v[k] = x; });
+                poll(fw + size_t(j - 1) * LW, cnt + waits.skew[WAIT_CORR - 1], [&](int k, float x) { v[k] = x; });
             if (pl >= 0 && pl < PL) {
 #pragma unroll
                 for (int k = 0; k < M; k++) {
@@ -655,7 +657,7 @@ __global__ void __launch_bounds__(ResLayout2<M, NW>::NT, 1)
 
 template <int M, int NW, int HAS_COND, int LOOP>
 cudaError_t launch_resident2(const fvm_ctx *c, const ResSys &sys, cudaStream_t st, int S, int apply, int check_done,
-                             int max_polls, unsigned skew, cudaGraphConditionalHandle cond)
+                             int max_polls, int skewed, cudaGraphConditionalHandle cond)
 {
     using Lay = ResLayout2<M, NW>;
     cudaLaunchConfig_t cfg = {};
@@ -668,8 +670,8 @@ cudaError_t launch_resident2(const fvm_ctx *c, const ResSys &sys, cudaStream_t s
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = c->res_coop ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k_pois32_resident2<M, NW, HAS_COND, LOOP>, c->d, sys, S, apply, check_done, max_polls,
-                              skew, cond);
+    return cudaLaunchKernelEx(&cfg, k_pois32_resident2<M, NW, HAS_COND, LOOP>, c->d, sys, S, apply, check_done,
+                              waits_of(max_polls, skewed), cond);
 }
 
 template <int M, int NW, int HAS_COND>
@@ -806,8 +808,9 @@ int launch_sys(fvm_ctx *c, const ResSys &sys, cudaStream_t st, int sweeps, int a
         constexpr int M_ = decltype(m)::value, NW_ = decltype(nw)::value;
         if constexpr (NW_ <= 2) {
             if (pairs) {
-                if (has_cond) e = launch_resident2<M_, NW_, 1, 0>(c, sys, st, sweeps, apply, check_done, polls, tag_skew, cond);
-                else e = launch_resident2<M_, NW_, 0, 0>(c, sys, st, sweeps, apply, check_done, polls, tag_skew, cond);
+                const int skewed = tag_skew ? WAIT_SWEEP : 0;
+                if (has_cond) e = launch_resident2<M_, NW_, 1, 0>(c, sys, st, sweeps, apply, check_done, polls, skewed, cond);
+                else e = launch_resident2<M_, NW_, 0, 0>(c, sys, st, sweeps, apply, check_done, polls, skewed, cond);
                 return;
             }
         }
@@ -840,13 +843,14 @@ int resident_sweeps(const Tgt &t, int sweeps, int apply, int max_polls, unsigned
 
 namespace {
 template <int LOOP>
-int launch_loop(fvm_ctx *c, const ResSys &sys)
+int launch_loop(fvm_ctx *c, const ResSys &sys, int max_polls, int skewed)
 {
     cudaError_t e = cudaErrorInvalidValue;
     dispatch_line(c->d.sP, [&](auto m, auto nw) {
         constexpr int M_ = decltype(m)::value, NW_ = decltype(nw)::value;
         if constexpr (NW_ <= 2)
-            e = launch_resident2<M_, NW_, 0, LOOP>(c, sys, c->stream, c->d.refine_sweeps, 0, 0, kResidentPolls, 0u, 0);
+            e = launch_resident2<M_, NW_, 0, LOOP>(c, sys, c->stream, c->d.refine_sweeps, 0, 0,
+                                                  max_polls > 0 ? max_polls : kResidentPolls, skewed, 0);
     });
     if (e != cudaSuccess) {
         c->err = std::string("resident Poisson loop launch: ") + cudaGetErrorString(e);
@@ -859,8 +863,11 @@ int launch_loop(fvm_ctx *c, const ResSys &sys)
 
 // The whole iteration whose source is in place: the forward pressure, and another system
 // of the context's line tile with the transposed cross term.
-int resident_loop(fvm_ctx *c) { return launch_loop<1>(c, forward_sys(c)); }
-int resident_loop_adjoint(fvm_ctx *c, const ResSys &sys) { return launch_loop<2>(c, sys); }
+int resident_loop(fvm_ctx *c, int max_polls, int skewed) { return launch_loop<1>(c, forward_sys(c), max_polls, skewed); }
+int resident_loop_adjoint(fvm_ctx *c, const ResSys &sys, int max_polls, int skewed)
+{
+    return launch_loop<2>(c, sys, max_polls, skewed);
+}
 
 // The same sweeps on another system of the context's line tile (the adjoint's
 // transposed Poisson equation); no graph condition, default wait bound.

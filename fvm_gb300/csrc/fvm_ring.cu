@@ -32,8 +32,11 @@
 // n+2 needs neighbours that needed the readers' sweep n+1.  While one colour is solved
 // the other colour's groups form their next cross terms.  The residual's block sums
 // travel the same way and every block adds them in the same order, so all blocks take
-// the same decision.  Every wait is bounded; one that runs out sets the fault flag, the
-// pressure is left alone and the host reports FVM_ERR_TIMEOUT.
+// the same decision.  Every wait is bounded; one that runs out sets the flag of its
+// phase (odd lines, even lines, residual), which the whole block reads after the phase's
+// barrier and nobody writes before another barrier, so that all threads leave together; the
+// pressure is left alone and the host reports FVM_ERR_TIMEOUT.  Waits::skew lets
+// the waits of one kind look for tags that no block publishes: the check of those exits.
 //
 // ADJ: the transposed equation of the adjoint, (A^T + G^T DD^T) mu = g (fvm_adjoint.cu).
 // Its lagged cross term at (i,j) reads mu^(n-1) at rows j and j+2 (wrapped), columns i and
@@ -92,13 +95,13 @@ __device__ __forceinline__ double of_words(unsigned long long a, unsigned long l
 // The M elements of a line that thread t owns, once their words carry the tag; false
 // when the wait ran out.  One L2 round trip per poll: all loads precede the tests.
 template <int M, int TG>
-__device__ __forceinline__ bool poll_line(const ulonglong2 *src, int t, int n, unsigned want, double (&out)[M])
+__device__ __forceinline__ bool poll_line(const ulonglong2 *src, int t, int n, unsigned want, int max_polls, double (&out)[M])
 {
     unsigned pending = 0;
 #pragma unroll
     for (int k = 0; k < M; k++)
         if (t * M + k < n) pending |= 1u << k;
-    for (int it = 0; pending && it < kRingPolls; it++) {
+    for (int it = 0; pending && it < max_polls; it++) {
         unsigned long long a[M], b[M];
 #pragma unroll
         for (int k = 0; k < M; k++) {
@@ -119,12 +122,13 @@ __device__ __forceinline__ bool poll_line(const ulonglong2 *src, int t, int n, u
 // (timing).
 template <int M, int NW, int ADJ>
 __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
-    k_ring64(const __grid_constant__ Dev d, const __grid_constant__ RingSys sys, int ppb, int mode, int count)
+    k_ring64(const __grid_constant__ Dev d, const __grid_constant__ RingSys sys, int ppb, int mode, int count,
+             const __grid_constant__ Waits waits)
 {
     using Lay = RingLayout<M, NW>;
     constexpr int TG = Lay::TG, LW = Lay::LW, CST = Lay::CST;
     extern __shared__ double shm[];
-    __shared__ int s_fault, s_nf;
+    __shared__ int s_fault[3], s_nf;   // a wait of the odd half-sweep, the even one, the residual ran out
     __shared__ double s_line[2 * 8], s_tot[2 * RING_MAX_BLOCKS], s_res;
     const int L = d.NJ - 1, n = d.sP.n;
     const int pairs = L / 2, p0 = blockIdx.x * ppb, nl = 2 * min(ppb, pairs - p0), j0 = 2 * p0 + 1;
@@ -143,7 +147,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
     double *fold = cst + size_t(CST) * TG;              // [Gtot | Htot | forward | backward][NW]
     auto line = [&](int ver, int q) { return own + (size_t(ver) * nlm + q) * LW; };
     auto wrap = [L](int q) { return q < 1 ? q + L : (q > L ? q - L : q); };
-    if (threadIdx.x == 0) s_fault = s_nf = 0;
+    if (threadIdx.x == 0) s_fault[0] = s_fault[1] = s_fault[2] = s_nf = 0;
 
     // operands of the line, in the chunk ownership of the solve (element e = t*M + k)
     double fi[M], fa[M], fb[M], an[M], as[M], dv[M], c1[M], c2[M], c3[M], c4[M], v[M], su[M], sun[M], w5 = 0.0, w6 = 0.0;
@@ -354,9 +358,11 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
         for (int k = 0; k < M; k++)
             if (t * M + k < n) st_words(dst + k * TG + t, v[k], cnt0 + unsigned(m));
     };
-    auto wait_line = [&](int q, int m) {
-        if (!poll_line<M, TG>(slot(cnt0 + unsigned(m), q), t, n, cnt0 + unsigned(m), hal)) s_fault = 1;
+    auto wait_into = [&](int kind, int q, int m, double (&x)[M]) {
+        const unsigned tag = cnt0 + unsigned(m);
+        if (!poll_line<M, TG>(slot(tag, q), t, n, tag + waits.skew[kind - 1], waits.max_polls, x)) s_fault[kind - 1] = 1;
     };
+    auto wait_line = [&](int kind, int q, int m) { wait_into(kind, q, m, hal); };
 
     if (act && odd) source(1, su);
     int m = 0, have = 0;   // sweeps done; have: group 0's halo already holds version m
@@ -369,7 +375,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
             const int vr = (m + 2) % 3, vw = m % 3;
             if (act) {
                 if (odd) {
-                    if (g == 0 && m > 1 && !have) wait_line(jm1, m - 1);
+                    if (g == 0 && m > 1 && !have) wait_line(WAIT_ODD, jm1, m - 1);
                     const double *pn = line(vr, g + 1), *ps = g == 0 ? nullptr : line(vr, g - 1);
 #pragma unroll
                     for (int k = 0; k < M; k++) {
@@ -388,8 +394,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
                         double x[M];
 #pragma unroll
                         for (int k = 0; k < M; k++) x[k] = 0.0;
-                        const unsigned want = cnt0 + unsigned(m - 1);
-                        if (!poll_line<M, TG>(slot(want, je), t, n, want, x)) s_fault = 1;
+                        wait_into(WAIT_ODD, je, m - 1, x);
 #pragma unroll
                         for (int k = 0; k < M; k++) hm1[size_t(vr) * LW + k * TG + t] = x[k];
                         bar();
@@ -400,10 +405,10 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
             }
             have = 0;
             __syncthreads();
-            if (s_fault) { bad = true; break; }   // uniform: read by every thread after the barrier
+            if (s_fault[0]) { bad = true; break; }   // uniform: this flag is next written after another barrier
             if (act) {
                 if (!odd) {
-                    if (g == nl - 1) wait_line(wrap(j + 1), m);
+                    if (g == nl - 1) wait_line(WAIT_EVEN, wrap(j + 1), m);
                     const double *pn = g == nl - 1 ? nullptr : line(vw, g + 1), *ps = line(vw, g - 1);
 #pragma unroll
                     for (int k = 0; k < M; k++) {
@@ -419,8 +424,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
                         double x[M];
 #pragma unroll
                         for (int k = 0; k < M; k++) x[k] = 0.0;
-                        const unsigned want = cnt0 + unsigned(m);
-                        if (!poll_line<M, TG>(slot(want, jo), t, n, want, x)) s_fault = 1;
+                        wait_into(WAIT_EVEN, jo, m, x);
 #pragma unroll
                         for (int k = 0; k < M; k++) hm2[size_t(vw) * LW + k * TG + t] = x[k];
                         bar();
@@ -430,7 +434,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
                 }
             }
             __syncthreads();
-            if (s_fault) { bad = true; break; }
+            if (s_fault[1]) { bad = true; break; }
         }
         if (bad || mode) break;
         // scaled-L1 residual of P^m with the last sweep's source (of mu^m with its own)
@@ -446,8 +450,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
                         double x[M];
 #pragma unroll
                         for (int k = 0; k < M; k++) x[k] = 0.0;
-                        const unsigned want = cnt0 + unsigned(m);
-                        if (!poll_line<M, TG>(slot(want, je), t, n, want, x)) s_fault = 1;
+                        wait_into(WAIT_RES, je, m, x);
 #pragma unroll
                         for (int k = 0; k < M; k++) hm1[size_t(vw) * LW + k * TG + t] = x[k];
                         bar();
@@ -463,7 +466,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
                 aw[k] = e < n ? sys.AW[c] : 0.0;
                 ap[k] = e < n ? sys.AP[c] : 0.0;
             }
-            if (g == 0) wait_line(jm1, m);
+            if (g == 0) wait_line(WAIT_RES, jm1, m);
             const double *self = line(vw, g);
 #pragma unroll
             for (int k = 0; k < M; k++) {
@@ -496,13 +499,14 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
         }
         for (int q = threadIdx.x; q < 2 * (int)gridDim.x; q += blockDim.x) {
             bool got = false;
-            for (int it = 0; !got && it < kRingPolls; it++) {
+            const unsigned want = rtag + waits.skew[WAIT_SUMS - 1];
+            for (int it = 0; !got && it < waits.max_polls; it++) {
                 unsigned long long a, b;
                 ld_words(ps + q, a, b);
-                got = unsigned(a >> 32) == rtag && unsigned(b >> 32) == rtag;
+                got = unsigned(a >> 32) == want && unsigned(b >> 32) == want;
                 if (got) s_tot[q] = of_words(a, b);
             }
-            if (!got) s_fault = 1;
+            if (!got) s_fault[2] = 1;
         }
         __syncthreads();
         if (threadIdx.x < WARP) {
@@ -513,7 +517,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
             }
         }
         __syncthreads();
-        if (s_fault) { bad = true; break; }
+        if (s_fault[2]) { bad = true; break; }
         resip = s_res;
         if (!(resip > d.resimax && m < d.nswpp)) break;
     }
@@ -607,7 +611,7 @@ int ring_setup(fvm_ctx *c)
 
 namespace {
 template <int ADJ>
-int launch(fvm_ctx *c, const RingSys &sys, int mode, int count)
+int launch(fvm_ctx *c, const RingSys &sys, int mode, int count, int max_polls, int skewed)
 {
     cudaError_t e = cudaErrorInvalidValue;
     dispatch_line(c->d.sP, [&](auto m, auto nw) {
@@ -623,7 +627,8 @@ int launch(fvm_ctx *c, const RingSys &sys, int mode, int count)
         at[0].val.cooperative = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, k_ring64<M_, NW_, ADJ>, c->d, sys, c->d.ring_ppb, mode, count);
+        e = cudaLaunchKernelEx(&cfg, k_ring64<M_, NW_, ADJ>, c->d, sys, c->d.ring_ppb, mode, count,
+                               waits_of(max_polls > 0 ? max_polls : kRingPolls, skewed));
     });
     if (e != cudaSuccess) {
         c->err = std::string("Poisson ring launch: ") + cudaGetErrorString(e);
@@ -635,15 +640,19 @@ int launch(fvm_ctx *c, const RingSys &sys, int mode, int count)
 }  // namespace
 
 // The FP64 Poisson iteration of a context whose source term is in place (mode 0), or
-// `count` sweeps on chip (mode 1).  Cooperative: all blocks resident at once.
-int ring_launch(fvm_ctx *c, int mode, int count)
+// `count` sweeps on chip (mode 1).  Cooperative: all blocks resident at once.  max_polls 0: the
+// default bound of a wait.
+int ring_launch(fvm_ctx *c, int mode, int count, int max_polls, int skewed)
 {
     const Dev &d = c->d;
     return launch<0>(c, RingSys{d.sP.invD, d.sP.fa, d.sP.fb, d.cP.AN, d.cP.AS, d.cP.AE, d.cP.AW, d.cP.AP, d.DIVDT, d.P, d.pctl,
-                                d.res_every}, mode, count);
+                                d.res_every}, mode, count, max_polls, skewed);
 }
 
 // The adjoint's transposed equation, its factors in the layout of the radial tile.
-int ring_launch_adjoint(fvm_ctx *c, const RingSys &sys) { return launch<1>(c, sys, 0, 0); }
+int ring_launch_adjoint(fvm_ctx *c, const RingSys &sys, int max_polls, int skewed)
+{
+    return launch<1>(c, sys, 0, 0, max_polls, skewed);
+}
 
 }  // namespace fvm

@@ -1093,7 +1093,26 @@ int run_resident_wait_test(fvm_ctx *c, int max_polls)
         return FVM_ERR_ARG;
     }
     // four sweeps: waits at sweeps 2-4 (one exchange per sweep) or at sweep 3 (per pair)
-    RC(resident_sweeps(tgt_of(c), 4, 0, max_polls, 0x40000000u, 0, 0, 0));
+    RC(resident_sweeps(tgt_of(c), 4, 0, max_polls, WAIT_SKEW, 0, 0, 0));
+    FVM_CUDA(c, cudaMemcpyAsync(c->h_pctl, c->d.pctl, sizeof(PCtl), cudaMemcpyDeviceToHost, c->stream));
+    FVM_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (!c->h_pctl->fault) {
+        c->err = "a wait that cannot be satisfied did not report";
+        return FVM_ERR_CUDA;
+    }
+    return resident_fault(c);
+}
+
+// The one-launch iteration with the waits of one kind (WAIT_*) looking for tags no block
+// publishes.  It leaves the unknown alone when one runs out.
+int run_loop_wait_test(fvm_ctx *c, int transposed, int wait, int max_polls)
+{
+    if (!c->ring_blocks && !c->res_loop) {
+        c->err = "the context's Poisson iteration is not one launch";
+        return FVM_ERR_ARG;
+    }
+    if (transposed) return run_adjoint_wait_test(c, wait, max_polls);
+    RC(c->ring_blocks ? ring_launch(c, 0, 0, max_polls, wait) : resident_loop(c, max_polls, wait));
     FVM_CUDA(c, cudaMemcpyAsync(c->h_pctl, c->d.pctl, sizeof(PCtl), cudaMemcpyDeviceToHost, c->stream));
     FVM_CUDA(c, cudaStreamSynchronize(c->stream));
     if (!c->h_pctl->fault) {

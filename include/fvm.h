@@ -239,6 +239,12 @@ int fvm_time_sweeps(struct fvm_ctx *ctx, int sweeps, double *ms_per_launch, long
  * state is unchanged and the exchange state cleared, so the context stays usable.
  * FVM_ERR_ARG if the context does not use the resident path. */
 int fvm_resident_wait_test(struct fvm_ctx *ctx, int max_polls);
+/* The same check of the waits of the one-launch Poisson iterations: the forward one, or
+ * (transposed != 0) the adjoint's.  wait: which of its waits looks for tags that no
+ * block publishes -- FP64: 1 lines of the odd half-sweep, 2 of the even one; MIXED: 1 lines
+ * of the sweeps (refine_sweeps >= 4), 2 the neighbours' corrections; both: 3 lines of
+ * the residual, 4 its block sums.  FVM_ERR_ARG if the iteration is not one launch. */
+int fvm_loop_wait_test(struct fvm_ctx *ctx, int transposed, int wait, int max_polls);
 /* Layout of the resident Poisson sweeps the context chose: lines per block (0: the
  * per-colour path), blocks, and sweeps per exchange of boundary lines (1 or 2). */
 int fvm_resident_info(struct fvm_ctx *ctx, int *lines_per_block, int *blocks, int *sweeps_per_exchange);
