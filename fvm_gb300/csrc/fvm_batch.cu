@@ -209,7 +209,8 @@ int build_graph(fvm_batch *b)
     if (clusters) {
         std::vector<int> list(cls[0]);
         list.insert(list.end(), cls[1].begin(), cls[1].end());
-        FVM_CUDA(sh, cudaMemcpy(b->d_cases, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice));
+        // on the stream that the graph is launched on: the default stream has no order with it
+        FVM_CUDA(sh, cudaMemcpyAsync(b->d_cases, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice, st));
     }
     FVM_CUDA(sh, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     sh->capturing = true;
@@ -452,7 +453,8 @@ int fvm_batch_autotune(fvm_batch *b, int sweeps, int *tiles, double *ms)
         nt = std::max(nt, c->NJ - 1);
     }
     // the flow state is kept: the timed kernels write only scratch (Poisson) or
-    // the U field, which is saved and restored around the circumferential timing
+    // the U field, which is saved and restored around the circumferential timing (on the
+    // timing's stream)
     std::vector<double *> saved(b->ncases, nullptr);
     fvm_ctx *sh = &b->shell;
     int rc = sync_cases(b);
@@ -460,7 +462,7 @@ int fvm_batch_autotune(fvm_batch *b, int sweeps, int *tiles, double *ms)
     for (int k = 0; k < b->ncases; k++) {
         fvm_ctx *c = b->cases[k];
         FVM_CUDA(sh, cudaMalloc(&saved[k], sizeof(double) * c->n));
-        FVM_CUDA(sh, cudaMemcpy(saved[k], c->d.U, sizeof(double) * c->n, cudaMemcpyDeviceToDevice));
+        FVM_CUDA(sh, cudaMemcpyAsync(saved[k], c->d.U, sizeof(double) * c->n, cudaMemcpyDeviceToDevice, sh->stream));
     }
     int cur[4];
     fvm_batch_tiles(b, cur);
@@ -489,8 +491,9 @@ int fvm_batch_autotune(fvm_batch *b, int sweeps, int *tiles, double *ms)
     for (int k = 0; k < b->ncases; k++) {
         if (!saved[k]) continue;
         if (rc == FVM_OK) {
-            cudaError_t e = cudaMemcpy(b->cases[k]->d.U, saved[k], sizeof(double) * b->cases[k]->n,
-                                       cudaMemcpyDeviceToDevice);
+            cudaError_t e = cudaMemcpyAsync(b->cases[k]->d.U, saved[k], sizeof(double) * b->cases[k]->n,
+                                            cudaMemcpyDeviceToDevice, sh->stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(sh->stream);
             if (e != cudaSuccess) rc = berr(b, cudaGetErrorString(e), FVM_ERR_CUDA);
         }
         cudaFree(saved[k]);
