@@ -153,7 +153,7 @@ void drop_graph(fvm_batch *b)
 // The mixed Poisson iteration with one cluster per case, captured on the batch's streams:
 // cases of 16 blocks in one launch, those of 8 in another beside it, each from the most to
 // the fewest cells so that the last to finish are small.  Returns false (nothing captured)
-// when a case has no cluster form.
+// when a case has no cluster form or the device cannot hold the clusters.
 bool cluster_plan(fvm_batch *b, std::vector<int> (&cls)[2], size_t (&smem)[2])
 {
     for (int k = 0; k < b->ncases; k++) {
@@ -163,6 +163,8 @@ bool cluster_plan(fvm_batch *b, std::vector<int> (&cls)[2], size_t (&smem)[2])
         cls[q].push_back(k);
         smem[q] = std::max(smem[q], n);
     }
+    for (int q = 0; q < 2; q++)
+        if (!cls[q].empty() && !fvm::cluster_fits(b->t.tr, q == 0 ? 16 : 8, smem[q])) return false;
     for (auto &v : cls)
         std::stable_sort(v.begin(), v.end(), [b](int x, int y) { return b->cases[x]->n > b->cases[y]->n; });
     return true;

@@ -247,14 +247,15 @@ size_t cluster_bytes(const fvm_ctx *c, const LineSys &tile)
 
 int cluster_blocks(const fvm_ctx *c) { return cluster_size(c->NJ - 1); }
 
-// The iteration of the `count` cases listed in device memory, `blocks` blocks a case with
-// `smem` bytes each.
-int cluster_launch(const Tgt &t, cudaStream_t st, const int *cases, int count, int blocks, size_t smem)
+namespace {
+// f(kernel, launch configuration) for clusters of `blocks` blocks with `smem` bytes each,
+// one per case.
+template <class F>
+cudaError_t with_cluster(const LineSys &tile, int blocks, size_t smem, int count, cudaStream_t st, F &&f)
 {
     cudaError_t e = cudaErrorInvalidValue;
-    dispatch_line(t.tr, [&](auto m, auto nw) {
-        constexpr int M_ = decltype(m)::value, NW_ = decltype(nw)::value;
-        auto k = k_cluster32<M_, NW_>;
+    dispatch_line(tile, [&](auto m, auto nw) {
+        auto k = k_cluster32<decltype(m)::value, decltype(nw)::value>;
         e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLUSTER_SMEM);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return;
@@ -269,7 +270,29 @@ int cluster_launch(const Tgt &t, cudaStream_t st, const int *cases, int count, i
         at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, k, t.tab, cases);
+        e = f(k, cfg);
+    });
+    return e;
+}
+}  // namespace
+
+// Whether the device can hold such a cluster (16 blocks are more than it must offer).
+bool cluster_fits(const LineSys &tile, int blocks, size_t smem)
+{
+    int most = 0;
+    const cudaError_t e = with_cluster(tile, blocks, smem, 1, nullptr, [&](auto k, const cudaLaunchConfig_t &cfg) {
+        return cudaOccupancyMaxActiveClusters(&most, k, &cfg);
+    });
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess && most >= 1;
+}
+
+// The iteration of the `count` cases listed in device memory, `blocks` blocks a case with
+// `smem` bytes each.
+int cluster_launch(const Tgt &t, cudaStream_t st, const int *cases, int count, int blocks, size_t smem)
+{
+    const cudaError_t e = with_cluster(t.tr, blocks, smem, count, st, [&](auto k, const cudaLaunchConfig_t &cfg) {
+        return cudaLaunchKernelEx(&cfg, k, t.tab, cases);
     });
     if (e != cudaSuccess) {
         t.c->err = std::string("batched Poisson launch: ") + cudaGetErrorString(e);

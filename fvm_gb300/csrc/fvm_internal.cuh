@@ -354,6 +354,7 @@ size_t exchange_words(const fvm_ctx *c);   // 64-bit words of d.XW
 // mixed Poisson iteration of a batch, one cluster per case (fvm_cluster.cu)
 size_t cluster_bytes(const fvm_ctx *c, const LineSys &tile);
 int cluster_blocks(const fvm_ctx *c);   // blocks per case: 8 or 16
+bool cluster_fits(const LineSys &tile, int blocks, size_t smem);
 int cluster_launch(const Tgt &t, cudaStream_t st, const int *cases, int count, int blocks, size_t smem);
 // state copies between caller buffers and the device (fvm_copy.cu)
 cudaError_t copy_arrays(double *const *dst, const double *const *src, int count, size_t n, cudaMemcpyKind kind,
