@@ -1195,11 +1195,16 @@ int adj_poisson(fvm_ctx *c)
 {
     fvm_adj *A = c->adj;
     const Adj &a = A->a;
-    const bool ring = c->ring_blocks != 0 || a.PC;   // the whole iteration in one launch
-    if (!ring) ARC(adj_poisson_graph(c));
+    auto one = [&] { return c->ring_blocks != 0 || (c->res_loop && a.PC); };   // the whole iteration in one launch
+    bool ring = one();
     k_adj_pctl_reset<<<1, 1, 0, c->stream>>>(a);
     if (ring) {
-        ARC(adj_one_launch(c, 0, 0));
+        const int rc = adj_one_launch(c, 0, 0);
+        ring = one();   // false: the launch was refused
+        if (rc && ring) return rc;
+    }
+    if (!ring) ARC(adj_poisson_graph(c));
+    if (ring) {
         FVM_CUDA(c, cudaMemcpyAsync(A->h_pctl, a.pctl, sizeof(PCtl), cudaMemcpyDeviceToHost, c->stream));
         FVM_CUDA(c, cudaStreamSynchronize(c->stream));
     }

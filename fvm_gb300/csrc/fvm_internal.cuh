@@ -220,6 +220,15 @@ struct fvm_ctx {
     int post_suspend = 0;   // recomputation passes of the adjoint: no post-processing
 };
 
+// A cooperative launch that the device refuses because its blocks cannot all be resident (the
+// process has been given a part of the SMs): nothing ran, the path without it serves.
+inline bool launch_refused(cudaError_t e)
+{
+    if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorLaunchOutOfResources && e != cudaErrorNotSupported) return false;
+    cudaGetLastError();
+    return true;
+}
+
 // Count one kernel launch of the context (into the graph being captured, if any).
 #define KCOUNT(c)                                             \
     do {                                                      \
@@ -346,7 +355,8 @@ int resident_retile(fvm_ctx *c);   // resident_setup of a context whose radial t
 int resident_sweeps_on(fvm_ctx *c, const ResSys &sys, int sweeps, int apply, int check_done);
 int resident_sweeps(const Tgt &t, int sweeps, int apply, int max_polls, unsigned tag_skew,
                     cudaGraphConditionalHandle cond, int has_cond, int check_done, int decide = 0);
-// the whole forward iteration (c->res_loop), and the same of the transposed equation
+// the whole forward iteration (c->res_loop; a refused launch clears it and c->res_lines), and
+// the same of the transposed equation
 int resident_loop(fvm_ctx *c, int max_polls = 0, int skewed = 0);
 int resident_loop_adjoint(fvm_ctx *c, const ResSys &sys, int max_polls = 0, int skewed = 0);
 int resident_reset(fvm_ctx *c);
@@ -370,6 +380,7 @@ struct RingSys {
     PCtl *pctl;
     int per;
 };
+// (a refused launch clears c->ring_blocks)
 int ring_launch(fvm_ctx *c, int mode, int count, int max_polls = 0, int skewed = 0);
 int ring_launch_adjoint(fvm_ctx *c, const RingSys &sys, int max_polls = 0, int skewed = 0);
 }  // namespace fvm

@@ -853,6 +853,10 @@ int launch_loop(fvm_ctx *c, const ResSys &sys, int max_polls, int skewed)
                                                   max_polls > 0 ? max_polls : kResidentPolls, skewed, 0);
     });
     if (e != cudaSuccess) {
+        if (launch_refused(e)) {   // nor would the per-interval launch of as many blocks fit
+            c->res_loop = false;
+            c->res_lines = 0;
+        }
         c->err = std::string("resident Poisson loop launch: ") + cudaGetErrorString(e);
         return FVM_ERR_CUDA;
     }

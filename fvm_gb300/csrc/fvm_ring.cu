@@ -631,6 +631,7 @@ int launch(fvm_ctx *c, const RingSys &sys, int mode, int count, int max_polls, i
                                waits_of(max_polls > 0 ? max_polls : kRingPolls, skewed));
     });
     if (e != cudaSuccess) {
+        if (launch_refused(e)) c->ring_blocks = 0;
         c->err = std::string("Poisson ring launch: ") + cudaGetErrorString(e);
         return FVM_ERR_CUDA;
     }

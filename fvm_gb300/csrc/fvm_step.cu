@@ -983,8 +983,15 @@ long long poisson_loop_kernels(fvm_ctx *c, int niter)
 int poisson_loop(fvm_ctx *c)
 {
     Dev &d = c->d;
-    if (c->ring_blocks) return ring_launch(c, 0, 0);
-    if (c->res_loop) return resident_loop(c);
+    // a refused launch leaves the context to the launches below, from this step on
+    if (c->ring_blocks) {
+        const int rc = ring_launch(c, 0, 0);
+        if (rc == FVM_OK || c->ring_blocks) return rc;
+    }
+    if (c->res_loop) {
+        const int rc = resident_loop(c);
+        if (rc == FVM_OK || c->res_loop) return rc;
+    }
     RC(poisson_graph(c));
     if (!c->p.poisson_host_loop) {
         FVM_CUDA(c, cudaGraphLaunch(c->pgraph, c->stream));
