@@ -170,7 +170,18 @@ bool cluster_plan(fvm_batch *b, std::vector<int> (&cls)[2], size_t (&smem)[2])
     return true;
 }
 
-int cluster_capture(fvm_batch *b, const std::vector<int> (&cls)[2], const size_t (&smem)[2])
+// The case lists of the plan to the device, in the order of the batch's stream (the default
+// stream has no order with it).
+int cluster_lists(fvm_batch *b, const std::vector<int> (&cls)[2])
+{
+    fvm_ctx *sh = &b->shell;
+    std::vector<int> list(cls[0]);
+    list.insert(list.end(), cls[1].begin(), cls[1].end());
+    FVM_CUDA(sh, cudaMemcpyAsync(b->d_cases, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice, sh->stream));
+    return FVM_OK;
+}
+
+int cluster_capture(fvm_batch *b, const std::vector<int> (&cls)[2], const size_t (&smem)[2], int timed)
 {
     fvm_ctx *sh = &b->shell;
     cudaStream_t st[2] = {sh->stream, sh->stream};
@@ -182,7 +193,7 @@ int cluster_capture(fvm_batch *b, const std::vector<int> (&cls)[2], const size_t
     int at = 0;
     for (int q = 0; q < 2; q++) {
         if (cls[q].empty()) continue;
-        const int rc = fvm::cluster_launch(b->t, st[q], b->d_cases + at, (int)cls[q].size(), q == 0 ? 16 : 8, smem[q]);
+        const int rc = fvm::cluster_launch(b->t, st[q], b->d_cases + at, (int)cls[q].size(), q == 0 ? 16 : 8, smem[q], timed);
         if (rc) return rc;
         at += (int)cls[q].size();
     }
@@ -209,10 +220,8 @@ int build_graph(fvm_batch *b)
     size_t smem[2] = {0, 0};
     const bool clusters = cluster_plan(b, cls, smem);
     if (clusters) {
-        std::vector<int> list(cls[0]);
-        list.insert(list.end(), cls[1].begin(), cls[1].end());
-        // on the stream that the graph is launched on: the default stream has no order with it
-        FVM_CUDA(sh, cudaMemcpyAsync(b->d_cases, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice, st));
+        const int rc = cluster_lists(b, cls);
+        if (rc) return rc;
     }
     FVM_CUDA(sh, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     sh->capturing = true;
@@ -222,7 +231,7 @@ int build_graph(fvm_batch *b)
     cudaError_t e = cudaSuccess;
     cudaGraphConditionalHandle h{};
     if (rc == FVM_OK && clusters) {
-        rc = cluster_capture(b, cls, smem);
+        rc = cluster_capture(b, cls, smem, 0);
     } else if (rc == FVM_OK) {
         cudaStreamCaptureStatus cs;
         cudaGraph_t cg = nullptr;
@@ -297,17 +306,30 @@ int apply_tiles(fvm_batch *b, int rw, int rm, int tw, int tm)
     return upload_table(b);
 }
 
-// Average time of one batched sweep pair (both colours) of `what` (0: Poisson,
-// 1: circumferential predictor lines of U), replayed in a graph.
+// Average time of one batched sweep (both colours) of `what`, replayed in a graph -- 0: Poisson, by
+// the kernels that a step of the batch takes in its tiles (a case's cluster with one
+// residual and `sweeps` sweeps, or the sweeps' launches); 1: circumferential predictor lines of U.
 int time_kernels(fvm_batch *b, int what, int sweeps, double *ms)
 {
     fvm_ctx *sh = &b->shell;
     cudaGraph_t g = nullptr;
     cudaGraphExec_t ge = nullptr;
+    std::vector<int> cls[2];
+    size_t smem[2] = {0, 0};
+    const bool clusters = what == 0 && cluster_plan(b, cls, smem);
+    if (clusters) {
+        const int rc = cluster_lists(b, cls);
+        if (rc) return rc;
+    }
+    const int before = sh->pgraph_kernels;
     FVM_CUDA(sh, cudaStreamBeginCapture(sh->stream, cudaStreamCaptureModeThreadLocal));
     sh->capturing = true;
-    int rc = what == 0 ? fvm::sweep_pairs(b->t, sweeps) : fvm::theta_pairs(b->t, FVM_FIELD_U, sweeps);
+    int rc;
+    if (clusters) rc = cluster_capture(b, cls, smem, sweeps);
+    else rc = what == 0 ? fvm::sweep_pairs(b->t, sweeps) : fvm::theta_pairs(b->t, FVM_FIELD_U, sweeps);
     sh->capturing = false;
+    const int kernels = sh->pgraph_kernels - before;
+    sh->pgraph_kernels = before;
     cudaError_t e = cudaStreamEndCapture(sh->stream, &g);
     if (rc || e != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -325,6 +347,10 @@ int time_kernels(fvm_batch *b, int what, int sweeps, double *ms)
     FVM_CUDA(sh, cudaEventElapsedTime(&t_ms, sh->ev_a, sh->ev_b));
     cudaGraphExecDestroy(ge);
     *ms = t_ms / sweeps;
+    if (what == 0) {
+        sh->tm.sweep_span_ms += t_ms;
+        sh->tm.sweep_span_launches += kernels;
+    }
     return FVM_OK;
 }
 

@@ -65,7 +65,7 @@ __device__ __forceinline__ void cluster_barrier()
 }
 
 template <int M, int NW>
-__global__ void __launch_bounds__(CT, 2) k_cluster32(DevTable tab, const int *cases)
+__global__ void __launch_bounds__(CT, 2) k_cluster32(DevTable tab, const int *cases, int timed)
 {
     using Lay = CluLayout<M, NW>;
     constexpr int TG = Lay::TG, LW = Lay::LW, G = Lay::G;
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(CT, 2) k_cluster32(DevTable tab, const int *ca
         }
     }
     cluster_barrier();   // every block has started: its shared memory may be written from now on
-    const int S = d.refine_sweeps;
+    const int S = timed ? timed : d.refine_sweeps;   // timed: one interval of so many sweeps, nothing written
     int it = 0;
     double resip = 0.0;
     for (;;) {
@@ -206,6 +206,7 @@ __global__ void __launch_bounds__(CT, 2) k_cluster32(DevTable tab, const int *ca
             }
             cluster_barrier();
         }
+        if (timed) return;   // uniform over the cluster; nobody writes to another block after the last barrier
         it += S;
         // the correction added to P on the own lines, BCP ghosts of each line
         for (int q = g; q < nl; q += G) {
@@ -288,11 +289,11 @@ bool cluster_fits(const LineSys &tile, int blocks, size_t smem)
 }
 
 // The iteration of the `count` cases listed in device memory, `blocks` blocks a case with
-// `smem` bytes each.
-int cluster_launch(const Tgt &t, cudaStream_t st, const int *cases, int count, int blocks, size_t smem)
+// `smem` bytes each; timed: one residual and that many sweeps, on chip only.
+int cluster_launch(const Tgt &t, cudaStream_t st, const int *cases, int count, int blocks, size_t smem, int timed)
 {
     const cudaError_t e = with_cluster(t.tr, blocks, smem, count, st, [&](auto k, const cudaLaunchConfig_t &cfg) {
-        return cudaLaunchKernelEx(&cfg, k, t.tab, cases);
+        return cudaLaunchKernelEx(&cfg, k, t.tab, cases, timed);
     });
     if (e != cudaSuccess) {
         t.c->err = std::string("batched Poisson launch: ") + cudaGetErrorString(e);

@@ -365,7 +365,7 @@ size_t exchange_words(const fvm_ctx *c);   // 64-bit words of d.XW
 size_t cluster_bytes(const fvm_ctx *c, const LineSys &tile);
 int cluster_blocks(const fvm_ctx *c);   // blocks per case: 8 or 16
 bool cluster_fits(const LineSys &tile, int blocks, size_t smem);
-int cluster_launch(const Tgt &t, cudaStream_t st, const int *cases, int count, int blocks, size_t smem);
+int cluster_launch(const Tgt &t, cudaStream_t st, const int *cases, int count, int blocks, size_t smem, int timed);
 // state copies between caller buffers and the device (fvm_copy.cu)
 cudaError_t copy_arrays(double *const *dst, const double *const *src, int count, size_t n, cudaMemcpyKind kind,
                         cudaStream_t st);

@@ -293,13 +293,15 @@ int fvm_batch_case(struct fvm_batch *b, int k, struct fvm_ctx **ctx);
  * circumferential warps, circumferential elements per thread}. */
 int fvm_batch_tiles(const struct fvm_batch *b, int *tiles);
 int fvm_batch_set_tiles(struct fvm_batch *b, const int *tiles);
-/* Times every tile that covers the batch's lines on the batch itself (`sweeps`
- * replays of the batched Poisson sweep for the radial family, of the batched
- * circumferential predictor sweep for the other) and keeps the fastest.  Needs
+/* Times every tile that covers the batch's lines on the batch itself (for the radial
+ * family `sweeps` Poisson sweeps by the kernels that a step takes in that tile, for the
+ * other `sweeps` circumferential predictor sweeps) and keeps the fastest.  Needs
  * every case's grid; the flow state is left unchanged.  tiles (4 ints) and ms
  * (2 doubles: best time per sweep of each family) may be NULL. */
 int fvm_batch_autotune(struct fvm_batch *b, int sweeps, int *tiles, double *ms);
-/* Average time of one batched Poisson sweep (both colours, state unchanged). */
+/* Average time of one batched Poisson sweep (both colours, state unchanged) by the kernels
+ * that a step of the batch takes; with one cluster per case one residual is among them.
+ * fvm_batch_get_timing's sweep span holds their time and launches. */
 int fvm_batch_time_sweeps(struct fvm_batch *b, int sweeps, double *ms_per_sweep);
 /* nsteps time steps of every case.  out (may be NULL) receives nsteps*ncases
  * records, step-major (out[s*ncases + k]); each case's fvm_history holds its own.
