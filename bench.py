@@ -238,10 +238,10 @@ def roofline_sweep(w, ms_per_colour, peaks, mixed, resident=False, layout=None):
     (80 B) and P written (8 B), plus the other colour's lagged P (8 B) and, for the
     second colour, its new P (8 B): 100 B x active cells on average.
     The per-colour kernels launch once per colour.  The FP64 ring runs a step's whole
-    iteration in one launch (achieved = 100 B x cells / time per sweep).  The resident kernel runs the
-    refine_sweeps sweeps of a refinement interval in one launch with its lines'
-    operands held on chip: its algorithmic bytes per launch are the same per-sweep
-    figure times the sweeps it runs, so achieved = 32 B x cells / time per sweep."""
+    iteration in one launch (achieved = 100 B x cells / time per sweep).  The resident kernel keeps its lines'
+    operands on chip; its figures are given per refinement interval of refine_sweeps sweeps: its algorithmic bytes per launch are the same per-sweep
+    figure times the sweeps it runs, so achieved = 32 B x cells / time per sweep.  Both are
+    timed as one launch of sweeps without residuals."""
     n_active = cells(w) // 2
     if not ms_per_colour or ms_per_colour <= 0:
         return None
@@ -266,8 +266,10 @@ def roofline_sweep(w, ms_per_colour, peaks, mixed, resident=False, layout=None):
         out.update({"kernel": "k_pois32_resident2" if pairs else "k_pois32_resident", "sweeps_per_launch": spl,
                     "avg_launch_us": 2 * ms_per_colour * 1e3 * spl, "bytes_per_launch": 2 * per_colour * spl,
                     "per_sweep_us": 2 * ms_per_colour * 1e3, "bytes_per_sweep": 2 * per_colour,
-                    "note": "lines' factors, couplings, right-hand side and correction stay on chip for the "
-                            "interval; one launch per refine_sweeps sweeps" +
+                    "note": "lines' factors, couplings, right-hand side and correction stay on chip; timed as "
+                            "one launch of sweeps without residuals (a step runs the iteration, residuals included, "
+                            "in one launch), given per refine_sweeps sweeps; traffic: ncu capture of a launch of one "
+                            "interval" +
                             ("; boundary lines exchanged once per two sweeps (three lines per block solved "
                              "again)" if pairs else ""),
                     "layout": layout})
@@ -881,7 +883,7 @@ def run_sweep_bench(args):
                       "poisson": f"zebra line GS to scaled-L1 {sw['resimax']:g}, cap NSWPP={sw['nswpp']}",
                       "sweeps_per_step": {"min": min(sweeps), "max": max(sweeps)},
                       "tiles": {"radial": tiles_used[:2], "circumferential": tiles_used[2:],
-                                "chosen_by": "autotuner (timed on this batch)"},
+                                "chosen_by": "autotuner (timed on this batch by the kernels of its step)"},
                       "partition": [len(p) for p in parts],
                       "setup_s_rank": setup_s,
                       "l2": "inputs larger than L2 (about 0.5 GB of case state)"},

@@ -925,7 +925,9 @@ __device__ __forceinline__ int edge_off(const Steps &o, int e)
 // (set: 0 for CW, 1 + s for CWA[s]): on a grid extruded along the span Q13, Q23, XIZ, ETZ,
 // ZTX and ZTY are zero but for the rounding of the face centres next to the wall and the
 // far field, which leaves the (i,j) pair of CW, CWA[0] and CWA[1] and nothing of CWA[2] --
-// 36 of the 48 weights' loads and FMAs saved, the same bits.
+// 36 of the 48 weights' loads and FMAs saved, the same bits for finite fields (0 x NaN is not
+// formed: a value that is not finite reaches its neighbours through the other terms and the wall
+// along its I line, in the same step).
 template <class T = double>
 __device__ __forceinline__ T cross_w(const D3 &d, double *const *W, int set, const double *f, int c, int i, const Steps &o)
 {

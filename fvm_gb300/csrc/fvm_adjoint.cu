@@ -1305,7 +1305,7 @@ void adj_graphs_free(fvm_adj *A)
 // the state before it (full arrays; d.U, d.V themselves or a copy that they are set to).
 // drag_scale: weight of this step's drag coefficient in the objective.  The launches before
 // and after the Poisson iteration go as two graphs from the second step on that finds the
-// context unchanged, as run_step's do (128 x 96 mixed: 962 -> 901 us; FP64 window of six
+// context unchanged, as run_step's do (128 x 96 mixed at the time: 962 -> 901 us; FP64 window of six
 // steps: 12.28 -> 11.82 ms).
 int adj_step(fvm_ctx *c, const double *ubase, const double *vbase, double drag_scale)
 {

@@ -3,15 +3,17 @@
 //
 // Each case is an ordinary context (its own device slab, geometry, factors and
 // state, set up through the single-context entry points).  A batch keeps a device
-// table of the cases' device views; every sub-step of the time step is one launch
-// over all cases (grid z = case, x/y extents = the largest case, surplus blocks of
-// smaller cases return at once), so small cases fill the GPU together.  The whole
-// step -- including the Poisson iteration as a device-side while loop that ends
-// when the last case has converged or reached its sweep cap -- is one CUDA graph,
-// launched once per step; CALCCOEF records of every case and step stay on the
+// table of the cases' device views; every sub-step of the time step but the Poisson
+// iteration is one launch over all cases (grid z = case, x/y extents = the largest case,
+// surplus blocks of smaller cases return at once), so small cases fill the GPU together.
+// The mixed Poisson iteration runs in one thread-block cluster per case (fvm_cluster.cu),
+// each until its case has ended; where a case has no such form (FP64, the cell's own cross
+// term, lines too long for a block's shared memory) it is a device-side while loop over
+// launches for all cases, which ends when the last case has converged or reached its sweep
+// cap.  The whole step is one CUDA graph, launched once per step; CALCCOEF records of every case and step stay on the
 // device until the call returns.  The cases share the line tiles (warps per line
 // group, elements per thread) of the radial and circumferential line families;
-// fvm_batch_autotune times the candidate tiles on the batch itself.
+// fvm_batch_autotune times the candidate tiles on the batch itself, by the kernels its step runs.
 #include <algorithm>
 #include <cmath>
 #include <cstring>

@@ -607,7 +607,7 @@ __device__ __forceinline__ void group_apply_r(T (&v)[M], const T (&fi)[M], const
 // where their factors are tiny: a value far below its neighbours along the line takes its
 // share from them alone, and a non-finite value fills the line.  (Without the stages whose
 // factors are at most 2^-60, and a branch on their number: 128 x 96, four steps of 512 sweeps
-// 2.83 ms against 2.60, 512 x 384, two steps of 2048 6.40 against 6.48.)  Groups of one or
+// 2.83 ms against 2.59, 512 x 384, two steps of 2048 6.40 against 6.42.)  Groups of one or
 // two warps.
 constexpr int SCAN_STAGES = 5;
 template <typename T>

@@ -17,7 +17,7 @@
 // ghost row 0 hold values one BCP older, so they are P^(n-2)(1,j) and P^(n-2)(i,NJ-1).
 // A line's pressure is therefore kept in three versions.  Every operation is k_pois64's
 // and k_pres64's in the same rounding order, but for scan stages whose factors are all at
-// most 2^-80, which are left out (3 to 7 % of a step): both paths give the same bits unless
+// most 2^-80, which are left out (2 to 7 % of a step): both paths give the same bits unless
 // a value lies 2^27 or more below another on its line, where they differ by at most 2^-80 of
 // the larger one a solve and, through later roundings, by units in the last place of the
 // largest.  A line with a value that is not finite is not finite throughout, as there.
@@ -52,7 +52,7 @@
 // factors that the line solve's scans carry are formed once per launch and kept in
 // shared memory: per sweep only the value part of the scans is left.
 // Measured (step with 512 or 2048 sweeps, residual every 8): 128 x 96 FP64 7.48 -> 2.17 ms
-// (14.3 -> 3.9 us per sweep), 512 x 384 39.8 -> 16.1 ms (18 -> 7.6 us; 196,608 cells x 11
+// (14.3 -> 3.9 us per sweep), 512 x 384 39.8 -> 15.9 ms (18 -> 7.5 us; 196,608 cells x 11
 // instructions at the chip's 0.63 T/s: 3.4 us).
 #include <algorithm>
 #include <type_traits>

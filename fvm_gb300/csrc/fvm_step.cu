@@ -1076,7 +1076,7 @@ int resident_fault(fvm_ctx *c)
 // last one left it (the launches carry it by value; whatever changes it -- a grid,
 // controls -- takes the step after it through the launches again).  A first step is not
 // worth a graph, which costs about as much to build.  Direct launches: 269 us for a step at
-// 32 x 24 FP64 against 221, 2940 us for four at 128 x 96 mixed against 2834.
+// 32 x 24 FP64 against 221, 2940 us for four at 128 x 96 mixed against 2834 at the time.
 template <class Body>
 int step_part(fvm_ctx *c, int k, Body body)
 {

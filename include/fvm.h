@@ -228,9 +228,9 @@ int fvm_get_timing(struct fvm_ctx *ctx, fvm_timing *out);
 /* Replays `sweeps` zebra sweeps of the Poisson sweep kernels of the context's
  * precision (touching only scratch arrays, the state is unchanged) in a graph
  * bracketed by CUDA events on the context's stream.  ms_per_launch: average time
- * per zebra colour (the per-colour path launches once per colour; the resident
- * path runs all sweeps in one launch, reported as 1 in *launches, and the figure
- * is its time divided by 2*sweeps). */
+ * per zebra colour (the per-colour path launches once per colour; the on-chip
+ * paths run all sweeps in one launch, without residuals, reported as 1 in *launches,
+ * and the figure is its time divided by 2*sweeps). */
 int fvm_time_sweeps(struct fvm_ctx *ctx, int sweeps, double *ms_per_launch, long long *launches);
 /* Check of the bounded waits of the resident sweeps (MIXED contexts using them):
  * four sweeps on scratch arrays with exchange tags that no block publishes, so
@@ -275,8 +275,9 @@ int fvm_poisson_residual_static(int ni, int nj, const double *p, const double *s
 /* ---------------------------------------------------------------------------
  * Batches: many independent cases (different grids, Re, Pr, dt, rotation,
  * tolerances) advanced together, each sub-step one launch over all cases and the
- * whole time step one CUDA graph (the Poisson loop runs on the device until the
- * last case has converged or reached its cap).  No reference counterpart: the
+ * whole time step one CUDA graph (the Poisson iteration runs on the device, MIXED: each
+ * case in a thread-block cluster of its own where that fits, else until the last
+ * case has converged or reached its cap).  No reference counterpart: the
  * reference runs one case per process (Main.f90:40-118 once per run).
  * --------------------------------------------------------------------------- */
 struct fvm_batch;
