@@ -32,10 +32,11 @@
 // n+2 needs neighbours that needed the readers' sweep n+1.  While one colour is solved
 // the other colour's groups form their next cross terms.  The residual's block sums
 // travel the same way and every block adds them in the same order, so all blocks take
-// the same decision.  Every wait is bounded; one that runs out sets the flag of its
-// phase (odd lines, even lines, residual), which the whole block reads after the phase's
-// barrier and nobody writes before another barrier, so that all threads leave together; the
-// pressure is left alone and the host reports FVM_ERR_TIMEOUT.  Waits::skew lets
+// the same decision.  Every wait is bounded; one that runs out sets a flag (one
+// per parity of the sweep, one for the residual) that the whole block reads after the
+// sweep's or the residual's last barrier and that nobody writes again before another
+// barrier, so that all threads leave together.  The block leaves its pressure alone, the
+// others' waits for it run out in turn, and the host reports FVM_ERR_TIMEOUT.  Waits::skew lets
 // the waits of one kind look for tags that no block publishes: the check of those exits.
 //
 // ADJ: the transposed equation of the adjoint, (A^T + G^T DD^T) mu = g (fvm_adjoint.cu).
@@ -52,7 +53,7 @@
 // factors that the line solve's scans carry are formed once per launch and kept in
 // shared memory: per sweep only the value part of the scans is left.
 // Measured (step with 512 or 2048 sweeps, residual every 8): 128 x 96 FP64 7.48 -> 2.17 ms
-// (14.3 -> 3.9 us per sweep), 512 x 384 39.8 -> 15.9 ms (18 -> 7.5 us; 196,608 cells x 11
+// (14.3 -> 3.9 us per sweep), 512 x 384 39.8 -> 16.1 ms (18 -> 7.6 us; 196,608 cells x 11
 // instructions at the chip's 0.63 T/s: 3.4 us).
 #include <algorithm>
 #include <type_traits>
@@ -93,7 +94,8 @@ __device__ __forceinline__ double of_words(unsigned long long a, unsigned long l
 }
 
 // The M elements of a line that thread t owns, once their words carry the tag; false
-// when the wait ran out.  One L2 round trip per poll: all loads precede the tests.
+// when the wait ran out.  One L2 round trip per poll: all loads precede the tests.  (Not unrolled:
+// 128 x 96 2.29 ms against 2.20.)
 template <int M, int TG>
 __device__ __forceinline__ bool poll_line(const ulonglong2 *src, int t, int n, unsigned want, int max_polls, double (&out)[M])
 {
@@ -101,6 +103,7 @@ __device__ __forceinline__ bool poll_line(const ulonglong2 *src, int t, int n, u
 #pragma unroll
     for (int k = 0; k < M; k++)
         if (t * M + k < n) pending |= 1u << k;
+#pragma unroll 4
     for (int it = 0; pending && it < max_polls; it++) {
         unsigned long long a[M], b[M];
 #pragma unroll
@@ -128,7 +131,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
     using Lay = RingLayout<M, NW>;
     constexpr int TG = Lay::TG, LW = Lay::LW, CST = Lay::CST;
     extern __shared__ double shm[];
-    __shared__ int s_fault[3], s_nf;   // a wait of the odd half-sweep, the even one, the residual ran out
+    __shared__ int s_fault[3], s_nf;   // a wait of an even sweep, an odd one, a residual ran out
     __shared__ double s_line[2 * 8], s_tot[2 * RING_MAX_BLOCKS], s_res;
     const int L = d.NJ - 1, n = d.sP.n;
     const int pairs = L / 2, p0 = blockIdx.x * ppb, nl = 2 * min(ppb, pairs - p0), j0 = 2 * p0 + 1;
@@ -358,11 +361,12 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
         for (int k = 0; k < M; k++)
             if (t * M + k < n) st_words(dst + k * TG + t, v[k], cnt0 + unsigned(m));
     };
-    auto wait_into = [&](int kind, int q, int m, double (&x)[M]) {
-        const unsigned tag = cnt0 + unsigned(m);
-        if (!poll_line<M, TG>(slot(tag, q), t, n, tag + waits.skew[kind - 1], waits.max_polls, x)) s_fault[kind - 1] = 1;
+    // line q of sweep v; flag: what s_fault tells of the wait
+    auto wait_into = [&](int kind, int flag, int q, int v, double (&x)[M]) {
+        const unsigned tag = cnt0 + unsigned(v);
+        if (!poll_line<M, TG>(slot(tag, q), t, n, tag + waits.skew[kind - 1], waits.max_polls, x)) s_fault[flag] = 1;
     };
-    auto wait_line = [&](int kind, int q, int m) { wait_into(kind, q, m, hal); };
+    auto wait_line = [&](int kind, int flag, int q, int v) { wait_into(kind, flag, q, v, hal); };
 
     if (act && odd) source(1, su);
     int m = 0, have = 0;   // sweeps done; have: group 0's halo already holds version m
@@ -375,7 +379,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
             const int vr = (m + 2) % 3, vw = m % 3;
             if (act) {
                 if (odd) {
-                    if (g == 0 && m > 1 && !have) wait_line(WAIT_ODD, jm1, m - 1);
+                    if (g == 0 && m > 1 && !have) wait_line(WAIT_ODD, m & 1, jm1, m - 1);
                     const double *pn = line(vr, g + 1), *ps = g == 0 ? nullptr : line(vr, g - 1);
 #pragma unroll
                     for (int k = 0; k < M; k++) {
@@ -394,7 +398,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
                         double x[M];
 #pragma unroll
                         for (int k = 0; k < M; k++) x[k] = 0.0;
-                        wait_into(WAIT_ODD, je, m - 1, x);
+                        wait_into(WAIT_ODD, m & 1, je, m - 1, x);
 #pragma unroll
                         for (int k = 0; k < M; k++) hm1[size_t(vr) * LW + k * TG + t] = x[k];
                         bar();
@@ -405,10 +409,9 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
             }
             have = 0;
             __syncthreads();
-            if (s_fault[0]) { bad = true; break; }   // uniform: this flag is next written after another barrier
             if (act) {
                 if (!odd) {
-                    if (g == nl - 1) wait_line(WAIT_EVEN, wrap(j + 1), m);
+                    if (g == nl - 1) wait_line(WAIT_EVEN, m & 1, wrap(j + 1), m);
                     const double *pn = g == nl - 1 ? nullptr : line(vw, g + 1), *ps = line(vw, g - 1);
 #pragma unroll
                     for (int k = 0; k < M; k++) {
@@ -424,7 +427,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
                         double x[M];
 #pragma unroll
                         for (int k = 0; k < M; k++) x[k] = 0.0;
-                        wait_into(WAIT_EVEN, jo, m, x);
+                        wait_into(WAIT_EVEN, m & 1, jo, m, x);
 #pragma unroll
                         for (int k = 0; k < M; k++) hm2[size_t(vw) * LW + k * TG + t] = x[k];
                         bar();
@@ -434,7 +437,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
                 }
             }
             __syncthreads();
-            if (s_fault[1]) { bad = true; break; }
+            if (s_fault[m & 1]) { bad = true; break; }   // uniform: next written after another barrier
         }
         if (bad || mode) break;
         // scaled-L1 residual of P^m with the last sweep's source (of mu^m with its own)
@@ -450,7 +453,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
                         double x[M];
 #pragma unroll
                         for (int k = 0; k < M; k++) x[k] = 0.0;
-                        wait_into(WAIT_RES, je, m, x);
+                        wait_into(WAIT_RES, 2, je, m, x);
 #pragma unroll
                         for (int k = 0; k < M; k++) hm1[size_t(vw) * LW + k * TG + t] = x[k];
                         bar();
@@ -466,7 +469,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
                 aw[k] = e < n ? sys.AW[c] : 0.0;
                 ap[k] = e < n ? sys.AP[c] : 0.0;
             }
-            if (g == 0) wait_line(WAIT_RES, jm1, m);
+            if (g == 0) wait_line(WAIT_RES, 2, jm1, m);
             const double *self = line(vw, g);
 #pragma unroll
             for (int k = 0; k < M; k++) {
@@ -492,7 +495,7 @@ __global__ void __launch_bounds__(RingLayout<M, NW>::MAXT, 1)
         __syncthreads();
         const unsigned rtag = cnt0 + unsigned(m);
         ulonglong2 *ps = psum + size_t(round & 1) * 2 * gridDim.x;
-        if (threadIdx.x == 0) {
+        if (threadIdx.x == 0 && !s_fault[2]) {   // without its lines the block has no sums
             pairs_sum2(s_line, nl, ra, pa);
             st_words(ps + 2 * blockIdx.x, ra, rtag);
             st_words(ps + 2 * blockIdx.x + 1, pa, rtag);
